@@ -9,12 +9,13 @@
 // 128^-1/2).  The output is RMS-normalised per head, scaled by a learned weight and gated by SiLU(z).
 //
 // Two kernels per layer and step:
-//   gdn_conv_kernel  one thread per projected column: folds the GEMV's split-K partials, and for the q / k / v
+//   gdn_conv_rows_kernel  four projected columns per thread: folds the GEMV's split-K partials, and for the q / k / v
 //                    columns applies the convolution over the slot's last three inputs (kept per slot) + SiLU;
-//   gdn_step_kernel  one CTA per value head, thread j owns column j of the state (128 fp32 registers): decay,
+//   gdn_step_kernel  one CTA per value head and slot, thread j owns column j of the state (128 fp32 registers): decay,
 //                    delta rule, read-out, gated norm; q and k are shared through shared memory.
-// Rows of a step are walked in order inside each thread, so several rows of one slot (a prompt chunk, verify
-// rows) see each other's state; a thread keeps the state in registers while consecutive rows stay on one slot.
+// Slots share nothing, so the step's kernels give every slot CTAs of its own: with 12 requests a step of 12 such layers and 4
+// of attention takes 2.59 ms, 3.12 when 48 + 65 CTAs walked the slots one after the other;
+// several rows of one slot (verify rows) are walked in order by one CTA, which keeps the state in registers.
 #include "common.cuh"
 
 using namespace b2;
@@ -73,6 +74,110 @@ __global__ void __launch_bounds__(256) gdn_conv_kernel(const GdnConvParams p) {
   }
 }
 
+// Row `m` of a step is its slot's first one: the CTAs of that row walk all rows of the slot, in order.
+__device__ __forceinline__ bool first_of_slot(const int* ctrl, int m, int slot) {
+  for (int i = 0; i < m; ++i)
+    if (ctrl[CTRL_ROW_REQ + i] == slot) return false;
+  return true;
+}
+
+__device__ __forceinline__ float4 conv_in(const GdnConvParams& p, int m, int n) {
+  float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int s = 0; s < p.splits; ++s) {
+    const float4 v = *reinterpret_cast<const float4*>(p.part + ((size_t)s * p.M + m) * p.N + n);
+    x.x += v.x; x.y += v.y; x.z += v.z; x.w += v.w;
+  }
+  return x;
+}
+__device__ __forceinline__ float conv_tap(const float4& w, float a, float b, float c, float x) {
+  const float y = w.x * a + w.y * b + w.z * c + w.w * x;
+  return y / (1.f + __expf(-y));
+}
+// Four columns' taps, and their last three inputs (a oldest) against the layout [channel][3]
+struct ConvTaps {
+  float4 w[4], a, b, c;
+  __device__ __forceinline__ void load(const float* st) {
+    const float4 s0 = reinterpret_cast<const float4*>(st)[0], s1 = reinterpret_cast<const float4*>(st)[1], s2 = reinterpret_cast<const float4*>(st)[2];
+    a = make_float4(s0.x, s0.w, s1.z, s2.y);
+    b = make_float4(s0.y, s1.x, s1.w, s2.z);
+    c = make_float4(s0.z, s1.y, s2.x, s2.w);
+  }
+  __device__ __forceinline__ void store(float* st) const {
+    reinterpret_cast<float4*>(st)[0] = make_float4(a.x, b.x, c.x, a.y);
+    reinterpret_cast<float4*>(st)[1] = make_float4(b.y, c.y, a.z, b.z);
+    reinterpret_cast<float4*>(st)[2] = make_float4(c.z, a.w, b.w, c.w);
+  }
+  __device__ __forceinline__ float4 step(const float4& x) {
+    const float4 y = make_float4(conv_tap(w[0], a.x, b.x, c.x, x.x), conv_tap(w[1], a.y, b.y, c.y, x.y),
+                                 conv_tap(w[2], a.z, b.z, c.z, x.z), conv_tap(w[3], a.w, b.w, c.w, x.w));
+    a = b; b = c; c = x;
+    return y;
+  }
+};
+
+// The same with four columns per thread and the rows spread over the CTAs.  A convolution of four taps depends on three
+// earlier rows and on nothing else, so the rows of a prompt chunk need not be walked one after the other: a CTA takes CONV_R of
+// them and reads three more ahead of them (cached: the CTA above reads them too).  The sequential walk had 65 CTAs on a
+// 16480-wide projection, each a chain of 3000 dependent row visits: 2070 us where the bytes take 60 (a 3000-token prompt
+// through 12 such layers and 4 of attention: 61.1 -> 41.7 ms).
+// Rows of a step (ctrl): the CTAs of a slot's first row walk that slot's rows; the others leave.
+constexpr int CONV_R = 16, CONV_T = 128, CONV_U = 8;
+__global__ void __launch_bounds__(CONV_T) gdn_conv_rows_kernel(const GdnConvParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int n = (blockIdx.x * CONV_T + threadIdx.x) * 4;
+  const bool conv = n < p.conv_ch;
+  ConvTaps t;
+  if (p.ctrl) {
+    const int slot = p.ctrl[CTRL_ROW_REQ + blockIdx.y];
+    if (n >= p.N || !first_of_slot(p.ctrl, blockIdx.y, slot)) return;
+    float* st = p.conv_state + ((size_t)slot * p.conv_ch + n) * (TAPS - 1);
+    if (conv) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) t.w[i] = reinterpret_cast<const float4*>(p.conv_w)[n + i];
+      t.load(st);
+    }
+    for (int m = blockIdx.y; m < p.M; ++m) {
+      if (p.ctrl[CTRL_ROW_REQ + m] != slot) continue;
+      const float4 x = conv_in(p, m, n);
+      *reinterpret_cast<float4*>(p.act + (size_t)m * p.N + n) = conv ? t.step(x) : x;
+    }
+    if (conv) t.store(st);
+    return;
+  }
+  if (n >= p.N) return;
+  const int m0 = blockIdx.y * CONV_R, m1 = min(p.M, m0 + CONV_R);
+  float* st = p.conv_state + ((size_t)p.slot * p.conv_ch + n) * (TAPS - 1);
+  if (conv) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) t.w[i] = reinterpret_cast<const float4*>(p.conv_w)[n + i];
+    if (m0 == 0) {
+      t.load(st);
+    } else {
+      t.a = conv_in(p, m0 - 3, n);
+      t.b = conv_in(p, m0 - 2, n);
+      t.c = conv_in(p, m0 - 1, n);
+    }
+  }
+  for (int m = m0; m < m1; m += CONV_U) {
+    float4 x[CONV_U];
+#pragma unroll
+    for (int u = 0; u < CONV_U; ++u)
+      if (m + u < m1) x[u] = conv_in(p, m + u, n);
+#pragma unroll
+    for (int u = 0; u < CONV_U; ++u)
+      if (m + u < m1) *reinterpret_cast<float4*>(p.act + (size_t)(m + u) * p.N + n) = conv ? t.step(x[u]) : x[u];
+  }
+  // the chunk's last three inputs become the slot's state: written by the CTA that read the old one
+  if (conv && m0 == 0) {
+    t.a = conv_in(p, p.M - 3, n);
+    t.b = conv_in(p, p.M - 2, n);
+    t.c = conv_in(p, p.M - 1, n);
+    t.store(st);
+  }
+}
+
 struct GdnStepParams {
   const float* act;    // [M][N]
   int M, N, n_k, n_v;
@@ -99,24 +204,17 @@ __global__ void __launch_bounds__(DH) gdn_step_kernel(const GdnStepParams p) {
   pdl_wait();
   pdl_launch_dependents();
   const int h = blockIdx.x, j = threadIdx.x;
+  const int slot = p.ctrl ? p.ctrl[CTRL_ROW_REQ + blockIdx.y] : p.slot;
+  if (p.ctrl && !first_of_slot(p.ctrl, blockIdx.y, slot)) return;
   const int hk = h / (p.n_v / p.n_k);
   const int kd = p.n_k * DH, vd = p.n_v * DH;
   const float a_neg = -__expf(p.a_log[h]), dtb = p.dt_bias[h], nw = p.norm_w[j];
   float S[DH];
-  int cur = -1;
-  for (int m = 0; m < p.M; ++m) {
-    const int slot = p.ctrl ? p.ctrl[CTRL_ROW_REQ + m] : p.slot;
-    if (slot != cur) {
-      if (cur >= 0) {
-        float* sp = p.state + ((size_t)cur * p.n_v + h) * DH * DH + j;
+  float* sp = p.state + ((size_t)slot * p.n_v + h) * DH * DH + j;
 #pragma unroll
-        for (int i = 0; i < DH; ++i) sp[(size_t)i * DH] = S[i];
-      }
-      cur = slot;
-      const float* sp = p.state + ((size_t)cur * p.n_v + h) * DH * DH + j;
-#pragma unroll
-      for (int i = 0; i < DH; ++i) S[i] = sp[(size_t)i * DH];
-    }
+  for (int i = 0; i < DH; ++i) S[i] = sp[(size_t)i * DH];
+  for (int m = blockIdx.y; m < p.M; ++m) {
+    if (p.ctrl && p.ctrl[CTRL_ROW_REQ + m] != slot) continue;
     const float* a = p.act + (size_t)m * p.N;
     const float qv = a[hk * DH + j], kv = a[kd + hk * DH + j];
     const float vj = a[2 * kd + h * DH + j], zj = a[2 * kd + vd + h * DH + j];
@@ -147,11 +245,8 @@ __global__ void __launch_bounds__(DH) gdn_step_kernel(const GdnStepParams p) {
     const float y = o * rsqrtf(ms + p.eps) * nw * (zj / (1.f + __expf(-zj)));
     p.out[(size_t)m * vd + h * DH + j] = __float2bfloat16(y);
   }
-  if (cur >= 0) {
-    float* sp = p.state + ((size_t)cur * p.n_v + h) * DH * DH + j;
 #pragma unroll
-    for (int i = 0; i < DH; ++i) sp[(size_t)i * DH] = S[i];
-  }
+  for (int i = 0; i < DH; ++i) sp[(size_t)i * DH] = S[i];
 }
 
 // ---- prompt chunks: the same layer as three kernels, so that everything that does not depend on the state runs
@@ -675,6 +770,13 @@ extern "C" int b2_gdn_conv(const float* part, int splits, int M, int N, int conv
                            const float* conv_w, float* conv_state, float* act, void* stream) {
   if (M < 1 || (ctrl && M > 64) || (!ctrl && slot < 0) || splits < 1 || conv_ch > N) return -1;
   GdnConvParams p{part, splits, M, N, conv_ch, ctrl, slot, conv_w, conv_state, act};
+  // four columns per thread need whole, aligned 16-byte pieces of every row; a chunk needs its last three inputs in itself.
+  // (The other shapes, odd numbers of value heads among them, keep one column per thread and the rows in order.)
+  const uintptr_t at = (uintptr_t)part | (uintptr_t)conv_w | (uintptr_t)conv_state | (uintptr_t)act;
+  if (N % 4 == 0 && conv_ch % 4 == 0 && at % 16 == 0 && (ctrl || M >= 3)) {
+    const dim3 grid((N / 4 + CONV_T - 1) / CONV_T, ctrl ? M : (M + CONV_R - 1) / CONV_R);
+    if (grid.y <= 65535u) return b2_launch(gdn_conv_rows_kernel, grid, dim3(CONV_T), 0, (cudaStream_t)stream, true, p);
+  }
   return b2_launch(gdn_conv_kernel, dim3((N + 255) / 256), dim3(256), 0, (cudaStream_t)stream, true, p);
 }
 
@@ -684,7 +786,7 @@ extern "C" int b2_gdn_step(const float* act, int M, int N, int n_k, int n_v, int
                            void* out, void* stream) {
   if (head_dim != DH || M < 1 || (ctrl && M > 64) || (!ctrl && slot < 0) || n_k < 1 || n_v % n_k != 0 || N != 2 * n_k * DH + 2 * n_v * DH + 2 * n_v) return -1;
   GdnStepParams p{act, M, N, n_k, n_v, ctrl, slot, a_log, dt_bias, norm_w, eps, state, (__nv_bfloat16*)out};
-  return b2_launch(gdn_step_kernel, dim3(n_v), dim3(DH), 0, (cudaStream_t)stream, true, p);
+  return b2_launch(gdn_step_kernel, dim3(n_v, ctrl ? M : 1), dim3(DH), 0, (cudaStream_t)stream, true, p);
 }
 
 // The same on the tensor cores, rows in chunks of 64: `ws` holds chunks x n_v blocks of b2_gdn_wy_block_bytes().
