@@ -671,6 +671,137 @@ __global__ void __launch_bounds__(256) quant_x_kernel(const GemvParams p, uint8_
   }
 }
 
+// ---- decode rows of several requests through routed experts: one CTA per (group of up to eight rows that chose one expert, run
+// of n-blocks).  The batched GEMV above reads an expert once per (row, slot); with 48 rows and 8 of 256 experts each that is
+// 384 readings of ~200 experts, and the eight token columns of the integer MMA hold one row.  Here the routing kernel's last
+// CTA leaves a table of groups (moe.cu), the rows of a group are quantised into shared memory once and every n-block's
+// weights stream past them.  Two groups of four consumer warps own alternate n-blocks, so a sum never leaves its warp and the
+// CTA has no barrier after the staging; a run is about 64 W4B blocks (280 KB), which keeps the fixed cost per CTA (table,
+// staging, ring fill: ~4 us with two CTAs per SM) below its stream time and leaves three to four waves to balance.  A step of
+// 48 rows through 16 layers (hidden 2048, experts of 512): 11.5 -> 4.3 ms, with the router's slices (moe.cu).
+struct ExpertGroups {
+  int n;           // groups in use
+  int pad[15];
+  struct Entry { int expert, rows, pair[8]; } e[1];   // pair: place of (row, slot) among row * slots + slot
+};
+
+struct ExpertParams {
+  GemvParams g;      // w, x, KG, N, x_mode, ldx, x_div, x_batch_bytes, out_batch, alt_w, alt_id, expert_bytes
+  const ExpertGroups* groups;
+  int nb, run;       // n-blocks of the matrix, n-blocks per CTA (even)
+};
+
+__global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const ExpertParams ep) {
+  const GemvParams& p = ep.g;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem0 = (smem_u32(smem_raw) + 127u) & ~127u;
+  const uint32_t ring = smem0, bars = smem0 + kRingBytes, full0 = bars, empty0 = bars + 8 * kStages;
+  const uint32_t gs0 = bars + 128, xs0 = gs0 + ((p.KG * 64 + 127) & ~127);
+  const int strideB = stride_words(p.KG) * 4;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_wait();                 // the table is the routing kernel's, the rows an earlier one's
+  pdl_launch_dependents();
+  if ((int)blockIdx.y >= ep.groups->n) return;
+  const ExpertGroups::Entry& en = ep.groups->e[blockIdx.y];
+  const int M = en.rows, nb0 = blockIdx.x * ep.run, nbs = min(ep.run, ep.nb - nb0);
+  const int spb = (p.KG + kG - 1) / kG;                        // ring stages per n-block
+  // stage order: the two warp groups' n-blocks in turn, a lone last block by itself
+  const int pairs2 = nbs / 2, nstage = nbs * spb;
+  auto block_of = [&](int i) { return i < pairs2 * 2 * spb ? i / (2 * spb) * 2 + (i & 1) : nbs - 1; };
+  auto part_of = [&](int i) { return i < pairs2 * 2 * spb ? i % (2 * spb) / 2 : i - pairs2 * 2 * spb; };
+  if (tid == 0) {
+    for (int i = 0; i < kStages; ++i) {
+      mbar_init(full0 + 8 * i, 1);
+      mbar_init(empty0 + 8 * i, 4);
+    }
+    mbar_fence_init();
+  }
+  __syncthreads();
+  if (warp == 8) {
+    if (lane == 0) {
+      const uint8_t* src = ((p.alt_w && en.expert == p.alt_id) ? p.alt_w : p.w + (size_t)en.expert * p.expert_bytes) +
+                           (size_t)nb0 * p.KG * kBlockBytes;
+      bool ok = true;
+      int issued = 0;
+      for (int i = 0; i < nstage && ok; ++i) {
+        if (i >= kStages) ok = mbar_wait(empty0 + 8 * (i % kStages), ((i / kStages) - 1) & 1, ERR_GEMV_EMPTY_WAIT);
+        if (!ok) break;
+        const int s = i % kStages, q = part_of(i) * kG;
+        const uint32_t bytes = min(kG, p.KG - q) * kBlockBytes;
+        mbar_expect_tx(full0 + 8 * s, bytes);
+        bulk_g2s(ring + s * kStageBytes, src + ((size_t)block_of(i) * p.KG + q) * kBlockBytes, bytes, full0 + 8 * s);
+        issued = i + 1;
+      }
+      if (!ok)   // wait (bounded) for the copies that were issued and possibly never consumed
+        for (int i = max(0, issued - kStages); i < issued; ++i)
+          mbar_wait(full0 + 8 * (i % kStages), (i / kStages) & 1, ERR_GEMV_FULL_WAIT);
+    }
+    return;
+  }
+  // ---- the group's rows as quantised operands; rows from M on alias the last one (their columns are not stored)
+  const int nvec = p.KG * 8;
+  for (int v0 = 0; v0 < M * nvec; v0 += kConsumerThreads) {   // a multiple of 8: lanes stay together in groups of 8
+    const int v = v0 + tid, row = v / nvec, col = v - row * nvec;
+    uint4 val = make_uint4(0, 0, 0, 0);
+    if (row < M)
+      val = stage_load(p, reinterpret_cast<const uint8_t*>(p.x) + (size_t)(en.pair[row] / p.x_div) * p.x_batch_bytes, 0, col * 8, 1.f);
+    const StagedVec sv = stage_quant(val);
+    if (row < M) {
+      const int vq = col & 7;
+      const uint32_t dst = xs0 + row * strideB + ((col >> 3) * 32 + stage_word(vq)) * 4;
+      sts32(dst, sv.w[0]);
+      sts32(dst + 16, sv.w[1]);
+      sts32(dst + 32, sv.w[2]);
+      sts32(dst + 48, sv.w[3]);
+      if (vq == 0)
+        asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(gs0 + ((col >> 3) * 8 + row) * 8), "r"(__float_as_uint(sv.scale)), "r"((uint32_t)sv.m8sum) : "memory");
+    }
+  }
+  consumer_sync();
+  const int g = lane >> 2, t = lane & 3, wgrp = warp >> 2, row16 = (warp & 3) * 2;
+  const uint32_t w_off = row16 * 512 + lane * 16, sc_off = 4096 + (row16 * 16 + 2 * g) * 2;
+  const uint32_t x_row = xs0 + min(g, M - 1) * strideB + t * 32, gs_t = gs0 + 2 * t * 8;
+  float acc[2][1][4] = {};
+  for (int i = 0; i < nstage; ++i) {
+    const int blk = block_of(i), q = part_of(i) * kG;
+    if ((blk & 1) != wgrp) continue;
+    const int s = i % kStages, ng = min(kG, p.KG - q);
+    if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, (i / kStages) & 1, ERR_GEMV_FULL_WAIT))) return;   // the rest is not stored; the producer gives up too and drains its copies
+    const uint32_t st = ring + s * kStageBytes;
+#pragma unroll 1
+    for (int q0 = 0; q0 < ng; q0 += 2) {
+      const uint32_t xa[1] = {x_row + (q + q0) * 128};
+      const uint32_t gsa = gs_t + (q + q0) * 64;
+      if (q0 + 1 < ng) {
+        group_mma<1, 2>(acc[0], st + q0 * kBlockBytes, w_off, sc_off, xa, gsa);
+        group_mma<1, 2>(acc[1], st + q0 * kBlockBytes, w_off + 512, sc_off + 32, xa, gsa);
+      } else {
+        group_mma<1, 1>(acc[0], st + q0 * kBlockBytes, w_off, sc_off, xa, gsa);
+        group_mma<1, 1>(acc[1], st + q0 * kBlockBytes, w_off + 512, sc_off + 32, xa, gsa);
+      }
+    }
+    __syncwarp();
+    if (lane == 0) mbar_arrive(empty0 + 8 * s);
+    if (q + ng == p.KG) {     // the n-block is complete
+      const int n0 = (nb0 + blk) * 128 + row16 * 16 + g;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int m = 2 * t + e;
+        if (m < M) {
+          float* o = p.out + (size_t)en.pair[m] * p.out_batch + n0;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (n0 + 16 * h < p.N) o[16 * h] = acc[h][0][e];
+            if (n0 + 16 * h + 8 < p.N) o[16 * h + 8] = acc[h][0][2 + e];
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) acc[h][0][0] = acc[h][0][1] = acc[h][0][2] = acc[h][0][3] = 0.f;
+    }
+  }
+}
+
 template <int T>
 int launch_t(GemvParams& p, cudaStream_t stream) {
   // staged rows and chunk length: as much of the split's k range as fits the activation budget
@@ -857,6 +988,35 @@ extern "C" int b2_gemv_w4_experts_alt(const void* w4b_stack, long long expert_by
                                       void* stream) {
   return gemv_w4_experts_impl(w4b_stack, expert_bytes, expert_ids, batches, x, x_div, x_batch_bytes, out, N, K, S, ldx, x_mode,
                               s_in, x_slice, 0, stream, alt_w, alt_id);
+}
+
+// Rows grouped by expert (table of b2_moe_router_rows): one slice per (row, slot), out[pair][N].  `max_groups`: groups that the
+// table can hold.  -9: the rows of a group do not fit in shared memory beside the ring.
+extern "C" int b2_gemv_w4_groups(const void* w4b_stack, long long expert_bytes, const void* groups, int max_groups, const void* x,
+                                 int x_div, long long x_batch_bytes, float* out, int N, int K, int ldx, int x_mode, int s_in,
+                                 long long x_slice, const void* alt_w, int alt_id, void* stream) {
+  if (max_groups < 1 || max_groups > 65535 || K % 64 != 0 || K < 64 || N < 1 || x_div < 1 || (x_mode != 0 && x_mode != 1) || !groups) return -1;
+  ExpertParams e = {};
+  GemvParams& p = e.g;
+  p.w = reinterpret_cast<const uint8_t*>(w4b_stack); p.x = x; p.out = out;
+  p.M = 8; p.N = N; p.KG = K / 64; p.ldx = ldx; p.ldo = N; p.x_mode = x_mode; p.s_in = s_in; p.x_slice = x_slice;
+  p.expert_bytes = expert_bytes; p.alt_w = reinterpret_cast<const uint8_t*>(alt_w); p.alt_id = alt_id;
+  p.x_div = x_div; p.x_batch_bytes = x_batch_bytes; p.out_batch = N;
+  e.groups = reinterpret_cast<const ExpertGroups*>(groups);
+  e.nb = (N + 127) / 128;
+  e.run = max(2, (64 / p.KG) & ~1);
+  const int smem = 128 + kRingBytes + 128 + ((p.KG * 64 + 127) & ~127) + 8 * stride_words(p.KG) * 4;
+  if (smem > 232448) return -9;
+  static int configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (configured[dev & 63] < smem) {
+    cudaError_t err = cudaFuncSetAttribute(gemv_w4_groups_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (err != cudaSuccess) return (int)err;
+    configured[dev & 63] = smem;
+  }
+  return b2_launch(gemv_w4_groups_kernel, dim3((e.nb + e.run - 1) / e.run, max_groups), dim3(kThreads), smem,
+                   reinterpret_cast<cudaStream_t>(stream), true, e);
 }
 
 // Quantise activation rows for x_mode 3.  Input modes as the GEMV's (0 bf16 rows, 1 SiLU*up of fp32 slices,

@@ -159,21 +159,65 @@ struct RouterRowsParams {
   RouteRule rule;
   int* topk_idx;            // [M][k + shared_slot]
   float* topk_w;
-  int* ticket;              // one zeroed word; left zero
+  int* ticket;              // zeroed words, left zero: one, or (gridDim.y > 1) one per slice of token rows and one for all
+  int* groups;              // table of (row, slot) pairs by expert (gemv_w4.cu: ExpertGroups), or nullptr
 };
+
+// The pairs of M rows x `stride` slots, ordered by expert, in groups of up to eight of one expert.  256 threads; the order of the
+// pairs inside an expert comes from an atomic counter (a pair's result does not depend on its neighbours).
+constexpr int kGroupIds = 544;      // expert ids: 512 routed and up to 32 runs of a shared expert
+__device__ void group_pairs(const int* topk_idx, int pairs, int* groups, int* s_count, int* s_first) {
+  const int tid = threadIdx.x;
+  for (int i = tid; i < kGroupIds; i += 256) s_count[i] = 0;
+  __syncthreads();
+  for (int i = tid; i < pairs; i += 256) atomicAdd(&s_count[__ldcg(topk_idx + i)], 1);
+  __syncthreads();
+  if (tid < 32) {
+    int run = 0;
+    for (int i0 = 0; i0 < kGroupIds; i0 += 32) {
+      const int n = (s_count[i0 + tid] + 7) >> 3;
+      int x = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, x, o);
+        if (tid >= o) x += v;
+      }
+      s_first[i0 + tid] = run + x - n;
+      run += __shfl_sync(0xffffffffu, x, 31);
+    }
+    if (tid == 0) groups[0] = run;
+  }
+  __syncthreads();
+  for (int e = tid; e < kGroupIds; e += 256) {
+    const int c = s_count[e];
+    for (int j = 0; 8 * j < c; ++j) {
+      groups[16 + (s_first[e] + j) * 10] = e;
+      groups[16 + (s_first[e] + j) * 10 + 1] = min(8, c - 8 * j);
+    }
+  }
+  __syncthreads();
+  for (int i = tid; i < kGroupIds; i += 256) s_count[i] = 0;
+  __syncthreads();
+  for (int i = tid; i < pairs; i += 256) {
+    const int e = __ldcg(topk_idx + i), r = atomicAdd(&s_count[e], 1);
+    groups[16 + (s_first[e] + (r >> 3)) * 10 + 2 + (r & 7)] = i;
+  }
+}
 
 template <bool PLAIN>
 __global__ void __launch_bounds__(256) moe_router_rows_kernel(const RouterRowsParams p) {
-  __shared__ int s_last;
+  __shared__ int s_last, s_count[kGroupIds], s_first[kGroupIds];
   pdl_wait();
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int r = blockIdx.x * 8 + warp;
+  // token rows of this CTA: all of them, or the slice of eight that blockIdx.y names
+  const int m_lo = gridDim.y > 1 ? blockIdx.y * 8 : 0, m_hi = gridDim.y > 1 ? min(p.M, m_lo + 8) : p.M;
   if (r < p.R) {
     const uint4* wr = reinterpret_cast<const uint4*>(p.w + (size_t)r * p.H);
     const int chunks = p.H / 8;                 // 16-byte pieces of a row; a lane takes every 32nd
-    for (int m0 = 0; m0 < p.M; m0 += 8) {
-      const int mt = min(8, p.M - m0);
+    for (int m0 = m_lo; m0 < m_hi; m0 += 8) {
+      const int mt = min(8, m_hi - m0);
       float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       for (int c0 = lane; c0 < chunks; c0 += 32 * 8) {
         // eight pieces of the router row in flight, then the token rows against them
@@ -213,15 +257,15 @@ __global__ void __launch_bounds__(256) moe_router_rows_kernel(const RouterRowsPa
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    const int t = atomicAdd(p.ticket, 1);
+    const int t = atomicAdd(p.ticket + blockIdx.y, 1);
     s_last = t == (int)gridDim.x - 1;
-    if (s_last) *p.ticket = 0;
+    if (s_last) p.ticket[blockIdx.y] = 0;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
   const int stride = p.k + p.shared_slot;
-  for (int m = warp; m < p.M; m += 8) {
+  for (int m = m_lo + warp; m < m_hi; m += 8) {
     const float* lrow = p.logits + (size_t)m * p.ld;
     route_row<PLAIN>(lrow, p.E, p.k, p.rule, p.topk_idx + (size_t)m * stride, p.topk_w + (size_t)m * stride, lane);
     for (int i = lane; i < p.shared_slot; i += 32) {
@@ -229,6 +273,21 @@ __global__ void __launch_bounds__(256) moe_router_rows_kernel(const RouterRowsPa
       p.topk_w[(size_t)m * stride + p.k + i] = p.has_gate ? 1.f / (1.f + __expf(-__ldcg(lrow + p.E))) : 1.f;
     }
   }
+  if (!p.groups) return;
+  // every slice has routed its rows: the CTA that sees that last makes the table
+  __threadfence();
+  __syncthreads();
+  if (gridDim.y > 1) {
+    if (threadIdx.x == 0) {
+      const int t = atomicAdd(p.ticket + gridDim.y, 1);
+      s_last = t == (int)gridDim.y - 1;
+      if (s_last) p.ticket[gridDim.y] = 0;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+  }
+  group_pairs(p.topk_idx, p.M * stride, p.groups, s_count, s_first);
 }
 
 // ---------------------------------------------------------------- count + rank
@@ -418,13 +477,17 @@ extern "C" int b2_moe_route(const float* logits, int ld, int T, int E, int k, in
 
 extern "C" int b2_moe_router_rows(const void* w, const void* x, float* logits, int M, int R, int H, int ld, int E, int k,
                                   int shared_slot, int has_gate, int sigmoid, int groups, int keep, int renorm,
-                                  int* topk_idx, float* topk_w, int* ticket, void* stream) {
+                                  int* topk_idx, float* topk_w, int* ticket, int n_tickets, int* table, void* stream) {
   const RouteRule rule{sigmoid, groups, keep, renorm};
   if (!route_ok(E, k, rule) || H % 8 || M < 1 || R < E + (has_gate ? 1 : 0) || ld < R || shared_slot < 0 || (has_gate && shared_slot > 1))
     return -1;
   RouterRowsParams p{(const __nv_bfloat16*)w, (const __nv_bfloat16*)x, logits, M, R, H, ld, E, k, shared_slot, has_gate,
-                     rule, topk_idx, topk_w, ticket};
-  return b2_launch(route_plain(rule) ? moe_router_rows_kernel<true> : moe_router_rows_kernel<false>, dim3((R + 7) / 8), dim3(256), 0, (cudaStream_t)stream, true, p);
+                     rule, topk_idx, topk_w, ticket, table};
+  if (table && E + shared_slot > kGroupIds) return -1;
+  // Slices of eight token rows have CTAs of their own, which also route them (a router of 257 rows is 33 CTAs: 48 token rows
+  // behind one another took 58 us of a layer's step).  Callers with a single ticket word keep one slice.
+  const int slices = (M + 7) / 8 < n_tickets ? (M + 7) / 8 : 1;
+  return b2_launch(route_plain(rule) ? moe_router_rows_kernel<true> : moe_router_rows_kernel<false>, dim3((R + 7) / 8, slices), dim3(256), 0, (cudaStream_t)stream, true, p);
 }
 
 // counts must hold E zeros on entry (the caller clears it on the stream).

@@ -52,14 +52,37 @@ def combine_rows(part, s, m, k, h, topk_w, shared_part, s_sh, gate_logit, gate_l
                                          K._stream()), "moe_combine_rows")
 
 
+def group_words(pairs: int) -> int:
+    """int32 words of a table of ``pairs`` (row, slot) pairs grouped by expert."""
+    return 16 + 10 * pairs
+
+
+def max_groups(pairs: int, experts: int) -> int:
+    """Groups of up to eight pairs of one expert that ``pairs`` pairs over ``experts`` can make at most."""
+    return min(pairs, (pairs + 7 * experts) // 8)
+
+
 def router_rows(w, x, logits, m, r, h, ld, e, k, shared_slot, has_gate, topk_idx, topk_w, ticket,
-                rule=SOFTMAX_RENORM):
+                rule=SOFTMAX_RENORM, groups=None):
     """Decode rows: router logits (``r`` rows of ``w``: the experts, then the shared expert's gate row) and the
     routing of every row in one launch.  ``shared_slot``: each row gets slot k = (expert id ``e``, sigmoid(gate logit)
     or 1), so ``topk_idx`` / ``topk_w`` hold k + 1 entries per row; a number above 1: that many more slots, ids ``e`` .. with
-    weight 1.  ``ticket``: one zeroed int32 word."""
+    weight 1.  ``ticket``: zeroed int32 words; one, or more than one per eight rows, whose slices then run side by side.
+    ``groups`` (int32, ``group_words`` of the pairs): the pairs by expert, for ``gemv_groups``."""
+    if groups is not None and groups.numel() < group_words(m * (k + int(shared_slot))):
+        raise ValueError("router_rows: the table of groups is too small")
     K._check(K.lib().b2_moe_router_rows(K._p(w), K._p(x), K._p(logits), m, r, h, ld, e, k, int(shared_slot), int(has_gate), *rule,
-                                        K._p(topk_idx), K._p(topk_w), K._p(ticket), K._stream()), "moe_router_rows")
+                                        K._p(topk_idx), K._p(topk_w), K._p(ticket), ticket.numel(), K._p(groups), K._stream()),
+             "moe_router_rows")
+
+
+def gemv_groups(w4b_stack, expert_bytes, groups, most, x, x_div, x_batch_bytes, out, n, k, ldx, x_mode=0, s_in=1, x_slice=0, alt_w=None,
+                alt_id=-1):
+    """Rows against the experts they chose, up to eight rows of an expert at a time; ``out`` is ``[pair][n]``.  ``groups``: the table of
+    ``router_rows``, of at most ``most`` groups."""
+    K._check(K.lib().b2_gemv_w4_groups(K._p(w4b_stack), ctypes.c_longlong(expert_bytes), K._p(groups), most, K._p(x), x_div,
+                                       ctypes.c_longlong(x_batch_bytes), K._p(out), n, k, ldx, x_mode, s_in, ctypes.c_longlong(x_slice),
+                                       K._p(alt_w), alt_id, K._stream()), "gemv_w4_groups")
 
 
 def gemv_experts(w4b_stack, expert_bytes, expert_ids, batches, x, x_div, x_batch_bytes, out, n, k, splits, ldx,

@@ -72,3 +72,58 @@ def test_delta_step_per_slot(slots):
     assert (st.double().cpu() - S).abs().max() < 1e-4 * S.abs().max()
     assert (out.double().cpu() - ref).abs().max() < 2.0 ** -8 * ref.abs().max() + 1e-4       # one rounding to bf16
     assert torch.equal(st[3].cpu(), state[3])
+
+
+# rows, slots per row, routed experts, shared slots, hidden, expert width: rows of an expert below, at and beyond a group of eight;
+# n-blocks in pairs and a lone one; widths whose last ring stage is short
+@pytest.mark.parametrize("m,k,e,shared,h,f", [(8, 2, 4, 0, 256, 128), (1, 1, 3, 1, 64, 192), (9, 4, 16, 1, 512, 256), (64, 8, 256, 1, 2048, 512),
+                                              (33, 8, 8, 1, 320, 64), (64, 1, 1, 1, 128, 320), (17, 3, 64, 0, 4096, 448)])
+def test_grouped_experts(m, k, e, shared, h, f):
+    """Routing in slices, the table of groups, and both matrices of every expert against its rows in fp64."""
+    from b200serve.ops import moe as M
+    from b200serve.utils import quant as Q
+    torch.manual_seed(m + h)
+    ks, dev = k + shared, "cuda"
+    ids = e + shared
+    w_r = torch.randn((e + shared + 7) // 8 * 8, h, device=dev).div_(h ** 0.5).bfloat16()
+    x = torch.randn(m, h, device=dev).bfloat16()
+    ld = w_r.shape[0]
+    logits, idx = torch.zeros(m, ld, device=dev), torch.full((m * ks,), -1, dtype=torch.int32, device=dev)
+    wt, tickets = torch.zeros(m * ks, device=dev), torch.zeros((m + 7) // 8 + 1, dtype=torch.int32, device=dev)
+    groups = torch.zeros(M.group_words(m * ks), dtype=torch.int32, device=dev)
+    for t in (tickets, torch.zeros(1, dtype=torch.int32, device=dev)):          # slices side by side, or one
+        groups.zero_()
+        M.router_rows(w_r, x, logits, m, e + shared, h, ld, e, k, bool(shared), bool(shared), idx, wt, t, groups=groups)
+        torch.cuda.synchronize()
+        ref = x.double() @ w_r.double().T
+        assert (logits.double() - ref)[:, : e + shared].abs().max() < 1e-4 and int(t.abs().sum()) == 0
+        n, tab = int(groups[0]), groups[16:].view(-1, 10).cpu()
+        seen = []
+        for g in tab[:n].tolist():
+            assert 1 <= g[1] <= 8
+            seen += g[2: 2 + g[1]]
+            assert all(int(idx[p]) == g[0] for p in g[2: 2 + g[1]])
+        assert sorted(seen) == list(range(m * ks)) and n <= M.max_groups(m * ks, ids)
+    gu, dn = (torch.cat([Q.random_w4b(r, c, dev, s0 + i) for i in range(ids)]) for r, c, s0 in ((2 * f, h, 100), (h, f, 5)))
+    per_gu, per_dn = gu.numel() // ids, dn.numel() // ids
+    up = torch.full((m * ks, 2 * f), float("nan"), device=dev)
+    out = torch.full((m * ks, h), float("nan"), device=dev)
+    most = M.max_groups(m * ks, ids)
+    alt = dict(alt_w=gu.view(-1)[e * per_gu:].clone(), alt_id=e) if shared else {}
+    M.gemv_groups(gu, per_gu, groups, most, x, ks, h * 2, up, 2 * f, h, h, **alt)
+    alt = dict(alt_w=dn.view(-1)[e * per_dn:].clone(), alt_id=e) if shared else {}
+    M.gemv_groups(dn, per_dn, groups, most, up, 1, 2 * f * 4, out, h, f, 2 * f, x_mode=1, **alt)
+    torch.cuda.synchronize()
+    K.check_status()
+    nb_gu, nb_dn = gu.shape[0] // ids, dn.shape[0] // ids
+    for i in sorted(set(idx.tolist())):
+        pick = (idx == i).nonzero().flatten()
+        wu = Q.dequant_w4b(gu[i * nb_gu: (i + 1) * nb_gu], 2 * f).double()
+        y = x[pick // ks].double() @ wu.T
+        # activations are 15-bit integers against the largest of 64: 2^-15 of it per product, averaged over the row
+        assert (up[pick].double() - y).norm() < 1e-4 * y.norm()
+        v = up[pick].double().view(len(pick), f // 16, 2, 16)
+        a = (F.silu(v[:, :, 0]) * v[:, :, 1]).reshape(len(pick), f)
+        z = a @ Q.dequant_w4b(dn[i * nb_dn: (i + 1) * nb_dn], h).double().T
+        # the product is rounded to bf16 on the way in, once per element: 2^-9 each, averaged over the row
+        assert (out[pick].double() - z).norm() < 2.0 ** -8 * z.norm()
