@@ -242,6 +242,7 @@ class DecoderModel:
         # fixed KV split spans make a row's attention bits independent of the rows it is verified with (speculation
         # then reproduces plain decoding exactly); off, the splits adapt to the context (fastest at any depth)
         self.attn_fixed_spans = False
+        self.attn_waves = 2
         self.fused = self.nccl is None and os.environ.get("B2_UNFUSED", "0") != "1"     # dense layers: residual folds and norms ride inside the GEMVs
         # whole-step kernel (one launch for embedding + all dense layers of a one-request step of up to 8 rows).
         # Off unless asked for (B2_MEGA=1, or the attribute): on the 27B shape at depth 4096 it takes 6.6 ms per
@@ -276,6 +277,18 @@ class DecoderModel:
             K.gemv_w4(ql.w4b, x, part, m, ql.n, ql.k, s, x_mode=x_mode, s_in=s_in, x_slice=x_slice)
         return part, s
 
+    def _attn_splits(self, m: int) -> int:
+        """KV splits of an attention launch of ``m`` rows: as many as keep ``attn_waves`` waves of CTAs busy, at most those that
+        the partial buffers are laid out for.  Rows of different requests fill the GPU by themselves; every split of a short
+        context is a CTA that costs its launch, its copies' latency and a partial to merge, for a handful of keys.  16 layers, 8 KV
+        heads, all splits / two waves: 40 requests at 600 positions 7.63 / 6.61 ms, 64 at 300 10.4 / 8.5, 8 at 4000 in int8 2.61 /
+        2.43, 16 at 1500 in int8 3.90 / 2.84; one wave and four are within 3 % of two."""
+        if self.attn_fixed_spans:
+            return self.nsplit_attn
+        rows = max(1, min(8, 64 // self.cfg.gqa))
+        ctas = self.cfg.n_kv_heads * ((m + rows - 1) // rows if self.rows_one_request and m > 1 else m)
+        return max(1, min(self.nsplit_attn, (self.attn_waves * 296 + ctas - 1) // ctas))
+
     def _attention(self, m: int, ctrl, block_table, max_blocks, kv: KVCache, kc, vc, ks, vs, window: int = 0,
                    quant_out: bool = False) -> bool:
         """Split-KV attention of the step's rows into ``buf.attn_out``.  Head size 128 (bf16 or int8 KV) goes to the
@@ -287,10 +300,11 @@ class DecoderModel:
             inkernel = m <= self.attn_merge_inkernel_rows    # few rows: the last split CTA merges; many: a merge launch
             # ``quant_out``: the caller's next launch is the o projection on pre-quantised rows; the merge writes them
             quant = quant_out and not inkernel and m >= self.prequant_rows and self.merge_quant
+            nsplit = self._attn_splits(m)
             K.attn_rows(b.q, kc, vc, block_table, ctrl, b.o_part, b.ml_part, b.attn_out, b.tickets if inkernel else None,
                         m, cfg.n_q_heads,
-                        cfg.n_kv_heads, cfg.head_dim, self.nsplit_attn, max_blocks, self.scale,
-                        span_pages=(max_blocks + self.nsplit_attn - 1) // self.nsplit_attn if self.attn_fixed_spans else 0,
+                        cfg.n_kv_heads, cfg.head_dim, nsplit, max_blocks, self.scale,
+                        span_pages=(max_blocks + nsplit - 1) // nsplit if self.attn_fixed_spans else 0,
                         k_scale=ks, v_scale=vs, kv_int8=kv.kv_int8, window=window, one_request=self.rows_one_request and m > 1,
                         xq=b.xq if quant else None, xq_gs=b.xq_gs if quant else None)
             return quant
