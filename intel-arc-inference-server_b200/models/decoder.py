@@ -62,6 +62,7 @@ class StepBuffers:
             self.gdn_act = torch.zeros(max_rows, cfg.gdn_proj_dim, dtype=f32, device=device)
             self.gdn_out = torch.zeros(max_rows, cfg.gdn_value_dim, dtype=bf, device=device)
         self.xq = torch.zeros(max_rows * (kmax // 64) * 128, dtype=torch.uint8, device=device)    # pre-quantised rows
+        self.xr = torch.zeros(K.rows_pad(max_rows) * kmax * 2, dtype=torch.uint8, device=device)   # rows of the tcgen05 form
         self.xq_gs = torch.zeros(K.quant_slots(max_rows) * (kmax // 64) * 2, dtype=torch.int32, device=device)   # {scale, -8 sum} per group and token slot
         self._parts = {}
         self.device = device
@@ -234,6 +235,8 @@ class DecoderModel:
         # from this many rows up the activations are quantised once by their own kernel instead of in every
         # CTA of the GEMV (whose prologue repeats the rows' work per 128 output columns)
         self.prequant_rows = int(os.environ.get("B2_PREQUANT_ROWS", "3"))
+        self.rows_min = 17      # rows from which the linears run on tcgen05 (16 layers, integer GEMV / tcgen05: 16 rows 2.43 / 3.10 ms, 17 rows
+        # 3.67 / 3.49, 40 rows 5.90 / 4.43, 64 rows 7.72 / 5.55)
         self.merge_quant = os.environ.get("B2_MERGE_QUANT", "1") == "1"   # the attention merge writes the o projection's quantised rows
         self.attn_rows_min = int(os.environ.get("B2_ATTN_ROWS_MIN", "1"))
         self.rows_one_request = False    # set by the engine around a step whose rows are one request's, consecutive
@@ -263,7 +266,27 @@ class DecoderModel:
             self._gather = torch.zeros(self.nccl[1], max_rows, 2, dtype=torch.float32, device=self.device)
 
     # ------------------------------------------------------------------ pieces
+    def _on_rows(self, m: int) -> bool:
+        """Steps of ``m`` rows take the tcgen05 form of the linears (``gemm_rows.cu``), whose sums are not the integer GEMV's bits:
+        never where a row's bits must not depend on its company, and on one GPU only (no fold over the wire)."""
+        return self.rows_min <= m <= 64 and not self.attn_fixed_spans and self.tp is None and self.nccl is None
+
+    def _gemm_rows(self, name: str, ql: QLinear, x, m: int, staged: bool = False, fold: bool = False, **stage):
+        b = self.buf
+        key = (ql.n, ql.k, "rows")
+        s = self._splits.get(key)
+        if s is None:
+            s = self._splits[key] = K.rows_splits(ql.n, ql.k)
+        part = b.part(name, s, ql.n)
+        if not staged:
+            K.stage_rows(x, m, ql.k, b.xr, **stage)
+        K.gemm_w4_rows(ql.w4b, b.xr, part, m, ql.n, ql.k, s, fold_tickets=b.fold_tickets if fold else None,
+                       fold_resid=b.resid if fold else None, fold_ssq=b.ssq if fold else None)
+        return part, s
+
     def _gemv(self, name: str, ql: QLinear, x: torch.Tensor, m: int, x_mode=0, s_in=1, x_slice=0):
+        if self._on_rows(m):
+            return self._gemm_rows(name, ql, x, m, x_mode=x_mode, s_in=s_in, x_slice=x_slice)
         key = (ql.n, ql.k)
         s = self._splits.get(key)
         if s is None:
@@ -299,14 +322,15 @@ class DecoderModel:
         if (m >= self.attn_rows_min or window == -1) and cfg.head_dim == 128 and self.nsplit_attn <= 64 and cfg.gqa <= 16:
             inkernel = m <= self.attn_merge_inkernel_rows    # few rows: the last split CTA merges; many: a merge launch
             # ``quant_out``: the caller's next launch is the o projection on pre-quantised rows; the merge writes them
-            quant = quant_out and not inkernel and m >= self.prequant_rows and self.merge_quant
+            wide = self._on_rows(m)
+            quant = quant_out and not inkernel and (wide or m >= self.prequant_rows) and self.merge_quant
             nsplit = self._attn_splits(m)
             K.attn_rows(b.q, kc, vc, block_table, ctrl, b.o_part, b.ml_part, b.attn_out, b.tickets if inkernel else None,
                         m, cfg.n_q_heads,
                         cfg.n_kv_heads, cfg.head_dim, nsplit, max_blocks, self.scale,
                         span_pages=(max_blocks + nsplit - 1) // nsplit if self.attn_fixed_spans else 0,
                         k_scale=ks, v_scale=vs, kv_int8=kv.kv_int8, window=window, one_request=self.rows_one_request and m > 1,
-                        xq=b.xq if quant else None, xq_gs=b.xq_gs if quant else None)
+                        xq=(b.xr if wide else b.xq) if quant else None, xq_gs=b.xq_gs if quant and not wide else None)
             return quant
         else:
             if window > 0:
@@ -351,13 +375,16 @@ class DecoderModel:
                     x_slice=0, tp_fold: bool = True, prequantised: bool = False):
         """``tp_fold`` False: a linear every rank holds whole (a draft head's front) folds locally, without the
         ranks' all-reduce."""
+        if self._on_rows(m):
+            return self._gemm_rows(name, ql, x, m, staged=prequantised, fold=fold, x_mode=x_mode, s_in=s_in, x_slice=x_slice, norm_w=norm_w,
+                                   norm_ssq=self.buf.ssq if norm_w is not None else None, norm_eps=self.cfg.rms_eps)
         key = (ql.n, ql.k)
         s = self._splits.get(key)
         if s is None:
             s = self._splits[key] = K.gemv_splits(ql.n, ql.k)
         b = self.buf
         part = b.part(name, s, ql.n)
-        if prequantised:        # ``buf.xq`` / ``buf.xq_gs`` already hold these rows (written by the attention merge)
+        if prequantised:        # ``buf.xq`` / ``buf.xq_gs`` (``buf.xr``) already hold these rows (written by the attention merge)
             x, x_mode, norm_w, xq_gs = b.xq, 3, None, b.xq_gs
         elif m >= self.prequant_rows:
             K.quant_x(x, m, ql.k, b.xq, b.xq_gs, x_mode=x_mode, s_in=s_in, x_slice=x_slice, norm_w=norm_w,

@@ -359,6 +359,17 @@ __device__ __forceinline__ StagedVec stage_quant(uint4 val) {
 // the vector's four words go to +0 (high, k 0..3), +4 (low), +8 (high, k 4..7), +12 (low).
 __device__ __forceinline__ int stage_word(int vq) { return (vq & 1) * 16 + (vq >> 2) * 2 + ((vq & 3) >> 1); }
 
+// ---------------------------------------------------------------- activation rows for the tcgen05 form (gemm_rows.cu)
+// Vector `v` (k = 8 v .. 8 v + 7) of a row into [K / 64][T][128 bytes]: a group's element 8 i + 2 t + e of the operand is
+// k = 32 (i >> 2) + 16 (i & 1) + 4 t + ((i >> 1) & 1) + 2 e, the order in which a W4B word's nibbles come apart in pairs; the
+// 16-byte chunk i of row r lies at chunk i ^ (r & 7), the 128-byte swizzle.
+__device__ __forceinline__ void store_row_vec(uint8_t* xr, int T, int row, int v, uint4 val) {
+  const int vq = v & 7, i = 4 * (vq >> 2) + ((vq >> 1) & 1);
+  uint8_t* dst = xr + ((size_t)(v >> 3) * T + row) * 128 + 8 * (vq & 1);
+  *reinterpret_cast<uint2*>(dst + ((i ^ (row & 7)) << 4)) = make_uint2(__byte_perm(val.x, val.y, 0x5410), __byte_perm(val.z, val.w, 0x5410));
+  *reinterpret_cast<uint2*>(dst + (((i + 2) ^ (row & 7)) << 4)) = make_uint2(__byte_perm(val.x, val.y, 0x7632), __byte_perm(val.z, val.w, 0x7632));
+}
+
 }  // namespace b2
 
 // Host-side launch helper: every kernel of the decode path is launched with the

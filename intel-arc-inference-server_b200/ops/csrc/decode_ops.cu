@@ -506,7 +506,8 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(const AttnDecParams p)
 
 // grid (n_q, M), D threads.  xq != nullptr (D = 128): the head's 128 outputs, as rounded to bf16, also leave as the two
 // quantised 64-k groups the o projection's integer GEMV reads (the work of quant_x_kernel on this row slice, same
-// bits), which saves that launch in a step of several rows.
+// bits), which saves that launch in a step of several rows; without xq_gs, as the bf16 rows of the tcgen05 form
+// (stage_rows_kernel, gs_rows token rows per group).
 __global__ void attn_merge_kernel(const float* o_part, const float* ml_part, __nv_bfloat16* out, int n_q, int nsplit,
                                   int D, uint8_t* xq, uint32_t* xq_gs, int gs_rows) {
   __shared__ float cw[64];
@@ -563,6 +564,10 @@ __global__ void attn_merge_kernel(const float* o_part, const float* ml_part, __n
     __syncthreads();
     if (d < 32) {   // lanes 0..15 hold the head's sixteen 16-byte vectors; every lane of the warp calls the quantiser
       const uint4 val = d < 16 ? reinterpret_cast<const uint4*>(srow)[d] : make_uint4(0, 0, 0, 0);
+      if (!xq_gs) {        // rows of the tcgen05 form
+        if (d < 16) store_row_vec(xq, gs_rows, m, h * 16 + d, val);
+        return;
+      }
       const StagedVec sv = stage_quant(val);
       if (d < 16) {
         const int KG = n_q * 2, group = h * 2 + (d >> 3), vq = d & 7;
@@ -973,10 +978,11 @@ extern "C" int b2_attn_merge(const float* o_part, const float* ml_part, void* ou
 }
 
 // The merge that also writes the rows' quantised form for the o projection (head size 128; xq [M][n_q * 2][128 B],
-// xq_gs [n_q * 2][gs_rows] {scale, -8 sum}: the layout of b2_quant_x for K = n_q * 128).
+// xq_gs [n_q * 2][gs_rows] {scale, -8 sum}: the layout of b2_quant_x for K = n_q * 128; xq_gs nullptr: that of b2_stage_rows,
+// xq [n_q * 2][gs_rows][128 B]).
 extern "C" int b2_attn_merge_quant(const float* o_part, const float* ml_part, void* out, int M, int n_q, int nsplit, int D,
                                    void* xq, void* xq_gs, int gs_rows, void* stream) {
-  if (D != 128 || !xq || !xq_gs || gs_rows < M) return -1;
+  if (D != 128 || !xq || gs_rows < M) return -1;
   return b2_launch(attn_merge_kernel, dim3(n_q, M), dim3(D), 0, (cudaStream_t)stream, true, o_part, ml_part,
                    (__nv_bfloat16*)out, n_q, nsplit, D, (uint8_t*)xq, (uint32_t*)xq_gs, gs_rows);
 }

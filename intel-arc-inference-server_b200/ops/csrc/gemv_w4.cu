@@ -802,6 +802,27 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
   }
 }
 
+// The rows as the tcgen05 form reads them (gemm_rows.cu): bf16, [KG][T][128 bytes] with the 128-byte swizzle, in its k order.
+// grid (ceil(KG / 32), M), 256 threads: one 16-byte vector per thread.
+__global__ void __launch_bounds__(256) stage_rows_kernel(const GemvParams p, uint8_t* xr) {
+  __shared__ float s_rinv;
+  pdl_wait();
+  pdl_launch_dependents();
+  const int row = blockIdx.y, tid = threadIdx.x;
+  if (p.x_mode == 2) {
+    if (tid < 32) {
+      float ss = 0.f;
+      for (int j = tid; j < p.norm_nb; j += 32) ss += p.norm_ssq[(size_t)row * p.norm_nb + j];
+      ss = warp_sum(ss);
+      if (tid == 0) s_rinv = rsqrtf(ss / (float)(p.KG * 64) + p.norm_eps);
+    }
+    __syncthreads();
+  }
+  const int v = blockIdx.x * 256 + tid;
+  if (v >= p.KG * 8) return;
+  store_row_vec(xr, p.rows, row, v, stage_load(p, reinterpret_cast<const uint8_t*>(p.x), row, v * 8, p.x_mode == 2 ? s_rinv : 1.f));
+}
+
 template <int T>
 int launch_t(GemvParams& p, cudaStream_t stream) {
   // staged rows and chunk length: as much of the split's k range as fits the activation budget
@@ -1031,6 +1052,18 @@ extern "C" int b2_quant_x(const void* x, int M, int K, int ldx, int x_mode, int 
   p.rows = M <= 8 ? 8 : (M <= 16 ? 16 : (M <= 32 ? 32 : 64));   // token slots per group in xq_gs (8 x the GEMV's tile count)
   dim3 grid((p.KG * 8 + 255) / 256, M);
   return b2_launch(quant_x_kernel, grid, dim3(256), 0, (cudaStream_t)stream, true, p, (uint8_t*)xq, (uint32_t*)xq_gs);
+}
+
+// Rows for b2_gemm_w4_rows, input modes as b2_quant_x; xr is [K / 64][M rounded up to 16][128] bytes (rows from M on are not written).
+extern "C" int b2_stage_rows(const void* x, int M, int K, int ldx, int x_mode, int s_in, long long x_slice, const float* norm_w,
+                             const float* norm_ssq, float norm_eps, void* xr, void* stream) {
+  if (M < 1 || M > 64 || K % 64 != 0 || x_mode < 0 || x_mode > 2) return -1;
+  if (x_mode == 2 && (K % 128 != 0 || !norm_w || !norm_ssq)) return -2;
+  GemvParams p = {};
+  p.x = x; p.M = M; p.KG = K / 64; p.ldx = ldx; p.x_mode = x_mode; p.s_in = s_in; p.x_slice = x_slice;
+  p.norm_w = norm_w; p.norm_ssq = norm_ssq; p.norm_nb = K / 128; p.norm_eps = norm_eps;
+  p.rows = (M + 15) & ~15;
+  return b2_launch(stage_rows_kernel, dim3((p.KG * 8 + 255) / 256, M), dim3(256), 0, (cudaStream_t)stream, true, p, (uint8_t*)xr);
 }
 
 B2_DEFINE_STATUS(gemv)

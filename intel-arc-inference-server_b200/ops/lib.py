@@ -17,7 +17,7 @@ import torch
 from . import build as _build
 
 _lib: Optional[ctypes.CDLL] = None
-_UNITS = ("gemv", "decode", "gemm", "attn", "attnrows", "moe", "comm", "ep", "spec", "sampler", "gdn", "mega", "dflash", "latent", "mlstm", "channel")
+_UNITS = ("gemv", "decode", "gemm", "attn", "attnrows", "moe", "comm", "ep", "spec", "sampler", "gdn", "mega", "dflash", "latent", "mlstm", "channel", "gemmrows")
 
 # Control block layout (int32 words) -- mirrors decode_ops.cu
 CTRL_N_ROWS = 0
@@ -196,6 +196,37 @@ def quant_x(x, m, k, xq, xq_gs, *, x_mode=0, s_in=1, x_slice=0, ldx=None, norm_w
     _check(rc, "quant_x")
 
 
+def rows_pad(m: int) -> int:
+    """Token rows per 64-k group that ``stage_rows`` lays out for ``m`` rows."""
+    return (m + 15) // 16 * 16
+
+
+def stage_rows(x, m, k, xr, *, x_mode=0, s_in=1, x_slice=0, ldx=None, norm_w=None, norm_ssq=None, norm_eps=0.0):
+    """``m`` activation rows as ``gemm_w4_rows`` reads them (``xr``: ``rows_pad(m)`` x ``k`` bf16); input modes as ``quant_x``."""
+    if ldx is None:
+        ldx = 2 * k if x_mode == 1 else k
+    if m > 64 or xr.numel() * xr.element_size() < rows_pad(m) * k * 2:
+        raise ValueError(f"stage_rows: buffer too small for {m} rows of {k}")
+    rc = lib().b2_stage_rows(_p(x), m, k, ldx, x_mode, s_in, ctypes.c_longlong(x_slice), _p(norm_w), _p(norm_ssq),
+                             ctypes.c_float(norm_eps), _p(xr), _stream())
+    _check(rc, "stage_rows")
+
+
+def rows_splits(n: int, k: int) -> int:
+    """k splits of ``gemm_w4_rows``: the GEMV's, less those that would be left without a group."""
+    kg = k // 64
+    per = (-(-kg // gemv_splits(n, k)) + 3) // 4 * 4
+    return -(-kg // per)
+
+
+def gemm_w4_rows(w4b, xr, out, m, n, k, splits, *, fold_tickets=None, fold_resid=None, fold_ssq=None):
+    """``out[s][m][n]`` fp32 partial sums of staged rows (``stage_rows``) against a W4B weight, on tcgen05; ``fold_*`` as in
+    ``gemv_w4_fused``."""
+    rc = lib().b2_gemm_w4_rows(_p(w4b), _p(xr), _p(out), m, n, k, splits, _p(fold_tickets), _p(fold_resid), _p(fold_resid),
+                               _p(fold_ssq), _stream())
+    _check(rc, "gemm_w4_rows")
+
+
 def decode_mega_sms() -> int:
     """CTAs of the whole-step decode kernel: one per SM of the current device."""
     n = lib().b2_decode_mega_sms()
@@ -281,7 +312,7 @@ def attn_rows(q, k_cache, v_cache, block_table, ctrl, o_part, ml_part, out, tick
     ``one_request``: the caller knows that all ``m`` rows are one request's, at consecutive positions; the launch then
     has one CTA column per group of rows instead of one per row (most of which would leave at once).
     ``xq`` / ``xq_gs`` (with ``tickets=None``): the merge also writes the rows in the quantised form of ``quant_x`` for
-    K = n_q * d, so that the o projection's GEMV can read them without that launch."""
+    K = n_q * d, so that the o projection's GEMV can read them without that launch; ``xq`` alone: in the form of ``stage_rows``."""
     rc = lib().b2_attn_rows(_p(q), _p(k_cache), _p(v_cache), _p(k_scale), _p(v_scale), 1 if kv_int8 else 0,
                             _p(block_table), _p(ctrl), _p(o_part), _p(ml_part),
                             _p(out), _p(tickets), m, n_q, n_kv, d, nsplit, max_blocks, ctypes.c_float(scale), span_pages,
@@ -290,7 +321,7 @@ def attn_rows(q, k_cache, v_cache, block_table, ctrl, o_part, ml_part, out, tick
     if tickets is None:     # many rows: the merge is its own launch, one CTA per row and head
         if xq is not None:
             rc = lib().b2_attn_merge_quant(_p(o_part), _p(ml_part), _p(out), m, n_q, nsplit, d, _p(xq), _p(xq_gs),
-                                           quant_slots(m), _stream())
+                                           quant_slots(m) if xq_gs is not None else rows_pad(m), _stream())
         else:
             rc = lib().b2_attn_merge(_p(o_part), _p(ml_part), _p(out), m, n_q, nsplit, d, _stream())
         _check(rc, "attn_merge")

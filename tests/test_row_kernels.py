@@ -127,3 +127,83 @@ def test_grouped_experts(m, k, e, shared, h, f):
         z = a @ Q.dequant_w4b(dn[i * nb_dn: (i + 1) * nb_dn], h).double().T
         # the product is rounded to bf16 on the way in, once per element: 2^-9 each, averaged over the row
         assert (out[pick].double() - z).norm() < 2.0 ** -8 * z.norm()
+
+
+# rows at the edges of the four instances (16 token rows each); splits with unequal and lone groups; n not a multiple of 128; fewer
+# blocks than the four sets take in turn; more items than SMs
+@pytest.mark.parametrize("m,n,k,splits", [(1, 128, 64, 1), (9, 256, 128, 2), (16, 300, 320, 1), (17, 128, 704, 3), (31, 1000, 1024, 4), (32, 5120, 640, 4),
+                                          (33, 640, 448, 7), (48, 128, 1088, 16), (49, 20480, 256, 2), (64, 384, 5120, 7)])
+@pytest.mark.parametrize("fold", [False, True])
+def test_linears_on_rows(m, n, k, splits, fold):
+    from b200serve.utils import quant as Q
+    torch.manual_seed(n + m)
+    dev, per = "cuda", (-(-(k // 64) // splits) + 3) // 4 * 4
+    splits = -(-(k // 64) // per)
+    w = Q.random_w4b(n, k, dev, 7)
+    wf = Q.dequant_w4b(w, n).double()
+    x = torch.randn(m, k, device=dev).bfloat16()
+    xr = torch.zeros(K.rows_pad(m) * k * 2, dtype=torch.uint8, device=dev)
+    xr.view(-1)[:] = 0xff          # rows that are not staged are NaN
+    part = torch.full((splits, m, n), float("nan"), device=dev)
+    K.stage_rows(x, m, k, xr)
+    nb = (n + 127) // 128
+    tickets, ssq = torch.zeros(nb, dtype=torch.int32, device=dev), torch.zeros(m, nb, device=dev)
+    resid = torch.randn(m, n, device=dev).bfloat16()
+    r0 = resid.clone()
+    args = dict(fold_tickets=tickets, fold_resid=resid, fold_ssq=ssq) if fold else {}
+    K.gemm_w4_rows(w, xr, part, m, n, k, splits, **args)
+    torch.cuda.synchronize()
+    K.check_status()
+    ref = x.double() @ wf.T
+    # exact products; k sums in fp32 whatever the order: a few 2^-24 of the terms' root sum of squares
+    bound = 16 * 2.0 ** -24 * (x.double().abs() @ wf.abs().T)
+    assert ((part.double().sum(0) - ref).abs() <= bound + 1e-12).all()
+    for s in range(splits):
+        lo, hi = s * per * 64, min(k, (s + 1) * per * 64)
+        assert (part[s].double() - x[:, lo:hi].double() @ wf[:, lo:hi].T).norm() < 1e-5 * ref.norm()
+    if fold:
+        want = r0.double() + ref
+        assert ((resid.double() - want).abs() <= 2.0 ** -8 * want.abs() + bound + 1e-6).all() and int(tickets.abs().sum()) == 0
+        sq = torch.nn.functional.pad(resid.double() ** 2, (0, nb * 128 - n)).view(m, nb, 128).sum(-1)
+        assert (ssq.double() - sq).abs().max() < 1e-5 * sq.max()
+
+
+@pytest.mark.parametrize("m", [3, 16, 40])
+def test_staged_rows_of_every_kind(m):
+    """SiLU(gate) * up of split sums, normalised residual rows, and the attention merge's own rows, each against a plain row form of the
+    same values."""
+    torch.manual_seed(m)
+    dev, k, s_in = "cuda", 640, 3
+    pad = K.rows_pad(m)
+
+    def unstaged(xr):
+        a = xr.view(torch.bfloat16).view(k // 64, pad, 8, 8)[:, :m]                   # [group][row][chunk][element]
+        rows = torch.arange(m, device=dev)
+        a = torch.stack([a[:, rows, (i ^ (rows & 7))] for i in range(8)], dim=2)      # chunks in order
+        out = torch.empty(m, k // 64, 64, dtype=torch.bfloat16, device=dev)
+        for i in range(8):
+            for t in range(4):
+                for e in range(2):
+                    out[:, :, 32 * (i >> 2) + 16 * (i & 1) + 4 * t + ((i >> 1) & 1) + 2 * e] = a[:, :, i, 2 * t + e].T
+        return out.view(m, k)
+    xr = torch.zeros(pad * k * 2, dtype=torch.uint8, device=dev)
+    x = torch.randn(m, k, device=dev).bfloat16()
+    K.stage_rows(x, m, k, xr)
+    assert torch.equal(unstaged(xr), x)
+    part = torch.randn(s_in, m, 2 * k, device=dev)
+    K.stage_rows(part, m, k, xr, x_mode=1, s_in=s_in, x_slice=m * 2 * k)
+    v = part.sum(0).double().view(m, k // 16, 2, 16)
+    want = (F.silu(v[:, :, 0]) * v[:, :, 1]).reshape(m, k)
+    assert ((unstaged(xr).double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5).all()
+    nw = 1 + 0.1 * torch.randn(k, device=dev)
+    ssq = (x.float() ** 2).view(m, k // 128, 128).sum(-1).contiguous()
+    K.stage_rows(x, m, k, xr, x_mode=2, norm_w=nw, norm_ssq=ssq, norm_eps=1e-6)
+    want = x.double() * torch.rsqrt((x.double() ** 2).mean(-1, keepdim=True) + 1e-6) * nw.double()
+    assert ((unstaged(xr).double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
+    heads, ns = k // 128, 5
+    o, ml = torch.randn(m, heads, ns, 128, device=dev), torch.rand(m, heads, ns, 2, device=dev) + 0.5
+    out = torch.zeros(m, k, dtype=torch.bfloat16, device=dev)
+    xr.zero_()
+    rc = K.lib().b2_attn_merge_quant(K._p(o), K._p(ml), K._p(out), m, heads, ns, 128, K._p(xr), None, pad, K._stream())
+    torch.cuda.synchronize()
+    assert rc == 0 and torch.equal(unstaged(xr), out) and out.abs().sum() > 0
