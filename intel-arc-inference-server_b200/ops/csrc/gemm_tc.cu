@@ -102,6 +102,116 @@ struct Cfg {
   static constexpr int THREADS = kThreads + (W4 ? kDequantWarps * 32 : 0);
 };
 
+// 32 accumulators of one row, columns n0 .. n0 + 31, through the epilogue into C
+__device__ __forceinline__ void store_chunk(const GemmParams& p, const uint32_t (&v)[32], int grow, int n0) {
+            float f[32];
+  #pragma unroll
+            for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+            if (p.epi == EPI_SILU_MUL || p.epi == EPI_GLU) {
+              // columns alternate 16 gate, 16 up: 16 outputs per 32 accumulator columns
+              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)grow * p.ldc + (n0 >> 1);
+              uint32_t o[8];
+              if (p.epi == EPI_GLU && p.glu.bias) {
+  #pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  const float4 b = __ldg(reinterpret_cast<const float4*>(p.glu.bias + n0) + j);
+                  f[4 * j] += b.x; f[4 * j + 1] += b.y; f[4 * j + 2] += b.z; f[4 * j + 3] += b.w;
+                }
+              }
+  #pragma unroll
+              for (int j = 0; j < 8; ++j)
+                o[j] = p.epi == EPI_GLU ? pack_bf16(glu(p.glu, f[2 * j], f[16 + 2 * j]), glu(p.glu, f[2 * j + 1], f[17 + 2 * j]))
+                                        : pack_bf16(silu(f[2 * j]) * f[16 + 2 * j], silu(f[2 * j + 1]) * f[17 + 2 * j]);
+              *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+              *reinterpret_cast<uint4*>(dst + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+            } else if (p.epi == EPI_F32) {
+              float* dst = reinterpret_cast<float*>(p.C) + (size_t)grow * p.ldc + n0;
+              if (n0 + 32 <= p.N) {
+  #pragma unroll
+                for (int j = 0; j < 8; ++j)
+                  *reinterpret_cast<float4*>(dst + 4 * j) = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+              } else {
+                for (int j = 0; j < 32 && n0 + j < p.N; ++j) dst[j] = f[j];
+              }
+            } else {
+              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)grow * p.ldc + n0;
+              if (p.epi == EPI_RESID_ADD) {
+                const __nv_bfloat16* rs = p.resid + (size_t)grow * p.ldc + n0;
+                if (n0 + 32 <= p.N) {
+  #pragma unroll
+                  for (int j = 0; j < 4; ++j) {
+                    const uint4 rv = *reinterpret_cast<const uint4*>(rs + 8 * j);
+                    const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
+  #pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                      f[8 * j + 2 * q] += bf16_lo(rw[q]);
+                      f[8 * j + 2 * q + 1] += bf16_hi(rw[q]);
+                    }
+                  }
+                } else {
+                  for (int j = 0; j < 32 && n0 + j < p.N; ++j) f[j] += __bfloat162float(rs[j]);
+                }
+              }
+              if (p.epi == EPI_RELU2) {
+  #pragma unroll
+                for (int j = 0; j < 32; ++j) f[j] = relu2(f[j]);
+              }
+              if (n0 + 32 <= p.N) {
+  #pragma unroll
+                for (int j = 0; j < 4; ++j)
+                  *reinterpret_cast<uint4*>(dst + 8 * j) =
+                      make_uint4(pack_bf16(f[8 * j], f[8 * j + 1]), pack_bf16(f[8 * j + 2], f[8 * j + 3]),
+                                 pack_bf16(f[8 * j + 4], f[8 * j + 5]), pack_bf16(f[8 * j + 6], f[8 * j + 7]));
+              } else {
+                for (int j = 0; j < 32 && n0 + j < p.N; ++j) dst[j] = __float2bfloat16(f[j]);
+              }
+            }
+}
+
+// Vector `u` of a stage's W4B blocks (256 vectors a block) -> sixteen 8-byte pieces of the bf16 B tile.  A vector holds rows g and
+// g + 8 of a 16-row tile, 64 k: low nibbles are k 4t..4t+3 of a 32-k step, high nibbles k + 16 (the operand order of the decode
+// GEMV); row r lies at r * 128 bytes, 16-byte chunk (k / 8) XOR (r mod 8) -- the 128-byte swizzle.
+__device__ __forceinline__ void expand_w4(int u, uint32_t raw, uint32_t sb) {
+            const int b = u >> 8, v = u & 255, j = v >> 5, l = v & 31, g = l >> 2, tq = l & 3;
+            uint4 wv;
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w)
+                         : "r"(raw + b * kW4Block + v * 16));
+            uint32_t sc2;
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc2) : "r"(raw + b * kW4Block + 4096 + (j * 16 + 2 * g) * 2));
+            const __half2 sh = *reinterpret_cast<const __half2*>(&sc2);
+            const float s_lo = __low2float(sh), s_hi = __high2float(sh);
+            const uint32_t wa[4] = {wv.x, wv.y, wv.z, wv.w};
+            uint64_t sc2x[2], off2;
+            asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[0]) : "f"(s_lo));
+            asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[1]) : "f"(s_hi));
+            asm("mov.b64 %0, {%1, %1};" : "=l"(off2) : "f"(-8388616.f));
+  #pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const int row = b * 128 + j * 16 + g + 8 * (c & 1);
+  #pragma unroll
+              for (int e = 0; e < 2; ++e) {
+                const uint32_t x = (wa[c] >> (4 * e)) & 0x0F0F0F0Fu;
+                // bytes -> floats through the 2^23 trick: 0x4B0000qq is 8388608 + q; q - 8 (exact) and the product with
+                // the scale run as packed pairs (add.f32x2 / mul.f32x2), the same floats as the scalar form
+                uint64_t f01, f23;
+                asm("mov.b64 %0, {%1, %2};" : "=l"(f01) : "r"(__byte_perm(x, 0x4B000000u, 0x7440)), "r"(__byte_perm(x, 0x4B000000u, 0x7441)));
+                asm("mov.b64 %0, {%1, %2};" : "=l"(f23) : "r"(__byte_perm(x, 0x4B000000u, 0x7442)), "r"(__byte_perm(x, 0x4B000000u, 0x7443)));
+                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(off2));
+                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(off2));
+                asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(sc2x[c & 1]));
+                asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(sc2x[c & 1]));
+                float g0, g1, g2, g3;
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(g0), "=f"(g1) : "l"(f01));
+                asm("mov.b64 {%0, %1}, %2;" : "=f"(g2), "=f"(g3) : "l"(f23));
+                const uint32_t p01 = pack_bf16(g0, g1);
+                const uint32_t p23 = pack_bf16(g2, g3);
+                const int k0 = 32 * (c >> 1) + 16 * e + 4 * tq;
+                const uint32_t dst = sb + row * 128 + ((((uint32_t)k0 >> 3) ^ ((uint32_t)row & 7u)) << 4) + (k0 & 7) * 2;
+                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst), "r"(p01), "r"(p23) : "memory");
+              }
+            }
+}
+
 template <int BN, bool I8, bool W4 = false>
 __global__ void __launch_bounds__(Cfg<BN, W4>::THREADS, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -234,9 +344,6 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else if (W4 && warp >= 6) {
     // ------------------------------------------------------------ W4 expansion (warps 6 .. 6 + kDequantWarps - 1)
-    // One 16-byte vector of a W4B block holds rows g and g + 8 of a 16-row tile, 64 k: low nibbles are k 4t..4t+3 of a
-    // 32-k step, high nibbles k + 16 (the operand order of the decode GEMV).  Each vector becomes sixteen 8-byte
-    // pieces of the B tile: row r at r * 128 bytes, 16-byte chunk (k / 8) XOR (r mod 8) -- the 128-byte swizzle.
     const int dt = threadIdx.x - 6 * 32;   // 0 .. 32 * kDequantWarps - 1
     int it = 0;
     bool ok = true;
@@ -249,46 +356,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (ok) ok = __all_sync(0xffffffffu, mbar_wait(rawfull0 + 8 * s, (it / C::STAGES) & 1, ERR_GEMM_FULL_WAIT));
         if (!ok) break;
         const uint32_t sb = smem_base + s * C::STAGE + C::A_BYTES, raw = raw_base + s * C::RAW;
-        for (int u = dt; u < nblk * 256; u += kDequantWarps * 32) {
-          const int b = u >> 8, v = u & 255, j = v >> 5, l = v & 31, g = l >> 2, tq = l & 3;
-          uint4 wv;
-          asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w)
-                       : "r"(raw + b * kW4Block + v * 16));
-          uint32_t sc2;
-          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc2) : "r"(raw + b * kW4Block + 4096 + (j * 16 + 2 * g) * 2));
-          const __half2 sh = *reinterpret_cast<const __half2*>(&sc2);
-          const float s_lo = __low2float(sh), s_hi = __high2float(sh);
-          const uint32_t wa[4] = {wv.x, wv.y, wv.z, wv.w};
-          uint64_t sc2x[2], off2;
-          asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[0]) : "f"(s_lo));
-          asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[1]) : "f"(s_hi));
-          asm("mov.b64 %0, {%1, %1};" : "=l"(off2) : "f"(-8388616.f));
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int row = b * 128 + j * 16 + g + 8 * (c & 1);
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const uint32_t x = (wa[c] >> (4 * e)) & 0x0F0F0F0Fu;
-              // bytes -> floats through the 2^23 trick: 0x4B0000qq is 8388608 + q; q - 8 (exact) and the product with
-              // the scale run as packed pairs (add.f32x2 / mul.f32x2), the same floats as the scalar form
-              uint64_t f01, f23;
-              asm("mov.b64 %0, {%1, %2};" : "=l"(f01) : "r"(__byte_perm(x, 0x4B000000u, 0x7440)), "r"(__byte_perm(x, 0x4B000000u, 0x7441)));
-              asm("mov.b64 %0, {%1, %2};" : "=l"(f23) : "r"(__byte_perm(x, 0x4B000000u, 0x7442)), "r"(__byte_perm(x, 0x4B000000u, 0x7443)));
-              asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(off2));
-              asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(off2));
-              asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(sc2x[c & 1]));
-              asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(sc2x[c & 1]));
-              float g0, g1, g2, g3;
-              asm("mov.b64 {%0, %1}, %2;" : "=f"(g0), "=f"(g1) : "l"(f01));
-              asm("mov.b64 {%0, %1}, %2;" : "=f"(g2), "=f"(g3) : "l"(f23));
-              const uint32_t p01 = pack_bf16(g0, g1);
-              const uint32_t p23 = pack_bf16(g2, g3);
-              const int k0 = 32 * (c >> 1) + 16 * e + 4 * tq;
-              const uint32_t dst = sb + row * 128 + ((((uint32_t)k0 >> 3) ^ ((uint32_t)row & 7u)) << 4) + (k0 & 7) * 2;
-              asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst), "r"(p01), "r"(p23) : "memory");
-            }
-          }
-        }
+        for (int u = dt; u < nblk * 256; u += kDequantWarps * 32) expand_w4(u, raw, sb);
         fence_proxy_async_smem();   // the MMA reads the tile through the async proxy
         __syncwarp();
         if (lane == 0) mbar_arrive(full0 + 8 * s);
@@ -378,68 +446,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
             __syncwarp();
           }
         } else if (row_ok && n0 < p.N) {
-          float f[32];
-#pragma unroll
-          for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-          if (p.epi == EPI_SILU_MUL || p.epi == EPI_GLU) {
-            // columns alternate 16 gate, 16 up: 16 outputs per 32 accumulator columns
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)grow * p.ldc + (n0 >> 1);
-            uint32_t o[8];
-            if (p.epi == EPI_GLU && p.glu.bias) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j) {
-                const float4 b = __ldg(reinterpret_cast<const float4*>(p.glu.bias + n0) + j);
-                f[4 * j] += b.x; f[4 * j + 1] += b.y; f[4 * j + 2] += b.z; f[4 * j + 3] += b.w;
-              }
-            }
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              o[j] = p.epi == EPI_GLU ? pack_bf16(glu(p.glu, f[2 * j], f[16 + 2 * j]), glu(p.glu, f[2 * j + 1], f[17 + 2 * j]))
-                                      : pack_bf16(silu(f[2 * j]) * f[16 + 2 * j], silu(f[2 * j + 1]) * f[17 + 2 * j]);
-            *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
-            *reinterpret_cast<uint4*>(dst + 8) = make_uint4(o[4], o[5], o[6], o[7]);
-          } else if (p.epi == EPI_F32) {
-            float* dst = reinterpret_cast<float*>(p.C) + (size_t)grow * p.ldc + n0;
-            if (n0 + 32 <= p.N) {
-#pragma unroll
-              for (int j = 0; j < 8; ++j)
-                *reinterpret_cast<float4*>(dst + 4 * j) = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-            } else {
-              for (int j = 0; j < 32 && n0 + j < p.N; ++j) dst[j] = f[j];
-            }
-          } else {
-            __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)grow * p.ldc + n0;
-            if (p.epi == EPI_RESID_ADD) {
-              const __nv_bfloat16* rs = p.resid + (size_t)grow * p.ldc + n0;
-              if (n0 + 32 <= p.N) {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const uint4 rv = *reinterpret_cast<const uint4*>(rs + 8 * j);
-                  const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
-#pragma unroll
-                  for (int q = 0; q < 4; ++q) {
-                    f[8 * j + 2 * q] += bf16_lo(rw[q]);
-                    f[8 * j + 2 * q + 1] += bf16_hi(rw[q]);
-                  }
-                }
-              } else {
-                for (int j = 0; j < 32 && n0 + j < p.N; ++j) f[j] += __bfloat162float(rs[j]);
-              }
-            }
-            if (p.epi == EPI_RELU2) {
-#pragma unroll
-              for (int j = 0; j < 32; ++j) f[j] = relu2(f[j]);
-            }
-            if (n0 + 32 <= p.N) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                *reinterpret_cast<uint4*>(dst + 8 * j) =
-                    make_uint4(pack_bf16(f[8 * j], f[8 * j + 1]), pack_bf16(f[8 * j + 2], f[8 * j + 3]),
-                               pack_bf16(f[8 * j + 4], f[8 * j + 5]), pack_bf16(f[8 * j + 6], f[8 * j + 7]));
-            } else {
-              for (int j = 0; j < 32 && n0 + j < p.N; ++j) dst[j] = __float2bfloat16(f[j]);
-            }
-          }
+          store_chunk(p, v, grow, n0);
         }
       }
       tc_fence_before();
@@ -465,6 +472,186 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, C::TMEM_COLS);
+  }
+}
+
+// ------------------------------------------------------------------ two SMs on one tile (cta_group::2)
+// A cluster of two CTAs computes 256 x 256 tiles: each holds 128 rows of A and 128 of the 256 rows of B in its shared memory and
+// 128 rows of the accumulator in its tensor memory; the even CTA issues the MMAs for both.  Per k block a CTA then fetches,
+// stores and reads 16 KB of B instead of 32: six stages fit instead of four, and the tensor core's operand reads fall from 96 to
+// 64 bytes a cycle.  bf16 GEMMs that are not grouped, with the local epilogues; the loads carry no multicast.
+// 4096 rows x 34816 x 5120: 986 -> 908 us (1.61 PFLOP/s); x 5120 x 17408: 573 -> 504; 900 rows x 34816 x 5120: 272 -> 247.
+struct PairCfg {
+  static constexpr int BN = 256, HALF = 128 * BKB, STAGE = 2 * HALF, STAGES = 6, BARS = 256;
+  static constexpr int SMEM = STAGES * STAGE + 1024 + BARS;
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_rank0(uint32_t addr) {     // the even CTA's copy of a shared-memory word
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(r) : "r"(addr));
+  return r;
+}
+// mbar_wait for a barrier on which threads of the other CTA arrive
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, unsigned int code) {
+  const long long t0 = clock64();
+  for (;;) {
+#pragma unroll 1
+    for (int i = 0; i < 256; ++i) {
+      uint32_t ok;
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, %3;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(ok)
+          : "r"(bar), "r"(parity), "r"(kSuspendHintNs)
+          : "memory");
+      if (ok) return true;
+    }
+    if (clock64() - t0 > kWaitCycles) {
+      record_error(code, (blockIdx.x << 8) | (threadIdx.x >> 5));
+      return false;
+    }
+  }
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t cluster_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];" ::"r"(dst),
+      "l"(map), "r"(cluster_bar), "r"(x), "r"(y)
+      : "memory");
+}
+__device__ __forceinline__ void umma_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {     // arrives on this barrier of both CTAs
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"((uint16_t)3)
+               : "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+  using C = PairCfg;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u, bars = smem + C::STAGES * C::STAGE;
+  const uint32_t full0 = bars, empty0 = full0 + 8 * C::STAGES, tfull0 = empty0 + 8 * C::STAGES, tempty0 = tfull0 + 16, slot = tempty0 + 16;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)cluster_rank();
+  const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM), tiles_n = (p.N + C::BN - 1) / C::BN, n_tiles = tiles_m * tiles_n;
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, KB = p.K * 2 / BKB;
+
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < C::STAGES; ++i) {
+      mbar_init(full0 + 8 * i, 1);           // used in the even CTA: both CTAs' bytes
+      mbar_init(empty0 + 8 * i, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(tfull0 + 8 * i, 1);
+      mbar_init(tempty0 + 8 * i, 8);         // used in the even CTA: both CTAs' epilogue warps
+    }
+    mbar_fence_init();
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(slot) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();            // both CTAs' barriers are there before anything arrives on them
+  tc_fence_after();
+  uint32_t tmem;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(slot));
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ copies: this CTA's halves of A and B
+    if (lane == 0) {
+      prefetch_tmap(&map_a);
+      prefetch_tmap(&map_b);
+      int it = 0;
+      bool ok = true;
+      for (int t = pair; t < n_tiles && ok; t += pairs) {
+        const int row0 = (t % tiles_m) * 2 * BM + rank * BM, n0 = (t / tiles_m) * C::BN + rank * (C::BN / 2);
+        for (int kb = 0; kb < KB; ++kb, ++it) {
+          const int s = it % C::STAGES;
+          if (it >= C::STAGES) ok = mbar_wait(empty0 + 8 * s, ((it / C::STAGES) - 1) & 1, ERR_GEMM_EMPTY_WAIT);
+          if (!ok) break;
+          const uint32_t sa = smem + s * C::STAGE, bar = map_rank0(full0 + 8 * s);
+          if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * C::STAGE);
+          tma_load_2d_pair(sa, &map_a, kb * (BKB / 2), row0, bar);
+          tma_load_2d_pair(sa + C::HALF, &map_b, kb * (BKB / 2), n0, bar);
+        }
+      }
+      // After a wait that ran out, the even CTA waits (bounded) for the bytes both have asked for; the odd one meets it at the
+      // cluster barrier below.
+      if (!ok && rank == 0)
+        for (int i = max(0, it - C::STAGES); i < it; ++i) mbar_wait(full0 + 8 * (i % C::STAGES), (i / C::STAGES) & 1, ERR_GEMM_FULL_WAIT);
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMAs, even CTA only
+    if (lane == 0 && rank == 0) {
+      constexpr uint32_t idesc = make_idesc(1, 1, 2 * BM, C::BN);
+      int it = 0, lt = 0;
+      bool ok = true;
+      for (int t = pair; t < n_tiles && ok; t += pairs, ++lt) {
+        const int a = lt & 1;
+        if (lt >= 2) ok = mbar_wait_cluster(tempty0 + 8 * a, ((lt >> 1) - 1) & 1, ERR_GEMM_TMEM_EMPTY_WAIT);
+        if (!ok) break;
+        tc_fence_after();
+        for (int kb = 0; kb < KB; ++kb, ++it) {
+          const int s = it % C::STAGES;
+          ok = mbar_wait_cluster(full0 + 8 * s, (it / C::STAGES) & 1, ERR_GEMM_FULL_WAIT);
+          if (!ok) break;
+          tc_fence_after();
+          const uint64_t da = make_desc_sw128(smem + s * C::STAGE), db = make_desc_sw128(smem + s * C::STAGE + C::HALF);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) umma_f16_pair(tmem + a * C::BN, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+          tc_commit_pair(empty0 + 8 * s);
+        }
+        if (ok) tc_commit_pair(tfull0 + 8 * a);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue (warps 2..5): this CTA's 128 rows
+    const int quarter = warp & 3;
+    int lt = 0;
+    for (int t = pair; t < n_tiles; t += pairs, ++lt) {
+      const int a = lt & 1, nt = t / tiles_m;
+      const int grow = (t % tiles_m) * 2 * BM + rank * BM + quarter * 32 + lane;
+      if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * a, (lt >> 1) & 1, ERR_GEMM_TMEM_FULL_WAIT))) break;
+      tc_fence_after();
+#pragma unroll 1
+      for (int c = 0; c < C::BN / 32; ++c) {
+        uint32_t v[32];
+        B2_TMEM_LD_32(tmem + a * C::BN + c * 32 + ((uint32_t)(quarter * 32) << 16), v);
+        tmem_ld_wait();
+        const int n0 = nt * C::BN + c * 32;
+        if (grow < p.M && n0 < p.N) store_chunk(p, v, grow, n0);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(map_rank0(tempty0 + 8 * a));
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();            // nothing of the other CTA is on its way here any more
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
   }
 }
 
@@ -605,6 +792,36 @@ int launch_w4(const CUtensorMap& ma, const GemmParams& p, int n_tiles_max, cudaS
   return (int)cudaGetLastError();
 }
 
+int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, cudaStream_t st) {
+  using C = PairCfg;
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    configured[dev & 63] = true;
+  }
+  const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + C::BN - 1) / C::BN), pairs = min(tiles, sm_count() / 2);
+  gemm_pair_kernel<<<2 * pairs, kThreads, C::SMEM, st>>>(ma, mb, p);
+  return (int)cudaGetLastError();
+}
+
+// Tile of a bf16 product that is not grouped: -256 the pair form, or 256 / 128 columns on one SM.  Waves of tiles times what a
+// wave takes (K = 5120, weights beyond L2): 256 x 256 on two SMs 30 us, 128 x 256 on one 33, 128 x 128 22; the narrow tile only
+// where it fits in one wave.  130 x 5120 x 17408: 110 / 78 us wide / narrow, 300 x 34816 x 5120: 128 / 116 pair / wide,
+// 512 x 5120 x 17408: 93 / 126, 4096 x 34816 x 5120: 908 / 986.
+int tile_of(int M, int N) {
+  const int sms = sm_count(), mt = (M + BM - 1) / BM, mp = (M + 2 * BM - 1) / (2 * BM);
+  const int wide = (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
+  if (N < 256) return wide;
+  const auto waves = [](int tiles, int at_once) { return (tiles + at_once - 1) / at_once; };
+  const int n256 = (N + 255) / 256, n128 = (N + 127) / 128;
+  const int pair = waves(mp * n256, sms / 2) * 30, one = waves(mt * n256, sms) * 33;
+  if (mt * n128 <= sms && 22 < min(pair, one)) return 128;
+  return pair <= one ? -256 : wide;
+}
+
 }  // namespace
 
 // C = A * W^T with W read as int4: a [M][K] bf16, w4b the W4B blocks [E][ceil(N / 128)][K / 64][4352] (E = 1 unless the
@@ -653,11 +870,15 @@ static int gemm_tc_impl(const void* a, const void* b, void* c, int M, int N, int
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.C = c; p.resid = (const __nv_bfloat16*)resid;
   p.a_scale = a_scale; p.b_scale = b_scale; p.epi = epi; p.glu = glu;
   p.blk_expert = blk_expert; p.blk_row0 = blk_row0; p.blk_rows = blk_rows; p.n_blk = n_blk; p.max_blk = max_blk;
-  if (bn != 128 && bn != 256) {
-    bn = (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
+  const bool local = !i8 && !blk_expert && !ag_cnt && epi != EPI_RS_PUSH && epi != EPI_EP_RETURN;
+  bool pair = local && bn == -256;
+  if (!pair && bn != 128 && bn != 256) {
+    bn = local ? tile_of(M, N) : (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
     // few rows: narrower tiles while they still fit in one wave
-    if (!blk_expert && ((M + BM - 1) / BM) * ((N + 127) / 128) <= sm_count()) bn = 128;
+    if (!local && !blk_expert && ((M + BM - 1) / BM) * ((N + 127) / 128) <= sm_count()) bn = 128;
+    pair = bn == -256;
   }
+  if (pair) bn = 128;       // B arrives in two halves
   CUtensorMap ma, mb;
   int rc = make_map(&ma, a, i8 != 0, (uint64_t)M, (uint64_t)K, 0, BM);
   if (rc) return rc;
@@ -666,6 +887,7 @@ static int gemm_tc_impl(const void* a, const void* b, void* c, int M, int N, int
   const int tiles_m = blk_expert ? max_blk : (M + BM - 1) / BM;
   const int n_tiles = tiles_m * ((N + bn - 1) / bn);
   cudaStream_t st = (cudaStream_t)stream;
+  if (pair) return launch_pair(ma, mb, p, st);
   if (bn == 256) return i8 ? launch<256, true>(ma, mb, p, n_tiles, st) : launch<256, false>(ma, mb, p, n_tiles, st);
   return i8 ? launch<128, true>(ma, mb, p, n_tiles, st) : launch<128, false>(ma, mb, p, n_tiles, st);
 }
