@@ -656,37 +656,44 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 }
 
 // ------------------------------------------------------------------ W4B -> bf16 [N][K] (two-pass prefill path)
-// grid (K/64, N/128), 256 threads: thread (tile j = warp, lane) expands its 16 bytes, the tile is
-// staged in shared memory and written as 128-byte row segments.
+// grid (ceil(K / 256), N / 128), 256 threads: a thread (tile j = warp, lane) expands its 16 bytes of four consecutive blocks, all
+// loaded at once.  The four lanes of a quad hold 32 contiguous bytes of a row, so they store whole sectors from registers;
+// through a shared-memory tile, one block per CTA, the pass ran at 4.6 TB/s.
+// 34816 x 5120: 98 -> 83 us (451 MB, 5.5 TB/s).
 __global__ void __launch_bounds__(256) dequant_w4b_kernel(const uint8_t* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                                           int N, int K) {
-  __shared__ __align__(16) uint32_t tile[128][33];  // [row][k pairs] (+1 pad)
-  const int kg = blockIdx.x, nb = blockIdx.y, KG = K / 64;
-  const uint8_t* blk = w + ((size_t)nb * KG + kg) * 4352;
+  constexpr int U = 4;
+  const int kg0 = blockIdx.x * U, nb = blockIdx.y, KG = K / 64;
+  const uint8_t* blk = w + ((size_t)nb * KG + kg0) * 4352;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const uint4 wv = *reinterpret_cast<const uint4*>(blk + warp * 512 + lane * 16);
-  const __half* sc = reinterpret_cast<const __half*>(blk + 4096) + warp * 16;
-  const float s_lo = __half2float(sc[2 * g]), s_hi = __half2float(sc[2 * g + 1]);  // scales are stored as (g, g + 8) pairs
-  const uint32_t wa[4] = {wv.x, wv.y, wv.z, wv.w};
+  uint4 wv[U];
+  uint32_t sc[U];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const int row = warp * 16 + g + 8 * (c & 1);
-    const float s = (c & 1) ? s_hi : s_lo;
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {  // e = 0: low nibbles (k = 4t + b of the 32-k step), 1: high nibbles (+ 16)
-      const uint32_t x = (wa[c] >> (4 * e)) & 0x0F0F0F0Fu;
-      const float f0 = (float)((int)(x & 0xFF) - 8) * s, f1 = (float)((int)((x >> 8) & 0xFF) - 8) * s;
-      const float f2 = (float)((int)((x >> 16) & 0xFF) - 8) * s, f3 = (float)((int)(x >> 24) - 8) * s;
-      const int kpair = (32 * (c >> 1) + 16 * e + 4 * t) >> 1;
-      tile[row][kpair] = pack_bf16(f0, f1);
-      tile[row][kpair + 1] = pack_bf16(f2, f3);
-    }
+  for (int u = 0; u < U; ++u) {
+    if (kg0 + u >= KG) break;
+    wv[u] = __ldg(reinterpret_cast<const uint4*>(blk + (size_t)u * 4352 + warp * 512 + lane * 16));
+    sc[u] = __ldg(reinterpret_cast<const uint32_t*>(blk + (size_t)u * 4352 + 4096) + warp * 8 + g);   // scales are stored as (g, g + 8) pairs
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 128 * 32; i += 256) {
-    const int row = i >> 5, kp = i & 31;
-    const int n = nb * 128 + row;
-    if (n < N) reinterpret_cast<uint32_t*>(out + (size_t)n * K + kg * 64)[kp] = tile[row][kp];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    if (kg0 + u >= KG) break;
+    const __half2 sh = *reinterpret_cast<const __half2*>(&sc[u]);
+    const uint32_t wa[4] = {wv[u].x, wv[u].y, wv[u].z, wv[u].w};
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int n = nb * 128 + warp * 16 + g + 8 * (c & 1);
+      const float s = (c & 1) ? __high2float(sh) : __low2float(sh);
+      if (n >= N) continue;
+      __nv_bfloat16* row = out + (size_t)n * K + (kg0 + u) * 64 + 32 * (c >> 1) + 4 * t;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {  // e = 0: low nibbles (k = 4t + b of the 32-k step), 1: high nibbles (+ 16)
+        const uint32_t x = (wa[c] >> (4 * e)) & 0x0F0F0F0Fu;
+        float f[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[i] = (float)((int)((x >> (8 * i)) & 0xFF) - 8) * s;
+        *reinterpret_cast<uint2*>(row + 16 * e) = make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]));
+      }
+    }
   }
 }
 
@@ -932,7 +939,8 @@ extern "C" int b2_gemm_tc_ep(const void* a, const void* b, void* c, int M, int N
 
 extern "C" int b2_dequant_w4b(const void* w4b, void* out_bf16, int N, int K, void* stream) {
   if (K % 64) return -1;
-  dim3 grid(K / 64, (N + 127) / 128);
+  if (((uintptr_t)w4b & 15) || ((uintptr_t)out_bf16 & 7)) return -3;
+  dim3 grid((K / 64 + 3) / 4, (N + 127) / 128);
   dequant_w4b_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const uint8_t*)w4b, (__nv_bfloat16*)out_bf16, N, K);
   return (int)cudaGetLastError();
 }

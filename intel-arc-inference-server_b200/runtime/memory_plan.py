@@ -114,10 +114,10 @@ def prefill_scratch_bytes(cfg: ModelConfig, chunk: int, backend: str) -> int:
     ffn = cfg.ffn if not cfg.is_moe else max(cfg.expert_ffn, cfg.shared_ffn)
     b = chunk * (2 * h * 2 + cfg.qkv_dim * 4 + 2 * cfg.q_dim * 2 + ffn * 2)
     biggest = max(cfg.qkv_dim * h, h * cfg.q_dim, 2 * ffn * h)
-    if backend in ("bf16", "auto"):
+    if backend in ("bf16", "auto", "w4", "int4", "w4a16"):
         b += biggest * 2
-        if cfg.is_moe:
-            b += cfg.n_experts * 3 * cfg.expert_ffn * h * 2
+    if backend in ("bf16", "auto") and cfg.is_moe:
+        b += cfg.n_experts * 3 * cfg.expert_ffn * h * 2
     if cfg.is_moe:
         rows = (chunk * cfg.top_k // 128 + cfg.n_experts) * 128
         b += rows * (2 * h + cfg.expert_ffn) * 2

@@ -11,6 +11,7 @@ with the residual add.  Only the last row of the last chunk goes through the hea
 Weight forms for the GEMMs:
   ``bf16``      W4B is dequantised to a bf16 slab right before each GEMM (two-pass, as the
                 reference's pf_dequant_slab + pf_gemm) -- no second resident copy of the model;
+  ``w4``        the same, except for few rows and for routed experts, whose GEMMs read the int4 blocks themselves;
   ``bf16-resident``  the dequantised matrices stay in HBM (a 27B model is 42 GB of the 180 GB);
   ``int8``      per-token int8 activations x per-row int8 weights on kind::i8, scales in the epilogue
                 (the reference's ``--prefill-backend l0-int8``, docs/16-int8-prefill.md).
@@ -62,6 +63,14 @@ class PhaseProfile:
         parts = ", ".join(f"{k} {v:.2f} ms ({100 * v / allms:.0f} %)" for k, v in sorted(tot.items(), key=lambda kv: -kv[1]))
         out.write(f"prefill profile: {tokens} tokens, {allms:.2f} ms in phases: {parts}\n")
         self.spans = []
+
+
+# Backend ``w4`` keeps no bf16 copy of the model.  Up to this many rows (one row of GEMM tiles) the GEMM expands the int4 blocks
+# inside its tiles; beyond that every further row of tiles would expand them again, and the weight is expanded once into the
+# workspace that the two-pass form uses, which holds the largest matrix.  16 layers of the 27B shape, fused / expanded first:
+# 130 rows 7.6 / 6.8 ms, 900 rows 22.3 / 13.9, 4000 rows 67 / 41; in runs of 64 MB that stay in the L2 the products of a run are
+# too narrow to fill the GPU (900 rows: 16.7).
+W4_FUSED_ROWS = 128
 
 
 class PrefillRunner:
@@ -140,7 +149,7 @@ class PrefillRunner:
             G.quant_rows_i8(a, a8, self.a_scale[:rows])
             w8, ws = self._w_i8(ql)
             G.gemm_i8(a8, w8, self.a_scale[:rows], ws, out, epi=epi, resid=resid)
-        elif self.backend == "w4":      # the GEMM reads the int4 blocks itself: nothing but the W4B weights is resident
+        elif self.backend == "w4" and a.shape[0] <= W4_FUSED_ROWS:
             G.gemm_w4(a, ql.w4b, ql.n, ql.k, out, epi=epi, resid=resid)
         else:
             G.gemm_bf16(a, self._w_bf16(ql), out, epi=epi, resid=resid)

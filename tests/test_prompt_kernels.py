@@ -5,6 +5,7 @@ import torch.nn.functional as F
 
 from b200serve.ops import gemm as G
 from b200serve.ops import lib as K
+from b200serve.utils import quant as Q
 
 pytestmark = pytest.mark.gpu
 
@@ -38,3 +39,13 @@ def test_two_sm_gemm(m, n, k, bn):
         v = ref.view(m, n // 32, 2, 16)
         want = (F.silu(v[:, :, 0]) * v[:, :, 1]).reshape(m, n // 2)
         assert ((act.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
+
+
+@pytest.mark.parametrize("n,k", [(128, 64), (100, 256), (1000, 320), (256, 4096), (5120, 1088)])
+def test_expanded_weights(n, k):
+    """Four blocks per CTA and what is left of them, rows behind the matrix untouched."""
+    w = Q.random_w4b(n, k, "cuda", 3)
+    out = torch.full((n + 1, k), float("nan"), dtype=torch.bfloat16, device="cuda")
+    G.dequant_w4b(w, n, k, out[:n])
+    torch.cuda.synchronize()
+    assert torch.equal(out[:n], Q.dequant_w4b(w, n).bfloat16()) and torch.isnan(out[n]).all()
