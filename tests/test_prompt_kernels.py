@@ -49,3 +49,45 @@ def test_expanded_weights(n, k):
     G.dequant_w4b(w, n, k, out[:n])
     torch.cuda.synchronize()
     assert torch.equal(out[:n], Q.dequant_w4b(w, n).bfloat16()) and torch.isnan(out[n]).all()
+
+
+@pytest.mark.parametrize("m,h", [(512, 64), (513, 2048), (600, 2056), (1000, 4096), (519, 5120), (700, 5128), (512, 8192), (530, 8200), (511, 5120)])
+def test_norm_of_prompt_rows(m, h):
+    torch.manual_seed(h)
+    r, w = (torch.randn(m + 1, h, device="cuda") * 3).bfloat16(), 1 + 0.1 * torch.randn(h, device="cuda")
+    x, keep = torch.full((m + 1, h), float("nan"), dtype=torch.bfloat16, device="cuda"), r.clone()
+    K.resid_norm(1, m, h, w, 1e-6, r, x, resid_in=r, splits=0)
+    torch.cuda.synchronize()
+    want = r[:m].double() * torch.rsqrt((r[:m].double() ** 2).mean(-1, keepdim=True) + 1e-6) * w.double()
+    # one rounding to bf16; the fp32 sum of h squares moves the factor by less than 2^-24 sqrt(h)
+    assert ((x[:m].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-30).all()
+    assert torch.equal(r, keep) and torch.isnan(x[m]).all()
+
+
+@pytest.mark.parametrize("m,pos0,nq,nkv,d", [(1, 0, 4, 2, 128), (3, 5, 8, 2, 64), (4, 16, 40, 8, 128), (37, 31, 3, 1, 256), (130, 1000, 16, 4, 128), (18, 7, 5, 5, 192)])
+def test_rope_append_of_prompt_rows(m, pos0, nq, nkv, d):
+    from b200serve.models.oracle import rope_tables
+    torch.manual_seed(m)
+    ld, blocks = (nq + 2 * nkv) * d, (pos0 + m + 15) // 16 + 1
+    qkv = torch.randn(m, ld, device="cuda")
+    cos, sin = (t.cuda().contiguous() for t in rope_tables(d, 1e6, pos0 + m + 4))
+    table = torch.randperm(blocks + 3, device="cuda")[:blocks].int().view(1, blocks).repeat(2, 1).contiguous()
+    kc, vc = (torch.full((blocks + 3, nkv, 16, d), 7.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    q = torch.zeros(m, nq * d, dtype=torch.bfloat16, device="cuda")
+    K.rope_append(qkv, 0, 1, m, None, table, blocks, cos, sin, nq, nkv, d, q, kc, vc, None, None, False, req=1, pos0=pos0)
+    torch.cuda.synchronize()
+    pos = torch.arange(pos0, pos0 + m, device="cuda")
+    c, s = (t[pos].double()[:, None] for t in (cos, sin))
+
+    def turned(x):
+        a, b = x[..., : d // 2], x[..., d // 2:]
+        return torch.cat([a * c - b * s, b * c + a * s], -1)
+    v = qkv.double()
+    close = lambda got, want: ((got.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()        # noqa: E731  one rounding
+    assert close(q.view(m, nq, d), turned(v[:, : nq * d].view(m, nq, d)))
+    at = table[1].long()[pos // 16], pos % 16
+    assert close(kc[at[0], :, at[1]], turned(v[:, nq * d: (nq + nkv) * d].view(m, nkv, d)))
+    assert torch.equal(vc[at[0], :, at[1]], qkv[:, (nq + nkv) * d:].view(m, nkv, d).bfloat16())
+    for t in (kc, vc):
+        t[at[0], :, at[1]] = 7.0
+        assert (t == 7.0).all()
