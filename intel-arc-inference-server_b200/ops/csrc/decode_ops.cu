@@ -899,6 +899,128 @@ __global__ void __launch_bounds__(64) head_gemv_mma_kernel(const HeadParams<__nv
   }
 }
 
+// The same for 17 to 64 rows in one pass over the weights (a pass per 16 rows read the head two to four times: 40 rows of a
+// 151936 x 5120 head 880 us; now 376, the bytes take 234).
+// Four warps of 32 weight rows; a k step's activations (MT x 16 rows x 64 k) are shared by them, so they are copied by the
+// whole CTA, one barrier a step, while the weights stay in the lanes' own slots.  The products of a (row, weight row) pair are
+// added in the order of the form above: the same bits.
+constexpr int kWideStages = 4;
+template <int MT>
+struct WideHead {
+  static constexpr int XB = MT * 16 * 128, WB = 4 * 8 * 512, STAGE = XB + WB, SMEM = kWideStages * STAGE;
+};
+template <int MT>
+__global__ void __launch_bounds__(128) head_gemv_wide_kernel(const HeadParams<__nv_bfloat16> p, int m0) {
+  using C = WideHead<MT>;
+  constexpr int NG = 4, KU = 2;
+  extern __shared__ __align__(16) unsigned char head_smem[];
+  __shared__ float sv[4][MT * 16];
+  __shared__ int si[4][MT * 16];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
+  const int row0 = blockIdx.x * 128 + warp * 8 * NG;
+  const __nv_bfloat16* wp[NG];
+#pragma unroll
+  for (int i = 0; i < NG; ++i) wp[i] = p.w + (size_t)min(row0 + 8 * i + g, p.N - 1) * p.K + t * 8;
+  // activations: vector (32-k half u, row r, piece c) at u * MT * 1024 + r * 64 + c * 16; thread tid copies c = tid & 3 of rows
+  // (tid >> 2) and + 32
+  const uint32_t smem = (uint32_t)__cvta_generic_to_shared(head_smem), xcol = (tid & 3) * 8;
+  const int steps = p.K / (32 * KU);
+  auto issue = [&](int step) {
+    if (step < steps) {
+      const int k = step * 32 * KU;
+      const uint32_t st = smem + (step % kWideStages) * C::STAGE, dst = st + C::XB + warp * 8 * 512 + lane * 16;
+#pragma unroll
+      for (int u = 0; u < KU; ++u) {
+#pragma unroll
+        for (int i = 0; i < NG; ++i)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + (u * NG + i) * 512), "l"(wp[i] + k + 32 * u) : "memory");
+#pragma unroll
+        for (int r = tid >> 2; r < MT * 16; r += 32)
+          asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(st + u * MT * 1024 + r * 64 + (tid & 3) * 16),
+                       "l"(p.x + (size_t)min(m0 + r, p.M - 1) * p.K + k + 32 * u + xcol)
+                       : "memory");
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");   // an empty group past the end keeps the count uniform
+  };
+  float acc[MT][NG][4];
+#pragma unroll
+  for (int a = 0; a < MT; ++a)
+#pragma unroll
+    for (int i = 0; i < NG; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[a][i][j] = 0.f;
+#pragma unroll
+  for (int s0 = 0; s0 < kWideStages - 1; ++s0) issue(s0);
+  for (int step = 0; step < steps; ++step) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kWideStages - 2) : "memory");
+    __syncthreads();       // everybody's copies of this step have landed, and everybody has read the step before
+    issue(step + kWideStages - 1);
+    const unsigned char* st = head_smem + (step % kWideStages) * C::STAGE;
+    const uint4* ws = reinterpret_cast<const uint4*>(st + C::XB + warp * 8 * 512) + lane;
+#pragma unroll
+    for (int u = 0; u < KU; ++u) {
+      uint4 wv[NG];
+#pragma unroll
+      for (int i = 0; i < NG; ++i) wv[i] = ws[(u * NG + i) * 32];
+      const uint4* xs = reinterpret_cast<const uint4*>(st + u * MT * 1024) + g * 4 + t;
+#pragma unroll
+      for (int a = 0; a < MT; ++a) {
+        const uint4 av = xs[a * 64], bv = xs[a * 64 + 32];
+#pragma unroll
+        for (int i = 0; i < NG; ++i) {
+          mma_bf16_16816(acc[a][i], av.x, bv.x, av.y, bv.y, wv[i].x, wv[i].y);
+          mma_bf16_16816(acc[a][i], av.z, bv.z, av.w, bv.w, wv[i].z, wv[i].w);
+        }
+      }
+    }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int a = 0; a < MT; ++a) {
+    float best[2] = {-INFINITY, -INFINITY};
+    int besti[2] = {0x7fffffff, 0x7fffffff};
+#pragma unroll
+    for (int grp = 0; grp < NG; ++grp)
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int n = row0 + grp * 8 + 2 * t + j;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m = m0 + a * 16 + g + 8 * h;
+          const float v = acc[a][grp][2 * h + j];
+          if (n < p.N && m < p.M) {
+            p.out[(size_t)m * p.ldo + n] = v;
+            if (n < p.n_valid && v > best[h]) { best[h] = v; besti[h] = n; }   // n ascends: ties keep the lower id
+          }
+        }
+      }
+    if (!p.cand_val) continue;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+#pragma unroll
+      for (int d = 1; d <= 2; d <<= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, best[h], d);
+        const int oi = __shfl_xor_sync(0xffffffffu, besti[h], d);
+        if (ov > best[h] || (ov == best[h] && oi < besti[h])) { best[h] = ov; besti[h] = oi; }
+      }
+      if (t == 0) { sv[warp][a * 16 + g + 8 * h] = best[h]; si[warp][a * 16 + g + 8 * h] = besti[h]; }
+    }
+  }
+  if (!p.cand_val) return;
+  __syncthreads();
+  const int nc = (p.N + 63) / 64;          // candidates stand for 64 weight rows, two warps
+  for (int i = tid; i < MT * 32; i += 128) {
+    const int m = i >> 1, c = blockIdx.x * 2 + (i & 1), w = (i & 1) * 2;
+    if (m0 + m >= p.M || c >= nc) continue;
+    const bool second = sv[w + 1][m] > sv[w][m];      // warps ascend in n
+    p.cand_val[(size_t)(m0 + m) * nc + c] = second ? sv[w + 1][m] : sv[w][m];
+    p.cand_idx[(size_t)(m0 + m) * nc + c] = second ? si[w + 1][m] : si[w][m];
+  }
+}
+
 // grid M, 256 threads: reduce the candidates; ties -> lower id; write control block.
 __global__ void __launch_bounds__(256) argmax_finish_kernel(const float* cand_val, const int* cand_idx, int ncand,
                                                             int* ctrl, int advance) {
@@ -1085,6 +1207,19 @@ extern "C" int b2_attn_merge_quant(const float* o_part, const float* ml_part, vo
                    (__nv_bfloat16*)out, n_q, nsplit, D, (uint8_t*)xq, (uint32_t*)xq_gs, gs_rows);
 }
 
+template <int MT>
+static int head_wide(const HeadParams<__nv_bfloat16>& p, int m0, cudaStream_t st) {
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    cudaError_t e = cudaFuncSetAttribute(head_gemv_wide_kernel<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideHead<MT>::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    configured[dev & 63] = true;
+  }
+  return b2_launch(head_gemv_wide_kernel<MT>, dim3((p.N + 127) / 128), dim3(128), WideHead<MT>::SMEM, st, true, p, m0);
+}
+
 template <typename WT>
 static int head_launch(const HeadParams<WT>& p, cudaStream_t st) {
   const int rows_per_cta = 64;
@@ -1100,6 +1235,13 @@ static int head_launch(const HeadParams<WT>& p, cudaStream_t st) {
         configured[dev & 63] = true;
       }
       for (int m0 = 0; m0 < p.M; m0 += 16) {
+        if (p.M - m0 > 16) {
+          const int mt = min(4, (p.M - m0 + 15) / 16);
+          int rc = mt == 2 ? head_wide<2>(p, m0, st) : mt == 3 ? head_wide<3>(p, m0, st) : head_wide<4>(p, m0, st);
+          if (rc) return rc;
+          m0 += (mt - 1) * 16;
+          continue;
+        }
         int rc = b2_launch(head_gemv_mma_kernel, grid, dim3(64), kHeadSmem, st, true, p, m0);
         if (rc) return rc;
       }

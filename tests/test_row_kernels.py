@@ -207,3 +207,23 @@ def test_staged_rows_of_every_kind(m):
     rc = K.lib().b2_attn_merge_quant(K._p(o), K._p(ml), K._p(out), m, heads, ns, 128, K._p(xr), None, pad, K._stream())
     torch.cuda.synchronize()
     assert rc == 0 and torch.equal(unstaged(xr), out) and out.abs().sum() > 0
+
+
+@pytest.mark.parametrize("m", [17, 31, 32, 33, 48, 49, 64])
+@pytest.mark.parametrize("n,k", [(64, 64), (100, 192), (1000, 512), (4160, 1024)])
+def test_head_of_many_rows(m, n, k):
+    """One pass for up to 64 rows: the bits of the 16-row form, and its arg-max candidates."""
+    torch.manual_seed(m + n)
+    w, x = (torch.randn(n, k, device="cuda") * 0.05).bfloat16(), torch.randn(m, k, device="cuda").bfloat16()
+    w[n // 2] = w[n // 3]                      # ties between rows
+    nc = K.head_ncand(n)
+    out, cv, ci = torch.full((m, n), float("nan"), device="cuda"), torch.zeros(m, nc, device="cuda"), torch.zeros(m, nc, dtype=torch.int32, device="cuda")
+    K.head_gemv(w, x, out, m, n, k, cv, ci, n_valid=n - 3)
+    for m0 in range(0, m, 16):
+        part = x[m0: m0 + 16].contiguous()
+        o1, v1, i1 = torch.zeros(len(part), n, device="cuda"), torch.zeros(len(part), nc, device="cuda"), torch.zeros(len(part), nc, dtype=torch.int32, device="cuda")
+        K.head_gemv(w, part, o1, len(part), n, k, v1, i1, n_valid=n - 3)
+        torch.cuda.synchronize()
+        assert torch.equal(out[m0: m0 + 16], o1) and torch.equal(cv[m0: m0 + 16], v1) and torch.equal(ci[m0: m0 + 16], i1)
+    ref = x.double() @ w.double().T
+    assert ((out.double() - ref).abs() <= 16 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 1e-9).all()
