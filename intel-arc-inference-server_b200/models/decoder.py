@@ -235,8 +235,9 @@ class DecoderModel:
         # from this many rows up the activations are quantised once by their own kernel instead of in every
         # CTA of the GEMV (whose prologue repeats the rows' work per 128 output columns)
         self.prequant_rows = int(os.environ.get("B2_PREQUANT_ROWS", "3"))
-        self.rows_min = 17      # rows from which the linears run on tcgen05 (16 layers, integer GEMV / tcgen05: 16 rows 2.43 / 3.10 ms, 17 rows
-        # 3.67 / 3.49, 40 rows 5.90 / 4.43, 64 rows 7.72 / 5.55)
+        # rows from which the linears run on tcgen05 (16 layers, integer GEMV / tcgen05: 16 rows 2.37 / 2.76 ms, 17 rows 3.66 / 2.96, 40 rows
+        # 5.89 / 4.13, 64 rows 7.71 / 4.93)
+        self.rows_min = 17
         self.merge_quant = os.environ.get("B2_MERGE_QUANT", "1") == "1"   # the attention merge writes the o projection's quantised rows
         self.attn_rows_min = int(os.environ.get("B2_ATTN_ROWS_MIN", "1"))
         self.rows_one_request = False    # set by the engine around a step whose rows are one request's, consecutive

@@ -12,18 +12,19 @@
 // summed in its own fp32 accumulator, which the workers scale by the rows' fp16 scales and add up in registers: one
 // FMA per row, token and group, no conversion, no quantised activation, no zero-point term.
 //
-// One persistent CTA per SM, 18 warps.  A stage is four consecutive blocks, one for each set of workers:
-//   warps 0-15  four sets of four warps (a warp per TMEM quarter): load the block's vectors, expand, store A; when the group's products
-//               are there, scale and add.  A set expands its next block while the MMAs of this one run (two A buffers, one
-//               accumulator: 4 x (2 x 32 + 64) = 512 TMEM columns), then meets at a named barrier and its first lane issues
-//               the next MMAs: issuing for four sets by one thread cost 1200 cycles a block (a lone thread retires an instruction
-//               every ten cycles), four threads do it side by side;
-//   warp 16     bulk copies of weights, 17 KB a stage;   warp 17  bulk copies of the token rows, 4 T x 128 bytes a stage.
-// At the end of an item (128 output rows x one k split) the sets' sums meet in shared memory in a fixed order.  A row's bits do
+// One persistent CTA per SM, 20 warps.  A ring stage is four consecutive blocks; even and odd blocks go through two pipelines of
+// the same roles, which meet nowhere but at barriers, so that expanding, multiplying and adding up different blocks overlap:
+//   warps 0-7    expand: four warps (one per TMEM quarter) a pipeline, its two blocks of a stage at a time; A buffers for two stages;
+//   warps 8-15   add up: wait for a block's products, scale, add; two accumulators a pipeline (2 x (4 x 32 + 2 x 64) TMEM columns);
+//   warp 16      bulk copies of weights, 17 KB a stage;   warp 17  bulk copies of the token rows, 4 T x 128 bytes a stage;
+//   warps 18-19  issue a pipeline's MMAs each (a lone thread retires an instruction every ten cycles or so).
+// At the end of an item (128 output rows x one k split) the pipelines' sums meet in shared memory, even blocks first, while the
+// other roles are ahead in the next item.  A row's bits do
 // not depend on the other rows of the step; they are not those of the integer GEMV, whose activations are 15-bit integers.
-// 34816 x 5120 / 5120 x 17408, us (integer GEMV in brackets): 17 - 32 rows 57 / 32 (88 / 46), 33 - 48 rows 68 / 38 (133 / 70), 64 rows
-// 84 / 50 (156 / 82); a step of 40 requests through 16 layers of the 27B shape 5.90 -> 4.43 ms.  The bytes would take 14 / 7: a stage
-// takes 2200 cycles, of which a set spends 580 expanding, 620 on its first lane's issue and 470 waiting for the products.
+// 34816 x 5120 / 5120 x 17408, us (integer GEMV in brackets): 17 - 32 rows 47 / 26 (88 / 46), 33 - 48 rows 61 / 34 (132 / 70), 64 rows
+// 65 / 36 (156 / 82).  The bytes would take 14 / 7: a stage takes 2100 to 3300 cycles in which no role is busy more than half the
+// time; they wait for one another's products.  (One role per warp set with a barrier per block, as first built: 57, 68 and 84 us.
+// One lane polling for its warp: 4 to 9 % slower.  One MMA in place of four: no change.)
 #include "common.cuh"
 
 using namespace b2;
@@ -31,7 +32,7 @@ using namespace b2;
 namespace {
 
 constexpr int kBlockBytes = 4352;
-constexpr int kSets = 4, kWorkers = kSets * 128, kThreads = kWorkers + 64;
+constexpr int kStageBlocks = 4, kThreads = 640;
 constexpr int kMaxSplits = 16;
 
 struct RowsParams {
@@ -47,16 +48,15 @@ struct RowsParams {
 
 template <int T>
 struct Cfg {
-  static constexpr int XB = kSets * T * 128, WB = kSets * kBlockBytes;      // a stage's token rows and weights
-  static constexpr int RED = 2 * (kSets - 1) * (T / 4) * 512;               // twice the sets' sums of a quarter of the token rows
-  static constexpr int NX = T <= 16 ? 9 : T <= 32 ? 6 : T <= 48 ? 4 : 3, NW = T <= 16 ? 7 : T <= 32 ? 6 : T <= 48 ? 5 : 4;
+  static constexpr int XB = kStageBlocks * T * 128, WB = kStageBlocks * kBlockBytes;      // a stage's token rows and weights
+  static constexpr int RED = T * 512;                                       // half the token rows of each pipeline's sums
+  static constexpr int NX = T <= 16 ? 9 : T <= 32 ? 6 : T <= 48 ? 4 : 3, NW = T <= 16 ? 7 : T <= 32 ? 6 : 5;
   static constexpr int OFF_RAW = NX * XB, OFF_RED = OFF_RAW + NW * WB, OFF_BAR = OFF_RED + RED;
-  static constexpr int BARS = (2 * NW + 2 * NX + kSets) * 8 + 16;
-  static constexpr int SMEM = 1024 + OFF_BAR + (BARS + 15) / 16 * 16 + 64 * 16;
+  static constexpr int BARS = (2 * NW + 2 * NX + 16) * 8 + 16;
+  static constexpr int SMEM = 1024 + OFF_BAR + BARS;
 };
 
-__device__ __forceinline__ void workers_sync() { asm volatile("bar.sync 1, 512;" ::: "memory"); }
-__device__ __forceinline__ void set_sync(int set) { asm volatile("bar.sync %0, 128;" ::"r"(2 + set) : "memory"); }
+__device__ __forceinline__ void adders_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 
 #define B2_TMEM_LD_16(taddr, r)                                                                                       \
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];" \
@@ -86,21 +86,27 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
   const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t xs0 = smem0, raw0 = smem0 + C::OFF_RAW, red0 = smem0 + C::OFF_RED, bars = smem0 + C::OFF_BAR;
   const uint32_t wfull0 = bars, wempty0 = wfull0 + 8 * C::NW, xfull0 = wempty0 + 8 * C::NW, xempty0 = xfull0 + 8 * C::NX;
-  const uint32_t dfull0 = xempty0 + 8 * C::NX, misc = dfull0 + 8 * kSets;      // misc: TMEM address, "last" flag
-  const uint32_t ss0 = bars + (C::BARS + 15) / 16 * 16;                        // [64][4] sums of squares of the fold
+  const uint32_t afull0 = xempty0 + 8 * C::NX, afree0 = afull0 + 32;           // [pipeline][stage parity]
+  const uint32_t dfull0 = afree0 + 32, dempty0 = dfull0 + 32;                  // [pipeline][block of the stage]
+  const uint32_t misc = dempty0 + 32;                                          // TMEM address, "last" flag
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int items = p.nb * p.S;
 
   if (tid == 0) {
     for (int i = 0; i < C::NW; ++i) {
       mbar_init(wfull0 + 8 * i, 1);
-      mbar_init(wempty0 + 8 * i, 4 * kSets);     // every worker warp has read its block
+      mbar_init(wempty0 + 8 * i, 16);            // expanding warps have read their vectors, adding warps their scales
     }
     for (int i = 0; i < C::NX; ++i) {
       mbar_init(xfull0 + 8 * i, 1);
-      mbar_init(xempty0 + 8 * i, kSets);         // every set's MMAs have read the token rows
+      mbar_init(xempty0 + 8 * i, 2);             // both pipelines' MMAs have read the token rows
     }
-    for (int i = 0; i < kSets; ++i) mbar_init(dfull0 + 8 * i, 1);
+    for (int i = 0; i < 4; ++i) {
+      mbar_init(afull0 + 8 * i, 4);
+      mbar_init(afree0 + 8 * i, 1);
+      mbar_init(dfull0 + 8 * i, 1);
+      mbar_init(dempty0 + 8 * i, 4);
+    }
     mbar_fence_init();
   }
   if (warp == 17) {
@@ -112,14 +118,51 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
   tc_fence_after();
   uint32_t tmem;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(misc));
+  const auto groups_of = [&](int item) { const int s = item % p.S; return min(p.KG, (s + 1) * p.gps) - s * p.gps; };
 
-  if (warp >= 16) {
+  if (warp >= 18) {
+    // ---------------------------------------------------------------- MMAs of pipeline warp - 18
+    if (lane == 0) {
+      const int pipe = warp - 18;
+      constexpr uint32_t idesc = make_idesc(1, 1, 128, T);
+      const uint64_t xdesc = make_desc_sw128(xs0 + pipe * T * 128);
+      const uint32_t xd_lo = (uint32_t)xdesc, xd_hi = (uint32_t)(xdesc >> 32), a0 = tmem + pipe * 256, d0 = a0 + 128;
+      const uint32_t af = afull0 + 16 * pipe, fr = afree0 + 16 * pipe, df = dfull0 + 16 * pipe, de = dempty0 + 16 * pipe;
+      int xs = 0, xp = 0, n = 0, used[2] = {0, 0};       // n: stages before
+      bool ok = true;
+      for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+        for (int left = groups_of(item) - pipe; left > -pipe && ok; left -= kStageBlocks, ++n) {      // blocks of the stage from this one on
+          const uint32_t par = n & 1;
+          ok = mbar_wait(xfull0 + 8 * xs, xp, ERR_GEMM_FULL_WAIT) && mbar_wait(af + 8 * par, (n >> 1) & 1, ERR_GEMM_TMEM_FULL_WAIT);
+          if (!ok) break;
+          const uint32_t xlo = xd_lo + xs * (C::XB >> 4), a = a0 + par * 64;
+          tc_fence_after();
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            if (left <= 2 * j) break;
+            if (used[j] > 0) {
+              ok = mbar_wait(de + 8 * j, (used[j] - 1) & 1, ERR_GEMM_TMEM_EMPTY_WAIT);
+              if (!ok) break;
+              tc_fence_after();
+            }
+            ++used[j];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) umma_f16_ts_w(d0 + j * 64, a + j * 32 + 8 * k, xlo + j * (2 * T * 128 >> 4) + 2 * k, xd_hi, idesc, k != 0);    // 16 k = 32 bytes a step
+            tc_commit(df + 8 * j);
+          }
+          if (left > 0) tc_commit(fr + 8 * par);
+          else mbar_arrive(fr + 8 * par);
+          if (++xs == C::NX) { xs = 0; xp ^= 1; }
+        }
+      }
+    }
+  } else if (warp >= 16) {
     // ---------------------------------------------------------------- copies
     if (lane == 0) {
       const bool wt = warp == 16;
       const int n = wt ? C::NW : C::NX, unit = wt ? kBlockBytes : T * 128;
       const uint32_t full0 = wt ? wfull0 : xfull0, empty0 = wt ? wempty0 : xempty0, dst0 = wt ? raw0 : xs0;
-      const uint32_t stage = kSets * unit;
+      const uint32_t stage = kStageBlocks * unit;
       if (!wt) pdl_wait();       // the weights depend on nothing: their first stages are asked for before the previous kernel is done
       int slot = 0, round = 0;   // stage of the ring, times it was filled before
       bool ok = true;
@@ -127,10 +170,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
         const int nblk = item / p.S, g0 = (item - nblk * p.S) * p.gps;
         int left = min(p.KG, g0 + p.gps) - g0;
         const uint8_t* src = wt ? p.w + ((size_t)nblk * p.KG + g0) * kBlockBytes : p.x + (size_t)g0 * (T * 128);
-        for (; left > 0; left -= kSets, src += stage) {
+        for (; left > 0; left -= kStageBlocks, src += stage) {
           if (round > 0) ok = mbar_wait(empty0 + 8 * slot, (round - 1) & 1, ERR_GEMM_EMPTY_WAIT);
           if (!ok) break;
-          const uint32_t bytes = min(left, kSets) * unit, bar = full0 + 8 * slot;
+          const uint32_t bytes = min(left, kStageBlocks) * unit, bar = full0 + 8 * slot;
           mbar_expect_tx(bar, bytes);
           bulk_g2s(dst0 + slot * stage, src, bytes, bar);
           if (++slot == n) { slot = 0; ++round; }
@@ -142,176 +185,171 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
           if (r >= 0) mbar_wait(full0 + 8 * i, r & 1, ERR_GEMM_FULL_WAIT);
         }
     }
-  } else {
-    // ---------------------------------------------------------------- workers
-    const int set = warp >> 2, q = warp & 3;
-    const uint32_t my_tmem = tmem + set * 128 + ((uint32_t)(32 * q) << 16), dfull = dfull0 + 8 * set;
-    const int row = 32 * q + lane;
-    const uint32_t v_off = set * kBlockBytes + 2 * q * 512 + lane * 16;
-    const uint32_t sc_off = set * kBlockBytes + 4096 + ((row >> 4) * 16 + 2 * (row & 7) + ((row >> 3) & 1)) * 2;
-    constexpr uint32_t idesc = make_idesc(1, 1, 128, T);
-    const uint64_t xdesc = make_desc_sw128(xs0 + set * T * 128);
-    const uint32_t xd_lo = (uint32_t)xdesc, xd_hi = (uint32_t)(xdesc >> 32);
-    pdl_wait();
-    pdl_launch_dependents();
-    int ws = 0, wp = 0, xs = 0, xp = 0;     // ring stages and their parities
-    int done = 0, read = 0;                 // blocks of this set expanded, accumulators read
+  } else if (warp < 8) {
+    // ---------------------------------------------------------------- expand
+    const int pipe = warp >> 2, q = warp & 3;
+    const uint32_t a0 = tmem + pipe * 256 + ((uint32_t)(32 * q) << 16), af = afull0 + 16 * pipe, fr = afree0 + 16 * pipe;
+    const uint32_t v_off = pipe * kBlockBytes + 2 * q * 512 + lane * 16;
+    int ws = 0, wp = 0, n = 0;
     bool ok = true;
-    float next_scale = 0.f;
-    // this set's block of the next weight stage into its A buffer; `has`: there is one
-    const auto expand = [&](bool has) {
-      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(wfull0 + 8 * ws, wp, ERR_GEMM_FULL_WAIT));
-      const uint32_t st = raw0 + ws * C::WB, empty = wempty0 + 8 * ws;
-      if (++ws == C::NW) { ws = 0; wp ^= 1; }
-      if (!ok) return;
-      if (!has) {
-        if (lane == 0) mbar_arrive(empty);
-        return;
-      }
-      uint4 v[2];
+    for (int item = blockIdx.x; item < items && ok; item += gridDim.x) {
+      for (int left = groups_of(item) - pipe; left > -pipe; left -= kStageBlocks, ++n) {
+        ok = __all_sync(0xffffffffu, mbar_wait(wfull0 + 8 * ws, wp, ERR_GEMM_FULL_WAIT));
+        if (!ok) break;
+        const uint32_t st = raw0 + ws * C::WB + v_off, par = n & 1;
+        uint4 v[2][2];
 #pragma unroll
-      for (int j = 0; j < 2; ++j)
-        asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[j].x), "=r"(v[j].y), "=r"(v[j].z), "=r"(v[j].w) : "r"(st + v_off + j * 512));
-      unsigned short h;
-      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(st + sc_off));
-      next_scale = __half2float(__ushort_as_half(h));
-      __syncwarp();
-      if (lane == 0) mbar_arrive(empty);
-      const uint32_t a = my_tmem + (done & 1) * 32;
+        for (int j = 0; j < 2; ++j)
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-        uint32_t r[16];
-        // column 4 i + t, i = 4 (32-k step) + 2 (low or high byte of a pair) + (nibble): k = 32 ks + 16 hi + 4 t + o + 2 e
+          for (int h = 0; h < 2; ++h)
+            if (left > 2 * j)
+              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v[j][h].x), "=r"(v[j][h].y), "=r"(v[j][h].z), "=r"(v[j][h].w) : "r"(st + j * 2 * kBlockBytes + h * 512));
+        __syncwarp();
+        if (lane == 0) mbar_arrive(wempty0 + 8 * ws);
+        if (++ws == C::NW) { ws = 0; wp ^= 1; }
+        if (n >= 2) ok = __all_sync(0xffffffffu, mbar_wait(fr + 8 * par, ((n >> 1) - 1) & 1, ERR_GEMM_TMEM_EMPTY_WAIT));
+        if (!ok) break;
+        tc_fence_after();
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int j = 0; j < 2; ++j) {
+          if (left <= 2 * j) break;
 #pragma unroll
-          for (int hf = 0; hf < 2; ++hf) r[2 * i + hf] = nibbles_bf16(w[2 * (i >> 2) + hf], 8 * ((i >> 1) & 1) + 4 * (i & 1));
-        B2_TMEM_ST_16X128_8(a + ((uint32_t)(16 * j) << 16), r);
-      }
-      tmem_st_wait();
-      ++done;
-    };
-    // the MMAs of the block that was expanded last, by the set's first lane once all four warps have stored it
-    const auto multiply = [&](bool has) {
-      tc_fence_before();
-      set_sync(set);
-      if (q == 0) {
-        if (ok && lane == 0) {
-          tc_fence_after();
-          const bool got = mbar_wait(xfull0 + 8 * xs, xp, ERR_GEMM_FULL_WAIT);
-          if (got && has) {
-            const uint32_t am = tmem + set * 128 + ((done - 1) & 1) * 32, dm = tmem + set * 128 + 64, lo = xd_lo + xs * (C::XB >> 4);
+          for (int h = 0; h < 2; ++h) {
+            const uint32_t w[4] = {v[j][h].x, v[j][h].y, v[j][h].z, v[j][h].w};
+            uint32_t r[16];
+            // column 4 i + t, i = 4 (32-k step) + 2 (low or high byte of a pair) + (nibble): k = 32 ks + 16 hi + 4 t + o + 2 e
 #pragma unroll
-            for (int k = 0; k < 4; ++k) umma_f16_ts_w(dm, am + 8 * k, lo + 2 * k, xd_hi, idesc, k != 0);    // 16 k = 32 bytes a step
-            tc_commit(dfull);
-          } else if (got) {
-            mbar_arrive(xempty0 + 8 * xs);
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+              for (int hf = 0; hf < 2; ++hf) r[2 * i + hf] = nibbles_bf16(w[2 * (i >> 2) + hf], 8 * ((i >> 1) & 1) + 4 * (i & 1));
+            B2_TMEM_ST_16X128_8(a0 + par * 64 + j * 32 + ((uint32_t)(16 * h) << 16), r);
           }
         }
+        tmem_st_wait();
+        tc_fence_before();
         __syncwarp();
+        if (lane == 0) mbar_arrive(af + 8 * par);
       }
-      if (++xs == C::NX) { xs = 0; xp ^= 1; }
-    };
+    }
+  } else {
+    // ---------------------------------------------------------------- add up
+    const int pipe = (warp - 8) >> 2, q = warp & 3;
+    const uint32_t d0 = tmem + pipe * 256 + 128 + ((uint32_t)(32 * q) << 16), df = dfull0 + 16 * pipe, de = dempty0 + 16 * pipe;
+    const int row = 32 * q + lane, at = tid - 256;
+    const uint32_t sc_off = pipe * kBlockBytes + 4096 + ((row >> 4) * 16 + 2 * (row & 7) + ((row >> 3) & 1)) * 2;
+    pdl_wait();
+    pdl_launch_dependents();
+    int ws = 0, wp = 0, xs = 0, xp = 0, used[2] = {0, 0};
+    bool ok = true;
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
       const int nblk = item / p.S, split = item - nblk * p.S;
-      const int ng = min(p.KG, (split + 1) * p.gps) - split * p.gps, ns = (ng + kSets - 1) / kSets;
-      const auto has = [&](int k) { return k * kSets + set < ng; };
       float acc[T];
 #pragma unroll
       for (int i = 0; i < T; ++i) acc[i] = 0.f;
-      expand(has(0));
-      multiply(has(0));
-      for (int k = 0; k < ns; ++k) {
-        const float scale = next_scale;
-        if (k + 1 < ns) expand(has(k + 1));
-        if (has(k)) {
-          if (ok) ok = __all_sync(0xffffffffu, mbar_wait(dfull, read & 1, ERR_GEMM_TMEM_FULL_WAIT));
-          if (ok && q == 0 && lane == 0) mbar_arrive(xempty0 + 8 * (xs == 0 ? C::NX - 1 : xs - 1));    // the MMAs have read the token rows
-          ++read;
-          if (ok) {
-            tc_fence_after();
+      for (int left = groups_of(item) - pipe; left > -pipe; left -= kStageBlocks) {
+        if (ok) ok = __all_sync(0xffffffffu, mbar_wait(wfull0 + 8 * ws, wp, ERR_GEMM_FULL_WAIT));
+        float scale[2] = {0.f, 0.f};
+        if (ok) {
 #pragma unroll
-            for (int c0 = 0; c0 < T; c0 += 16) {
-              uint32_t d[16];
-              B2_TMEM_LD_16(my_tmem + 64 + c0, d);
-              tmem_ld_wait();
-#pragma unroll
-              for (int i = 0; i < 16; ++i) acc[c0 + i] = fmaf(scale, __uint_as_float(d[i]), acc[c0 + i]);
-            }
+          for (int j = 0; j < 2; ++j) {
+            unsigned short h = 0;
+            if (left > 2 * j) asm volatile("ld.shared.u16 %0, [%1];" : "=h"(h) : "r"(raw0 + ws * C::WB + j * 2 * kBlockBytes + sc_off));
+            scale[j] = __half2float(__ushort_as_half(h));
           }
+          __syncwarp();
+          if (lane == 0) mbar_arrive(wempty0 + 8 * ws);
         }
-        if (k + 1 < ns) multiply(has(k + 1));
+        if (++ws == C::NW) { ws = 0; wp ^= 1; }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          if (left <= 2 * j) break;
+          if (ok) ok = __all_sync(0xffffffffu, mbar_wait(df + 8 * j, used[j] & 1, ERR_GEMM_TMEM_FULL_WAIT));
+          ++used[j];
+          if (!ok) continue;
+          tc_fence_after();
+#pragma unroll
+          for (int c0 = 0; c0 < T; c0 += 16) {
+            uint32_t d[16];
+            B2_TMEM_LD_16(d0 + j * 64 + c0, d);
+            tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < 16; ++i) acc[c0 + i] = fmaf(scale[j], __uint_as_float(d[i]), acc[c0 + i]);
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(de + 8 * j);
+        }
+        // the stage's token rows have been read by this pipeline's MMAs (which its products say; without one, the copy has to have
+        // landed before the stage may be handed back)
+        if (ok && q == 0) {
+          if (left <= 0) ok = __all_sync(0xffffffffu, mbar_wait(xfull0 + 8 * xs, xp, ERR_GEMM_FULL_WAIT));
+          if (ok && lane == 0) mbar_arrive(xempty0 + 8 * xs);
+        }
+        if (++xs == C::NX) { xs = 0; xp ^= 1; }
       }
-      // ---- the sets' sums, a quarter of the token rows at a time: set h takes quarter h from the others' buffers, in set order
-      constexpr int Q = T / 4;
+      // ---- the pipelines' sums: each takes half of the token rows from the other, even blocks first
+      constexpr int H = T / 2;
       const uint32_t col = red0 + (uint32_t)row * 4;
       const int n = nblk * 128 + row;
+      adders_sync();              // what was in the buffers before has been read
 #pragma unroll
-      for (int h = 0; h < kSets; ++h) {
-        const uint32_t buf = col + (h & 1) * ((kSets - 1) * Q * 512);      // two rounds' buffers in turn
-        if (set != h) {
+      for (int i = 0; i < H; ++i) {
+        const float give = pipe ? acc[i] : acc[H + i];
+        asm volatile("st.shared.f32 [%0], %1;" ::"r"(col + (pipe * H + i) * 512), "f"(give) : "memory");
+      }
+      adders_sync();
+      float* o = p.out + ((size_t)split * p.M + pipe * H) * p.N + n;
 #pragma unroll
-          for (int i = 0; i < Q; ++i) asm volatile("st.shared.f32 [%0], %1;" ::"r"(buf + ((set < h ? set : set - 1) * Q + i) * 512), "f"(acc[h * Q + i]) : "memory");
-        }
-        workers_sync();
-        if (set == h) {
-          float* o = p.out + ((size_t)split * p.M + h * Q) * p.N + n;
-#pragma unroll
-          for (int i = 0; i < Q; ++i) {
-            float sum = 0.f;
-#pragma unroll
-            for (int j = 0; j < kSets; ++j) {
-              float v = acc[h * Q + i];
-              if (j != h) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(buf + ((j < h ? j : j - 1) * Q + i) * 512));
-              sum = j ? sum + v : v;
-            }
-            if (h * Q + i < p.M && n < p.N) o[(size_t)i * p.N] = sum;
-          }
-        }
+      for (int i = 0; i < H; ++i) {
+        float other;
+        asm volatile("ld.shared.f32 %0, [%1];" : "=f"(other) : "r"(col + ((pipe ^ 1) * H + i) * 512));
+        const float mine = pipe ? acc[H + i] : acc[i];
+        if (pipe * H + i < p.M && n < p.N) o[(size_t)i * p.N] = pipe ? other + mine : mine + other;
       }
       if (p.fold_tickets == nullptr) continue;
       // ---- the last split of an n-block adds the slices in split order to the residual rows and leaves the sums of squares of
-      // its 128 columns (the arithmetic and order of the integer GEMV's fold).  Four rows are in flight per thread.
+      // its 128 columns.
       __threadfence();
-      workers_sync();
-      if (tid == 0) {
+      adders_sync();
+      if (at == 0) {
         const int last = atomicAdd(&p.fold_tickets[nblk], 1) == p.S - 1;
         if (last) p.fold_tickets[nblk] = 0;
         asm volatile("st.shared.u32 [%0], %1;" ::"r"(misc + 4), "r"(last) : "memory");
       }
-      workers_sync();
+      adders_sync();
       int last;
       asm volatile("ld.shared.u32 %0, [%1];" : "=r"(last) : "r"(misc + 4));
       if (!last) continue;
       __threadfence();
-      const int c = tid & 127, rsub = tid >> 7, fn = nblk * 128 + c;     // four rows of 128 columns at a time
-      for (int m0 = rsub; m0 < p.M; m0 += 16) {
-        float v[4] = {0.f, 0.f, 0.f, 0.f};
+      const int fn = nblk * 128 + lane * 4;       // a warp per row, four columns per lane, the slices' loads in flight together
+      for (int m = warp - 8; m < p.M; m += 8) {
+        float f[4] = {0.f, 0.f, 0.f, 0.f};
+        if (p.N % 4 == 0 && fn + 4 <= p.N) {
+          const uint2 r = *reinterpret_cast<const uint2*>(p.fold_resid_in + (size_t)m * p.N + fn);
+          f[0] = bf16_lo(r.x); f[1] = bf16_hi(r.x); f[2] = bf16_lo(r.y); f[3] = bf16_hi(r.y);
+#pragma unroll 1
+          for (int s0 = 0; s0 < p.S; s0 += 8) {
+            float4 v[8];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
-          if (m0 + 4 * u < p.M && fn < p.N) v[u] = __bfloat162float(p.fold_resid_in[(size_t)(m0 + 4 * u) * p.N + fn]);
-#pragma unroll 4
-        for (int sp = 0; sp < p.S; ++sp)
+            for (int u = 0; u < 8; ++u)
+              v[u] = s0 + u < p.S ? __ldcg(reinterpret_cast<const float4*>(p.out + ((size_t)(s0 + u) * p.M + m) * p.N + fn)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-          for (int u = 0; u < 4; ++u)
-            if (m0 + 4 * u < p.M && fn < p.N) v[u] += __ldcg(p.out + ((size_t)sp * p.M + m0 + 4 * u) * p.N + fn);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int m = m0 + 4 * u;
-          if (m >= p.M) break;
-          const __nv_bfloat16 rb = __float2bfloat16(v[u]);
-          if (fn < p.N) p.fold_resid_out[(size_t)m * p.N + fn] = rb;
-          const float rf = fn < p.N ? __bfloat162float(rb) : 0.f;
-          const float ss = warp_sum(rf * rf);
-          if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(ss0 + (m * 4 + (c >> 5)) * 4), "f"(ss) : "memory");
+            for (int u = 0; u < 8; ++u) { f[0] += v[u].x; f[1] += v[u].y; f[2] += v[u].z; f[3] += v[u].w; }
+          }
+          const uint2 o2 = make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]));
+          *reinterpret_cast<uint2*>(p.fold_resid_out + (size_t)m * p.N + fn) = o2;
+          f[0] = bf16_lo(o2.x); f[1] = bf16_hi(o2.x); f[2] = bf16_lo(o2.y); f[3] = bf16_hi(o2.y);
+        } else {
+          for (int i = 0; i < 4 && fn + i < p.N; ++i) {
+            f[i] = __bfloat162float(p.fold_resid_in[(size_t)m * p.N + fn + i]);
+            for (int sp = 0; sp < p.S; ++sp) f[i] += __ldcg(p.out + ((size_t)sp * p.M + m) * p.N + fn + i);
+            const __nv_bfloat16 rb = __float2bfloat16(f[i]);
+            p.fold_resid_out[(size_t)m * p.N + fn + i] = rb;
+            f[i] = __bfloat162float(rb);
+          }
         }
-      }
-      workers_sync();
-      if (tid < p.M) {
-        float4 q4;
-        asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(q4.x), "=f"(q4.y), "=f"(q4.z), "=f"(q4.w) : "r"(ss0 + tid * 16));
-        p.fold_ssq[(size_t)tid * p.nb + nblk] = ((q4.x + q4.y) + q4.z) + q4.w;
+        const float ss = warp_sum((f[0] * f[0] + f[1] * f[1]) + (f[2] * f[2] + f[3] * f[3]));
+        if (lane == 0) p.fold_ssq[(size_t)m * p.nb + nblk] = ss;
       }
     }
   }
@@ -344,11 +382,11 @@ int launch_rows(const RowsParams& p, cudaStream_t stream) {
 extern "C" int b2_gemm_w4_rows(const void* w4b, const void* x, float* out, int M, int N, int K, int S, int* fold_tickets,
                                const void* fold_resid_in, void* fold_resid_out, float* fold_ssq, void* stream) {
   if (M < 1 || M > 64 || N < 1 || K < 64 || K % 64 != 0 || S < 1 || S > kMaxSplits) return -1;
-  if (((uintptr_t)w4b | (uintptr_t)x) & 15) return -4;
+  if ((((uintptr_t)w4b | (uintptr_t)x | (uintptr_t)out) & 15) || (((uintptr_t)fold_resid_in | (uintptr_t)fold_resid_out) & 7)) return -4;
   RowsParams p;
   p.w = (const uint8_t*)w4b; p.x = (const uint8_t*)x; p.out = out;
   p.M = M; p.N = N; p.KG = K / 64; p.S = S; p.nb = (N + 127) / 128;
-  p.gps = ((p.KG + S - 1) / S + kSets - 1) / kSets * kSets;    // whole stages
+  p.gps = ((p.KG + S - 1) / S + kStageBlocks - 1) / kStageBlocks * kStageBlocks;    // whole stages
   if (p.gps * (S - 1) >= p.KG) return -2;                      // every split has groups
   p.fold_tickets = fold_tickets; p.fold_resid_in = (const __nv_bfloat16*)fold_resid_in;
   p.fold_resid_out = (__nv_bfloat16*)fold_resid_out; p.fold_ssq = fold_ssq;
