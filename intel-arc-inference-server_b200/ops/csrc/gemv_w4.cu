@@ -238,11 +238,12 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
   const uint32_t gsB = (p.xcg * 8 * T * 8 + 127) & ~127;   // bytes of one buffer's group scales
   const uint32_t xsB = (uint32_t)p.rows * strideB;          // bytes of one buffer's rows
 
-  // One token tile (M <= 8): the eight consumer warps form two groups of four that take alternate ring stages, a warp
+  // One or two token tiles (M <= 16): the eight consumer warps form two groups of four that take alternate ring stages, a warp
   // owning 32 rows of the block as two 16-row tiles.  Two stages of a CTA (four of an SM) are then in work at a time
   // and a warp has twice the independent MMA chains per wait; with all eight warps on every stage the loop was bound
-  // by the latency of one stage's wait -> load -> MMA -> hand-back chain, not by HBM.
-  constexpr bool kSplit = T == 1;
+  // by the latency of one stage's wait -> load -> MMA -> hand-back chain, not by HBM.  (Two token tiles: a step of 9 / 16 rows, 16
+  // layers of the 27B shape, 2.17 -> 2.13 / 2.42 -> 2.36 ms; with four tiles a warp has no registers for a second row tile.)
+  constexpr bool kSplit = T <= 2;
   constexpr int RT = kSplit ? 2 : 1;   // row tiles per warp
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nblk = blockIdx.x, split = blockIdx.y;
@@ -429,22 +430,20 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
       for (int tt = 0; tt < T; ++tt) xa[tt] = x_row[tt] + xb * xsB + gi * 128;
       const uint32_t gsa = gs_t + xb * gsB;
       const int ng = min(kG, cg - gi);   // groups of this stage
-      constexpr int NGq = T <= 2 ? 2 : 1;   // groups whose MMA chains are interleaved
+      constexpr int NGq = T == 1 ? 2 : 1;   // groups whose MMA chains are interleaved (two token tiles have chains enough, and no registers)
 #pragma unroll 1
       for (int q0 = 0; q0 < ng; q0 += NGq) {
         if (kSplit) {
-          float (&a0)[1][4] = *reinterpret_cast<float (*)[1][4]>(&acc[0]);
-          float (&a1)[1][4] = *reinterpret_cast<float (*)[1][4]>(&acc[T]);
-          const uint32_t (&xa1)[1] = *reinterpret_cast<const uint32_t (*)[1]>(&xa[0]);
-          if (q0 + 1 < ng) {
-            group_mma<1, 2>(a0, st + q0 * kBlockBytes, w_off, sc_off, xa1, gsa + (gi + q0) * 8 * T * 8);
-            group_mma<1, 2>(a1, st + q0 * kBlockBytes, w_off + 512, sc_off + 32, xa1, gsa + (gi + q0) * 8 * T * 8);
+          float (&a0)[T][4] = *reinterpret_cast<float (*)[T][4]>(&acc[0]);
+          float (&a1)[T][4] = *reinterpret_cast<float (*)[T][4]>(&acc[T]);
+          if (NGq == 2 && q0 + 1 < ng) {
+            group_mma<T, NGq>(a0, st + q0 * kBlockBytes, w_off, sc_off, xa, gsa + (gi + q0) * 8 * T * 8);
+            group_mma<T, NGq>(a1, st + q0 * kBlockBytes, w_off + 512, sc_off + 32, xa, gsa + (gi + q0) * 8 * T * 8);
           } else {
-            group_mma<1, 1>(a0, st + q0 * kBlockBytes, w_off, sc_off, xa1, gsa + (gi + q0) * 8 * T * 8);
-            group_mma<1, 1>(a1, st + q0 * kBlockBytes, w_off + 512, sc_off + 32, xa1, gsa + (gi + q0) * 8 * T * 8);
+            group_mma<T, 1>(a0, st + q0 * kBlockBytes, w_off, sc_off, xa, gsa + (gi + q0) * 8 * T * 8);
+            group_mma<T, 1>(a1, st + q0 * kBlockBytes, w_off + 512, sc_off + 32, xa, gsa + (gi + q0) * 8 * T * 8);
           }
-        } else if (NGq == 2 && q0 + 1 < ng) group_mma<T, NGq>(*reinterpret_cast<float (*)[T][4]>(&acc[0]), st + q0 * kBlockBytes, w_off, sc_off, xa, gsa + (gi + q0) * 8 * T * 8);
-        else group_mma<T, 1>(*reinterpret_cast<float (*)[T][4]>(&acc[0]), st + q0 * kBlockBytes, w_off, sc_off, xa, gsa + (gi + q0) * 8 * T * 8);
+        } else group_mma<T, 1>(*reinterpret_cast<float (*)[T][4]>(&acc[0]), st + q0 * kBlockBytes, w_off, sc_off, xa, gsa + (gi + q0) * 8 * T * 8);
 #pragma unroll
         for (int tt = 0; tt < T; ++tt) xa[tt] += 128 * NGq;
       }
@@ -463,16 +462,16 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
     // the two groups hold the sums of alternate stages of the same rows: they meet in shared memory (the ring is
     // free now: every stage has been waited for and consumed), group 0 first, so the order of the sum is fixed
     consumer_sync();
-    const uint32_t scr = ring + ((warp & 3) * 32 + lane) * 32;   // 8 floats per thread of a group
+    const uint32_t scr = ring + ((warp & 3) * 32 + lane) * (16 * T * RT);   // 4 T RT floats per thread of a group
     if (wgrp == 1) {
 #pragma unroll
-      for (int h = 0; h < RT; ++h)
+      for (int h = 0; h < T * RT; ++h)
         asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(scr + 16 * h), "f"(acc[h][0]), "f"(acc[h][1]), "f"(acc[h][2]), "f"(acc[h][3]) : "memory");
     }
     consumer_sync();
     if (wgrp == 0) {
 #pragma unroll
-      for (int h = 0; h < RT; ++h) {
+      for (int h = 0; h < T * RT; ++h) {
         float4 o;
         asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(scr + 16 * h));
         acc[h][0] += o.x; acc[h][1] += o.y; acc[h][2] += o.z; acc[h][3] += o.w;
@@ -486,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
 #pragma unroll
     for (int tt = 0; tt < T; ++tt) {
       const int m0 = tt * 8 + 2 * t, m1 = m0 + 1;
-      const float (&a)[4] = acc[kSplit ? h : tt];
+      const float (&a)[4] = acc[h * T + tt];
       if (m0 < p.M) {
         if (n_lo < p.N) outp[(size_t)m0 * p.ldo + n_lo] = a[0];
         if (n_hi < p.N) outp[(size_t)m0 * p.ldo + n_hi] = a[2];

@@ -227,3 +227,22 @@ def test_head_of_many_rows(m, n, k):
         assert torch.equal(out[m0: m0 + 16], o1) and torch.equal(cv[m0: m0 + 16], v1) and torch.equal(ci[m0: m0 + 16], i1)
     ref = x.double() @ w.double().T
     assert ((out.double() - ref).abs() <= 16 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 1e-9).all()
+
+
+# two token tiles: k blocks around what a stage and the two groups of warps take in turn, ends of blocks and of the row tiles
+@pytest.mark.parametrize("m", [9, 15, 16])
+@pytest.mark.parametrize("n,k,splits", [(128, 64, 1), (300, 320, 1), (256, 704, 3), (1000, 1088, 2), (5120, 1024, 4)])
+def test_integer_gemv_of_two_token_tiles(m, n, k, splits):
+    from b200serve.utils import quant as Q
+    torch.manual_seed(n + m)
+    w, x = Q.random_w4b(n, k, "cuda", 7), torch.randn(m, k, device="cuda").bfloat16()
+    wf = Q.dequant_w4b(w, n).double()
+    out, again, one = (torch.full((splits, m, n), float("nan"), device="cuda") for _ in range(3))
+    K.gemv_w4(w, x, out, m, n, k, splits)
+    K.gemv_w4(w, x, again, m, n, k, splits)
+    torch.cuda.synchronize()
+    K.check_status()
+    # activations are 15-bit integers per 64-k group: half a step of the group's largest, 2^-15, on every weight; fp32 sums
+    top = x.double().abs().view(m, k // 64, 64).amax(-1).repeat_interleave(64, -1)
+    bound = 2.0 ** -14 * (top @ wf.abs().T) + 16 * 2.0 ** -24 * (x.double().abs() @ wf.abs().T)
+    assert ((out.double().sum(0) - x.double() @ wf.T).abs() <= bound).all() and torch.equal(out, again)
