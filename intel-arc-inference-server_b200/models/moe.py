@@ -143,6 +143,13 @@ class _PrefillScratch:
         self.slab_gu = self.slab_dn = None
 
 
+# Prompt chunks of up to this many rows per expert read the experts' int4 blocks whatever the backend: with less than a tile of
+# rows an expert is bound by its bytes.  256 experts, 8 per row, 16 layers, bf16 copies / int4 blocks: 300 rows 8.4 / 7.1 ms, 1400 10.0 /
+# 8.6, 2048 10.8 / 9.4, 3000 (94 rows an expert) 12.7 / 11.2; 4000 (125) 15.6 / 15.5, and from a whole tile on the copies cost
+# no more than expanding the blocks for each further tile.
+W4_EXPERT_ROWS = 112
+
+
 def _expert_bf16(runner, lw: LayerWeights, sc: _PrefillScratch):
     """bf16 ``[E][N][K]`` forms of the stacked experts: resident when asked for, else dequantised into
     slabs that the next layer overwrites."""
@@ -184,7 +191,8 @@ def moe_block_prefill(runner, lw: LayerWeights, c: int):
            sc.blk_rows, sc.n_blk, sc.total_rows)
     M.scatter(sc.topk_idx, sc.rank, sc.expert_base, c, k, x, h, sc.row_of, sc.xs)
     blocks = (sc.blk_expert, sc.blk_row0, sc.blk_rows, sc.n_blk, sc.max_blk)
-    if runner.backend == "w4":      # grouped GEMMs over the experts' int4 blocks (a quarter of the bf16 bytes from HBM)
+    # grouped GEMMs over the experts' int4 blocks: a quarter of the bf16 bytes from HBM, at the price of expanding them (the same bits)
+    if runner.backend == "w4" or c * k <= W4_EXPERT_ROWS * e:
         G.gemm_w4(sc.xs, lw.experts_gate_up_w4b, 2 * i, h, sc.act, epi=G.EPI_SILU_MUL, blocks=blocks, n_experts=e)
         G.gemm_w4(sc.act, lw.experts_down_w4b, h, i, sc.y, epi=G.EPI_BF16, blocks=blocks, n_experts=e)
     else:

@@ -91,3 +91,39 @@ def test_rope_append_of_prompt_rows(m, pos0, nq, nkv, d):
     for t in (kc, vc):
         t[at[0], :, at[1]] = 7.0
         assert (t == 7.0).all()
+
+
+# k blocks around the depths of the tile ring and of the ring of int4 blocks, both tile widths, one tile per CTA and several
+@pytest.mark.parametrize("kb", [1, 3, 5, 7, 8, 10, 11, 29])
+@pytest.mark.parametrize("m,n,bn", [(130, 776, 256), (2049, 2560, 256), (130, 328, 128), (1500, 2176, 128)])
+def test_int4_block_ring(m, n, bn, kb):
+    torch.manual_seed(kb)
+    k = 64 * kb
+    w, a = Q.random_w4b(n, k, "cuda", 5), torch.randn(m, k, device="cuda").bfloat16()
+    wb = G.dequant_w4b(w, n, k)
+    out = torch.full((m + 1, n), float("nan"), device="cuda")
+    G.gemm_w4(a, w, n, k, out[:m], epi=G.EPI_F32, bn=bn)
+    torch.cuda.synchronize()
+    K.check_status()
+    ref, bound = a.double() @ wb.double().T, 16 * 2.0 ** -24 * (a.double().abs() @ wb.double().abs().T)
+    assert ((out[:m].double() - ref).abs() <= bound + 1e-9).all() and torch.isnan(out[m]).all()
+
+
+@pytest.mark.parametrize("over", [-400, 0, 1])
+def test_experts_from_int4_or_copies(over, monkeypatch):
+    """Prompt chunks on both sides of the rule: expanding a tile's blocks gives the bits of the bf16 copies."""
+    from b200serve.models import moe
+    from b200serve.models.config import small_moe
+    from b200serve.models.weights import random_weights
+    from b200serve.runtime.engine import Engine
+    cfg = small_moe()
+    rows = moe.W4_EXPERT_ROWS * cfg.n_experts // cfg.top_k + over
+    prompt = torch.randint(0, cfg.vocab, (rows,), generator=torch.Generator().manual_seed(rows)).tolist()
+    got = []
+    for limit in (moe.W4_EXPERT_ROWS, 0, 1 << 20):
+        monkeypatch.setattr(moe, "W4_EXPERT_ROWS", limit)
+        eng = Engine(random_weights(cfg, device="cuda", seed=4), max_seqs=1, max_len=1024, prefill_backend="bf16")
+        first = eng.prefill(0, prompt, chunk=1024)
+        K.check_status()
+        got.append((first, eng.logits(1)[0].clone()))
+    assert all(g[0] == got[0][0] and torch.equal(g[1], got[0][1]) for g in got)
