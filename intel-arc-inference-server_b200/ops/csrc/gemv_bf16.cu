@@ -33,7 +33,10 @@ struct GemvBfParams {
   Glu glu;                   // EPI_GLU
 };
 
-constexpr int kStages = 4, kWarps = 4, NG = 4, KU = 2;
+// Three stages a warp let three CTAs share an SM, as many bytes in flight as four stages in two, and finer waves (688 CTAs of a
+// 22016-wide projection).  8 layers of width 4096, step of 1 / 8 / 16 rows: 843 / 1002 / 1251 us, with four stages 932 / 1093 / 1296,
+// with two 922 / 1094 / 1292.
+constexpr int kStages = 3, kWarps = 4, NG = 4, KU = 2;
 
 template <int MH>
 constexpr int stage_bytes() { return (KU * NG + KU * MH) * 512; }

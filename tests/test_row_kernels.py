@@ -246,3 +246,18 @@ def test_integer_gemv_of_two_token_tiles(m, n, k, splits):
     top = x.double().abs().view(m, k // 64, 64).amax(-1).repeat_interleave(64, -1)
     bound = 2.0 ** -14 * (top @ wf.abs().T) + 16 * 2.0 ** -24 * (x.double().abs() @ wf.abs().T)
     assert ((out.double().sum(0) - x.double() @ wf.T).abs() <= bound).all() and torch.equal(out, again)
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("n,k,splits", [(32, 64, 1), (40, 256, 1), (72, 768, 1), (64, 832, 2), (1000, 2112, 3)])
+def test_bf16_gemv_ring(m, n, k, splits):
+    """Steps per warp below, at and above the ring's depth, warps without a step, columns that end inside a tile."""
+    from b200serve.ops import latent as L
+    torch.manual_seed(k + m)
+    w, x = (torch.randn(n, k, device="cuda") * 0.05).bfloat16(), torch.randn(m, k, device="cuda").bfloat16()
+    out = torch.full((splits, m, n), float("nan"), device="cuda")
+    L.gemv_bf16(w, x, out, m, n, k, splits)
+    torch.cuda.synchronize()
+    K.check_status()
+    bound = 16 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
+    assert ((out.double().sum(0) - x.double() @ w.double().T).abs() <= bound + 1e-9).all()
