@@ -17,8 +17,11 @@
 //     slices are merged in slice order through shared memory before the split's partial is written;
 //   * split-KV partials and the in-kernel merge by the last CTA ("ticket") have the layout and the fixed
 //     split order of the per-row kernel, so either kernel can serve a row.
-// An int8 cache (one fp32 scale per row) is staged as int8 and expanded to bf16 in shared memory by the thread
-// that owns the key, then takes the same path.
+// An int8 cache (one fp32 scale per row) is staged as int8.  Groups of up to 32 query rows multiply it as it is: a warp reads the
+// bytes of its own keys in the MMA's layout and makes them integers in bf16, which are exact, in registers; K's scale goes on
+// the products and V's on the probabilities, both in fp32.  Nothing is written back to shared memory, so it holds three
+// batches in flight.  Beyond 32 query rows, where several warps would make the same integers, the thread that owns a key
+// expands its row to bf16 tiles and the bf16 path follows.
 // The role of the reference's verify attention (src/kernels/attn_verify_dpas.cl) and of its decode
 // attention's GQA packing (src/kernels/attn_v2.cl).
 #include "common.cuh"
@@ -81,6 +84,14 @@ __device__ __forceinline__ uint32_t tile_off(int row, int d) {
 }
 
 // NKS: key slices per batch (1, 2 or 4); the four warps are NKS slices x (4 / NKS) groups of 16 query rows.
+// int8 as bf16 integers: even bytes of w as a pair.  With b's low seven bits as mantissa of 2^7, 128 + (b & 127) less 128 or, where
+// the sign is set, 256.
+__device__ __forceinline__ uint32_t bytes_bf16(uint32_t w) {
+  uint32_t lo = (w & 0x007f007fu) | 0x43004300u, hi = (w & 0x00800080u) | 0x43004300u, d;
+  asm("sub.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+
 template <bool I8, int NKS>
 __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t* smem_raw, const int* s_pos, int* s_last_p, int* s_bt,
                                                const int req, const int rows, const int QR, const int ctx_max, const int z) {
@@ -92,6 +103,10 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
   const uint32_t bar0 = k8s0 + (I8 ? p.nbuf * stageB : 0);
   float* scratch = reinterpret_cast<float*>(smem_raw + (base - smem_u32(smem_raw)));  // merges reuse the K / V tiles
   int& s_last = *s_last_p;
+  // The bytes go into the MMA's operands from registers (8 requests at up to 4000 positions, 16 layers: a step of 2.38 -> 2.13 ms;
+  // the expansion took longer than the bytes' way from HBM and everything else waited for it)
+  constexpr bool kDirect = I8 && NKS > 1;
+  const int nst = 2 + p.nbuf;     // then: batches in flight, in the tiles' memory too
   constexpr int NRG = 4 / NKS;    // groups of 16 query rows
   constexpr int KW = KB / NKS;              // keys per warp and batch
   constexpr int KS = KW > kPassKeys ? kPassKeys : KW;   // keys per pass over the warp's slice
@@ -121,8 +136,7 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
   const int* bt = bt_smem ? s_bt : btg;
 
   if (tid == 0) {
-    mbar_init(bar0, 1);
-    mbar_init(bar0 + 8, 1);
+    for (int i = 0; i < (kDirect ? nst : 2); ++i) mbar_init(bar0 + 8 * i, 1);
     mbar_fence_init();
   }
   __syncthreads();
@@ -141,6 +155,13 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
     const __nv_bfloat16* qp = p.q + (size_t)m * p.n_q * D + (size_t)(kh * p.gqa + h) * D;
 #pragma unroll
     for (int kk = 0; kk < 8; ++kk) {
+      if (kDirect) {    // step kk takes dims 32 t + 4 kk + (0, 2) and + (1, 3): the even and odd bytes of a word of the key's row
+        const uint32_t* qw = reinterpret_cast<const uint32_t*>(qp + 32 * t + 4 * kk);
+        const uint32_t q0 = ok ? qw[0] : 0u, q1 = ok ? qw[1] : 0u;
+        qa[kk][hf] = __byte_perm(q0, q1, 0x5410);
+        qa[kk][2 + hf] = __byte_perm(q0, q1, 0x7632);
+        continue;
+      }
       qa[kk][hf] = ok ? *reinterpret_cast<const uint32_t*>(qp + 16 * kk + 2 * t) : 0u;          // k = 2t, 2t + 1
       qa[kk][2 + hf] = ok ? *reinterpret_cast<const uint32_t*>(qp + 16 * kk + 8 + 2 * t) : 0u;  // k + 8
     }
@@ -152,6 +173,110 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
 
   bool okw = true;
   const int nbatch = (max(key1 - key0, 0) + KB - 1) / KB;
+  if constexpr (kDirect) {
+    auto issue = [&](int b, int slot) {     // warp 0: one copy per page, of K and of V
+      const int kb0 = b * KB, npages = (min(KB, key1 - key0 - kb0) + 15) >> 4;
+      const uint32_t bar = bar0 + 8 * slot, st = base + slot * stageB;
+      if (lane == 0) mbar_expect_tx(bar, (uint32_t)npages * 4096u);
+      __syncwarp();
+      if ((lane >> 1) < npages) {
+        const int pi = lane >> 1, row = (bt[(kb0 >> 4) + pi] * p.n_kv + kh) * 16;
+        tma_load_2d(st + (lane & 1) * (KB * D) + pi * 2048, (lane & 1) ? &p.v_map : &p.k_map, 0, row, bar);
+      }
+    };
+    if (warp == 0)
+      for (int b = 0; b < min(nst, nbatch); ++b) issue(b, b);
+    // the scales of this thread's keys (columns 2 t, 2 t + 1 of each n8 tile), a batch ahead of their use; keys behind the split's end: 0
+    float kn[NJ][2], vn[NJ][2];
+    auto scales = [&](int b) {
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int key = b * KB + ksl * KW + 8 * j + 2 * t + e;
+          const bool in = key < key1 - key0;
+          const size_t row = in ? ((size_t)bt[key >> 4] * p.n_kv + kh) * 16 + (key & 15) : 0;
+          kn[j][e] = in ? p.k_scale[row] : 0.f;
+          vn[j][e] = in ? p.v_scale[row] : 0.f;
+        }
+    };
+    if (active && nbatch > 0) scales(0);
+    int slot = 0, par = 0;
+    for (int batch = 0; batch < nbatch; ++batch) {
+      const int kb0 = key0 + batch * KB, nk = min(KB, key1 - kb0), kofs = ksl * KW;
+      if (okw) okw = mbar_wait(bar0 + 8 * slot, par, ERR_ATTN_WAIT);
+      if (okw && active && kofs < nk) {
+        const uint32_t k8 = base + slot * stageB, v8 = k8 + KB * D;
+        float vs[NJ][2], s[NJ][4];
+        // ---- S = Q K^T: the thread's key is row g of the tile, its dims 32 t .. 32 t + 31
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) {
+          s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+          uint32_t w[8];
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w[4 * u]), "=r"(w[4 * u + 1]), "=r"(w[4 * u + 2]), "=r"(w[4 * u + 3])
+                         : "r"(k8 + (kofs + 8 * j + g) * 128 + (((2 * t + u) ^ g) << 4)));
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk)
+            mma_bf16_16816(s[j], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], bytes_bf16(w[kk]), bytes_bf16(w[kk] >> 8));
+        }
+        float mnew[2] = {mx[0], mx[1]};
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int key = kb0 + kofs + 8 * j + 2 * t + (e & 1), hf = e >> 1;
+            s[j][e] = key < ctx[hf] && key < key1 && key >= wlo[hf] ? s[j][e] * (kn[j][e & 1] * p.scale_log2) : -INFINITY;
+            mnew[hf] = fmaxf(mnew[hf], s[j][e]);
+          }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j) vs[j][0] = vn[j][0], vs[j][1] = vn[j][1];
+        if (batch + 1 < nbatch) scales(batch + 1);
+        float corr[2];
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+          mnew[hf] = fmaxf(mnew[hf], __shfl_xor_sync(0xffffffffu, mnew[hf], 1));
+          mnew[hf] = fmaxf(mnew[hf], __shfl_xor_sync(0xffffffffu, mnew[hf], 2));
+          corr[hf] = mnew[hf] == -INFINITY ? 1.f : exp2f(mx[hf] - mnew[hf]);   // mx = -inf on the first keys -> 0
+          lsum[hf] *= corr[hf];
+          mx[hf] = mnew[hf];
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1];
+        }
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float pe = mnew[e >> 1] == -INFINITY ? 0.f : exp2f(s[j][e] - mnew[e >> 1]);
+            lsum[e >> 1] += pe;
+            s[j][e] = pe * vs[j][e & 1];
+          }
+        // ---- O += (P scale) V: a 16-bit column of the transposed load is two dims of a key, so its even bytes are the operand of
+        // an n8 tile over even dims and its odd bytes of one over odd dims: o[2 c + h] column n is dim 16 c + 2 n + h
+#pragma unroll
+        for (int kk = 0; kk < NJ / 2; ++kk) {
+          const uint32_t pa0 = pack_bf16(s[2 * kk][0], s[2 * kk][1]), pa1 = pack_bf16(s[2 * kk][2], s[2 * kk][3]);
+          const uint32_t pa2 = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]), pa3 = pack_bf16(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+#pragma unroll
+          for (int c = 0; c < 8; c += 2) {
+            uint32_t r0, r1, r2, r3;
+            const int mi = lane >> 3, key = kofs + 16 * kk + 8 * (mi & 1) + (lane & 7);
+            ldsm_x4_trans(v8 + key * 128 + (((c + (mi >> 1)) ^ (key & 7)) << 4), r0, r1, r2, r3);
+            mma_bf16_16816(o[2 * c], pa0, pa1, pa2, pa3, bytes_bf16(r0), bytes_bf16(r1));
+            mma_bf16_16816(o[2 * c + 1], pa0, pa1, pa2, pa3, bytes_bf16(r0 >> 8), bytes_bf16(r1 >> 8));
+            mma_bf16_16816(o[2 * c + 2], pa0, pa1, pa2, pa3, bytes_bf16(r2), bytes_bf16(r3));
+            mma_bf16_16816(o[2 * c + 3], pa0, pa1, pa2, pa3, bytes_bf16(r2 >> 8), bytes_bf16(r3 >> 8));
+          }
+        }
+      }
+      __syncthreads();    // the batch is consumed: its memory may be filled again
+      if (warp == 0 && batch + nst < nbatch) issue(batch + nst, slot);
+      if (++slot == nst) { slot = 0; par ^= 1; }
+    }
+  } else {
   float ksc[2] = {0.f, 0.f}, vsc[2] = {0.f, 0.f};
   // The pages of batch b into buffer b % nbuf: lanes of warp 0 issue one tiled copy each (page, K or V, half).
   auto issue = [&](int b) {
@@ -313,6 +438,7 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
     }
     }  // pass
   }
+  }
 
   // ---- this split's partials: unnormalised O against the running maximum, (max, sum)
 #pragma unroll
@@ -329,7 +455,13 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
       for (int hf = 0; hf < 2; ++hf) {
         float* dst = scratch + (size_t)(ksl * (NRG * 16) + rg * 16 + g + 8 * hf) * SROW;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) *reinterpret_cast<float2*>(dst + 8 * j + 2 * t) = make_float2(o[j][2 * hf], o[j][2 * hf + 1]);
+        for (int j = 0; j < 16; j += 2)
+          if (kDirect) {
+            *reinterpret_cast<float4*>(dst + 8 * j + 4 * t) = make_float4(o[j][2 * hf], o[j + 1][2 * hf], o[j][2 * hf + 1], o[j + 1][2 * hf + 1]);
+          } else {
+            *reinterpret_cast<float2*>(dst + 8 * j + 2 * t) = make_float2(o[j][2 * hf], o[j][2 * hf + 1]);
+            *reinterpret_cast<float2*>(dst + 8 * j + 8 + 2 * t) = make_float2(o[j + 1][2 * hf], o[j + 1][2 * hf + 1]);
+          }
         if (t == 0) {
           dst[D] = mx[hf];
           dst[D + 1] = lsum[hf];

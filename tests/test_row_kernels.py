@@ -261,3 +261,47 @@ def test_bf16_gemv_ring(m, n, k, splits):
     K.check_status()
     bound = 16 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T)
     assert ((out.double().sum(0) - x.double() @ w.double().T).abs() <= bound + 1e-9).all()
+
+
+# contexts at the edges of pages, of a warp's keys and of a batch, more batches than are in flight; one, two and four groups of 16
+# query rows (the last goes through expanded tiles); rows behind a context hold NaN scales
+@pytest.mark.parametrize("ctx", [1, 16, 33, 127, 129, 512, 513, 1900])
+@pytest.mark.parametrize("nq,nkv,rows,window", [(5, 1, 1, 0), (16, 4, 4, 0), (16, 1, 1, 0), (20, 4, 5, 100), (12, 2, 5, 0), (16, 2, 8, 0)])
+@pytest.mark.parametrize("splits", [1, 3])
+def test_attention_on_int8_cache(ctx, nq, nkv, rows, window, splits):
+    torch.manual_seed(ctx)
+    d, gqa, dev = 128, nq // nkv, "cuda"
+    spec = [(0, p) for p in range(max(0, ctx - rows), ctx)] + [(1, ctx // 2)]
+    m, blocks = len(spec), ctx // 16 + 2
+    table = (torch.randperm(2 * blocks, device=dev) + 1).int().view(2, blocks).contiguous()
+    k8, v8 = (torch.randint(-127, 128, (2 * blocks + 1, nkv, 16, d), dtype=torch.int8, device=dev) for _ in range(2))
+    ks, vs = (torch.rand(2 * blocks + 1, nkv, 16, device=dev) * 0.03 for _ in range(2))
+    for req, last in ((0, ctx - 1), (1, ctx // 2)):       # nothing is stored behind the last position
+        pos = torch.arange(last + 1, blocks * 16, device=dev)
+        for t in (ks, vs):
+            t[table[req].long()[pos // 16], :, pos % 16] = float("nan")
+    q = torch.randn(m, nq * d, device=dev).bfloat16()
+    ctrl = _ctrl([r for r, _ in spec])
+    ctrl[K.CTRL_ROW_POS: K.CTRL_ROW_POS + m] = torch.tensor([p for _, p in spec], dtype=torch.int32, device=dev)
+    part, ml = torch.full((m * nq * splits * d,), float("nan"), device=dev), torch.full((m * nq * splits * 2,), float("nan"), device=dev)
+    out = torch.full((m, nq * d), float("nan"), dtype=torch.bfloat16, device=dev)
+    K.attn_rows(q, k8, v8, table, ctrl, part, ml, out, None, m, nq, nkv, d, splits, blocks, d ** -0.5, k_scale=ks, v_scale=vs, kv_int8=True,
+                window=window)
+    torch.cuda.synchronize()
+    K.check_status()
+    for i, (req, pos) in enumerate(spec):
+        at = torch.arange(max(0, pos + 1 - window) if window else 0, pos + 1, device=dev)
+        pg = table[req].long()[at // 16]
+        kk, vv = (c[pg, :, at % 16].double() * s[pg, :, at % 16].double()[..., None] for c, s in ((k8, ks), (v8, vs)))
+        qq = q[i].double().view(nkv, gqa, d)
+        s = torch.einsum("hgd,khd->hgk", qq, kk) * d ** -0.5
+        p = s.softmax(-1)
+        want, size = torch.einsum("hgk,khd->hgd", p, vv), torch.einsum("hgk,khd->hgd", p, vv.abs())
+        # probabilities (times V's scale) and the result are rounded to bf16, which has eight significant bits: 2^-8 of the
+        # value each, 2^-7 together, and a little for fp32 scores and sums.  Expanded tiles round K and V too: 2^-8 of V,
+        # and of every product of a score
+        bound = 1.05 * 2.0 ** -7 * size
+        if rows * gqa > 32:
+            ds = 2.0 ** -8 * torch.einsum("hgd,khd->hgk", qq.abs(), kk.abs()).amax(-1, keepdim=True) * d ** -0.5
+            bound = bound + (2.0 ** -8 + 2 * ds) * size
+        assert ((out[i].double().view(nkv, gqa, d) - want).abs() <= bound + 1e-9).all()
