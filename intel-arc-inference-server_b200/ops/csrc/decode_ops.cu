@@ -125,14 +125,20 @@ __global__ void __launch_bounds__(256) norm_rows_kernel(const ResidNormParams p,
   uint4 v[NV];
 #pragma unroll
   for (int i = 0; i < NV; ++i) v[i] = lane + 32 * i < H8 ? src[lane + 32 * i] : make_uint4(0, 0, 0, 0);
-  float ss = 0.f;
+  // the order of the form above, whose warp i had these 32 pieces: a sum per piece, over the lanes, over the pieces (the same bits)
+  float tot = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+    float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) ss += bf16_lo(w[j]) * bf16_lo(w[j]) + bf16_hi(w[j]) * bf16_hi(w[j]);
+    for (int j = 0; j < 4; ++j) {
+      const float f0 = bf16_lo(w[j]), f1 = bf16_hi(w[j]);
+      ss += f0 * f0 + f1 * f1;
+    }
+    tot += warp_sum(ss);
   }
-  const float rinv = rsqrtf(warp_sum(ss) / (float)p.H + p.eps);
+  const float rinv = rsqrtf(tot / (float)p.H + p.eps);
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = lane + 32 * i;

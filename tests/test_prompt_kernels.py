@@ -62,6 +62,9 @@ def test_norm_of_prompt_rows(m, h):
     # one rounding to bf16; the fp32 sum of h squares moves the factor by less than 2^-24 sqrt(h)
     assert ((x[:m].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-30).all()
     assert torch.equal(r, keep) and torch.isnan(x[m]).all()
+    few = torch.empty(100, h, dtype=torch.bfloat16, device="cuda")       # a CTA per row: the same bits
+    K.resid_norm(1, 100, h, w, 1e-6, r, few, resid_in=r, splits=0)
+    assert torch.equal(x[:100], few)
 
 
 @pytest.mark.parametrize("m,pos0,nq,nkv,d", [(1, 0, 4, 2, 128), (3, 5, 8, 2, 64), (4, 16, 40, 8, 128), (37, 31, 3, 1, 256), (130, 1000, 16, 4, 128), (18, 7, 5, 5, 192)])
