@@ -306,7 +306,8 @@ class DecoderModel:
         the partial buffers are laid out for.  Rows of different requests fill the GPU by themselves; every split of a short
         context is a CTA that costs its launch, its copies' latency and a partial to merge, for a handful of keys.  16 layers, 8 KV
         heads, all splits / two waves: 40 requests at 600 positions 7.63 / 6.61 ms, 64 at 300 10.4 / 8.5, 8 at 4000 in int8 2.61 /
-        2.43, 16 at 1500 in int8 3.90 / 2.84; one wave and four are within 3 % of two."""
+        2.43, 16 at 1500 in int8 3.90 / 2.84; one wave and four are within 3 % of two from 8
+        requests on, and 5 to 8 % behind it at 4 requests of 4000."""
         if self.attn_fixed_spans:
             return self.nsplit_attn
         rows = max(1, min(8, 64 // self.cfg.gqa))
