@@ -49,11 +49,13 @@ __device__ __forceinline__ void route_row(const float* __restrict__ lrow, int E,
 #pragma unroll
   for (int i = 0; i < PER; ++i) {
     if (!PLAIN && 32 * i >= E) { v[i] = -1.f; continue; }
-    // softmax: unnormalised probabilities; -1 marks "taken / absent"
+    // softmax: unnormalised probabilities; -1 marks "taken / absent", -1/2 a score that is NaN: it is taken after all others (a
+    // row's ids index weights and tables, so they are E's whatever the logits) and makes the row's weights NaN
     const bool in = (lane + 32 * i) < E;
     if (!PLAIN && rule.sigmoid) v[i] = in ? 1.f / (1.f + expf(-v[i])) : -1.f;
     else v[i] = in ? __expf(v[i] - mx) : -1.f;
     if (!PLAIN) total += in ? v[i] : 0.f;
+    v[i] = fmaxf(v[i], in ? -0.5f : -1.f);
   }
   if (!PLAIN && rule.groups > 1) {
     const int size = E / rule.groups;
@@ -117,6 +119,7 @@ __device__ __forceinline__ void route_row(const float* __restrict__ lrow, int E,
       if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
     }
     if ((bi & 31) == lane) v[bi >> 5] = -1.f;
+    if (bv < 0.f) bv = __int_as_float(0x7fc00000);
     wsum += bv;
     if (lane == r) { myw = bv; myid = bi; }
   }

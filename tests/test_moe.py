@@ -34,6 +34,62 @@ def test_route_matches_oracle_rule(t, e, k):
     assert (w.cpu().reshape(t, k)[clear] - ref_w[clear]).abs().max() < 1e-5
 
 
+@pytest.mark.parametrize("e,k,rule", [(8, 2, (0, 1, 1, 1)), (256, 8, (0, 1, 1, 1)), (64, 6, (1, 1, 1, 1)), (40, 4, (1, 1, 1, 0)), (64, 6, (1, 8, 3, 1)),
+                                      (33, 3, (0, 1, 1, 0)), (512, 32, (0, 1, 1, 1))])
+def test_route_of_rows_that_are_not_numbers(e, k, rule):
+    """A row without enough scores that are numbers gets distinct ids of the experts and NaN weights; the rows beside it, and rows with
+    a few NaN scores, are routed as if those experts were not there."""
+    from b200serve.ops import moe as M
+    torch.manual_seed(e + k)
+    logits = torch.randn(9, e)
+    logits[1] = float("nan")
+    logits[2, torch.randperm(e)[: e - k + 1]] = float("nan")      # one number too few
+    logits[3] = -float("inf")
+    logits[4] = float("inf")
+    logits[5, torch.randperm(e)[: e // 8]] = float("nan")
+    clean = logits.clone()
+    clean[5] = torch.where(clean[5].isnan(), -30.0, clean[5])
+    got, ref = [], []
+    for t, out in ((logits, got), (clean, ref)):
+        idx, w = torch.full((9 * k,), -1, dtype=torch.int32, device="cuda"), torch.zeros(9 * k, device="cuda")
+        M.route(t.cuda(), e, 9, e, k, idx, w, rule=rule)
+        torch.cuda.synchronize()
+        out += [idx.view(9, k).cpu(), w.view(9, k).cpu()]
+    assert all(0 <= int(i) < e for i in got[0].flatten()) and all(len(set(r)) == k for r in got[0].tolist())
+    assert got[1][1:3].isnan().any(-1).all()
+    for r in (0, 6, 7, 8):
+        assert torch.equal(got[0][r], ref[0][r]) and torch.equal(got[1][r], ref[1][r]) and got[1][r].isfinite().all()
+    if rule[1] == 1:
+        assert torch.equal(got[0][5], ref[0][5])
+        if rule[0] or rule[3]:          # (a softmax over all scores has no normaliser)
+            assert torch.allclose(got[1][5], ref[1][5], rtol=1e-5, atol=0)
+
+
+def test_grouped_step_with_a_row_that_is_not_a_number():
+    """The other rows of a step get the bits they get beside a row of numbers."""
+    from b200serve.ops import lib as K
+    from b200serve.ops import moe as M
+    torch.manual_seed(5)
+    m, e, k, h = 12, 16, 4, 256
+    w, x = torch.randn(e, h, device="cuda").bfloat16(), torch.randn(m, h, device="cuda").bfloat16()
+    out = []
+    for bad in (False, True):
+        xx = x.clone()
+        if bad:
+            xx[7] = float("nan")
+        logits, idx, wt = torch.zeros(m, e, device="cuda"), torch.full((m * k,), -1, dtype=torch.int32, device="cuda"), torch.zeros(m * k, device="cuda")
+        tickets, groups = (torch.zeros(n, dtype=torch.int32, device="cuda") for n in (3, M.group_words(m * k)))
+        M.router_rows(w, xx, logits, m, e, h, e, e, k, False, False, idx, wt, tickets, groups=groups)
+        torch.cuda.synchronize()
+        K.check_status()
+        tab = groups[16:].view(-1, 10)[: int(groups[0])].tolist()
+        assert all(0 <= g[0] < e and 1 <= g[1] <= 8 for g in tab)
+        assert sorted(p for g in tab for p in g[2: 2 + g[1]]) == list(range(m * k))
+        out.append((idx.view(m, k).cpu(), wt.view(m, k).cpu()))
+    rows = [r for r in range(m) if r != 7]
+    assert torch.equal(out[0][0][rows], out[1][0][rows]) and torch.equal(out[0][1][rows], out[1][1][rows]) and out[1][1][7].isnan().all()
+
+
 def _teacher_forced(oracle, prompt, toks, margin):
     kv = OracleKV(oracle.cfg)
     logits = oracle.forward(prompt, kv, 0)[-1]
