@@ -48,6 +48,8 @@ class StepBuffers:
         self.attn_out = torch.zeros(max_rows, cfg.q_dim, dtype=bf, device=device)
         self.o_part = torch.zeros(max_rows * cfg.n_q_heads * nsplit_attn * cfg.head_dim, dtype=f32, device=device)
         self.ml_part = torch.zeros(max_rows * cfg.n_q_heads * nsplit_attn * 2, dtype=f32, device=device)
+        # KV splits of a step's rows, for full attention and for windowed layers
+        self.attn_plan, self.attn_plan_win = (torch.zeros(K.attn_plan_words(max_rows, cfg.n_kv_heads), dtype=torch.int32, device=device) for _ in range(2))
         self.logits = torch.zeros(max_rows, head_rows, dtype=f32, device=device)
         self.ncand = K.head_ncand(head_rows)
         self.cand_val = torch.zeros(max_rows * self.ncand, dtype=f32, device=device)
@@ -81,6 +83,9 @@ def attn_splits(n_kv_heads: int, depth: int) -> int:
     depth 1024 1.41 / 1.43 / 1.45 ms with 16 / 32 / 37 splits, depth 4096 1.50 / 1.49 ms with 32 / 37, depth
     32768 (8 layers) 1.10 / 1.17 ms with 37 / 64."""
     return max(4, min(64, 296 // max(1, n_kv_heads), max(depth, 64) // 64))
+
+
+ATTN_WAVES = 2      # of 2 x 148 CTAs of decode attention, see ``DecoderModel._attn_splits``
 
 
 class ListedBuffers:
@@ -241,12 +246,12 @@ class DecoderModel:
         self.merge_quant = os.environ.get("B2_MERGE_QUANT", "1") == "1"   # the attention merge writes the o projection's quantised rows
         self.attn_rows_min = int(os.environ.get("B2_ATTN_ROWS_MIN", "1"))
         self.rows_one_request = False    # set by the engine around a step whose rows are one request's, consecutive
+        self._planned = False            # the step's attention takes its splits from ``buf.attn_plan``
         self.block_rows = False      # set by a block drafter around its layers: flagged rows attend non-causally
         self.attn_merge_inkernel_rows = int(os.environ.get("B2_ATTN_MERGE_INKERNEL_ROWS", "0"))
         # fixed KV split spans make a row's attention bits independent of the rows it is verified with (speculation
         # then reproduces plain decoding exactly); off, the splits adapt to the context (fastest at any depth)
         self.attn_fixed_spans = False
-        self.attn_waves = 2
         self.fused = self.nccl is None and os.environ.get("B2_UNFUSED", "0") != "1"     # dense layers: residual folds and norms ride inside the GEMVs
         # whole-step kernel (one launch for embedding + all dense layers of a one-request step of up to 8 rows).
         # Off unless asked for (B2_MEGA=1, or the attribute): on the 27B shape at depth 4096 it takes 6.6 ms per
@@ -302,17 +307,36 @@ class DecoderModel:
         return part, s
 
     def _attn_splits(self, m: int) -> int:
-        """KV splits of an attention launch of ``m`` rows: as many as keep ``attn_waves`` waves of CTAs busy, at most those that
-        the partial buffers are laid out for.  Rows of different requests fill the GPU by themselves; every split of a short
-        context is a CTA that costs its launch, its copies' latency and a partial to merge, for a handful of keys.  16 layers, 8 KV
-        heads, all splits / two waves: 40 requests at 600 positions 7.63 / 6.61 ms, 64 at 300 10.4 / 8.5, 8 at 4000 in int8 2.61 /
-        2.43, 16 at 1500 in int8 3.90 / 2.84; one wave and four are within 3 % of two from 8
-        requests on, and 5 to 8 % behind it at 4 requests of 4000."""
+        """KV splits of an attention launch of ``m`` rows of one request, which share a context: as many as keep ``ATTN_WAVES`` waves
+        of CTAs busy, at most those that the partial buffers are laid out for."""
         if self.attn_fixed_spans:
             return self.nsplit_attn
         rows = max(1, min(8, 64 // self.cfg.gqa))
-        ctas = self.cfg.n_kv_heads * ((m + rows - 1) // rows if self.rows_one_request and m > 1 else m)
-        return max(1, min(self.nsplit_attn, (self.attn_waves * 296 + ctas - 1) // ctas))
+        ctas = self.cfg.n_kv_heads * ((m + rows - 1) // rows)
+        return max(1, min(self.nsplit_attn, (ATTN_WAVES * 296 + ctas - 1) // ctas))
+
+    def _attn_rows_ok(self, m: int) -> bool:
+        """Steps of ``m`` rows have the multi-row attention kernel."""
+        cfg = self.cfg
+        return m >= self.attn_rows_min and cfg.head_dim == 128 and self.nsplit_attn <= 64 and cfg.gqa <= 16
+
+    def _start(self, m: int, ctrl, lw: Optional[LayerWeights] = None):
+        """A walk's first launch: the rows' embeddings into ``buf.resid``, normed for layer ``lw`` into ``buf.x`` (None: the residual
+        rows are there), and the attention's splits where the rows are several requests'.  Those go by lengths, which only
+        the device knows."""
+        cfg, b = self.cfg, self.buf
+        self._planned = m > 1 and not self.rows_one_request and not self.attn_fixed_spans and self._attn_rows_ok(m)
+        heads, win = (cfg.n_q_heads, cfg.n_kv_heads, self.nsplit_attn), max(0, cfg.sliding_window)
+        if lw is None:
+            if self._planned:
+                K.attn_plan(ctrl, m, *heads, b.attn_plan)
+                if win:
+                    K.attn_plan(ctrl, m, *heads, b.attn_plan_win, window=win)
+        elif self._planned:
+            K.embed_plan(m, cfg.hidden, lw.input_norm, cfg.rms_eps, b.resid, b.x, self.w.embed, ctrl, cfg.vocab, b.flag, *heads, b.attn_plan,
+                         window=win, plan_win=b.attn_plan_win if win else None)
+        else:
+            K.resid_norm(0, m, cfg.hidden, lw.input_norm, cfg.rms_eps, b.resid, b.x, embed=self.w.embed, ctrl=ctrl, vocab=cfg.vocab, flag=b.flag)
 
     def _attention(self, m: int, ctrl, block_table, max_blocks, kv: KVCache, kc, vc, ks, vs, window: int = 0,
                    quant_out: bool = False) -> bool:
@@ -321,18 +345,19 @@ class DecoderModel:
         cfg, b = self.cfg, self.buf
         if window == -1 and (cfg.head_dim != 128 or self.nsplit_attn > 64 or cfg.gqa > 16):
             raise NotImplementedError("block rows need the multi-row attention kernel (head size 128)")
-        if (m >= self.attn_rows_min or window == -1) and cfg.head_dim == 128 and self.nsplit_attn <= 64 and cfg.gqa <= 16:
+        if self._attn_rows_ok(m) or window == -1:
             inkernel = m <= self.attn_merge_inkernel_rows    # few rows: the last split CTA merges; many: a merge launch
             # ``quant_out``: the caller's next launch is the o projection on pre-quantised rows; the merge writes them
             wide = self._on_rows(m)
             quant = quant_out and not inkernel and (wide or m >= self.prequant_rows) and self.merge_quant
-            nsplit = self._attn_splits(m)
+            plan = (b.attn_plan_win if window > 0 else b.attn_plan) if self._planned else None
+            nsplit = self.nsplit_attn if plan is not None else self._attn_splits(m)
             K.attn_rows(b.q, kc, vc, block_table, ctrl, b.o_part, b.ml_part, b.attn_out, b.tickets if inkernel else None,
                         m, cfg.n_q_heads,
                         cfg.n_kv_heads, cfg.head_dim, nsplit, max_blocks, self.scale,
                         span_pages=(max_blocks + nsplit - 1) // nsplit if self.attn_fixed_spans else 0,
                         k_scale=ks, v_scale=vs, kv_int8=kv.kv_int8, window=window, one_request=self.rows_one_request and m > 1,
-                        xq=(b.xr if wide else b.xq) if quant else None, xq_gs=b.xq_gs if quant and not wide else None)
+                        xq=(b.xr if wide else b.xq) if quant else None, xq_gs=b.xq_gs if quant and not wide else None, plan=plan)
             return quant
         else:
             if window > 0:
@@ -572,6 +597,8 @@ class DecoderModel:
         pend = None
         embedded = False
         self.rows_one_request = bool(one_request)     # the attention launch then counts row groups, not rows
+        if resid_ready or not first_from_embed:
+            self._start(m, ctrl)
         if self.fused and resid_ready and all(lw.gate_up is not None and lw.gdn is None for lw in layers) and h % 128 == 0:
             for i, lw in enumerate(layers):
                 self.dense_layer_fused(lw, kv_layer0 + i, m, ctrl, block_table, max_blocks, kv, x_ready=False)
@@ -583,8 +610,7 @@ class DecoderModel:
                 self.mega_layers(layers, m, ctrl, block_table, max_blocks, kv, plan, kv_layer0)
                 return None, 0
         if self.fused and first_from_embed and all(lw.gate_up is not None and lw.gdn is None for lw in layers) and h % 128 == 0:
-            K.resid_norm(0, m, h, layers[0].input_norm, cfg.rms_eps, b.resid, b.x, embed=self.w.embed, ctrl=ctrl,
-                         vocab=cfg.vocab, flag=b.flag)
+            self._start(m, ctrl, layers[0])
             for i, lw in enumerate(layers):
                 self.dense_layer_fused(lw, kv_layer0 + i, m, ctrl, block_table, max_blocks, kv, x_ready=(i == 0))
             return None, 0      # the residual stream is already folded
@@ -592,8 +618,7 @@ class DecoderModel:
                 any(lw.gdn is not None for lw in layers) and all(lw.gate_up is not None for lw in layers) and
                 cfg.gdn_value_dim % 64 == 0):
             # hybrid model: gated delta-net layers and attention layers, both on their fused forms
-            K.resid_norm(0, m, h, layers[0].input_norm, cfg.rms_eps, b.resid, b.x, embed=self.w.embed, ctrl=ctrl,
-                         vocab=cfg.vocab, flag=b.flag)
+            self._start(m, ctrl, layers[0])
             for i, lw in enumerate(layers):
                 if lw.gdn is not None:
                     self.gdn_layer_fused(lw, kv_layer0 + i, m, ctrl, kv, x_ready=(i == 0))
@@ -601,8 +626,7 @@ class DecoderModel:
                     self.dense_layer_fused(lw, kv_layer0 + i, m, ctrl, block_table, max_blocks, kv, x_ready=(i == 0))
             return None, 0
         if first_from_embed and self._moe_fusable(layers):
-            K.resid_norm(0, m, h, layers[0].input_norm, cfg.rms_eps, b.resid, b.x, embed=self.w.embed, ctrl=ctrl,
-                         vocab=cfg.vocab, flag=b.flag)
+            self._start(m, ctrl, layers[0])
             for i, lw in enumerate(layers):
                 self.moe_layer_fused(lw, kv_layer0 + i, m, ctrl, block_table, max_blocks, kv, x_ready=(i == 0))
             return None, 0      # the residual stream is already folded
@@ -612,8 +636,7 @@ class DecoderModel:
             if pend is None:
                 if first_from_embed and not embedded:
                     embedded = True
-                    K.resid_norm(0, m, h, lw.input_norm, cfg.rms_eps, b.resid, b.x, embed=self.w.embed, ctrl=ctrl,
-                                 vocab=cfg.vocab, flag=b.flag)
+                    self._start(m, ctrl, lw)
                 else:   # resid already holds the layer input
                     K.resid_norm(1, m, h, lw.input_norm, cfg.rms_eps, b.resid, b.x, resid_in=b.resid, splits=0)
             else:

@@ -24,6 +24,7 @@
 // expands its row to bf16 tiles and the bf16 path follows.
 // The role of the reference's verify attention (src/kernels/attn_verify_dpas.cl) and of its decode
 // attention's GQA packing (src/kernels/attn_v2.cl).
+#include "attn_plan.cuh"
 #include "common.cuh"
 
 #include <cstdlib>
@@ -66,6 +67,8 @@ struct AttnRowsParams {
   int one_slice;   // 1: never cut a batch's keys over idle warps (a row's bits then do not depend on the group's size)
   int span_pages;  // > 0: every split covers this many pages whatever the context (a row's bits then do not depend
                    // on which rows share its CTA); 0: the group's context is cut into nsplit equal parts
+  const int* plan; // [64] splits of every row, then what entry blockIdx.y of the grid stands for (attn_plan.cuh); nullptr: every
+                   // group has nsplit splits
   float scale_log2;
 };
 
@@ -94,7 +97,8 @@ __device__ __forceinline__ uint32_t bytes_bf16(uint32_t w) {
 
 template <bool I8, int NKS>
 __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t* smem_raw, const int* s_pos, int* s_last_p, int* s_bt,
-                                               const int req, const int rows, const int QR, const int ctx_max, const int z) {
+                                               const int req, const int rows, const int QR, const int ctx_max, const int z,
+                                               const int split, const int nsp) {
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;   // the swizzle pattern repeats every 1024 bytes
   // bf16 form: nbuf pairs of operand tiles.  int8 form: one pair of operand tiles, nbuf pairs of staged int8 rows.
   const int ntile = I8 ? 1 : p.nbuf;
@@ -111,7 +115,7 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
   constexpr int KW = KB / NKS;              // keys per warp and batch
   constexpr int KS = KW > kPassKeys ? kPassKeys : KW;   // keys per pass over the warp's slice
   constexpr int NJ = KS / 8;                // n8 tiles of keys per pass
-  const int kh = blockIdx.x, split = blockIdx.y;   // z: the group's first row
+  const int kh = blockIdx.x;   // z: the group's first row; split of nsp (partials have p.nsplit places)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int rg = warp % NRG, ksl = warp / NRG;
   const int total_pages = (ctx_max + 15) >> 4;
@@ -122,8 +126,8 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
     pps = p.span_pages;
     key0 = max(split * pps, page0) * 16;
     key1 = min(ctx_max, (split + 1) * pps * 16);
-  } else {                  // the pages from the window's first one on, in nsplit equal parts
-    pps = (total_pages - page0 + p.nsplit - 1) / p.nsplit;
+  } else {                  // the pages from the window's first one on, in nsp equal parts
+    pps = (total_pages - page0 + nsp - 1) / nsp;
     key0 = (page0 + split * pps) * 16;
     key1 = min(ctx_max, key0 + pps * 16);
   }
@@ -518,27 +522,27 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
   __syncthreads();
   if (tid == 0) {
     const int tk = atomicAdd(&p.tickets[z * p.n_kv + kh], 1);
-    s_last = (tk == p.nsplit - 1);
+    s_last = (tk == nsp - 1);
     if (s_last) p.tickets[z * p.n_kv + kh] = 0;
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  float* cw = scratch;  // [QR][nsplit] weights of the splits
+  float* cw = scratch;  // [QR][nsp] weights of the splits
   for (int i = tid; i < QR; i += kThreads) {
     const int m = z + i / p.gqa, h = i % p.gqa;
     const size_t pb = ((size_t)m * p.n_q + kh * p.gqa + h) * p.nsplit;
     float mm = -INFINITY;
-    for (int sp = 0; sp < p.nsplit; ++sp) mm = fmaxf(mm, __ldcg(p.ml_part + (pb + sp) * 2));
+    for (int sp = 0; sp < nsp; ++sp) mm = fmaxf(mm, __ldcg(p.ml_part + (pb + sp) * 2));
     float lt = 0.f;
-    for (int sp = 0; sp < p.nsplit; ++sp) {
+    for (int sp = 0; sp < nsp; ++sp) {
       const float ms = __ldcg(p.ml_part + (pb + sp) * 2);
       const float c = (ms == -INFINITY) ? 0.f : exp2f(ms - mm);
       lt += __ldcg(p.ml_part + (pb + sp) * 2 + 1) * c;
-      cw[i * p.nsplit + sp] = c;
+      cw[i * nsp + sp] = c;
     }
     const float inv = lt > 0.f ? 1.f / lt : 0.f;
-    for (int sp = 0; sp < p.nsplit; ++sp) cw[i * p.nsplit + sp] *= inv;
+    for (int sp = 0; sp < nsp; ++sp) cw[i * nsp + sp] *= inv;
   }
   __syncthreads();
   for (int i = tid; i < QR * (D / 4); i += kThreads) {
@@ -546,14 +550,14 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
     const int m = z + qr / p.gqa, h = qr % p.gqa;
     const float* src = p.o_part + (((size_t)m * p.n_q + kh * p.gqa + h) * p.nsplit) * D + d4;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int s0 = 0; s0 < p.nsplit; s0 += 4) {
+    for (int s0 = 0; s0 < nsp; s0 += 4) {
       float4 v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        v[u] = (s0 + u < p.nsplit) ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)(s0 + u) * D)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        v[u] = (s0 + u < nsp) ? __ldcg(reinterpret_cast<const float4*>(src + (size_t)(s0 + u) * D)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        const float c = (s0 + u < p.nsplit) ? cw[qr * p.nsplit + s0 + u] : 0.f;
+        const float c = (s0 + u < nsp) ? cw[qr * nsp + s0 + u] : 0.f;
         acc.x = fmaf(v[u].x, c, acc.x); acc.y = fmaf(v[u].y, c, acc.y);
         acc.z = fmaf(v[u].z, c, acc.z); acc.w = fmaf(v[u].w, c, acc.w);
       }
@@ -565,11 +569,18 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
   }
 }
 
+__global__ void __launch_bounds__(64) attn_plan_kernel(const AttnPlanParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
+  attn_plan(p);
+}
+
 template <bool I8>
 __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const __grid_constant__ AttnRowsParams p) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ int s_last;
-  const int z = p.one_group ? blockIdx.z * min(kMaxRows, 64 / p.gqa) : blockIdx.z, tid = threadIdx.x;
+  const int tid = threadIdx.x;
+  int z = p.one_group ? blockIdx.z * min(kMaxRows, 64 / p.gqa) : blockIdx.z, split = blockIdx.y, nsp = p.nsplit;
   if (tid == 0) {   // the descriptors are launch parameters: their fetch overlaps the wait for the previous kernel
     prefetch_tmap(&p.k_map);
     prefetch_tmap(&p.v_map);
@@ -579,12 +590,19 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const __grid_con
   // ---- the group: consecutive rows of one request; this CTA is its leader or leaves.  The rows' request
   // ids and positions are read once, in parallel, into shared memory.
   __shared__ int s_req[64], s_pos[64], s_bt[kBtSmem];
+  const int entry = p.plan ? __ldcg(p.plan + 64 + blockIdx.y) : 0;
   if (tid < 64) {
     s_req[tid] = tid < p.M ? p.ctrl[CTRL_ROW_REQ + tid] : -1;
     s_pos[tid] = tid < p.M ? p.ctrl[CTRL_ROW_POS + tid] : 0;
   }
   const bool blk = p.block && tid < p.M && p.ctrl[CTRL_ROW_BLOCK + tid] != 0;
   __syncthreads();
+  if (p.plan) {
+    if (entry < 0) return;
+    z = entry & 255;
+    split = (entry >> 8) & 255;
+    nsp = entry >> 16;
+  }
   const int req = s_req[z];
   int gs = z;
   while (gs > 0 && s_req[gs - 1] == req) --gs;
@@ -603,11 +621,11 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const __grid_con
     __syncthreads();
   }
   if (QR <= 16 && !p.one_slice)
-    attn_rows_body<I8, 4>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z);
+    attn_rows_body<I8, 4>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z, split, nsp);
   else if (QR <= 32 && !p.one_slice)
-    attn_rows_body<I8, 2>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z);
+    attn_rows_body<I8, 2>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z, split, nsp);
   else
-    attn_rows_body<I8, 1>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z);
+    attn_rows_body<I8, 1>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z, split, nsp);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
@@ -664,16 +682,26 @@ int cache_map(CUtensorMap* out, const void* ptr, uint64_t rows, int i8) {
 
 }  // namespace
 
+// Splits by length for b2_attn_rows over the same rows (`ctrl`, M, heads, nsplit the most of a row, window): plan is 64 + entries
+// words, entries >= M of them for what the grid's CTAs stand for.  (A step that starts from its tokens: b2_embed_plan.)
+extern "C" int b2_attn_plan(const int* ctrl, int M, int n_q, int n_kv, int nsplit, int window, int* plan, int entries, void* stream) {
+  AttnPlanParams p;
+  if (!attn_plan_params(p, ctrl, M, n_q, n_kv, nsplit, window, plan, entries)) return -1;
+  return b2_launch(attn_plan_kernel, dim3(1), dim3(64), 0, (cudaStream_t)stream, true, p);
+}
+
 // Rows of a request that follow one another in the control block are served together.  bf16 or int8 KV, head size 128,
 // nsplit <= 64, GQA <= 16.  tickets [M][n_kv] (zeroed once; the kernel leaves them zero): the last split CTA of a
 // group merges in the kernel; nullptr: the partials are left for b2_attn_merge.
+// plan (no fixed spans, no one_group): table of b2_attn_plan for these rows; the merge is b2_attn_merge_counted then.
 extern "C" int b2_attn_rows(const void* q, const void* k_cache, const void* v_cache, const float* k_scale,
                             const float* v_scale, int kv_int8, const int* block_table,
                             const int* ctrl, float* o_part, float* ml_part, void* out, int* tickets, int M, int n_q,
                             int n_kv, int D_, int nsplit, int max_blocks, float scale, int span_pages, int num_pages,
-                            int window, int one_group, void* stream) {
+                            int window, int one_group, const int* plan, int entries, void* stream) {
   if (D_ != D || nsplit < 1 || nsplit > 64 || n_q % n_kv != 0 || n_q / n_kv > 16 || M > 64 || num_pages < 1) return -1;
   if (((uintptr_t)k_cache | (uintptr_t)v_cache) & 15) return -4;
+  if (plan && (entries < M || entries > 65535 || span_pages > 0 || one_group)) return -5;
   AttnRowsParams p;
   p.q = (const __nv_bfloat16*)q; p.k_scale = k_scale; p.v_scale = v_scale;
   const uint64_t cache_rows = (uint64_t)num_pages * n_kv * 16;
@@ -685,6 +713,7 @@ extern "C" int b2_attn_rows(const void* q, const void* k_cache, const void* v_ca
   p.tickets = tickets; p.M = M; p.n_q = n_q; p.n_kv = n_kv; p.gqa = n_q / n_kv; p.nsplit = nsplit; p.max_blocks = max_blocks;
   p.scale_log2 = scale * 1.4426950408889634f;
   p.span_pages = span_pages;
+  p.plan = plan;
   p.window = window > 0 ? window : 0;
   p.block = window == -1 ? 1 : 0;          // window -1: rows flagged in the control block are non-causal block rows
   p.one_slice = span_pages > 0 ? 1 : 0;   // fixed spans promise bits that do not depend on the group
@@ -710,9 +739,10 @@ extern "C" int b2_attn_rows(const void* q, const void* k_cache, const void* v_ca
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = 1;
   }
+  const dim3 grid = plan ? dim3(n_kv, entries, 1) : dim3(n_kv, nsplit, gz);
   if (kv_int8)
-    return b2_launch(attn_rows_kernel<true>, dim3(n_kv, nsplit, gz), dim3(kThreads), smem, (cudaStream_t)stream, true, p);
-  return b2_launch(attn_rows_kernel<false>, dim3(n_kv, nsplit, gz), dim3(kThreads), smem, (cudaStream_t)stream, true, p);
+    return b2_launch(attn_rows_kernel<true>, grid, dim3(kThreads), smem, (cudaStream_t)stream, true, p);
+  return b2_launch(attn_rows_kernel<false>, grid, dim3(kThreads), smem, (cudaStream_t)stream, true, p);
 }
 
 B2_DEFINE_STATUS(attnrows)

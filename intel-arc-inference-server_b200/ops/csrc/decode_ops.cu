@@ -12,6 +12,7 @@
 // attn_v2.cl, gemv_bf16.cl, gemv_i8w.cl and argmax.cl.  All of them read the row
 // table of the device-resident control block, so a captured CUDA graph replays
 // without host writes (the reference's central idea: docs/04-architecture.md:214-228).
+#include "attn_plan.cuh"
 #include "common.cuh"
 
 using namespace b2;
@@ -44,13 +45,18 @@ struct ResidNormParams {
   int* flag;
 };
 
+struct EmbedPlanParams {     // a step's start: ResidNormParams of mode 0, and CTAs behind the rows' that plan its attention
+  ResidNormParams r;
+  AttnPlanParams plan;
+  int window;                // of a second table, for windowed layers
+  int* plan_win;
+};
+
 // blockDim = H/8 rounded up to a warp (at most 1024): each thread owns 8 consecutive elements per
 // pass, and the S slice loads of a pass are independent, so they are all in flight together.
-__global__ void __launch_bounds__(1024) resid_norm_kernel(const ResidNormParams p) {
+__device__ __forceinline__ void resid_norm_row(const ResidNormParams& p) {
   extern __shared__ float vals[];
   __shared__ float red[32];
-  pdl_wait();
-  pdl_launch_dependents();
   const int m = blockIdx.x, tid = threadIdx.x, nthr = blockDim.x;
   const int H8 = p.H >> 3;
   float ss = 0.f;
@@ -109,6 +115,27 @@ __global__ void __launch_bounds__(1024) resid_norm_kernel(const ResidNormParams 
       reinterpret_cast<uint4*>(p.x_out + (size_t)m * p.H)[i] = o;
     }
   }
+}
+
+__global__ void __launch_bounds__(1024) resid_norm_kernel(const ResidNormParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
+  resid_norm_row(p);
+}
+
+__global__ void __launch_bounds__(1024) embed_plan_kernel(const EmbedPlanParams p) {
+  pdl_wait();
+  pdl_launch_dependents();
+  if (blockIdx.x < p.plan.M) {
+    resid_norm_row(p.r);
+    return;
+  }
+  AttnPlanParams a = p.plan;
+  if (blockIdx.x > p.plan.M) {
+    a.window = p.window;
+    a.plan = p.plan_win;
+  }
+  attn_plan(a);
 }
 
 // Norm of a prompt's rows (no partials to fold): a warp per row, the row in registers, its loads all in flight, no barrier
@@ -597,9 +624,11 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(const AttnDecParams p)
 // grid (n_q, M), D threads.  xq != nullptr (D = 128): the head's 128 outputs, as rounded to bf16, also leave as the two
 // quantised 64-k groups the o projection's integer GEMV reads (the work of quant_x_kernel on this row slice, same
 // bits), which saves that launch in a step of several rows; without xq_gs, as the bf16 rows of the tcgen05 form
-// (stage_rows_kernel, gs_rows token rows per group).
+// (stage_rows_kernel, gs_rows token rows per group).  counts: [M] splits that a row has of the nsplit (<= 64) places, or nullptr:
+// all of them.
+template <int V>
 __global__ void attn_merge_kernel(const float* o_part, const float* ml_part, __nv_bfloat16* out, int n_q, int nsplit,
-                                  int D, uint8_t* xq, uint32_t* xq_gs, int gs_rows) {
+                                  int D, uint8_t* xq, uint32_t* xq_gs, int gs_rows, const int* counts) {
   __shared__ float cw[64];
   __shared__ __align__(16) __nv_bfloat16 srow[128];
   pdl_wait();
@@ -608,31 +637,47 @@ __global__ void attn_merge_kernel(const float* o_part, const float* ml_part, __n
   const size_t base = ((size_t)m * n_q + h) * nsplit;
   float merged;
   if (nsplit <= 64) {
-    // weights of the splits once per CTA (one lane per split), then every thread's loads are independent
+    // weights of the splits once per CTA (one lane per split), then every thread's loads are independent.  The first 32 splits'
+    // values are requested before the weights are known: one round trip for both; of places that may not be a row's, eight
+    const int n = counts ? counts[m] : nsplit, sure = counts ? min(nsplit, 8) : nsplit;
+    const float* src = o_part + base * D + d;
+    float v0[V];
+#pragma unroll
+    for (int u = 0; u < V; ++u) v0[u] = u < sure ? src[(size_t)u * D] : 0.f;
+    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
     if (d < 32) {
-      float m0 = d < nsplit ? ml_part[(base + d) * 2] : -INFINITY, m1 = d + 32 < nsplit ? ml_part[(base + d + 32) * 2] : -INFINITY;
+      if (d < nsplit) m0 = ml_part[(base + d) * 2], l0 = ml_part[(base + d) * 2 + 1];
+      if (d + 32 < nsplit) m1 = ml_part[(base + d + 32) * 2], l1 = ml_part[(base + d + 32) * 2 + 1];
+    }
+    if (counts) {
+#pragma unroll
+      for (int u = 0; u < V; ++u) {
+        if (u >= n) v0[u] = 0.f;
+        else if (u >= 8) v0[u] = src[(size_t)u * D];
+      }
+      if (d >= n) m0 = -INFINITY;
+      if (d + 32 >= n) m1 = -INFINITY;
+    }
+    if (d < 32) {
       const float mm = warp_max(fmaxf(m0, m1));
       const float c0 = m0 == -INFINITY ? 0.f : exp2f(m0 - mm), c1 = m1 == -INFINITY ? 0.f : exp2f(m1 - mm);
-      float l = (d < nsplit ? ml_part[(base + d) * 2 + 1] * c0 : 0.f) + (d + 32 < nsplit ? ml_part[(base + d + 32) * 2 + 1] * c1 : 0.f);
+      float l = (d < n ? l0 * c0 : 0.f) + (d + 32 < n ? l1 * c1 : 0.f);
       // a fixed-shape tree over the lanes: the same bits on every run
       l = warp_sum(l);
       const float inv = l > 0.f ? 1.f / l : 0.f;
       cw[d] = c0 * inv;
       cw[d + 32] = c1 * inv;
     }
-    // the first 32 splits' values are requested before the weights are known: one round trip for both
-    float v0[32];
-#pragma unroll
-    for (int u = 0; u < 32; ++u) v0[u] = u < nsplit ? o_part[(base + u) * D + d] : 0.f;
     __syncthreads();
     float o = 0.f;
 #pragma unroll
-    for (int u = 0; u < 32; ++u) o = fmaf(v0[u], u < nsplit ? cw[u] : 0.f, o);
-    if (nsplit > 32) {
+    for (int u = 0; u < V; ++u) o = fmaf(v0[u], u < n ? cw[u] : 0.f, o);
+#pragma unroll 1
+    for (int s0 = V; s0 < n; s0 += V) {
 #pragma unroll
-      for (int u = 0; u < 32; ++u) v0[u] = 32 + u < nsplit ? o_part[(base + 32 + u) * D + d] : 0.f;
+      for (int u = 0; u < V; ++u) v0[u] = s0 + u < n ? src[(size_t)(s0 + u) * D] : 0.f;
 #pragma unroll
-      for (int u = 0; u < 32; ++u) o = fmaf(v0[u], 32 + u < nsplit ? cw[32 + u] : 0.f, o);
+      for (int u = 0; u < V; ++u) o = fmaf(v0[u], s0 + u < n ? cw[s0 + u] : 0.f, o);
     }
     merged = o;
   } else {
@@ -1124,6 +1169,20 @@ extern "C" int b2_resid_norm(const void* embed, const int* ctrl, const void* res
   return b2_launch(resid_norm_kernel, dim3(M), dim3(threads), (size_t)H * 4, (cudaStream_t)stream, true, p);
 }
 
+// A step's start: the rows' embeddings (mode 0 of b2_resid_norm) and, in CTAs beside them, the splits of its attention
+// (b2_attn_plan; plan_win: the same for windowed layers, or nullptr).
+extern "C" int b2_embed_plan(const void* embed, const int* ctrl, int M, int H, int vocab, const float* w, float eps, void* resid_out,
+                             void* x_out, int* flag, int n_q, int n_kv, int nsplit, int entries, int* plan, int window, int* plan_win,
+                             void* stream) {
+  EmbedPlanParams p = {};
+  p.r.embed = (const __nv_bfloat16*)embed; p.r.ctrl = ctrl; p.r.H = H; p.r.vocab = vocab; p.r.w = w; p.r.eps = eps;
+  p.r.resid_out = (__nv_bfloat16*)resid_out; p.r.x_out = (__nv_bfloat16*)x_out; p.r.flag = flag;
+  p.window = window; p.plan_win = plan_win;
+  if (H % 8 || (plan_win && window < 1) || !attn_plan_params(p.plan, ctrl, M, n_q, n_kv, nsplit, 0, plan, entries)) return -1;
+  const int threads = min(1024, max(64, (H / 8 + 31) / 32 * 32));
+  return b2_launch(embed_plan_kernel, dim3(M + (plan_win ? 2 : 1)), dim3(threads), (size_t)H * 4, (cudaStream_t)stream, true, p);
+}
+
 extern "C" int b2_draft_front(const void* embed, const int* ctrl, int vocab, const void* hidden, long long hidden_ld,
                               const float* w_e, const float* w_h, float eps, int M, int H, void* xcat, int* flag,
                               void* stream) {
@@ -1165,6 +1224,15 @@ static int attn_decode_dispatch(int gqa, const AttnDecParams& p, dim3 grid, cuda
   return -3;
 }
 
+// Few rows of many splits: all values of 32 splits in flight.  Rows enough to fill the GPU, or few splits: 16 at a time leave room for
+// twice the CTAs (121 / 56 registers).  Attention and merge of 5 rows of 40 heads in 37 splits 16.9 -> 14.1 us, whose values were asked for
+// behind the weights before; of 64 rows in 2 splits 37.9 -> 34.2.
+static int merge_launch(const float* o_part, const float* ml_part, void* out, int M, int n_q, int nsplit, int D, void* xq, void* xq_gs,
+                        int gs_rows, const int* counts, cudaStream_t st) {
+  return b2_launch(counts || nsplit <= 16 ? attn_merge_kernel<16> : attn_merge_kernel<32>, dim3(n_q, M), dim3(D), 0, st, true, o_part, ml_part,
+                   (__nv_bfloat16*)out, n_q, nsplit, D, (uint8_t*)xq, (uint32_t*)xq_gs, gs_rows, counts);
+}
+
 extern "C" int b2_attn_decode(const void* q, const void* k_cache, const void* v_cache, const float* k_scale,
                               const float* v_scale, const int* block_table, const int* ctrl, float* o_part,
                               float* ml_part, void* out, int M, int n_q, int n_kv, int D, int nsplit, int max_blocks,
@@ -1182,8 +1250,7 @@ extern "C" int b2_attn_decode(const void* q, const void* k_cache, const void* v_
   else if (D == 64) rc = attn_decode_dispatch<64>(n_q / n_kv, p, grid, st);
   else return -2;
   if (rc || tickets) return rc;
-  return b2_launch(attn_merge_kernel, dim3(n_q, M), dim3(D), 0, st, true, (const float*)o_part, (const float*)ml_part,
-                   (__nv_bfloat16*)out, n_q, nsplit, D, (uint8_t*)nullptr, (uint32_t*)nullptr, 0);
+  return merge_launch(o_part, ml_part, out, M, n_q, nsplit, D, nullptr, nullptr, 0, nullptr, st);
 }
 
 extern "C" int b2_kv_convert(void* k16, void* v16, const int* table16, void* k8, void* v8, float* ks, float* vs,
@@ -1199,8 +1266,7 @@ extern "C" int b2_kv_convert(void* k16, void* v16, const int* table16, void* k8,
 // Merge of split-KV partials as its own launch (one CTA per row and query head).
 extern "C" int b2_attn_merge(const float* o_part, const float* ml_part, void* out, int M, int n_q, int nsplit, int D,
                              void* stream) {
-  return b2_launch(attn_merge_kernel, dim3(n_q, M), dim3(D), 0, (cudaStream_t)stream, true, o_part, ml_part,
-                   (__nv_bfloat16*)out, n_q, nsplit, D, (uint8_t*)nullptr, (uint32_t*)nullptr, 0);
+  return merge_launch(o_part, ml_part, out, M, n_q, nsplit, D, nullptr, nullptr, 0, nullptr, (cudaStream_t)stream);
 }
 
 // The merge that also writes the rows' quantised form for the o projection (head size 128; xq [M][n_q * 2][128 B],
@@ -1209,8 +1275,14 @@ extern "C" int b2_attn_merge(const float* o_part, const float* ml_part, void* ou
 extern "C" int b2_attn_merge_quant(const float* o_part, const float* ml_part, void* out, int M, int n_q, int nsplit, int D,
                                    void* xq, void* xq_gs, int gs_rows, void* stream) {
   if (D != 128 || !xq || gs_rows < M) return -1;
-  return b2_launch(attn_merge_kernel, dim3(n_q, M), dim3(D), 0, (cudaStream_t)stream, true, o_part, ml_part,
-                   (__nv_bfloat16*)out, n_q, nsplit, D, (uint8_t*)xq, (uint32_t*)xq_gs, gs_rows);
+  return merge_launch(o_part, ml_part, out, M, n_q, nsplit, D, xq, xq_gs, gs_rows, nullptr, (cudaStream_t)stream);
+}
+
+// Either merge of rows that have counts[m] of the nsplit <= 64 places (b2_attn_rows with a budget); xq nullptr: plain rows only.
+extern "C" int b2_attn_merge_counted(const float* o_part, const float* ml_part, void* out, int M, int n_q, int nsplit, int D,
+                                     const int* counts, void* xq, void* xq_gs, int gs_rows, void* stream) {
+  if (D != 128 || nsplit < 1 || nsplit > 64 || !counts || (xq && gs_rows < M)) return -1;
+  return merge_launch(o_part, ml_part, out, M, n_q, nsplit, D, xq, xq_gs, gs_rows, counts, (cudaStream_t)stream);
 }
 
 template <int MT>
@@ -1338,8 +1410,7 @@ extern "C" int b2_attn_decode_static(const void* q, const void* k_cache, const v
   if (D == 128) rc = attn_decode_dispatch<128>(n_q / n_kv, p, grid, st);
   else rc = attn_decode_dispatch<64>(n_q / n_kv, p, grid, st);
   if (rc) return rc;
-  return b2_launch(attn_merge_kernel, dim3(n_q, M), dim3(D), 0, st, true, (const float*)o_part, (const float*)ml_part,
-                   (__nv_bfloat16*)out, n_q, nsplit, D, (uint8_t*)nullptr, (uint32_t*)nullptr, 0);
+  return merge_launch(o_part, ml_part, out, M, n_q, nsplit, D, nullptr, nullptr, 0, nullptr, st);
 }
 
 B2_DEFINE_STATUS(decode)

@@ -302,9 +302,37 @@ def attn_decode(q, k_cache, v_cache, block_table, ctrl, o_part, ml_part, out, m,
     _check(rc, "attn_decode")
 
 
+def attn_plan_entries(m: int, n_kv: int) -> int:
+    """KV splits over all rows that a planned attention launch of ``m`` rows has room for: two waves of CTAs, or one beside a split of
+    each row."""
+    wave = -(-296 // n_kv)
+    return max(2 * wave, m + wave)
+
+
+def attn_plan_words(max_rows: int, n_kv: int) -> int:
+    return 64 + attn_plan_entries(max_rows, n_kv)
+
+
+def attn_plan(ctrl, m, n_q, n_kv, nsplit, plan, window: int = 0):
+    """KV splits of ``m`` rows of several requests by their lengths, at most ``nsplit`` of a row, into ``plan`` (int32,
+    ``attn_plan_words``) for ``attn_rows``."""
+    if plan.numel() < attn_plan_words(m, n_kv):
+        raise ValueError(f"attn_plan: the table is too small for {m} rows")
+    _check(lib().b2_attn_plan(_p(ctrl), m, n_q, n_kv, nsplit, window, _p(plan), attn_plan_entries(m, n_kv), _stream()), "attn_plan")
+
+
+def embed_plan(m, h, w, eps, resid_out, x_out, embed, ctrl, vocab, flag, n_q, n_kv, nsplit, plan, window: int = 0, plan_win=None):
+    """``resid_norm`` from the embedding and, in the same launch, ``attn_plan`` of the rows (``plan_win``: of windowed layers too)."""
+    if min(t.numel() for t in (plan, plan if plan_win is None else plan_win)) < attn_plan_words(m, n_kv):
+        raise ValueError(f"embed_plan: the table is too small for {m} rows")
+    rc = lib().b2_embed_plan(_p(embed), _p(ctrl), m, h, vocab, _p(w), ctypes.c_float(eps), _p(resid_out), _p(x_out), _p(flag), n_q, n_kv,
+                             nsplit, attn_plan_entries(m, n_kv), _p(plan), window, _p(plan_win), _stream())
+    _check(rc, "embed_plan")
+
+
 def attn_rows(q, k_cache, v_cache, block_table, ctrl, o_part, ml_part, out, tickets, m, n_q, n_kv, d, nsplit,
               max_blocks, scale, span_pages: int = 0, k_scale=None, v_scale=None, kv_int8: bool = False, window: int = 0,
-              one_request: bool = False, xq=None, xq_gs=None):
+              one_request: bool = False, xq=None, xq_gs=None, plan=None):
     """Decode / verify attention that serves consecutive rows of one request together on the tensor cores
     (bf16 or int8 KV, head size 128); same split-KV partial buffers and in-kernel merge as ``attn_decode``.
     ``window`` > 0: every row attends to its last ``window`` positions only; ``window`` = -1: the rows are a block whose
@@ -312,14 +340,18 @@ def attn_rows(q, k_cache, v_cache, block_table, ctrl, o_part, ml_part, out, tick
     ``one_request``: the caller knows that all ``m`` rows are one request's, at consecutive positions; the launch then
     has one CTA column per group of rows instead of one per row (most of which would leave at once).
     ``xq`` / ``xq_gs`` (with ``tickets=None``): the merge also writes the rows in the quantised form of ``quant_x`` for
-    K = n_q * d, so that the o projection's GEMV can read them without that launch; ``xq`` alone: in the form of ``stage_rows``."""
+    K = n_q * d, so that the o projection's GEMV can read them without that launch; ``xq`` alone: in the form of ``stage_rows``.
+    ``plan`` (neither ``span_pages`` nor ``one_request``): table of ``attn_plan`` for these rows, ``nsplit`` and window."""
     rc = lib().b2_attn_rows(_p(q), _p(k_cache), _p(v_cache), _p(k_scale), _p(v_scale), 1 if kv_int8 else 0,
                             _p(block_table), _p(ctrl), _p(o_part), _p(ml_part),
                             _p(out), _p(tickets), m, n_q, n_kv, d, nsplit, max_blocks, ctypes.c_float(scale), span_pages,
-                            k_cache.numel() // (n_kv * 16 * d), window, 1 if one_request else 0, _stream())
+                            k_cache.numel() // (n_kv * 16 * d), window, 1 if one_request else 0, _p(plan), attn_plan_entries(m, n_kv), _stream())
     _check(rc, "attn_rows")
     if tickets is None:     # many rows: the merge is its own launch, one CTA per row and head
-        if xq is not None:
+        if plan is not None:
+            rc = lib().b2_attn_merge_counted(_p(o_part), _p(ml_part), _p(out), m, n_q, nsplit, d, _p(plan), _p(xq), _p(xq_gs),
+                                             quant_slots(m) if xq_gs is not None else rows_pad(m), _stream())
+        elif xq is not None:
             rc = lib().b2_attn_merge_quant(_p(o_part), _p(ml_part), _p(out), m, n_q, nsplit, d, _p(xq), _p(xq_gs),
                                            quant_slots(m) if xq_gs is not None else rows_pad(m), _stream())
         else:

@@ -105,6 +105,26 @@ def test_attention_split_rule_and_quantiser_slots():
     assert [quant_slots(m) for m in (1, 8, 9, 16, 17, 33, 64)] == [8, 8, 16, 16, 32, 64, 64]
 
 
+def test_splits_of_a_step():
+    """One request's rows get equal splits, counted by the groups that share a CTA; rows of several are planned on the device, with
+    room for one split of each row and a wave of CTAs beside."""
+    from types import SimpleNamespace
+    from b200serve.models.decoder import DecoderModel
+    from b200serve.ops.lib import attn_plan_entries, attn_plan_words
+
+    def splits(m, kv_heads=8, gqa=5, most=37, fixed=False):
+        cfg = SimpleNamespace(n_kv_heads=kv_heads, gqa=gqa)
+        return DecoderModel._attn_splits(SimpleNamespace(cfg=cfg, nsplit_attn=most, attn_fixed_spans=fixed), m)
+    assert splits(1) == splits(5) == splits(16) == 37 and splits(64) == 10          # 8 groups: ceil(592 / 64)
+    assert splits(64, gqa=16) == 5                                                  # groups of four rows
+    assert splits(64, kv_heads=64, fixed=True) == 37 and splits(64, kv_heads=64) == 2
+    assert attn_plan_entries(2, 8) == 74 and attn_plan_entries(40, 8) == 77 and attn_plan_entries(64, 64) == 69
+    for kv in (1, 2, 3, 8, 16, 64):
+        assert all(m <= attn_plan_entries(m, kv) <= attn_plan_words(64, kv) - 64 for m in range(1, 65))
+
+
+
+
 def test_quant_x_refuses_buffers_that_are_too_small():
     """The binding checks the sizes before the kernel runs: 3 rows still need 8 token slots per 64-k group."""
     import pytest

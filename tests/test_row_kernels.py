@@ -305,3 +305,118 @@ def test_attention_on_int8_cache(ctx, nq, nkv, rows, window, splits):
             ds = 2.0 ** -8 * torch.einsum("hgd,khd->hgk", qq.abs(), kk.abs()).amax(-1, keepdim=True) * d ** -0.5
             bound = bound + (2.0 ** -8 + 2 * ds) * size
         assert ((out[i].double().view(nkv, gqa, d) - want).abs() <= bound + 1e-9).all()
+
+
+def _shares(spec, gqa, nkv, most, window):
+    """Splits of every row: groups of up to eight consecutive rows of a request, by the pages each reads; of all spans that give the
+    longest group 1, 2, .. splits the one whose longest piece, or waves of 296 CTAs times the mean piece, takes least."""
+    rmax, groups, i = min(8, 64 // gqa), [], 0
+    while i < len(spec):
+        j = i
+        while j < len(spec) and spec[j][0] == spec[i][0] and j - i < rmax:
+            j += 1
+        last, first = max(p for _, p in spec[i:j]), spec[i][1]
+        groups.append((j - i, max(1, last // 16 + 1 - (max(0, first + 1 - window) // 16 if window else 0))))
+        i = j
+    pages, best = [p for _, p in groups], None
+    for k in range(1, min(most, max(pages)) + 1):
+        span = -(-max(pages) // k)
+        n = [min(most, -(-p // span)) for p in pages]
+        if sum(n) <= K.attn_plan_entries(len(spec), nkv):
+            t = max(8 + max(-(-p // c) for p, c in zip(pages, n)), -(-sum(n) * nkv // 296) * (8 - (-sum(pages) // sum(n))))
+            if best is None or t < best[0]:
+                best = (t, n)
+    return [c for (r, _), c in zip(groups, best[1]) for _ in range(r)]
+
+
+# one long context among short ones, the most splits a row may have, several rows of some requests, groups at the 32nd row and behind,
+# lone pages, one split of everything, more heads than slots of a wave, a window
+@pytest.mark.parametrize("spec,nq,nkv,most,window", [
+    ([(i, 40 + 3 * i) for i in range(7)] + [(7, 2900)], 5, 1, 37, 0), ([(0, 2900)] + [(i, 15) for i in range(1, 33)], 4, 2, 16, 0),
+    ([(3, p) for p in range(500, 560)] + [(i, 1800 + i) for i in (0, 1, 2, 4)], 10, 2, 64, 0), ([(i, 200 - 3 * i) for i in range(64)], 8, 4, 8, 0),
+    ([(i // 3, 100 * (i // 3) + i % 3) for i in range(60)], 16, 1, 12, 0), ([(0, 0), (1, 16)], 2, 2, 37, 0), ([(i, 50 * i) for i in range(9)], 2, 1, 1, 0),
+    ([(i, 700) for i in range(33)] + [(i, 5) for i in range(33, 64)], 16, 16, 18, 0), ([(0, 2000), (1, 90), (2, 700), (2, 701), (2, 702)], 6, 2, 9, 100)])
+@pytest.mark.parametrize("kv", ["bf16", "int8"])
+def test_attention_splits_by_length(spec, nq, nkv, most, window, kv):
+    torch.manual_seed(len(spec) + most)
+    d, gqa, dev, m = 128, nq // nkv, "cuda", len(spec)
+    seqs, blocks = 1 + max(r for r, _ in spec), max(p for _, p in spec) // 16 + 2
+    pages = seqs * blocks
+    table = (torch.randperm(pages, device=dev) + 1).int().view(seqs, blocks).contiguous()
+    if kv == "int8":
+        k, v = (torch.randint(-127, 128, (pages + 1, nkv, 16, d), dtype=torch.int8, device=dev) for _ in range(2))
+        ks, vs = (torch.rand(pages + 1, nkv, 16, device=dev) * 0.03 for _ in range(2))
+    else:
+        k, v = (torch.randn(pages + 1, nkv, 16, d, device=dev).bfloat16() for _ in range(2))
+        ks = vs = None
+    q = torch.randn(m, nq * d, device=dev).bfloat16()
+    ctrl = _ctrl([r for r, _ in spec])
+    ctrl[K.CTRL_ROW_POS: K.CTRL_ROW_POS + m] = torch.tensor([p for _, p in spec], dtype=torch.int32, device=dev)
+    plan = torch.full((K.attn_plan_words(m, nkv),), 1 << 20, dtype=torch.int32, device=dev)
+    K.attn_plan(ctrl, m, nq, nkv, most, plan, window=window)
+    want = _shares(spec, gqa, nkv, most, window)
+    assert plan[:m].tolist() == want
+    entries = [(e & 255, e >> 8 & 255, e >> 16) for e in plan[64:].tolist() if e >= 0]
+    lead = [i for i in range(m) if i == 0 or spec[i][0] != spec[i - 1][0] or (i - next(j for j in range(m) if spec[j][0] == spec[i][0])) % min(8, 64 // gqa) == 0]
+    assert sorted(entries) == [(i, c, want[i]) for i in lead for c in range(want[i])]
+    kw = dict(k_scale=ks, v_scale=vs, kv_int8=kv == "int8", window=window)
+    pad, kq = K.rows_pad(m), nq * d
+    rows, quant = torch.zeros(pad * kq * 2, dtype=torch.uint8, device=dev), torch.zeros(m * kq * 2, dtype=torch.uint8, device=dev)
+    gs = torch.zeros(K.quant_slots(m) * kq // 64 * 2, dtype=torch.int32, device=dev)
+    outs, tickets = [], torch.zeros(m * nkv, dtype=torch.int32, device=dev)
+    for extra in ({}, {"xq": rows}, {"xq": quant, "xq_gs": gs}, None):         # None: the last split's CTA merges
+        merge, extra = (tickets, {}) if extra is None else (None, extra)
+        part, ml = torch.full((m * nq * most * d,), float("nan"), device=dev), torch.full((m * nq * most * 2,), float("nan"), device=dev)
+        out = torch.full((m, kq), float("nan"), dtype=torch.bfloat16, device=dev)
+        K.attn_rows(q, k, v, table, ctrl, part, ml, out, merge, m, nq, nkv, d, most, blocks, d ** -0.5, plan=plan, **kw, **extra)
+        torch.cuda.synchronize()
+        K.check_status()
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2]) and int(tickets.abs().sum()) == 0
+    again, gs2 = torch.zeros_like(rows), torch.zeros_like(gs)         # the rows as their own launches make them
+    K.stage_rows(outs[0], m, kq, again)
+    live = [t.view(kq // 64, pad, 128)[:, :m] for t in (rows, again)]
+    assert torch.equal(*live)
+    again = torch.zeros_like(quant)
+    K.quant_x(outs[0], m, kq, again, gs2)
+    assert torch.equal(quant, again) and torch.equal(gs, gs2)
+    if not window and max(want) == 1:      # nothing is cut: the even form with one split
+        even = torch.empty_like(outs[0])
+        K.attn_rows(q, k, v, table, ctrl, part, ml, even, None, m, nq, nkv, d, 1, blocks, d ** -0.5, **kw)
+        assert torch.equal(even, outs[0])
+    for i, (req, pos) in enumerate(spec):
+        at = torch.arange(max(0, pos + 1 - window) if window else 0, pos + 1, device=dev)
+        pg = table[req].long()[at // 16]
+        kk, vv = (c[pg, :, at % 16].double() * (1 if s is None else s[pg, :, at % 16].double()[..., None]) for c, s in ((k, ks), (v, vs)))
+        qq = q[i].double().view(nkv, gqa, d)
+        p = (torch.einsum("hgd,khd->hgk", qq, kk) * d ** -0.5).softmax(-1)
+        want, size = torch.einsum("hgk,khd->hgd", p, vv), torch.einsum("hgk,khd->hgd", p, vv.abs())
+        # probabilities (times an int8 V's scale) and the result are rounded to bf16: 2^-8 of the value each, and a little for fp32 sums.
+        # Groups above 32 query rows round an int8 cache's K and V too: 2^-8 of V, and of every product of a score
+        bound = 1.05 * 2.0 ** -7 * size
+        if kv == "int8" and min(8, 64 // gqa, sum(r == req for r, _ in spec)) * gqa > 32:
+            ds = 2.0 ** -8 * torch.einsum("hgd,khd->hgk", qq.abs(), kk.abs()).amax(-1, keepdim=True) * d ** -0.5
+            bound = bound + (2.0 ** -8 + 2 * ds) * size
+        for got in (outs[0], outs[3]):
+            assert ((got[i].double().view(nkv, gqa, d) - want).abs() <= bound + 1e-9).all()
+
+
+@pytest.mark.parametrize("m,h,window", [(2, 64, 0), (17, 512, 0), (64, 5120, 300), (5, 9000, 64)])
+def test_plan_beside_the_embedding(m, h, window):
+    """One launch with the rows and the tables of the launches it stands for."""
+    torch.manual_seed(m)
+    nq, nkv, most, vocab = 10, 2, 37, 50
+    ctrl = _ctrl([i // 2 for i in range(m)])
+    ctrl[K.CTRL_ROW_POS: K.CTRL_ROW_POS + m] = torch.randint(0, 30000, (m,), dtype=torch.int32, device="cuda")
+    ctrl[K.CTRL_CUR_TOKEN: K.CTRL_CUR_TOKEN + m] = torch.randint(0, vocab, (m,), dtype=torch.int32, device="cuda")
+    embed, w, flag = torch.randn(vocab, h, device="cuda").bfloat16(), 1 + 0.1 * torch.randn(h, device="cuda"), torch.zeros(4, dtype=torch.int32, device="cuda")
+    r0, x0, r1, x1 = (torch.full((m, h), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4))
+    p0, w0, p1, w1 = (torch.full((K.attn_plan_words(m, nkv),), 7, dtype=torch.int32, device="cuda") for _ in range(4))
+    K.resid_norm(0, m, h, w, 1e-6, r0, x0, embed=embed, ctrl=ctrl, vocab=vocab, flag=flag)
+    K.attn_plan(ctrl, m, nq, nkv, most, p0)
+    K.attn_plan(ctrl, m, nq, nkv, most, w0, window=max(1, window))
+    K.embed_plan(m, h, w, 1e-6, r1, x1, embed, ctrl, vocab, flag, nq, nkv, most, p1, window=window, plan_win=w1 if window else None)
+    torch.cuda.synchronize()
+    rows = 64 + K.attn_plan_entries(m, nkv)
+    assert torch.equal(r0, r1) and torch.equal(x0, x1) and torch.equal(p0[64:rows], p1[64:rows]) and torch.equal(p0[:m], p1[:m])
+    assert (torch.equal(w0[64:rows], w1[64:rows]) and torch.equal(w0[:m], w1[:m])) if window else (w1 == 7).all()
