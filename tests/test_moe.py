@@ -122,7 +122,7 @@ def test_tiny_moe_rows_path_matches_oracle():
     _teacher_forced(oracle, prompt, toks, 0.03)
 
 
-@pytest.mark.parametrize("backend", ["bf16", "bf16-resident"])
+@pytest.mark.parametrize("backend", ["bf16", "bf16-resident", "w4"])
 def test_small_moe_prompt_path_matches_oracle(backend):
     from b200serve.ops import lib as K
     from b200serve.runtime.engine import Engine

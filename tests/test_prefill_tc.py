@@ -50,7 +50,7 @@ def test_attn_prefill_matches_softmax(c, pos0, n_q, n_kv, window):
     assert (got - ref).abs().max() < 0.02 * ref.abs().max() + 2e-3
 
 
-@pytest.mark.parametrize("backend", ["bf16", "bf16-resident", "int8", "bf16-windowed", "bf16-hybrid", "int8-hybrid"])
+@pytest.mark.parametrize("backend", ["bf16", "bf16-resident", "int8", "w4", "bf16-windowed", "bf16-hybrid", "int8-hybrid", "w4-hybrid"])
 def test_prefill_runner_matches_oracle(backend):
     from b200serve.runtime.engine import Engine
     from b200serve.ops import lib as K
@@ -90,6 +90,31 @@ def test_prefill_runner_matches_oracle(backend):
         if t != want:
             assert float(logits[want] - logits[t]) < margin, (i, t, want)
         logits = oracle.forward(torch.tensor([t]), kv, len(prompt) + i)[0]
+
+
+# chunks at and around the row count up to which the GEMM expands the int4 blocks itself: whole prompts on either side, prompts whose
+# last chunk falls to the other side, a chunk of one row; matrices of different sizes in turn through the workspace
+@pytest.mark.gpu
+@pytest.mark.parametrize("family", ["small-dense", "small-hybrid", "small-moe"])
+@pytest.mark.parametrize("n,chunk", [(128, 128), (129, 256), (129, 128), (300, 256), (300, 128)])
+def test_int4_prompt_backend_has_the_bits_of_bf16(family, n, chunk):
+    from b200serve.models.config import preset
+    from b200serve.ops import lib as K
+    from b200serve.runtime.engine import Engine
+    from b200serve.runtime.prefill import W4_FUSED_ROWS
+    assert W4_FUSED_ROWS == 128
+    cfg = preset(family)
+    prompt = torch.randint(0, cfg.vocab, (n,), generator=torch.Generator().manual_seed(n)).tolist()
+    got = []
+    for backend in ("bf16", "w4", "w4a16"):
+        eng = Engine(random_weights(cfg, device="cuda", seed=3), max_seqs=2, max_len=1024, prefill_backend=backend, nsplit_attn=4)
+        first = eng.prefill(1, prompt, chunk=chunk)
+        K.check_status()
+        assert eng._prefill.backend == ("bf16" if backend == "bf16" else "w4")
+        assert (eng._prefill._slab is None) == (backend != "bf16" and min(n, chunk) <= W4_FUSED_ROWS)
+        got.append((first, eng.logits(1)[0].clone(), {k: t.clone() for k, t in {**eng.kv.page_tensors(), **eng.kv.states}.items()}))
+    for g in got[1:]:
+        assert g[0] == got[0][0] and torch.equal(g[1], got[0][1]) and all(torch.equal(t, got[0][2][k]) for k, t in g[2].items())
 
 
 @pytest.mark.gpu
