@@ -143,11 +143,24 @@ class _PrefillScratch:
         self.slab_gu = self.slab_dn = None
 
 
-# Prompt chunks of up to this many rows per expert read the experts' int4 blocks whatever the backend: with less than a tile of
+# Prompt chunks of up to this many rows per expert read the experts' int4 blocks where that is a choice: with less than a tile of
 # rows an expert is bound by its bytes.  256 experts, 8 per row, 16 layers, bf16 copies / int4 blocks: 300 rows 8.4 / 7.1 ms, 1400 10.0 /
 # 8.6, 2048 10.8 / 9.4, 3000 (94 rows an expert) 12.7 / 11.2; 4000 (125) 15.6 / 15.5, and from a whole tile on the copies cost
 # no more than expanding the blocks for each further tile.
 W4_EXPERT_ROWS = 112
+# Copies that are resident already are the better form while the experts' tiles (one of 128 rows x 256 columns each) are few: a
+# wave of tiles is bound by the chain of one tile, which expanding makes longer, not by bytes.  4 layers of hidden 2048, copies / int4 blocks:
+# 8 experts of 2048 (128 tiles) 200 rows 909 / 937 us, 448 rows 942 / 993; 32 of 768 (192) 200 rows 971 / 1019, 896 1128 / 1171; 64 of 512 (256)
+# 200 rows 1063 / 1062, 597 1154 / 1156; 64 of 1408 (704) 200 rows 1577 / 1520, 896 1762 / 1681; 128 of 768 (768) 200 rows 1778 / 1646.
+W4_EXPERT_TILES = 2 * 148
+
+
+def experts_from_int4(backend: str, c: int, k: int, e: int, width: int) -> bool:
+    """The experts' GEMMs of a prompt chunk of ``c`` rows, ``k`` of ``e`` experts each, read int4 blocks (else bf16 copies: the same
+    bits)."""
+    if backend == "w4":          # there are no copies
+        return True
+    return c * k <= W4_EXPERT_ROWS * e and (backend != "bf16-resident" or e * ((2 * width + 255) // 256) > W4_EXPERT_TILES)
 
 
 def _expert_bf16(runner, lw: LayerWeights, sc: _PrefillScratch):
@@ -192,7 +205,7 @@ def moe_block_prefill(runner, lw: LayerWeights, c: int):
     M.scatter(sc.topk_idx, sc.rank, sc.expert_base, c, k, x, h, sc.row_of, sc.xs)
     blocks = (sc.blk_expert, sc.blk_row0, sc.blk_rows, sc.n_blk, sc.max_blk)
     # grouped GEMMs over the experts' int4 blocks: a quarter of the bf16 bytes from HBM, at the price of expanding them (the same bits)
-    if runner.backend == "w4" or c * k <= W4_EXPERT_ROWS * e:
+    if experts_from_int4(runner.backend, c, k, e, i):
         G.gemm_w4(sc.xs, lw.experts_gate_up_w4b, 2 * i, h, sc.act, epi=G.EPI_SILU_MUL, blocks=blocks, n_experts=e)
         G.gemm_w4(sc.act, lw.experts_down_w4b, h, i, sc.y, epi=G.EPI_BF16, blocks=blocks, n_experts=e)
     else:

@@ -105,6 +105,17 @@ def test_attention_split_rule_and_quantiser_slots():
     assert [quant_slots(m) for m in (1, 8, 9, 16, 17, 33, 64)] == [8, 8, 16, 16, 32, 64, 64]
 
 
+def test_form_of_a_prompts_experts():
+    """Int4 blocks below a tile of rows an expert; where copies are resident, only from more tiles than two waves on."""
+    from b200serve.models.moe import experts_from_int4
+    assert experts_from_int4("w4", 100000, 8, 256, 512)
+    for backend in ("bf16", "int8"):
+        assert experts_from_int4(backend, 448, 2, 8, 2048) and not experts_from_int4(backend, 449, 2, 8, 2048)
+    assert not experts_from_int4("bf16-resident", 100, 2, 8, 2048) and not experts_from_int4("bf16-resident", 896, 4, 32, 768)
+    assert experts_from_int4("bf16-resident", 100, 6, 64, 1408) and not experts_from_int4("bf16-resident", 1195, 6, 64, 1408)
+    assert experts_from_int4("bf16-resident", 3584, 8, 256, 512) and not experts_from_int4("bf16-resident", 3585, 8, 256, 512)
+
+
 def test_splits_of_a_step():
     """One request's rows get equal splits, counted by the groups that share a CTA; rows of several are planned on the device, with
     room for one split of each row and a wave of CTAs beside."""

@@ -130,3 +130,22 @@ def test_experts_from_int4_or_copies(over, monkeypatch):
         K.check_status()
         got.append((first, eng.logits(1)[0].clone()))
     assert all(g[0] == got[0][0] and torch.equal(g[1], got[0][1]) for g in got)
+
+
+@pytest.mark.parametrize("tiles", [0, 1 << 20])
+def test_resident_copies_or_int4(tiles, monkeypatch):
+    """A resident model's experts from its copies or from the blocks: the bits of the model that makes copies anew."""
+    from b200serve.models import moe
+    from b200serve.models.config import small_moe
+    from b200serve.models.weights import random_weights
+    from b200serve.runtime.engine import Engine
+    cfg = small_moe()
+    monkeypatch.setattr(moe, "W4_EXPERT_TILES", tiles)
+    prompt = torch.randint(0, cfg.vocab, (200,), generator=torch.Generator().manual_seed(8)).tolist()
+    got = []
+    for backend in ("bf16", "bf16-resident"):
+        eng = Engine(random_weights(cfg, device="cuda", seed=4), max_seqs=1, max_len=1024, prefill_backend=backend)
+        got.append((eng.prefill(0, prompt), eng.logits(1)[0].clone()))
+        K.check_status()
+    assert (getattr(eng.model.w.layers[0], "_experts_bf16", None) is None) == (tiles == 0)
+    assert got[0][0] == got[1][0] and torch.equal(got[0][1], got[1][1])
