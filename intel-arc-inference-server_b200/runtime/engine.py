@@ -168,7 +168,10 @@ class Engine:
         c[K.CTRL_N_ROWS] = m
         for at, values in ((K.CTRL_ROW_REQ, [r.slot for r in rows]), (K.CTRL_ROW_POS, [r.pos for r in rows]),
                            (K.CTRL_CUR_TOKEN, [r.token for r in rows]), (K.CTRL_ROW_BLOCK, [r.block for r in rows])):
-            c[at: at + m] = values
+            try:
+                c[at: at + m] = values
+            except (TypeError, ValueError):      # device scalars (an arg-max that was not read), one-element tensors
+                c[at: at + m] = [int(v) for v in values]
         self._one_request = all(r.slot == rows[0].slot and r.pos == rows[0].pos + i for i, r in enumerate(rows))
         self.ctrl_stage.push(self.ctrl)
 

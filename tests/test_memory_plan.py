@@ -173,3 +173,26 @@ def test_every_step_buffer_is_known_to_the_planner(name):
     buf.surprise = torch.zeros(4)               # a buffer nobody told the planner about
     with pytest.raises(AssertionError, match="surprise"):
         R.audit(buf, kv, cfg, "bf16", max_seqs=2)
+
+
+@pytest.mark.parametrize("device", ["cpu", pytest.param("cuda", marks=pytest.mark.gpu)])
+def test_control_block_takes_numbers_and_scalar_tensors(device):
+    """A row's token may be the arg-max of the last step's logits, on the device and unread, or a one-element tensor."""
+    import numpy as np
+    import torch
+    from types import SimpleNamespace
+    from b200serve.ops import lib as K
+    from b200serve.runtime.engine import Engine, Row
+    from b200serve.utils.staging import Staged
+    eng = SimpleNamespace(ctrl_stage=Staged((K.CTRL_WORDS,), torch.int32), ctrl=torch.zeros(K.CTRL_WORDS, dtype=torch.int32, device=device))
+    logits = torch.tensor([0.0, 3.0, 1.0, 2.0], device=device)
+    for tokens in ([5, 7, 9], [logits.argmax(), 7, logits[2:].argmax()], [torch.tensor([5], device=device)] * 3, [np.int64(5), 7, torch.tensor(9)]):
+        rows = [Row(4 - i, 10 * i, t, i & 1) for i, t in enumerate(tokens)]
+        Engine._write_rows(eng, rows)
+        c = eng.ctrl.tolist()
+        assert c[K.CTRL_N_ROWS] == 3 and c[K.CTRL_ROW_REQ: K.CTRL_ROW_REQ + 3] == [4, 3, 2] and c[K.CTRL_ROW_POS: K.CTRL_ROW_POS + 3] == [0, 10, 20]
+        assert c[K.CTRL_CUR_TOKEN: K.CTRL_CUR_TOKEN + 3] == [int(t) for t in tokens] and c[K.CTRL_ROW_BLOCK: K.CTRL_ROW_BLOCK + 3] == [0, 1, 0]
+        assert not eng._one_request
+    for bad, error in (([2 ** 31, 0, 0], OverflowError), ([None, 0, 0], TypeError)):
+        with pytest.raises(error):
+            Engine._write_rows(eng, [Row(0, i, t) for i, t in enumerate(bad)])
