@@ -685,7 +685,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // grid (ceil(K / 256), N / 128), 256 threads: a thread (tile j = warp, lane) expands its 16 bytes of four consecutive blocks, all
 // loaded at once.  The four lanes of a quad hold 32 contiguous bytes of a row, so they store whole sectors from registers;
 // through a shared-memory tile, one block per CTA, the pass ran at 4.6 TB/s.
-// 34816 x 5120: 98 -> 83 us (451 MB, 5.5 TB/s).
+// 34816 x 5120: 98 -> 83 us (451 MB, 5.5 TB/s).  PAIRS: 4-byte stores, for an output that is aligned to no more.
+template <bool PAIRS>
 __global__ void __launch_bounds__(256) dequant_w4b_kernel(const uint8_t* __restrict__ w, __nv_bfloat16* __restrict__ out,
                                                           int N, int K) {
   constexpr int U = 4;
@@ -717,7 +718,13 @@ __global__ void __launch_bounds__(256) dequant_w4b_kernel(const uint8_t* __restr
         float f[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) f[i] = (float)((int)((x >> (8 * i)) & 0xFF) - 8) * s;
-        *reinterpret_cast<uint2*>(row + 16 * e) = make_uint2(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]));
+        const uint32_t lo = pack_bf16(f[0], f[1]), hi = pack_bf16(f[2], f[3]);
+        if (PAIRS) {
+          reinterpret_cast<uint32_t*>(row + 16 * e)[0] = lo;
+          reinterpret_cast<uint32_t*>(row + 16 * e)[1] = hi;
+        } else {
+          *reinterpret_cast<uint2*>(row + 16 * e) = make_uint2(lo, hi);
+        }
       }
     }
   }
@@ -965,9 +972,10 @@ extern "C" int b2_gemm_tc_ep(const void* a, const void* b, void* c, int M, int N
 
 extern "C" int b2_dequant_w4b(const void* w4b, void* out_bf16, int N, int K, void* stream) {
   if (K % 64) return -1;
-  if (((uintptr_t)w4b & 15) || ((uintptr_t)out_bf16 & 7)) return -3;
+  if (((uintptr_t)w4b & 15) || ((uintptr_t)out_bf16 & 3)) return -3;
   dim3 grid((K / 64 + 3) / 4, (N + 127) / 128);
-  dequant_w4b_kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const uint8_t*)w4b, (__nv_bfloat16*)out_bf16, N, K);
+  const auto kernel = ((uintptr_t)out_bf16 & 7) ? dequant_w4b_kernel<true> : dequant_w4b_kernel<false>;
+  kernel<<<grid, 256, 0, (cudaStream_t)stream>>>((const uint8_t*)w4b, (__nv_bfloat16*)out_bf16, N, K);
   return (int)cudaGetLastError();
 }
 

@@ -51,6 +51,18 @@ def test_expanded_weights(n, k):
     assert torch.equal(out[:n], Q.dequant_w4b(w, n).bfloat16()) and torch.isnan(out[n]).all()
 
 
+@pytest.mark.parametrize("n,k", [(100, 256), (1000, 320)])
+def test_expanded_weights_into_a_view(n, k):
+    """An output that starts in the middle of an 8-byte word."""
+    w = Q.random_w4b(n, k, "cuda", 3)
+    flat = torch.full((n * k + 4,), float("nan"), dtype=torch.bfloat16, device="cuda")
+    G.dequant_w4b(w, n, k, flat[2: 2 + n * k].view(n, k))
+    torch.cuda.synchronize()
+    assert torch.equal(flat[2: 2 + n * k].view(n, k), Q.dequant_w4b(w, n).bfloat16()) and torch.isnan(flat[:2]).all() and torch.isnan(flat[-2:]).all()
+    with pytest.raises(RuntimeError):
+        G.dequant_w4b(w, n, k, flat[1: 1 + n * k].view(n, k))
+
+
 @pytest.mark.parametrize("m,h", [(512, 64), (513, 2048), (600, 2056), (1000, 4096), (519, 5120), (700, 5128), (512, 8192), (530, 8200), (511, 5120)])
 def test_norm_of_prompt_rows(m, h):
     torch.manual_seed(h)
