@@ -85,6 +85,9 @@ def attn_splits(n_kv_heads: int, depth: int) -> int:
     return max(4, min(64, 296 // max(1, n_kv_heads), max(depth, 64) // 64))
 
 
+# Rows from which the linears run on tcgen05 (27B shape, 16 layers, integer GEMV / tcgen05: 16 rows 2.37 / 2.76 ms, 17 rows 3.66 / 2.96,
+# 40 rows 5.89 / 4.13, 64 rows 7.71 / 4.93)
+ROWS_MIN = 17
 ATTN_WAVES = 2      # of 2 x 148 CTAs of decode attention, see ``DecoderModel._attn_splits``
 
 
@@ -240,9 +243,6 @@ class DecoderModel:
         # from this many rows up the activations are quantised once by their own kernel instead of in every
         # CTA of the GEMV (whose prologue repeats the rows' work per 128 output columns)
         self.prequant_rows = int(os.environ.get("B2_PREQUANT_ROWS", "3"))
-        # rows from which the linears run on tcgen05 (16 layers, integer GEMV / tcgen05: 16 rows 2.37 / 2.76 ms, 17 rows 3.66 / 2.96, 40 rows
-        # 5.89 / 4.13, 64 rows 7.71 / 4.93)
-        self.rows_min = 17
         self.merge_quant = os.environ.get("B2_MERGE_QUANT", "1") == "1"   # the attention merge writes the o projection's quantised rows
         self.attn_rows_min = int(os.environ.get("B2_ATTN_ROWS_MIN", "1"))
         self.rows_one_request = False    # set by the engine around a step whose rows are one request's, consecutive
@@ -275,7 +275,7 @@ class DecoderModel:
     def _on_rows(self, m: int) -> bool:
         """Steps of ``m`` rows take the tcgen05 form of the linears (``gemm_rows.cu``), whose sums are not the integer GEMV's bits:
         never where a row's bits must not depend on its company, and on one GPU only (no fold over the wire)."""
-        return self.rows_min <= m <= 64 and not self.attn_fixed_spans and self.tp is None and self.nccl is None
+        return ROWS_MIN <= m <= 64 and not self.attn_fixed_spans and self.tp is None and self.nccl is None
 
     def _gemm_rows(self, name: str, ql: QLinear, x, m: int, staged: bool = False, fold: bool = False, **stage):
         b = self.buf

@@ -50,7 +50,7 @@ template <int T>
 struct Cfg {
   static constexpr int XB = kStageBlocks * T * 128, WB = kStageBlocks * kBlockBytes;      // a stage's token rows and weights
   static constexpr int RED = T * 512;                                       // half the token rows of each pipeline's sums
-  static constexpr int NX = T <= 16 ? 9 : T <= 32 ? 6 : T <= 48 ? 4 : 3, NW = T <= 16 ? 7 : T <= 32 ? 6 : 5;
+  static constexpr int NX = T <= 32 ? 6 : T <= 48 ? 4 : 3, NW = T <= 32 ? 6 : 5;
   static constexpr int OFF_RAW = NX * XB, OFF_RED = OFF_RAW + NW * WB, OFF_BAR = OFF_RED + RED;
   static constexpr int BARS = (2 * NW + 2 * NX + 16) * 8 + 16;
   static constexpr int SMEM = 1024 + OFF_BAR + BARS;
@@ -378,7 +378,7 @@ int launch_rows(const RowsParams& p, cudaStream_t stream) {
 
 }  // namespace
 
-// ``x``: b2_stage_rows of the same M and K.  S <= 16 splits of whole fours of groups, none of them empty.
+// ``x``: b2_stage_rows of the same M and K, whose rows are padded to 32, 48 or 64 (decode steps come here from 17 rows on).  S <= 16 splits of whole fours of groups, none of them empty.
 extern "C" int b2_gemm_w4_rows(const void* w4b, const void* x, float* out, int M, int N, int K, int S, int* fold_tickets,
                                const void* fold_resid_in, void* fold_resid_out, float* fold_ssq, void* stream) {
   if (M < 1 || M > 64 || N < 1 || K < 64 || K % 64 != 0 || S < 1 || S > kMaxSplits) return -1;
@@ -391,7 +391,6 @@ extern "C" int b2_gemm_w4_rows(const void* w4b, const void* x, float* out, int M
   p.fold_tickets = fold_tickets; p.fold_resid_in = (const __nv_bfloat16*)fold_resid_in;
   p.fold_resid_out = (__nv_bfloat16*)fold_resid_out; p.fold_ssq = fold_ssq;
   cudaStream_t st = (cudaStream_t)stream;
-  if (M <= 16) return launch_rows<16>(p, st);
   if (M <= 32) return launch_rows<32>(p, st);
   if (M <= 48) return launch_rows<48>(p, st);
   return launch_rows<64>(p, st);

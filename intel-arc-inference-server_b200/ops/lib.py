@@ -198,7 +198,7 @@ def quant_x(x, m, k, xq, xq_gs, *, x_mode=0, s_in=1, x_slice=0, ldx=None, norm_w
 
 def rows_pad(m: int) -> int:
     """Token rows per 64-k group that ``stage_rows`` lays out for ``m`` rows."""
-    return (m + 15) // 16 * 16
+    return max(32, (m + 15) // 16 * 16)
 
 
 def stage_rows(x, m, k, xr, *, x_mode=0, s_in=1, x_slice=0, ldx=None, norm_w=None, norm_ssq=None, norm_eps=0.0):

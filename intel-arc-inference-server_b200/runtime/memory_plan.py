@@ -100,7 +100,7 @@ def step_scratch_bytes(cfg: ModelConfig, max_rows: int = 64, nsplit: int = 32) -
     b += 16 * max_rows * (cfg.qkv_dim + 2 * h + 2 * max(cfg.ffn, cfg.expert_ffn * max(cfg.top_k, 1))) * 4
     kmax = max(2 * h, cfg.q_dim, cfg.ffn, cfg.expert_ffn, cfg.shared_ffn, cfg.gdn_value_dim)
     b += max_rows * (kmax // 64) * (128 + 8) + (1 << 16)      # quantised rows + group scales, small control words
-    b += (max_rows + 15) // 16 * 16 * kmax * 2                # rows of the tcgen05 form
+    b += max(32, (max_rows + 15) // 16 * 16) * kmax * 2       # rows of the tcgen05 form
     if cfg.n_gdn_layers:
         b += max_rows * (cfg.gdn_proj_dim * 4 + cfg.gdn_value_dim * 2)
     return int(b)

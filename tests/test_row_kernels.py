@@ -129,8 +129,8 @@ def test_grouped_experts(m, k, e, shared, h, f):
         assert (out[pick].double() - z).norm() < 2.0 ** -8 * z.norm()
 
 
-# rows at the edges of the four instances (16 token rows each); splits with unequal and lone groups; n not a multiple of 128; fewer
-# blocks than the four sets take in turn; more items than SMs
+# rows at the edges of the three instances (32, 48 and 64 token rows); splits with unequal and lone groups: stages of which one pipeline has
+# no block; n not a multiple of 128; more items than SMs
 @pytest.mark.parametrize("m,n,k,splits", [(1, 128, 64, 1), (9, 256, 128, 2), (16, 300, 320, 1), (17, 128, 704, 3), (31, 1000, 1024, 4), (32, 5120, 640, 4),
                                           (33, 640, 448, 7), (48, 128, 1088, 16), (49, 20480, 256, 2), (64, 384, 5120, 7)])
 @pytest.mark.parametrize("fold", [False, True])
