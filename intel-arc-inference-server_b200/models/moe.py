@@ -52,10 +52,13 @@ class _RowScratch:
         self.groups = torch.zeros(M.group_words(mr * (k + 1)), dtype=torch.int32, device=dev)
 
 
-# Steps of this many rows and more run their experts by groups of rows (one reading of an expert per eight rows), shorter ones by
-# (row, slot), whose split sums keep more CTAs busy.  16 layers of 256 experts, 8 per row: 1.47 ms by groups against 1.55 with 4
-# rows, 1.72 against 2.38 with 8, 2.96 against 7.01 with 32, 4.15 against 13.06 with 64.
+# Steps of this many rows and more whose (row, slot) pairs would read this many bytes run their experts by groups of rows (one reading of
+# an expert per eight rows), others by pair, whose split sums keep more CTAs busy; the table of groups and its rows' staging cost some 4 us a
+# layer.  Us by pair / by groups, hidden 2048, 4 layers: 256 experts of 512, 8 per row, 4 rows (60 MB) 486 / 428, 8 rows 680 / 496, 48
+# rows 2470 / 839; 32 of 768, 4 per row, 3 rows (30 MB) 377 / 378, 4 rows (40 MB) 425 / 390; 8 of 2048, 2 per row, 2 rows (27 MB) 364 / 379, 4 rows
+# 461 / 418.  Hidden 512, 2 layers, 16 of 256, 4 per row: 8 rows (8 MB) 145 / 155, 12 rows (13 MB) 158 / 162, 24 rows (25 MB) 182 / 166.
 GROUP_ROWS = 4
+GROUP_BYTES = 24_000_000
 
 
 def moe_block_rows(model, lw: LayerWeights, m: int, fold: bool = False):
@@ -75,7 +78,8 @@ def moe_block_rows(model, lw: LayerWeights, m: int, fold: bool = False):
         # ride along as an alternative tensor for its slot id -- and the weighted sum.
         ks = k + (1 if lw.shared is not None else 0)
         # (grouped, the slices of a split sum are added in another order: not where a row's bits must not depend on its company)
-        grouped = m >= GROUP_ROWS and not model.attn_fixed_spans and h <= 4096 and i <= 4096
+        grouped = (m >= GROUP_ROWS and m * ks * (gu_bytes + dn_bytes) >= GROUP_BYTES and not model.attn_fixed_spans and h <= 4096 and
+                   i <= 4096)
         M.router_rows(rc, b.x, sc.logits, m, e + (1 if lw.shared_gate is not None else 0), h, sc.ld, e, k,
                       lw.shared is not None, lw.shared_gate is not None, sc.topk_idx, sc.topk_w, sc.ticket,
                       groups=sc.groups if grouped else None)

@@ -675,9 +675,10 @@ __global__ void __launch_bounds__(256) quant_x_kernel(const GemvParams p, uint8_
 // 384 readings of ~200 experts, and the eight token columns of the integer MMA hold one row.  Here the routing kernel's last
 // CTA leaves a table of groups (moe.cu), the rows of a group are quantised into shared memory once and every n-block's
 // weights stream past them.  Two groups of four consumer warps own alternate n-blocks, so a sum never leaves its warp and the
-// CTA has no barrier after the staging; a run is about 64 W4B blocks (280 KB), which keeps the fixed cost per CTA (table,
-// staging, ring fill: ~4 us with two CTAs per SM) below its stream time and leaves three to four waves to balance.  A step of
-// 48 rows through 16 layers (hidden 2048, experts of 512): 11.5 -> 4.3 ms, with the router's slices (moe.cu).
+// CTA has no barrier after the staging; a run is at most about 64 W4B blocks (280 KB), which keeps the fixed cost per CTA (table,
+// staging, ring fill: ~4 us with two CTAs per SM) below its stream time, and shorter where the groups would not fill a wave of 296
+// CTAs.  A step of 48 rows through 16 layers (hidden 2048, experts of 512): 11.5 -> 4.3 ms, with the router's slices (moe.cu); 4 layers, 8
+// rows, runs of 64 blocks whatever the groups / as here: experts of 512 500 / 496 us, hidden 512 with 16 of 256 (2 layers) 164 / 155.
 struct ExpertGroups {
   int n;           // groups in use
   int pad[15];
@@ -1024,7 +1025,7 @@ extern "C" int b2_gemv_w4_groups(const void* w4b_stack, long long expert_bytes, 
   p.x_div = x_div; p.x_batch_bytes = x_batch_bytes; p.out_batch = N;
   e.groups = reinterpret_cast<const ExpertGroups*>(groups);
   e.nb = (N + 127) / 128;
-  e.run = max(2, (64 / p.KG) & ~1);
+  e.run = max(2, min(64 / p.KG, (int)((long long)e.nb * max_groups / 296)) & ~1);
   const int smem = 128 + kRingBytes + 128 + ((p.KG * 64 + 127) & ~127) + 8 * stride_words(p.KG) * 4;
   if (smem > 232448) return -9;
   static int configured[64] = {};

@@ -122,6 +122,35 @@ def test_tiny_moe_rows_path_matches_oracle():
     _teacher_forced(oracle, prompt, toks, 0.03)
 
 
+@pytest.mark.parametrize("rows", [4, 9, 24])
+def test_steps_by_groups_or_by_pairs(rows, monkeypatch):
+    """Both forms of a step's experts in the engine, and which one a step takes."""
+    from b200serve.models import moe
+    from b200serve.ops import lib as K
+    from b200serve.ops import moe as M
+    from b200serve.runtime.engine import Engine, Row
+    cfg = small_moe()
+    g = torch.Generator().manual_seed(rows)
+    ids = torch.randint(0, cfg.vocab, (rows,), generator=g)
+    ref = OracleModel(random_weights(cfg, seed=4)).forward(ids)
+    calls = []
+    real = M.gemv_groups
+    monkeypatch.setattr(M, "gemv_groups", lambda *a, **kw: (calls.append(1), real(*a, **kw)))
+    got = []
+    for least in (0, moe.GROUP_BYTES, 1 << 60):
+        monkeypatch.setattr(moe, "GROUP_BYTES", least)
+        calls.clear()
+        eng = Engine(random_weights(cfg, device="cuda", seed=4), max_seqs=1, max_len=256, use_graphs=False, nsplit_attn=4)
+        eng.forward_rows([Row(0, i, int(t)) for i, t in enumerate(ids)])
+        K.check_status()
+        got.append(eng.logits(rows).float().cpu().clone())
+        # a row's experts are 5 x 209 KB of int4: 24 rows read 25 MB by pair
+        assert (len(calls) == 2 * cfg.n_layers) == (least == 0 or (least < 1 << 60 and rows == 24)) and len(calls) in (0, 2 * cfg.n_layers)
+        err = (got[-1] - ref).abs().amax(dim=1) / ref.abs().max()       # a near-tie between experts may flip under bf16 activations
+        assert (err < 0.04).float().mean() >= 0.7 and err.max() < 0.25, err
+    assert torch.equal(got[1], got[0 if rows == 24 else 2])
+
+
 @pytest.mark.parametrize("backend", ["bf16", "bf16-resident", "w4"])
 def test_small_moe_prompt_path_matches_oracle(backend):
     from b200serve.ops import lib as K
