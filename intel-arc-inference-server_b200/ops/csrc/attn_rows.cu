@@ -86,7 +86,6 @@ __device__ __forceinline__ uint32_t tile_off(int row, int d) {
   return (uint32_t)((d >> 6) * HALFB + row * 128 + ((((d & 63) >> 3) ^ (row & 7)) << 4));
 }
 
-// NKS: key slices per batch (1, 2 or 4); the four warps are NKS slices x (4 / NKS) groups of 16 query rows.
 // int8 as bf16 integers: even bytes of w as a pair.  With b's low seven bits as mantissa of 2^7, 128 + (b & 127) less 128 or, where
 // the sign is set, 256.
 __device__ __forceinline__ uint32_t bytes_bf16(uint32_t w) {
@@ -95,6 +94,7 @@ __device__ __forceinline__ uint32_t bytes_bf16(uint32_t w) {
   return d;
 }
 
+// NKS: key slices per batch (1, 2 or 4); the four warps are NKS slices x (4 / NKS) groups of 16 query rows.
 template <bool I8, int NKS>
 __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t* smem_raw, const int* s_pos, int* s_last_p, int* s_bt,
                                                const int req, const int rows, const int QR, const int ctx_max, const int z,
@@ -281,167 +281,167 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
       if (++slot == nst) { slot = 0; par ^= 1; }
     }
   } else {
-  float ksc[2] = {0.f, 0.f}, vsc[2] = {0.f, 0.f};
-  // The pages of batch b into buffer b % nbuf: lanes of warp 0 issue one tiled copy each (page, K or V, half).
-  auto issue = [&](int b) {
-    const int kb0 = key0 + b * KB, nk = min(KB, key1 - kb0), buf = b % p.nbuf;
-    const int npages = (nk + 15) >> 4;
-    const uint32_t bar = bar0 + 8 * buf;
-    if (tid == 0) mbar_expect_tx(bar, (uint32_t)npages * (I8 ? 4096u : 8192u));
-    __syncthreads();
-    const uint32_t kt = ks0 + (I8 ? 0 : buf) * tileB, vt = vs0 + (I8 ? 0 : buf) * tileB;
-    if (tid < 32) {
-      const int pi = tid >> 2, which = tid & 3;   // which: 0 K low dims, 1 K high dims, 2 V low, 3 V high
-      if (pi < npages && (!I8 || !(which & 1))) {
-        const int page = bt[((kb0 - key0) >> 4) + pi];
-        const int row = (page * p.n_kv + kh) * 16;
-        const CUtensorMap* map = (which & 2) ? &p.v_map : &p.k_map;
-        if (I8)
-          tma_load_2d(((which & 2) ? v8s0 : k8s0) + buf * stageB + pi * 2048, map, 0, row, bar);
-        else
-          tma_load_2d(((which & 2) ? vt : kt) + (which & 1) * HALFB + pi * 2048, map, (which & 1) * 64, row, bar);
+    float ksc[2] = {0.f, 0.f}, vsc[2] = {0.f, 0.f};
+    // The pages of batch b into buffer b % nbuf: lanes of warp 0 issue one tiled copy each (page, K or V, half).
+    auto issue = [&](int b) {
+      const int kb0 = key0 + b * KB, nk = min(KB, key1 - kb0), buf = b % p.nbuf;
+      const int npages = (nk + 15) >> 4;
+      const uint32_t bar = bar0 + 8 * buf;
+      if (tid == 0) mbar_expect_tx(bar, (uint32_t)npages * (I8 ? 4096u : 8192u));
+      __syncthreads();
+      const uint32_t kt = ks0 + (I8 ? 0 : buf) * tileB, vt = vs0 + (I8 ? 0 : buf) * tileB;
+      if (tid < 32) {
+        const int pi = tid >> 2, which = tid & 3;   // which: 0 K low dims, 1 K high dims, 2 V low, 3 V high
+        if (pi < npages && (!I8 || !(which & 1))) {
+          const int page = bt[((kb0 - key0) >> 4) + pi];
+          const int row = (page * p.n_kv + kh) * 16;
+          const CUtensorMap* map = (which & 2) ? &p.v_map : &p.k_map;
+          if (I8)
+            tma_load_2d(((which & 2) ? v8s0 : k8s0) + buf * stageB + pi * 2048, map, 0, row, bar);
+          else
+            tma_load_2d(((which & 2) ? vt : kt) + (which & 1) * HALFB + pi * 2048, map, (which & 1) * 64, row, bar);
+        }
       }
-    }
-    if (I8) {
-      if (tid < nk) {
-        const int key = kb0 + tid;
-        const size_t row = ((size_t)bt[(key - key0) >> 4] * p.n_kv + kh) * 16 + (key & 15);
-        ksc[buf] = p.k_scale[row];
-        vsc[buf] = p.v_scale[row];
-      }
-    } else if (tid >= npages * 16) {
-      // rows of pages that are not fetched: V must be finite (its products are multiplied by P = 0)
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(vt + (i >> 3) * HALFB + tid * 128 + 16 * (i & 7)), "r"(0) : "memory");
-    }
-  };
-  if (p.nbuf == 2 && nbatch > 0) issue(0);
-  for (int batch = 0; batch < nbatch; ++batch) {
-    const int kb0 = key0 + batch * KB;
-    const int nk = min(KB, key1 - kb0);
-    const int buf = batch % p.nbuf;
-    const uint32_t ks = ks0 + (I8 ? 0 : buf) * tileB, vs = vs0 + (I8 ? 0 : buf) * tileB;
-    const uint32_t k8s = k8s0 + buf * stageB, v8s = v8s0 + buf * stageB, bar = bar0 + 8 * buf;
-    __syncthreads();  // the previous batch is consumed: its buffer may be refilled
-    if (p.nbuf == 2) {
-      if (batch + 1 < nbatch) issue(batch + 1);
-    } else {
-      issue(batch);
-    }
-    if (okw) okw = mbar_wait(bar, (batch / p.nbuf) & 1, ERR_ATTN_WAIT);
-    if (I8) {
-      // every thread expands its own key's row: int8 x per-row scale -> bf16 into the operand tiles
-      if (tid >= nk) {   // rows without a key: V must be finite (its products are multiplied by P = 0)
+      if (I8) {
+        if (tid < nk) {
+          const int key = kb0 + tid;
+          const size_t row = ((size_t)bt[(key - key0) >> 4] * p.n_kv + kh) * 16 + (key & 15);
+          ksc[buf] = p.k_scale[row];
+          vsc[buf] = p.v_scale[row];
+        }
+      } else if (tid >= npages * 16) {
+        // rows of pages that are not fetched: V must be finite (its products are multiplied by P = 0)
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(vs + (i >> 3) * HALFB + tid * 128 + 16 * (i & 7)), "r"(0) : "memory");
+          asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(vt + (i >> 3) * HALFB + tid * 128 + 16 * (i & 7)), "r"(0) : "memory");
       }
-      if (okw && tid < nk) {
+    };
+    if (p.nbuf == 2 && nbatch > 0) issue(0);
+    for (int batch = 0; batch < nbatch; ++batch) {
+      const int kb0 = key0 + batch * KB;
+      const int nk = min(KB, key1 - kb0);
+      const int buf = batch % p.nbuf;
+      const uint32_t ks = ks0 + (I8 ? 0 : buf) * tileB, vs = vs0 + (I8 ? 0 : buf) * tileB;
+      const uint32_t k8s = k8s0 + buf * stageB, v8s = v8s0 + buf * stageB, bar = bar0 + 8 * buf;
+      __syncthreads();  // the previous batch is consumed: its buffer may be refilled
+      if (p.nbuf == 2) {
+        if (batch + 1 < nbatch) issue(batch + 1);
+      } else {
+        issue(batch);
+      }
+      if (okw) okw = mbar_wait(bar, (batch / p.nbuf) & 1, ERR_ATTN_WAIT);
+      if (I8) {
+        // every thread expands its own key's row: int8 x per-row scale -> bf16 into the operand tiles
+        if (tid >= nk) {   // rows without a key: V must be finite (its products are multiplied by P = 0)
 #pragma unroll
-        for (int which = 0; which < 2; ++which) {
-          const uint32_t src = (which ? v8s : k8s) + tid * D, dst = which ? vs : ks;
-          const float sc = which ? vsc[buf] : ksc[buf];
+          for (int i = 0; i < 16; ++i)
+            asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(vs + (i >> 3) * HALFB + tid * 128 + 16 * (i & 7)), "r"(0) : "memory");
+        }
+        if (okw && tid < nk) {
 #pragma unroll
-          for (int i = 0; i < D / 16; ++i) {
-            uint32_t w0, w1, w2, w3;
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w0), "=r"(w1), "=r"(w2), "=r"(w3) : "r"(src + ((i ^ (tid & 7)) << 4)));
-            const uint32_t ww[4] = {w0, w1, w2, w3};
-            uint32_t o[8];
+          for (int which = 0; which < 2; ++which) {
+            const uint32_t src = (which ? v8s : k8s) + tid * D, dst = which ? vs : ks;
+            const float sc = which ? vsc[buf] : ksc[buf];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              // int8 -> fp32 without the conversion unit (a quarter-rate pipe that capped this loop): the byte, biased
-              // to 0..255, dropped into the mantissa of 2^23 is 8388608 + u, and subtracting 8388736 leaves the signed
-              // value exactly -- the same floats as (float)(int8_t), so the same products
-              const uint32_t u = ww[j] ^ 0x80808080u;
-              const float f0 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7540)) - 8388736.f;
-              const float f1 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7541)) - 8388736.f;
-              const float f2 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7542)) - 8388736.f;
-              const float f3 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7543)) - 8388736.f;
-              o[2 * j] = pack_bf16(f0 * sc, f1 * sc);
-              o[2 * j + 1] = pack_bf16(f2 * sc, f3 * sc);
+            for (int i = 0; i < D / 16; ++i) {
+              uint32_t w0, w1, w2, w3;
+              asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(w0), "=r"(w1), "=r"(w2), "=r"(w3) : "r"(src + ((i ^ (tid & 7)) << 4)));
+              const uint32_t ww[4] = {w0, w1, w2, w3};
+              uint32_t o[8];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                // int8 -> fp32 without the conversion unit (a quarter-rate pipe that capped this loop): the byte, biased
+                // to 0..255, dropped into the mantissa of 2^23 is 8388608 + u, and subtracting 8388736 leaves the signed
+                // value exactly -- the same floats as (float)(int8_t), so the same products
+                const uint32_t u = ww[j] ^ 0x80808080u;
+                const float f0 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7540)) - 8388736.f;
+                const float f1 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7541)) - 8388736.f;
+                const float f2 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7542)) - 8388736.f;
+                const float f3 = __uint_as_float(__byte_perm(u, 0x4B000000u, 0x7543)) - 8388736.f;
+                o[2 * j] = pack_bf16(f0 * sc, f1 * sc);
+                o[2 * j + 1] = pack_bf16(f2 * sc, f3 * sc);
+              }
+              asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + tile_off(tid, 16 * i)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
+              asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + tile_off(tid, 16 * i + 8)), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
             }
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + tile_off(tid, 16 * i)), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]) : "memory");
-            asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(dst + tile_off(tid, 16 * i + 8)), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
           }
         }
       }
-    }
-    __syncthreads();
-    if (!okw || !active) continue;
+      __syncthreads();
+      if (!okw || !active) continue;
 #pragma unroll 1
-    for (int sub = 0; sub < KW / KS; ++sub) {
-    const int kofs = ksl * KW + sub * KS;   // this warp's slice of the batch, this pass
-    if (kofs >= nk) break;
+      for (int sub = 0; sub < KW / KS; ++sub) {
+      const int kofs = ksl * KW + sub * KS;   // this warp's slice of the batch, this pass
+      if (kofs >= nk) break;
 
-    // ---- S = Q K^T for this pass's keys: NJ n8 tiles x 8 k16 steps
-    float s[NJ][4];
+      // ---- S = Q K^T for this pass's keys: NJ n8 tiles x 8 k16 steps
+      float s[NJ][4];
 #pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+      for (int j = 0; j < NJ; ++j) {
+        s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
 #pragma unroll
-      for (int kk = 0; kk < 8; kk += 2) {
-        uint32_t b0, b1, b2, b3;
-        // matrices: (keys 8j.., d 16kk..), (d 16kk + 8..), (d 16(kk+1)..), (d 16(kk+1) + 8..)
-        ldsm_x4(ks + tile_off(kofs + 8 * j + (lane & 7), 16 * kk + 8 * (lane >> 3)), b0, b1, b2, b3);
-        mma_bf16_16816(s[j], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b0, b1);
-        mma_bf16_16816(s[j], qa[kk + 1][0], qa[kk + 1][1], qa[kk + 1][2], qa[kk + 1][3], b2, b3);
+        for (int kk = 0; kk < 8; kk += 2) {
+          uint32_t b0, b1, b2, b3;
+          // matrices: (keys 8j.., d 16kk..), (d 16kk + 8..), (d 16(kk+1)..), (d 16(kk+1) + 8..)
+          ldsm_x4(ks + tile_off(kofs + 8 * j + (lane & 7), 16 * kk + 8 * (lane >> 3)), b0, b1, b2, b3);
+          mma_bf16_16816(s[j], qa[kk][0], qa[kk][1], qa[kk][2], qa[kk][3], b0, b1);
+          mma_bf16_16816(s[j], qa[kk + 1][0], qa[kk + 1][1], qa[kk + 1][2], qa[kk + 1][3], b2, b3);
+        }
       }
-    }
-    // ---- scale, causal mask per row, online softmax (rows g and g + 8 of the tile)
-    float mnew[2] = {mx[0], mx[1]};
+      // ---- scale, causal mask per row, online softmax (rows g and g + 8 of the tile)
+      float mnew[2] = {mx[0], mx[1]};
 #pragma unroll
-    for (int j = 0; j < NJ; ++j)
+      for (int j = 0; j < NJ; ++j)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int key = kb0 + kofs + 8 * j + 2 * t + (e & 1);
-        const int hf = e >> 1;
-        const float v = key < ctx[hf] && key < key1 && key >= wlo[hf] ? s[j][e] * p.scale_log2 : -INFINITY;
-        s[j][e] = v;
-        mnew[hf] = fmaxf(mnew[hf], v);
+        for (int e = 0; e < 4; ++e) {
+          const int key = kb0 + kofs + 8 * j + 2 * t + (e & 1);
+          const int hf = e >> 1;
+          const float v = key < ctx[hf] && key < key1 && key >= wlo[hf] ? s[j][e] * p.scale_log2 : -INFINITY;
+          s[j][e] = v;
+          mnew[hf] = fmaxf(mnew[hf], v);
+        }
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        mnew[hf] = fmaxf(mnew[hf], __shfl_xor_sync(0xffffffffu, mnew[hf], 1));
+        mnew[hf] = fmaxf(mnew[hf], __shfl_xor_sync(0xffffffffu, mnew[hf], 2));
+      }
+      float corr[2];
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        corr[hf] = mnew[hf] == -INFINITY ? 1.f : exp2f(mx[hf] - mnew[hf]);   // mx = -inf on the first keys -> 0
+        lsum[hf] *= corr[hf];
+        mx[hf] = mnew[hf];
       }
 #pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      mnew[hf] = fmaxf(mnew[hf], __shfl_xor_sync(0xffffffffu, mnew[hf], 1));
-      mnew[hf] = fmaxf(mnew[hf], __shfl_xor_sync(0xffffffffu, mnew[hf], 2));
-    }
-    float corr[2];
-#pragma unroll
-    for (int hf = 0; hf < 2; ++hf) {
-      corr[hf] = mnew[hf] == -INFINITY ? 1.f : exp2f(mx[hf] - mnew[hf]);   // mx = -inf on the first keys -> 0
-      lsum[hf] *= corr[hf];
-      mx[hf] = mnew[hf];
-    }
-#pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1];
-    }
-#pragma unroll
-    for (int j = 0; j < NJ; ++j)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int hf = e >> 1;
-        const float pe = mnew[hf] == -INFINITY ? 0.f : exp2f(s[j][e] - mnew[hf]);
-        s[j][e] = pe;
-        lsum[hf] += pe;
+      for (int j = 0; j < 16; ++j) {
+        o[j][0] *= corr[0]; o[j][1] *= corr[0]; o[j][2] *= corr[1]; o[j][3] *= corr[1];
       }
-    // ---- O += P V: NJ / 2 k16 steps over this warp's keys, 16 n8 tiles over d
 #pragma unroll
-    for (int kk = 0; kk < NJ / 2; ++kk) {
-      const uint32_t pa0 = pack_bf16(s[2 * kk][0], s[2 * kk][1]), pa1 = pack_bf16(s[2 * kk][2], s[2 * kk][3]);
-      const uint32_t pa2 = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]), pa3 = pack_bf16(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+      for (int j = 0; j < NJ; ++j)
 #pragma unroll
-      for (int jd = 0; jd < 16; jd += 2) {
-        uint32_t b0, b1, b2, b3;
-        // matrices: (keys 16kk.., d 8jd..), (keys 16kk + 8.., d 8jd..), (keys 16kk.., d 8(jd+1)..), (keys + 8, d 8(jd+1)..)
-        const int mi = lane >> 3;
-        ldsm_x4_trans(vs + tile_off(kofs + 16 * kk + 8 * (mi & 1) + (lane & 7), 8 * (jd + (mi >> 1))), b0, b1, b2, b3);
-        mma_bf16_16816(o[jd], pa0, pa1, pa2, pa3, b0, b1);
-        mma_bf16_16816(o[jd + 1], pa0, pa1, pa2, pa3, b2, b3);
+        for (int e = 0; e < 4; ++e) {
+          const int hf = e >> 1;
+          const float pe = mnew[hf] == -INFINITY ? 0.f : exp2f(s[j][e] - mnew[hf]);
+          s[j][e] = pe;
+          lsum[hf] += pe;
+        }
+      // ---- O += P V: NJ / 2 k16 steps over this warp's keys, 16 n8 tiles over d
+#pragma unroll
+      for (int kk = 0; kk < NJ / 2; ++kk) {
+        const uint32_t pa0 = pack_bf16(s[2 * kk][0], s[2 * kk][1]), pa1 = pack_bf16(s[2 * kk][2], s[2 * kk][3]);
+        const uint32_t pa2 = pack_bf16(s[2 * kk + 1][0], s[2 * kk + 1][1]), pa3 = pack_bf16(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+#pragma unroll
+        for (int jd = 0; jd < 16; jd += 2) {
+          uint32_t b0, b1, b2, b3;
+          // matrices: (keys 16kk.., d 8jd..), (keys 16kk + 8.., d 8jd..), (keys 16kk.., d 8(jd+1)..), (keys + 8, d 8(jd+1)..)
+          const int mi = lane >> 3;
+          ldsm_x4_trans(vs + tile_off(kofs + 16 * kk + 8 * (mi & 1) + (lane & 7), 8 * (jd + (mi >> 1))), b0, b1, b2, b3);
+          mma_bf16_16816(o[jd], pa0, pa1, pa2, pa3, b0, b1);
+          mma_bf16_16816(o[jd + 1], pa0, pa1, pa2, pa3, b2, b3);
+        }
       }
+      }  // pass
     }
-    }  // pass
-  }
   }
 
   // ---- this split's partials: unnormalised O against the running maximum, (max, sum)

@@ -20,13 +20,14 @@
 // Tiles are walked M-fastest so CTAs that run together share one weight tile in L2.
 //
 // W4 form (template parameter W4): B is never materialised in global memory.  The producer fetches the W4B blocks of
-// a stage (4352 bytes per 128 rows x 64 k: nibbles + fp16 group scales) with bulk copies; eight more warps expand them
+// a stage (4352 bytes per 128 rows x 64 k: nibbles + fp16 group scales) with bulk copies; sixteen more warps expand them
 // to bf16 -- bf16_rne((q - 8) * scale), the same rounding as the dequantising pass -- straight into the stage's
 // B tile in the 128-byte-swizzled K-major layout the MMA descriptors expect, fence the generic stores against the
-// async proxy and complete the stage's barrier.  The weights cross HBM as int4 (a quarter of the bf16 bytes) and
-// no bf16 copy of the model is resident.  The role of the reference's direct-int4 GEMMs
+// async proxy and complete the stage's barrier.  The weights cross HBM as int4 (a quarter of the bf16 bytes), once per row of
+// tiles; chunks of several rows of tiles expand a weight once with dequant_w4b_kernel instead, into a workspace of the largest matrix, and
+// experts of a whole tile of rows and more read such copies.  The role of the reference's direct-int4 GEMMs
 // (src/kernels/prefill/pf_gemm_q4.cl, src/kernels/prefill/pf_moe_q4gemm.cl:1-40).  The blocks have a ring of their own,
-// seven k blocks deep and filled by a warp of its own: tied to the three tile stages, every block's trip from HBM was
+// seven k blocks deep (ten with 128 columns) and filled by a warp of its own: tied to the three tile stages, every block's trip from HBM was
 // part of the loop (2048 rows over 256 experts in 16 layers: 10.07 -> 9.71 ms).
 #include "common.cuh"
 #include "wire.cuh"
@@ -107,112 +108,112 @@ struct Cfg {
 
 // 32 accumulators of one row, columns n0 .. n0 + 31, through the epilogue into C
 __device__ __forceinline__ void store_chunk(const GemmParams& p, const uint32_t (&v)[32], int grow, int n0) {
-            float f[32];
-  #pragma unroll
-            for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
-            if (p.epi == EPI_SILU_MUL || p.epi == EPI_GLU) {
-              // columns alternate 16 gate, 16 up: 16 outputs per 32 accumulator columns
-              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)grow * p.ldc + (n0 >> 1);
-              uint32_t o[8];
-              if (p.epi == EPI_GLU && p.glu.bias) {
-  #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                  const float4 b = __ldg(reinterpret_cast<const float4*>(p.glu.bias + n0) + j);
-                  f[4 * j] += b.x; f[4 * j + 1] += b.y; f[4 * j + 2] += b.z; f[4 * j + 3] += b.w;
-                }
-              }
-  #pragma unroll
-              for (int j = 0; j < 8; ++j)
-                o[j] = p.epi == EPI_GLU ? pack_bf16(glu(p.glu, f[2 * j], f[16 + 2 * j]), glu(p.glu, f[2 * j + 1], f[17 + 2 * j]))
-                                        : pack_bf16(silu(f[2 * j]) * f[16 + 2 * j], silu(f[2 * j + 1]) * f[17 + 2 * j]);
-              *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
-              *reinterpret_cast<uint4*>(dst + 8) = make_uint4(o[4], o[5], o[6], o[7]);
-            } else if (p.epi == EPI_F32) {
-              float* dst = reinterpret_cast<float*>(p.C) + (size_t)grow * p.ldc + n0;
-              if (n0 + 32 <= p.N) {
-  #pragma unroll
-                for (int j = 0; j < 8; ++j)
-                  *reinterpret_cast<float4*>(dst + 4 * j) = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
-              } else {
-                for (int j = 0; j < 32 && n0 + j < p.N; ++j) dst[j] = f[j];
-              }
-            } else {
-              __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)grow * p.ldc + n0;
-              if (p.epi == EPI_RESID_ADD) {
-                const __nv_bfloat16* rs = p.resid + (size_t)grow * p.ldc + n0;
-                if (n0 + 32 <= p.N) {
-  #pragma unroll
-                  for (int j = 0; j < 4; ++j) {
-                    const uint4 rv = *reinterpret_cast<const uint4*>(rs + 8 * j);
-                    const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
-  #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                      f[8 * j + 2 * q] += bf16_lo(rw[q]);
-                      f[8 * j + 2 * q + 1] += bf16_hi(rw[q]);
-                    }
-                  }
-                } else {
-                  for (int j = 0; j < 32 && n0 + j < p.N; ++j) f[j] += __bfloat162float(rs[j]);
-                }
-              }
-              if (p.epi == EPI_RELU2) {
-  #pragma unroll
-                for (int j = 0; j < 32; ++j) f[j] = relu2(f[j]);
-              }
-              if (n0 + 32 <= p.N) {
-  #pragma unroll
-                for (int j = 0; j < 4; ++j)
-                  *reinterpret_cast<uint4*>(dst + 8 * j) =
-                      make_uint4(pack_bf16(f[8 * j], f[8 * j + 1]), pack_bf16(f[8 * j + 2], f[8 * j + 3]),
-                                 pack_bf16(f[8 * j + 4], f[8 * j + 5]), pack_bf16(f[8 * j + 6], f[8 * j + 7]));
-              } else {
-                for (int j = 0; j < 32 && n0 + j < p.N; ++j) dst[j] = __float2bfloat16(f[j]);
-              }
-            }
+  float f[32];
+#pragma unroll
+  for (int j = 0; j < 32; ++j) f[j] = __uint_as_float(v[j]);
+  if (p.epi == EPI_SILU_MUL || p.epi == EPI_GLU) {
+    // columns alternate 16 gate, 16 up: 16 outputs per 32 accumulator columns
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)grow * p.ldc + (n0 >> 1);
+    uint32_t o[8];
+    if (p.epi == EPI_GLU && p.glu.bias) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 b = __ldg(reinterpret_cast<const float4*>(p.glu.bias + n0) + j);
+        f[4 * j] += b.x; f[4 * j + 1] += b.y; f[4 * j + 2] += b.z; f[4 * j + 3] += b.w;
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      o[j] = p.epi == EPI_GLU ? pack_bf16(glu(p.glu, f[2 * j], f[16 + 2 * j]), glu(p.glu, f[2 * j + 1], f[17 + 2 * j]))
+                              : pack_bf16(silu(f[2 * j]) * f[16 + 2 * j], silu(f[2 * j + 1]) * f[17 + 2 * j]);
+    *reinterpret_cast<uint4*>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4*>(dst + 8) = make_uint4(o[4], o[5], o[6], o[7]);
+  } else if (p.epi == EPI_F32) {
+    float* dst = reinterpret_cast<float*>(p.C) + (size_t)grow * p.ldc + n0;
+    if (n0 + 32 <= p.N) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<float4*>(dst + 4 * j) = make_float4(f[4 * j], f[4 * j + 1], f[4 * j + 2], f[4 * j + 3]);
+    } else {
+      for (int j = 0; j < 32 && n0 + j < p.N; ++j) dst[j] = f[j];
+    }
+  } else {
+    __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.C) + (size_t)grow * p.ldc + n0;
+    if (p.epi == EPI_RESID_ADD) {
+      const __nv_bfloat16* rs = p.resid + (size_t)grow * p.ldc + n0;
+      if (n0 + 32 <= p.N) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint4 rv = *reinterpret_cast<const uint4*>(rs + 8 * j);
+          const uint32_t rw[4] = {rv.x, rv.y, rv.z, rv.w};
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            f[8 * j + 2 * q] += bf16_lo(rw[q]);
+            f[8 * j + 2 * q + 1] += bf16_hi(rw[q]);
+          }
+        }
+      } else {
+        for (int j = 0; j < 32 && n0 + j < p.N; ++j) f[j] += __bfloat162float(rs[j]);
+      }
+    }
+    if (p.epi == EPI_RELU2) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) f[j] = relu2(f[j]);
+    }
+    if (n0 + 32 <= p.N) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<uint4*>(dst + 8 * j) =
+            make_uint4(pack_bf16(f[8 * j], f[8 * j + 1]), pack_bf16(f[8 * j + 2], f[8 * j + 3]),
+                       pack_bf16(f[8 * j + 4], f[8 * j + 5]), pack_bf16(f[8 * j + 6], f[8 * j + 7]));
+    } else {
+      for (int j = 0; j < 32 && n0 + j < p.N; ++j) dst[j] = __float2bfloat16(f[j]);
+    }
+  }
 }
 
 // Vector `u` of a stage's W4B blocks (256 vectors a block) -> sixteen 8-byte pieces of the bf16 B tile.  A vector holds rows g and
 // g + 8 of a 16-row tile, 64 k: low nibbles are k 4t..4t+3 of a 32-k step, high nibbles k + 16 (the operand order of the decode
 // GEMV); row r lies at r * 128 bytes, 16-byte chunk (k / 8) XOR (r mod 8) -- the 128-byte swizzle.
 __device__ __forceinline__ void expand_w4(int u, uint32_t raw, uint32_t sb) {
-            const int b = u >> 8, v = u & 255, j = v >> 5, l = v & 31, g = l >> 2, tq = l & 3;
-            uint4 wv;
-            asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w)
-                         : "r"(raw + b * kW4Block + v * 16));
-            uint32_t sc2;
-            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc2) : "r"(raw + b * kW4Block + 4096 + (j * 16 + 2 * g) * 2));
-            const __half2 sh = *reinterpret_cast<const __half2*>(&sc2);
-            const float s_lo = __low2float(sh), s_hi = __high2float(sh);
-            const uint32_t wa[4] = {wv.x, wv.y, wv.z, wv.w};
-            uint64_t sc2x[2], off2;
-            asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[0]) : "f"(s_lo));
-            asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[1]) : "f"(s_hi));
-            asm("mov.b64 %0, {%1, %1};" : "=l"(off2) : "f"(-8388616.f));
-  #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const int row = b * 128 + j * 16 + g + 8 * (c & 1);
-  #pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const uint32_t x = (wa[c] >> (4 * e)) & 0x0F0F0F0Fu;
-                // bytes -> floats through the 2^23 trick: 0x4B0000qq is 8388608 + q; q - 8 (exact) and the product with
-                // the scale run as packed pairs (add.f32x2 / mul.f32x2), the same floats as the scalar form
-                uint64_t f01, f23;
-                asm("mov.b64 %0, {%1, %2};" : "=l"(f01) : "r"(__byte_perm(x, 0x4B000000u, 0x7440)), "r"(__byte_perm(x, 0x4B000000u, 0x7441)));
-                asm("mov.b64 %0, {%1, %2};" : "=l"(f23) : "r"(__byte_perm(x, 0x4B000000u, 0x7442)), "r"(__byte_perm(x, 0x4B000000u, 0x7443)));
-                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(off2));
-                asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(off2));
-                asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(sc2x[c & 1]));
-                asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(sc2x[c & 1]));
-                float g0, g1, g2, g3;
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(g0), "=f"(g1) : "l"(f01));
-                asm("mov.b64 {%0, %1}, %2;" : "=f"(g2), "=f"(g3) : "l"(f23));
-                const uint32_t p01 = pack_bf16(g0, g1);
-                const uint32_t p23 = pack_bf16(g2, g3);
-                const int k0 = 32 * (c >> 1) + 16 * e + 4 * tq;
-                const uint32_t dst = sb + row * 128 + ((((uint32_t)k0 >> 3) ^ ((uint32_t)row & 7u)) << 4) + (k0 & 7) * 2;
-                asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst), "r"(p01), "r"(p23) : "memory");
-              }
-            }
+  const int b = u >> 8, v = u & 255, j = v >> 5, l = v & 31, g = l >> 2, tq = l & 3;
+  uint4 wv;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(wv.x), "=r"(wv.y), "=r"(wv.z), "=r"(wv.w)
+               : "r"(raw + b * kW4Block + v * 16));
+  uint32_t sc2;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc2) : "r"(raw + b * kW4Block + 4096 + (j * 16 + 2 * g) * 2));
+  const __half2 sh = *reinterpret_cast<const __half2*>(&sc2);
+  const float s_lo = __low2float(sh), s_hi = __high2float(sh);
+  const uint32_t wa[4] = {wv.x, wv.y, wv.z, wv.w};
+  uint64_t sc2x[2], off2;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[0]) : "f"(s_lo));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[1]) : "f"(s_hi));
+  asm("mov.b64 %0, {%1, %1};" : "=l"(off2) : "f"(-8388616.f));
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int row = b * 128 + j * 16 + g + 8 * (c & 1);
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const uint32_t x = (wa[c] >> (4 * e)) & 0x0F0F0F0Fu;
+      // bytes -> floats through the 2^23 trick: 0x4B0000qq is 8388608 + q; q - 8 (exact) and the product with
+      // the scale run as packed pairs (add.f32x2 / mul.f32x2), the same floats as the scalar form
+      uint64_t f01, f23;
+      asm("mov.b64 %0, {%1, %2};" : "=l"(f01) : "r"(__byte_perm(x, 0x4B000000u, 0x7440)), "r"(__byte_perm(x, 0x4B000000u, 0x7441)));
+      asm("mov.b64 %0, {%1, %2};" : "=l"(f23) : "r"(__byte_perm(x, 0x4B000000u, 0x7442)), "r"(__byte_perm(x, 0x4B000000u, 0x7443)));
+      asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(off2));
+      asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(off2));
+      asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(sc2x[c & 1]));
+      asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(sc2x[c & 1]));
+      float g0, g1, g2, g3;
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(g0), "=f"(g1) : "l"(f01));
+      asm("mov.b64 {%0, %1}, %2;" : "=f"(g2), "=f"(g3) : "l"(f23));
+      const uint32_t p01 = pack_bf16(g0, g1);
+      const uint32_t p23 = pack_bf16(g2, g3);
+      const int k0 = 32 * (c >> 1) + 16 * e + 4 * tq;
+      const uint32_t dst = sb + row * 128 + ((((uint32_t)k0 >> 3) ^ ((uint32_t)row & 7u)) << 4) + (k0 & 7) * 2;
+      asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst), "r"(p01), "r"(p23) : "memory");
+    }
+  }
 }
 
 template <int BN, bool I8, bool W4 = false>
