@@ -10,7 +10,7 @@
 // start, first copies and partials cost about as much as kFixedPages.  It ranks what was measured: 24 requests at 1000 to 2000
 // positions with 1, 2, 3, 4 splits each 57, 51, 46, 51 us, 8 at 2000 to 4000 with 1, 2, 4, 8, 10 73, 42, 39, 41, 47.
 // One CTA of at least 64 threads, thread i standing for row i and for k = i + 1.  As a launch of its own of 1024 threads, which tried all k at
-// once, it took 8 us of every step; as one more CTA of the embedding's launch it takes up to 1.
+// once, it took 8 us of every step; as one more CTA of the embedding's launch it adds 1 (2 to 8 rows) to 4 (40 rows).
 #pragma once
 #include "common.cuh"
 
@@ -28,6 +28,7 @@ __device__ __forceinline__ void attn_plan(const AttnPlanParams& p) {
   constexpr int kReq = 16, kPos = 80;      // words of the control block
   __shared__ int s_req[64], s_pos[64], s_pages[64], s_n[64], s_piece[64];
   __shared__ unsigned s_best[2], s_start[2];
+  __shared__ int s_top[2], s_sum[2];
   const int i = threadIdx.x;
   if (i < 64) {
     s_req[i] = i < p.M ? __ldcg(p.ctrl + kReq + i) : -1;
@@ -51,22 +52,22 @@ __device__ __forceinline__ void attn_plan(const AttnPlanParams& p) {
     }
   }
   s_pages[i] = pages;
+  const int top = __reduce_max_sync(0xffffffffu, pages), sum = __reduce_add_sync(0xffffffffu, pages);
+  if ((i & 31) == 0) s_top[i >> 5] = top, s_sum[i >> 5] = sum;
   sync();
-  int longest = 0, total = 0;
-  for (int j = 0; j < p.M; ++j) {
-    longest = max(longest, s_pages[j]);
-    total += s_pages[j];
-  }
+  const int longest = max(s_top[0], s_top[1]), total = s_sum[0] + s_sum[1];
   const auto ceil_div = [](int a, int b) { return (a + b - 1) / b; };
   unsigned best = ~0u;
   if (i < min(p.nsplit, longest)) {
     const int span = ceil_div(longest, i + 1);
     const float inv = 1.f / (float)span;
     int n = 0;
-    for (int j = 0; j < p.M; ++j) {         // ceil(pages / span): a quotient that is off by one at most, put right
-      const int a = s_pages[j], q = (int)((float)a * inv), r = a - q * span;
-      n += q + (r > 0) + (r > span);
-    }
+    for (int j0 = 0; j0 < p.M; j0 += 8)
+#pragma unroll
+      for (int j = j0; j < j0 + 8; ++j) {   // ceil(pages / span): a quotient that is off by one at most, put right
+        const int a = s_pages[j], q = (int)((float)a * inv), r = a - q * span;
+        n += q + (r > 0) + (r > span);
+      }
     if (n <= p.entries) best = (unsigned)max(kPlanFixedPages + span, ceil_div(n * p.n_kv, kPlanSlots) * (kPlanFixedPages + ceil_div(total, n))) << 7 | (i + 1);
   }
   best = __reduce_min_sync(0xffffffffu, best);
@@ -79,7 +80,9 @@ __device__ __forceinline__ void attn_plan(const AttnPlanParams& p) {
   sync();
   for (int r = 0; r < rows; ++r) p.plan[i + r] = n;
   int at = 0;                               // longest pieces first
-  for (int j = 0; j < p.M; ++j) at += s_piece[j] > piece || (s_piece[j] == piece && j < i) ? s_n[j] : 0;
+  for (int j0 = 0; j0 < p.M; j0 += 8)
+#pragma unroll
+    for (int j = j0; j < j0 + 8; ++j) at += s_piece[j] > piece || (s_piece[j] == piece && j < i) ? s_n[j] : 0;
   for (int s = 0; s < n; ++s) p.plan[64 + at + s] = i | s << 8 | n << 16;
 }
 
