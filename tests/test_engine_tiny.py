@@ -167,3 +167,35 @@ def test_qkv_gemv_with_rope_and_kv_append_fold_matches_separate_kernel():
     ta, tb = a.generate(prompt, 16), b.generate(prompt, 16)
     assert ta == tb
     assert torch.equal(a.logits(1), b.logits(1))
+
+
+@pytest.mark.parametrize("family,kv", [("small-dense", "bf16"), ("small-dense", "int8"), ("small-windowed", "bf16"), ("small-hybrid", "bf16")])
+@pytest.mark.parametrize("graphs", [False, True])
+def test_step_of_uneven_requests(family, kv, graphs):
+    """Contexts of 3 to 900 positions in one step, then one request with several rows beside others: every row's logits as alone."""
+    from b200serve.models.config import preset
+    from b200serve.ops import lib as K
+    from b200serve.runtime.engine import Engine, Row
+    cfg = preset(family)
+    lengths = [3, 900, 17, 64, 250, 1]
+    g = torch.Generator().manual_seed(7)
+    ids = [torch.randint(0, cfg.vocab, (n + 5,), generator=g).tolist() for n in lengths]
+    eng = Engine(random_weights(cfg, device="cuda", seed=3), max_seqs=len(ids), max_len=1024, kv_dtype=kv, use_graphs=graphs)
+    alone = Engine(random_weights(cfg, device="cuda", seed=3), max_seqs=len(ids), max_len=1024, kv_dtype=kv, use_graphs=graphs)
+    for e in (eng, alone):
+        for s, t in enumerate(ids):
+            e.prefill(s, t[: lengths[s]])
+    for rows_of in ([1] * 6, [1, 1, 4, 1, 2, 1], [1, 2, 0, 1, 2, 0]):
+        rows = [Row(s, eng.seq_len[s] + i, ids[s][(eng.seq_len[s] + i) % len(ids[s])]) for s, n in enumerate(rows_of) for i in range(n)]
+        eng.forward_rows(rows)
+        got = eng.logits(len(rows)).clone()
+        want = []
+        for s in range(len(ids)):
+            mine = [r for r in rows if r.slot == s]
+            if mine:
+                alone.forward_rows(mine)
+                want.append(alone.logits(len(mine)).clone())
+        want = torch.cat(want)
+        K.check_status()
+        # bf16 activations in every layer, products of int8 rows: as far as the oracle's comparisons allow
+        assert (got - want).abs().max() < 0.04 * want.abs().max()
