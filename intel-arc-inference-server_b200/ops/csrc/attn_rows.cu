@@ -17,11 +17,13 @@
 //     slices are merged in slice order through shared memory before the split's partial is written;
 //   * split-KV partials and the in-kernel merge by the last CTA ("ticket") have the layout and the fixed
 //     split order of the per-row kernel, so either kernel can serve a row.
-// An int8 cache (one fp32 scale per row) is staged as int8.  Groups of up to 32 query rows multiply it as it is: a warp reads the
+// An int8 cache (one fp32 scale per row) is staged as int8.  Groups of up to 16 query rows multiply it as it is: a warp reads the
 // bytes of its own keys in the MMA's layout and makes them integers in bf16, which are exact, in registers; K's scale goes on
 // the products and V's on the probabilities, both in fp32.  Nothing is written back to shared memory, so it holds three
-// batches in flight.  Beyond 32 query rows, where several warps would make the same integers, the thread that owns a key
-// expands its row to bf16 tiles and the bf16 path follows.
+// batches in flight.  Beyond 16 query rows several warps would make the same integers: the thread that owns a key
+// expands its row to bf16 tiles and the bf16 path follows, with integers and scales as before up to 32 query rows, with scaled values
+// beyond.  One request, 40 / 8 heads, 5 rows (25 query rows) at 500, 4000 and 16000 positions: 9.8 / 11.9 / 31.0 us from registers,
+// 9.2 / 10.8 / 28.5 from tiles; one row 6.4 / 7.5 / 18.4 from registers, 7.4 / 8.5 / 22.6 from tiles.
 // The role of the reference's verify attention (src/kernels/attn_verify_dpas.cl) and of its decode
 // attention's GQA packing (src/kernels/attn_v2.cl).
 #include "attn_plan.cuh"
@@ -98,7 +100,7 @@ __device__ __forceinline__ uint32_t bytes_bf16(uint32_t w) {
 template <bool I8, int NKS>
 __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t* smem_raw, const int* s_pos, int* s_last_p, int* s_bt,
                                                const int req, const int rows, const int QR, const int ctx_max, const int z,
-                                               const int split, const int nsp) {
+                                               const int split, const int nsp, float* s_scale) {
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;   // the swizzle pattern repeats every 1024 bytes
   // bf16 form: nbuf pairs of operand tiles.  int8 form: one pair of operand tiles, nbuf pairs of staged int8 rows.
   const int ntile = I8 ? 1 : p.nbuf;
@@ -109,7 +111,8 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
   int& s_last = *s_last_p;
   // The bytes go into the MMA's operands from registers (8 requests at up to 4000 positions, 16 layers: a step of 2.38 -> 2.13 ms;
   // the expansion took longer than the bytes' way from HBM and everything else waited for it)
-  constexpr bool kDirect = I8 && NKS > 1;
+  constexpr bool kDirect = I8 && NKS == 4;
+  constexpr bool kExact = I8 && NKS == 2;   // integers in the tiles, their scales in s_scale ([2][KB]: K's with the softmax's factor, V's)
   const int nst = 2 + p.nbuf;     // then: batches in flight, in the tiles' memory too
   constexpr int NRG = 4 / NKS;    // groups of 16 query rows
   constexpr int KW = KB / NKS;              // keys per warp and batch
@@ -331,11 +334,15 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
       }
       if (okw) okw = mbar_wait(bar, (batch / p.nbuf) & 1, ERR_ATTN_WAIT);
       if (I8) {
-        // every thread expands its own key's row: int8 x per-row scale -> bf16 into the operand tiles
+        // every thread expands its own key's row: int8 (x per-row scale) -> bf16 into the operand tiles
         if (tid >= nk) {   // rows without a key: V must be finite (its products are multiplied by P = 0)
 #pragma unroll
           for (int i = 0; i < 16; ++i)
             asm volatile("st.shared.v4.u32 [%0], {%1,%1,%1,%1};" ::"r"(vs + (i >> 3) * HALFB + tid * 128 + 16 * (i & 7)), "r"(0) : "memory");
+        }
+        if (kExact) {
+          s_scale[tid] = tid < nk ? ksc[buf] * p.scale_log2 : 0.f;
+          s_scale[KB + tid] = tid < nk ? vsc[buf] : 0.f;
         }
         if (okw && tid < nk) {
 #pragma unroll
@@ -350,6 +357,12 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
               uint32_t o[8];
 #pragma unroll
               for (int j = 0; j < 4; ++j) {
+                if (kExact) {
+                  const uint32_t ev = bytes_bf16(ww[j]), od = bytes_bf16(ww[j] >> 8);
+                  o[2 * j] = __byte_perm(ev, od, 0x5410);
+                  o[2 * j + 1] = __byte_perm(ev, od, 0x7632);
+                  continue;
+                }
                 // int8 -> fp32 without the conversion unit (a quarter-rate pipe that capped this loop): the byte, biased
                 // to 0..255, dropped into the mantissa of 2^23 is 8388608 + u, and subtracting 8388736 leaves the signed
                 // value exactly -- the same floats as (float)(int8_t), so the same products
@@ -396,7 +409,8 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
         for (int e = 0; e < 4; ++e) {
           const int key = kb0 + kofs + 8 * j + 2 * t + (e & 1);
           const int hf = e >> 1;
-          const float v = key < ctx[hf] && key < key1 && key >= wlo[hf] ? s[j][e] * p.scale_log2 : -INFINITY;
+          const float sc = kExact ? s_scale[kofs + 8 * j + 2 * t + (e & 1)] : p.scale_log2;
+          const float v = key < ctx[hf] && key < key1 && key >= wlo[hf] ? s[j][e] * sc : -INFINITY;
           s[j][e] = v;
           mnew[hf] = fmaxf(mnew[hf], v);
         }
@@ -422,7 +436,7 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
         for (int e = 0; e < 4; ++e) {
           const int hf = e >> 1;
           const float pe = mnew[hf] == -INFINITY ? 0.f : exp2f(s[j][e] - mnew[hf]);
-          s[j][e] = pe;
+          s[j][e] = kExact ? pe * s_scale[KB + kofs + 8 * j + 2 * t + (e & 1)] : pe;
           lsum[hf] += pe;
         }
       // ---- O += P V: NJ / 2 k16 steps over this warp's keys, 16 n8 tiles over d
@@ -611,6 +625,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const __grid_con
   int rows = 1;
   while (rows < rmax && z + rows < p.M && s_req[z + rows] == req) ++rows;
   const int QR = rows * p.gqa;
+  __shared__ float s_scale[2 * KB];
   int ctx_max = 0;
   for (int r = 0; r < rows; ++r) ctx_max = max(ctx_max, s_pos[z + r] + 1);
   if (p.block) {           // a block row sees every position of its REQUEST's rows in this step, also those a
@@ -621,11 +636,11 @@ __global__ void __launch_bounds__(kThreads, 2) attn_rows_kernel(const __grid_con
     __syncthreads();
   }
   if (QR <= 16 && !p.one_slice)
-    attn_rows_body<I8, 4>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z, split, nsp);
+    attn_rows_body<I8, 4>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z, split, nsp, s_scale);
   else if (QR <= 32 && !p.one_slice)
-    attn_rows_body<I8, 2>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z, split, nsp);
+    attn_rows_body<I8, 2>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z, split, nsp, s_scale);
   else
-    attn_rows_body<I8, 1>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z, split, nsp);
+    attn_rows_body<I8, 1>(p, smem_raw, s_pos, &s_last, s_bt, req, rows, QR, ctx_max, z, split, nsp, s_scale);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
