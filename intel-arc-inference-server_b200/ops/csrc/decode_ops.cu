@@ -626,11 +626,12 @@ __global__ void __launch_bounds__(256) attn_decode_kernel(const AttnDecParams p)
 // bits), which saves that launch in a step of several rows; without xq_gs, as the bf16 rows of the tcgen05 form
 // (stage_rows_kernel, gs_rows token rows per group).  counts: [M] splits that a row has of the nsplit (<= 64) places, or nullptr:
 // all of them.
-template <int V>
+template <int V, int DIM, bool COUNTED>
 __global__ void attn_merge_kernel(const float* o_part, const float* ml_part, __nv_bfloat16* out, int n_q, int nsplit,
-                                  int D, uint8_t* xq, uint32_t* xq_gs, int gs_rows, const int* counts) {
+                                  int dim, uint8_t* xq, uint32_t* xq_gs, int gs_rows, const int* counts) {
   __shared__ float cw[64];
   __shared__ __align__(16) __nv_bfloat16 srow[128];
+  const int D = DIM ? DIM : dim;
   pdl_wait();
   pdl_launch_dependents();
   const int h = blockIdx.x, m = blockIdx.y, d = threadIdx.x;
@@ -639,7 +640,7 @@ __global__ void attn_merge_kernel(const float* o_part, const float* ml_part, __n
   if (nsplit <= 64) {
     // weights of the splits once per CTA (one lane per split), then every thread's loads are independent.  The first 32 splits'
     // values are requested before the weights are known: one round trip for both; of places that may not be a row's, eight
-    const int n = counts ? counts[m] : nsplit, sure = counts ? min(nsplit, 8) : nsplit;
+    const int n = COUNTED ? counts[m] : nsplit, sure = COUNTED ? min(nsplit, 8) : nsplit;
     const float* src = o_part + base * D + d;
     float v0[V];
 #pragma unroll
@@ -649,7 +650,7 @@ __global__ void attn_merge_kernel(const float* o_part, const float* ml_part, __n
       if (d < nsplit) m0 = ml_part[(base + d) * 2], l0 = ml_part[(base + d) * 2 + 1];
       if (d + 32 < nsplit) m1 = ml_part[(base + d + 32) * 2], l1 = ml_part[(base + d + 32) * 2 + 1];
     }
-    if (counts) {
+    if (COUNTED) {
 #pragma unroll
       for (int u = 0; u < V; ++u) {
         if (u >= n) v0[u] = 0.f;
@@ -1225,11 +1226,13 @@ static int attn_decode_dispatch(int gqa, const AttnDecParams& p, dim3 grid, cuda
 }
 
 // Few rows of many splits: all values of 32 splits in flight.  Rows enough to fill the GPU, or few splits: 16 at a time leave room for
-// twice the CTAs (121 / 56 registers).  Attention and merge of 5 rows of 40 heads in 37 splits 16.9 -> 14.1 us, whose values were asked for
-// behind the weights before; of 64 rows in 2 splits 37.9 -> 34.2.
+// more CTAs (56 / 40 registers; with a head size that is known only at run time, whose 32 addresses are computed, it took 121 and stood in the
+// way of the next attention's CTAs).  Merge of 5 / 64 rows of 40 heads in 37 splits 3.6 / 13.1 -> 2.8 / 8.5 us; attention and merge of 5 rows at
+// 1500 positions 16.9 -> 14.1, at 4000 17.9 -> 15.2.
 static int merge_launch(const float* o_part, const float* ml_part, void* out, int M, int n_q, int nsplit, int D, void* xq, void* xq_gs,
                         int gs_rows, const int* counts, cudaStream_t st) {
-  return b2_launch(counts || nsplit <= 16 ? attn_merge_kernel<16> : attn_merge_kernel<32>, dim3(n_q, M), dim3(D), 0, st, true, o_part, ml_part,
+  const auto kernel = D != 128 ? attn_merge_kernel<16, 0, false> : counts ? attn_merge_kernel<16, 128, true> : nsplit <= 16 ? attn_merge_kernel<16, 128, false> : attn_merge_kernel<32, 128, false>;
+  return b2_launch(kernel, dim3(n_q, M), dim3(D), 0, st, true, o_part, ml_part,
                    (__nv_bfloat16*)out, n_q, nsplit, D, (uint8_t*)xq, (uint32_t*)xq_gs, gs_rows, counts);
 }
 
