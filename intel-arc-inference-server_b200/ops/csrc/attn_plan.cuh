@@ -24,11 +24,17 @@ struct AttnPlanParams {
 
 constexpr int kPlanFixedPages = 8, kPlanSlots = 296;
 
-__device__ __forceinline__ void attn_plan(const AttnPlanParams& p) {
+struct AttnPlanShared {      // the caller's: beside an embedding it takes the place of a row's values, whose width may need all there is
+  int req[64], pos[64], pages[64], n[64], piece[64];
+  unsigned best[2], start[2];
+  int top[2], sum[2];
+};
+
+__device__ __forceinline__ void attn_plan(const AttnPlanParams& p, AttnPlanShared& sh) {
   constexpr int kReq = 16, kPos = 80;      // words of the control block
-  __shared__ int s_req[64], s_pos[64], s_pages[64], s_n[64], s_piece[64];
-  __shared__ unsigned s_best[2], s_start[2];
-  __shared__ int s_top[2], s_sum[2];
+  auto &s_req = sh.req, &s_pos = sh.pos, &s_pages = sh.pages, &s_n = sh.n, &s_piece = sh.piece;
+  auto &s_best = sh.best, &s_start = sh.start;
+  auto &s_top = sh.top, &s_sum = sh.sum;
   const int i = threadIdx.x;
   if (i < 64) {
     s_req[i] = i < p.M ? __ldcg(p.ctrl + kReq + i) : -1;

@@ -584,9 +584,10 @@ __device__ __forceinline__ void attn_rows_body(const AttnRowsParams& p, uint8_t*
 }
 
 __global__ void __launch_bounds__(64) attn_plan_kernel(const AttnPlanParams p) {
+  __shared__ AttnPlanShared shared;
   pdl_wait();
   pdl_launch_dependents();
-  attn_plan(p);
+  attn_plan(p, shared);
 }
 
 template <bool I8>

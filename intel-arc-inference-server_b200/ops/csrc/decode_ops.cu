@@ -124,6 +124,7 @@ __global__ void __launch_bounds__(1024) resid_norm_kernel(const ResidNormParams 
 }
 
 __global__ void __launch_bounds__(1024) embed_plan_kernel(const EmbedPlanParams p) {
+  extern __shared__ float vals[];
   pdl_wait();
   pdl_launch_dependents();
   if (blockIdx.x < p.plan.M) {
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(1024) embed_plan_kernel(const EmbedPlanParams 
     a.window = p.window;
     a.plan = p.plan_win;
   }
-  attn_plan(a);
+  attn_plan(a, *reinterpret_cast<AttnPlanShared*>(vals));
 }
 
 // Norm of a prompt's rows (no partials to fold): a warp per row, the row in registers, its loads all in flight, no barrier
@@ -1181,7 +1182,7 @@ extern "C" int b2_embed_plan(const void* embed, const int* ctrl, int M, int H, i
   p.window = window; p.plan_win = plan_win;
   if (H % 8 || (plan_win && window < 1) || !attn_plan_params(p.plan, ctrl, M, n_q, n_kv, nsplit, 0, plan, entries)) return -1;
   const int threads = min(1024, max(64, (H / 8 + 31) / 32 * 32));
-  return b2_launch(embed_plan_kernel, dim3(M + (plan_win ? 2 : 1)), dim3(threads), (size_t)H * 4, (cudaStream_t)stream, true, p);
+  return b2_launch(embed_plan_kernel, dim3(M + (plan_win ? 2 : 1)), dim3(threads), max((size_t)H * 4, sizeof(AttnPlanShared)), (cudaStream_t)stream, true, p);
 }
 
 extern "C" int b2_draft_front(const void* embed, const int* ctrl, int vocab, const void* hidden, long long hidden_ld,

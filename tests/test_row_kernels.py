@@ -401,9 +401,9 @@ def test_attention_splits_by_length(spec, nq, nkv, most, window, kv):
             assert ((got[i].double().view(nkv, gqa, d) - want).abs() <= bound + 1e-9).all()
 
 
-@pytest.mark.parametrize("m,h,window", [(2, 64, 0), (17, 512, 0), (64, 5120, 300), (5, 9000, 64)])
+@pytest.mark.parametrize("m,h,window", [(2, 64, 0), (17, 512, 0), (64, 5120, 300), (5, 9000, 64), (3, 12224, 0), (3, 12224, 64)])
 def test_plan_beside_the_embedding(m, h, window):
-    """One launch with the rows and the tables of the launches it stands for."""
+    """One launch with the rows and the tables of the launches it stands for, up to the widest row that those take."""
     torch.manual_seed(m)
     nq, nkv, most, vocab = 10, 2, 37, 50
     ctrl = _ctrl([i // 2 for i in range(m)])
