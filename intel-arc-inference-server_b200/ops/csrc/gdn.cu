@@ -771,9 +771,11 @@ extern "C" int b2_gdn_conv(const float* part, int splits, int M, int N, int conv
   if (M < 1 || (ctrl && M > 64) || (!ctrl && slot < 0) || splits < 1 || conv_ch > N) return -1;
   GdnConvParams p{part, splits, M, N, conv_ch, ctrl, slot, conv_w, conv_state, act};
   // four columns per thread need whole, aligned 16-byte pieces of every row; a chunk needs its last three inputs in itself.
-  // (The other shapes, odd numbers of value heads among them, keep one column per thread and the rows in order.)
+  // (The other shapes, odd numbers of value heads among them, keep one column per thread and the rows in order.  So does a chunk
+  // that is convolved in place: its rows would be replaced before the CTA below them has read them.)
+  const bool apart = act + (size_t)M * N <= part || part + (size_t)splits * M * N <= act;
   const uintptr_t at = (uintptr_t)part | (uintptr_t)conv_w | (uintptr_t)conv_state | (uintptr_t)act;
-  if (N % 4 == 0 && conv_ch % 4 == 0 && at % 16 == 0 && (ctrl || M >= 3)) {
+  if (N % 4 == 0 && conv_ch % 4 == 0 && at % 16 == 0 && (ctrl || (M >= 3 && apart))) {
     const dim3 grid((N / 4 + CONV_T - 1) / CONV_T, ctrl ? M : (M + CONV_R - 1) / CONV_R);
     if (grid.y <= 65535u) return b2_launch(gdn_conv_rows_kernel, grid, dim3(CONV_T), 0, (cudaStream_t)stream, true, p);
   }

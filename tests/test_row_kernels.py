@@ -45,6 +45,23 @@ def test_convolution_over_rows(rows, nk, nv, splits):
     assert (st.double().cpu() - ref_state).abs().max() < 1e-5
 
 
+@pytest.mark.parametrize("rows", [3, 40, 700, [1, 0, 1, 1, 2]])
+def test_convolution_in_place(rows):
+    """The activations in the projection's own memory: the values of a buffer of its own."""
+    torch.manual_seed(rows if isinstance(rows, int) else 5)
+    slots = rows if isinstance(rows, list) else [1] * rows
+    m, cc = len(slots), 1024
+    n = cc + 520
+    part, conv_w, state = torch.randn(m, n, device="cuda"), torch.randn(cc, 4, device="cuda") * 0.5, torch.randn(3, cc, 3, device="cuda")
+    ctrl = _ctrl(slots) if isinstance(rows, list) else None
+    act, st, here = torch.empty_like(part), state.clone(), part.clone()
+    K.gdn_conv(part, 1, m, n, cc, ctrl, conv_w, st, act, slot=1)
+    K.gdn_conv(here, 1, m, n, cc, ctrl, conv_w, state, here, slot=1)
+    torch.cuda.synchronize()
+    # four products and a SiLU of values up to ~10, which one form may contract to fmas where the other does not
+    assert (act - here).abs().max() < 1e-5 and torch.equal(st, state)
+
+
 @pytest.mark.parametrize("slots", [[0], [2, 0, 1], [1, 1, 1, 0, 0, 2], [0, 1, 0, 2, 1, 0], list(range(3)) * 5])
 def test_delta_step_per_slot(slots):
     """Slots interleaved in any order: every slot's rows in order, no slot touched that has none."""
