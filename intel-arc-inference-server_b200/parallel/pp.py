@@ -25,6 +25,7 @@ from ..models.config import ModelConfig
 from ..models.weights import ModelWeights, random_weights
 from ..ops import lib as K
 from ..runtime.engine import Engine, Row
+from ..utils.graphs import capture
 
 
 def split_layers(n_layers: int, stages: int, head_cost: float = 1.5) -> List[Tuple[int, int]]:
@@ -115,9 +116,7 @@ class PipelineEngine(Engine):
             if rows_in is not None:
                 b.resid[:m].copy_(rows_in[0])
                 b.ssq.copy_(rows_in[1])
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
-                self._stage_body(m, advance)
+            g = capture(lambda: self._stage_body(m, advance))
             self.ctrl.copy_(saved)
             self._stage_graph[key] = g
         g.replay()

@@ -11,7 +11,6 @@ sequence is.
 """
 from __future__ import annotations
 
-import gc
 from dataclasses import dataclass
 from typing import Dict, List, Optional, Sequence, Tuple
 
@@ -22,6 +21,7 @@ from ..models.config import ModelConfig
 from ..models.decoder import DecoderModel, KVCache, attn_splits
 from ..models.weights import ModelWeights
 from ..ops import lib as K
+from ..utils.graphs import capture
 from ..utils.staging import Staged
 from .kv_pool import KvPool
 
@@ -242,17 +242,7 @@ class Engine:
             self.ctrl.copy_(saved)
             for n, t in saved_states.items():
                 self.kv.states[n].copy_(t)
-            g = torch.cuda.CUDAGraph()
-            # no garbage collection while the stream captures: a dead engine's graphs and buffers released in the middle
-            # of it abort the process
-            collects = gc.isenabled()
-            gc.disable()
-            try:
-                with torch.cuda.graph(g):
-                    self._enqueue(m, advance)
-            finally:
-                if collects:
-                    gc.enable()
+            g = capture(lambda: self._enqueue(m, advance))
             self.ctrl.copy_(saved)
             self.graphs[key] = g
         g.replay()

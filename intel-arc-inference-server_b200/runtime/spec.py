@@ -28,6 +28,7 @@ from ..models.weights import MtpWeights, QLinear, _norm_weight, _rand_layer
 from ..ops import dflash as DF
 from ..ops import gemm as G
 from ..ops import lib as K
+from ..utils.graphs import capture
 from .engine import Engine, Row
 
 
@@ -223,9 +224,7 @@ class DraftHead:
             torch.cuda.current_stream().synchronize()
             for dst, src in zip((eng.ctrl, self.hid_in, self.draft_n, self.draft_list), saved):
                 dst.copy_(src)
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g):
-                self._enqueue(n, chain, block)
+            g = capture(lambda: self._enqueue(n, chain, block))
             for dst, src in zip((eng.ctrl, self.hid_in, self.draft_n, self.draft_list), saved):
                 dst.copy_(src)               # KV rows written by the warm-up and the capture are rewritten by the replay
             self.graphs[key] = g

@@ -199,3 +199,28 @@ def test_step_of_uneven_requests(family, kv, graphs):
         K.check_status()
         # bf16 activations in every layer, products of int8 rows: as far as the oracle's comparisons allow
         assert (got - want).abs().max() < 0.04 * want.abs().max()
+
+
+def test_capture_beside_a_thread_that_frees_graphs():
+    """A step is captured while another thread lets go of a dead engine's graphs."""
+    import threading
+    from b200serve.models.config import small_dense
+    from b200serve.ops import lib as K
+    from b200serve.runtime.engine import Engine
+    cfg = small_dense()
+    make = lambda **kw: Engine(random_weights(cfg, device="cuda", seed=2), max_seqs=1, max_len=256, nsplit_attn=4, **kw)
+    prompt = torch.randint(0, cfg.vocab, (20,), generator=torch.Generator().manual_seed(1)).tolist()
+    want = make(use_graphs=False).generate(prompt, 6)
+    dead, eng, freed = make(), make(), []
+    assert dead.generate(prompt, 6) == want
+    enqueue = eng._enqueue
+
+    def beside(*a):
+        if torch.cuda.is_current_stream_capturing():
+            t = threading.Thread(target=lambda: freed.append(len(dead.graphs)) or dead.graphs.clear())
+            t.start()
+            t.join()
+        return enqueue(*a)
+    eng._enqueue = beside
+    assert eng.generate(prompt, 6) == want and freed[0] > 0 and not dead.graphs
+    K.check_status()

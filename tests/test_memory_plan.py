@@ -196,3 +196,21 @@ def test_control_block_takes_numbers_and_scalar_tensors(device):
     for bad, error in (([2 ** 31, 0, 0], OverflowError), ([None, 0, 0], TypeError)):
         with pytest.raises(error):
             Engine._write_rows(eng, [Row(0, i, t) for i, t in enumerate(bad)])
+
+
+def test_collector_rests_until_the_last_capture_ends():
+    import gc
+    from b200serve.utils import graphs
+    assert gc.isenabled()
+    for first in (True, False):       # two captures that overlap; one in a process that collects by itself
+        try:
+            if not first:
+                gc.disable()
+            graphs._hold(1)
+            graphs._hold(1)
+            graphs._hold(-1)
+            assert not gc.isenabled()
+            graphs._hold(-1)
+            assert gc.isenabled() == first
+        finally:
+            gc.enable()
