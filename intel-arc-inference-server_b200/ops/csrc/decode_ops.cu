@@ -1282,7 +1282,7 @@ extern "C" int b2_attn_merge_quant(const float* o_part, const float* ml_part, vo
   return merge_launch(o_part, ml_part, out, M, n_q, nsplit, D, xq, xq_gs, gs_rows, nullptr, (cudaStream_t)stream);
 }
 
-// Either merge of rows that have counts[m] of the nsplit <= 64 places (b2_attn_rows with a budget); xq nullptr: plain rows only.
+// Either merge of rows that have counts[m] of the nsplit <= 64 places (b2_attn_rows with a plan); xq nullptr: plain rows only.
 extern "C" int b2_attn_merge_counted(const float* o_part, const float* ml_part, void* out, int M, int n_q, int nsplit, int D,
                                      const int* counts, void* xq, void* xq_gs, int gs_rows, void* stream) {
   if (D != 128 || nsplit < 1 || nsplit > 64 || !counts || (xq && gs_rows < M)) return -1;
