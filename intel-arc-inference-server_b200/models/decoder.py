@@ -85,9 +85,10 @@ def attn_splits(n_kv_heads: int, depth: int) -> int:
     return max(4, min(64, 296 // max(1, n_kv_heads), max(depth, 64) // 64))
 
 
-# Rows from which the linears run on tcgen05 (27B shape, 16 layers, integer GEMV / tcgen05: 16 rows 2.37 / 2.76 ms, 17 rows 3.66 / 2.96,
-# 40 rows 5.89 / 4.13, 64 rows 7.71 / 4.93)
-ROWS_MIN = 17
+# Rows from which the linears run on tcgen05 (16 layers, one request, integer GEMV / tcgen05: dense 27B shape 5 rows 1.58 / 1.65 ms, 8 rows 1.73 / 1.76,
+# 9 rows 2.17 / 1.88, 16 rows 2.38 / 1.96; hybrid, 12 requests 2.33 / 1.95; the MoE's linears of hidden 2048 1.51 / 1.45 with 8 requests: up to
+# eight rows the GEMV reads them in one tile, and there a row's bits are those of plain decoding)
+ROWS_MIN = 9
 ATTN_WAVES = 2      # of 2 x 148 CTAs of decode attention, see ``DecoderModel._attn_splits``
 
 

@@ -1054,7 +1054,7 @@ extern "C" int b2_quant_x(const void* x, int M, int K, int ldx, int x_mode, int 
   return b2_launch(quant_x_kernel, grid, dim3(256), 0, (cudaStream_t)stream, true, p, (uint8_t*)xq, (uint32_t*)xq_gs);
 }
 
-// Rows for b2_gemm_w4_rows, input modes as b2_quant_x; xr is [K / 64][M rounded up to 16, 32 at least][128] bytes (rows from M on are not written).
+// Rows for b2_gemm_w4_rows, input modes as b2_quant_x; xr is [K / 64][M rounded up to 16][128] bytes (rows from M on are not written).
 extern "C" int b2_stage_rows(const void* x, int M, int K, int ldx, int x_mode, int s_in, long long x_slice, const float* norm_w,
                              const float* norm_ssq, float norm_eps, void* xr, void* stream) {
   if (M < 1 || M > 64 || K % 64 != 0 || x_mode < 0 || x_mode > 2) return -1;
@@ -1062,7 +1062,7 @@ extern "C" int b2_stage_rows(const void* x, int M, int K, int ldx, int x_mode, i
   GemvParams p = {};
   p.x = x; p.M = M; p.KG = K / 64; p.ldx = ldx; p.x_mode = x_mode; p.s_in = s_in; p.x_slice = x_slice;
   p.norm_w = norm_w; p.norm_ssq = norm_ssq; p.norm_nb = K / 128; p.norm_eps = norm_eps;
-  p.rows = max(32, (M + 15) & ~15);
+  p.rows = (M + 15) & ~15;
   return b2_launch(stage_rows_kernel, dim3((p.KG * 8 + 255) / 256, M), dim3(256), 0, (cudaStream_t)stream, true, p, (uint8_t*)xr);
 }
 

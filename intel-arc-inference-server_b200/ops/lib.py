@@ -198,7 +198,7 @@ def quant_x(x, m, k, xq, xq_gs, *, x_mode=0, s_in=1, x_slice=0, ldx=None, norm_w
 
 def rows_pad(m: int) -> int:
     """Token rows per 64-k group that ``stage_rows`` lays out for ``m`` rows."""
-    return max(32, (m + 15) // 16 * 16)
+    return (m + 15) // 16 * 16
 
 
 def stage_rows(x, m, k, xr, *, x_mode=0, s_in=1, x_slice=0, ldx=None, norm_w=None, norm_ssq=None, norm_eps=0.0):
@@ -213,10 +213,17 @@ def stage_rows(x, m, k, xr, *, x_mode=0, s_in=1, x_slice=0, ldx=None, norm_w=Non
 
 
 def rows_splits(n: int, k: int) -> int:
-    """k splits of ``gemm_w4_rows``: the GEMV's, less those that would be left without a group."""
-    kg = k // 64
-    per = (-(-kg // gemv_splits(n, k)) + 3) // 4 * 4
-    return -(-kg // per)
+    """k splits of ``gemm_w4_rows``: those with which the longest CTA (pairs of 128-row blocks x splits over 148 CTAs, whole fours of groups a
+    split, and what beginning and ending an item costs in groups) has least to do."""
+    kg, pairs = k // 64, ((n + 127) // 128 + 1) // 2
+    best = None
+    for s in range(1, 17):
+        per = (-(-kg // s) + 3) // 4 * 4
+        s = -(-kg // per)
+        cost = -(-pairs * s // 148) * (per + 12)
+        if best is None or cost < best[0]:
+            best = cost, s
+    return best[1]
 
 
 def gemm_w4_rows(w4b, xr, out, m, n, k, splits, *, fold_tickets=None, fold_resid=None, fold_ssq=None):

@@ -185,6 +185,29 @@ def test_linears_on_rows(m, n, k, splits, fold):
         assert (ssq.double() - sq).abs().max() < 1e-5 * sq.max()
 
 
+@pytest.mark.parametrize("m,n,k", [(16, 38500, 192), (17, 19300, 64), (48, 19100, 320), (64, 38016, 128)])
+def test_linears_on_rows_keep_every_weight(m, n, k):
+    """Unit rows give the weights themselves, bit by bit: all sixteen nibbles in every place, scales of any size; more pairs of blocks than
+    SMs, the last one alone in odd numbers."""
+    from b200serve.utils import quant as Q
+    w = Q.random_w4b(n, k, "cuda", m)
+    blocks = w.view(-1, 4352)
+    blocks[:, :4096] = torch.randint(0, 256, (len(blocks), 4096), device="cuda", dtype=torch.uint8)
+    scales = blocks[:, 4096:].view(torch.float16)
+    scales[:] = (torch.randn_like(scales, dtype=torch.float32) * 2.0 ** torch.randint(-20, 14, scales.shape, device="cuda")).half()
+    wf = Q.dequant_w4b(w, n)
+    part, xr = torch.empty(1, m, n, device="cuda"), torch.zeros(K.rows_pad(m) * k * 2, dtype=torch.uint8, device="cuda")
+    for at in range(0, k, m):
+        x = torch.eye(k, device="cuda")[at: at + m]
+        x = torch.nn.functional.pad(x, (0, 0, 0, m - len(x))).bfloat16()
+        part.fill_(float("nan"))
+        K.stage_rows(x, m, k, xr)
+        K.gemm_w4_rows(w, xr, part, m, n, k, 1)
+        torch.cuda.synchronize()
+        assert torch.equal(part[0, : min(m, k - at)], wf[:, at: at + m].T.float())
+    K.check_status()
+
+
 @pytest.mark.parametrize("m", [3, 16, 40])
 def test_staged_rows_of_every_kind(m):
     """SiLU(gate) * up of split sums, normalised residual rows, and the attention merge's own rows, each against a plain row form of the
