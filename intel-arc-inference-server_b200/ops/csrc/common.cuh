@@ -93,9 +93,11 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // short system time limit passes, so the loop is not a hot spin.  The bound is kept on the SM's own
 // cycle counter (%clock64 costs a few cycles; %globaltimer is a slow read that, taken on every
 // wait, delayed each wake-up by most of a microsecond) and is only consulted after 256 failed
-// polls: about 4e9 cycles, i.e. roughly two seconds at 2 GHz.
+// polls: about 4e9 cycles, i.e. roughly two seconds at 2 GHz.  The first look, without a time limit, is all that stays inline: it costs 70 cycles where the
+// loop takes twice that for a phase that is over, and hot loops that hold its code several times outgrow the instruction caches (32 dense layers, one
+// request 2.52 -> 2.47 ms).
 constexpr long long kWaitCycles = 4000000000ll;
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned int code) {
+static __device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, unsigned int code) {
 #pragma unroll 1
   for (int i = 0; i < 256; ++i)
     if (mbar_try(bar, parity)) return true;
@@ -109,6 +111,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigne
       return false;
     }
   }
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned int code) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok || mbar_wait_long(bar, parity, code);
 }
 
 // ---------------------------------------------------------------- proxies / fences
