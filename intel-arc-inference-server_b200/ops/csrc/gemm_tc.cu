@@ -27,8 +27,9 @@
 // tiles; chunks of several rows of tiles expand a weight once with dequant_w4b_kernel instead, into a workspace of the largest matrix, and
 // experts of a whole tile of rows and more read such copies.  The role of the reference's direct-int4 GEMMs
 // (src/kernels/prefill/pf_gemm_q4.cl, src/kernels/prefill/pf_moe_q4gemm.cl:1-40).  The blocks have a ring of their own,
-// seven k blocks deep (ten with 128 columns) and filled by a warp of its own: tied to the three tile stages, every block's trip from HBM was
-// part of the loop (2048 rows over 256 experts in 16 layers: 10.07 -> 9.71 ms).
+// filled by a warp of its own, and so have the tiles of A: tied to the tiles of B, every trip from HBM was part of the loop.
+// 2048 rows over 256 experts (64 rows each), gate||up 1024 x 2048 / down 2048 x 512, us: 189 / 97 -> 157 / 89 with A apart, columns of tiles innermost, no rows fetched beyond
+// a block's last, and groups of expanding warps on alternate k blocks.
 #include "common.cuh"
 #include "wire.cuh"
 
@@ -43,6 +44,7 @@ namespace {
 constexpr int BM = 128;
 constexpr int BKB = 128;  // bytes of K per stage row (64 bf16 or 128 int8)
 constexpr int kThreads = 192;
+constexpr int kGroupBox = 32;   // grouped form: rows of a copy of A; a block's rows beyond its last such box are not fetched
 
 enum Epi : int { EPI_BF16 = 0, EPI_F32 = 1, EPI_SILU_MUL = 2, EPI_RESID_ADD = 3, EPI_RS_PUSH = 4, EPI_EP_RETURN = 5, EPI_GLU = 6, EPI_RELU2 = 7 };
 
@@ -88,8 +90,11 @@ struct GemmParams {
 };
 
 constexpr int kW4Block = 4352;     // one W4B block: 128 rows x 64 k of nibbles (4096 B) + 128 fp16 scales
-constexpr int kDequantWarps = 16;  // W4 form: warps that expand the blocks into the B tile (one 16-byte vector per thread and
-                                   // stage at BN = 256: eight warps left a third of the issue slots empty on dependent chains)
+constexpr int kDequantWarps = 16;  // W4 form: warps that expand the blocks into the B tile
+
+// The expanding warps are four groups on alternate k blocks: a k block's chain (wait, load, expand, store, fence, hand over) is longer than its share of any
+// pipe, and with all warps on every k block it was the loop (256 experts of 64 rows, 1024 x 2048, us: one group 175, two 164, four 157).
+constexpr int kDequantGroups = 4, kGroupWarps = kDequantWarps / kDequantGroups;
 
 template <int BN, bool W4 = false>
 struct Cfg {
@@ -97,11 +102,14 @@ struct Cfg {
   static constexpr int B_BYTES = BN * BKB;
   static constexpr int STAGE = A_BYTES + B_BYTES;
   static constexpr int RAW = W4 ? (BN / 128) * kW4Block : 0;   // a k block's W4B blocks
-  static constexpr int STAGES = W4 ? ((BN == 256) ? 3 : 5) : ((BN == 256) ? 4 : 6);
-  static constexpr int RAWS = W4 ? ((BN == 256) ? 7 : 10) : 0; // k blocks of the ring of W4B blocks
+  static constexpr int STAGES = W4 ? ((BN == 256) ? 4 : 5) : ((BN == 256) ? 4 : 6);
+  static constexpr int ASTAGES = W4 ? ((BN == 256) ? 3 : 6) : 0;   // W4: tiles of A, a ring of their own too
+  static constexpr int RAWS = W4 ? ((BN == 256) ? 4 : 10) : 0; // k blocks of the ring of W4B blocks
+  static_assert(!W4 || (STAGES >= kDequantGroups && RAWS >= kDequantGroups));   // else a group could meet a barrier two phases behind: the parity lies
   static constexpr int PUSH_STAGE = W4 ? 0 : 4 * 32 * 144;  // per epilogue warp: 32 rows x (128 B + 16 B pad) for coalesced peer stores
-  static constexpr int BARS = 384;
-  static constexpr int SMEM = STAGES * STAGE + 1024 /*align*/ + BARS + PUSH_STAGE + RAWS * RAW;
+  static constexpr int BARS = 512;
+  static constexpr int TILES = W4 ? STAGES * B_BYTES + ASTAGES * A_BYTES : STAGES * STAGE;
+  static constexpr int SMEM = TILES + 1024 /*align*/ + BARS + PUSH_STAGE + RAWS * RAW;
   static constexpr int TMEM_COLS = 2 * BN;  // two accumulators
   static constexpr int THREADS = kThreads + (W4 ? (kDequantWarps + 1) * 32 : 0);
 };
@@ -172,9 +180,22 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const uint32_t 
   }
 }
 
+// A weight's scale, times 64, as two bf16 of five significant bits whose sum it is (an fp16 has eleven: the rest behind the first five is
+// at most half a unit of them, so five bits or a power of two), each in both halves of a word.
+__device__ __forceinline__ void split_scale(float s, uint32_t& hi, uint32_t& lo) {
+  s *= 64.f;
+  const uint32_t h = (__float_as_uint(s) + 0x00040000u) & 0xFFF80000u;
+  const float rest = s - __uint_as_float(h);
+  hi = __byte_perm(h, 0, 0x3232);
+  lo = __byte_perm(__float_as_uint(fabsf(s) < __int_as_float(0x7f800000) ? rest : 0.f), 0, 0x3232);
+}
+
 // Vector `u` of a stage's W4B blocks (256 vectors a block) -> sixteen 8-byte pieces of the bf16 B tile.  A vector holds rows g and
 // g + 8 of a 16-row tile, 64 k: low nibbles are k 4t..4t+3 of a 32-k step, high nibbles k + 16 (the operand order of the decode
 // GEMV); row r lies at r * 128 bytes, 16-byte chunk (k / 8) XOR (r mod 8) -- the 128-byte swizzle.
+// Two bytes of a word go into the halves of a register, where each nibble already is a bf16 (up to 255 the bits are an integer times
+// 2^-133, denormal or not); a fused multiply-add makes it (q - 8) / 64, and with the scale in two exact parts v s_lo is exact and
+// v s_hi + v s_lo is rounded once: bf16_rne((q - 8) * scale), packed all the way.
 __device__ __forceinline__ void expand_w4(int u, uint32_t raw, uint32_t sb) {
   const int b = u >> 8, v = u & 255, j = v >> 5, l = v & 31, g = l >> 2, tq = l & 3;
   uint4 wv;
@@ -183,35 +204,31 @@ __device__ __forceinline__ void expand_w4(int u, uint32_t raw, uint32_t sb) {
   uint32_t sc2;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(sc2) : "r"(raw + b * kW4Block + 4096 + (j * 16 + 2 * g) * 2));
   const __half2 sh = *reinterpret_cast<const __half2*>(&sc2);
-  const float s_lo = __low2float(sh), s_hi = __high2float(sh);
-  const uint32_t wa[4] = {wv.x, wv.y, wv.z, wv.w};
-  uint64_t sc2x[2], off2;
-  asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[0]) : "f"(s_lo));
-  asm("mov.b64 %0, {%1, %1};" : "=l"(sc2x[1]) : "f"(s_hi));
-  asm("mov.b64 %0, {%1, %1};" : "=l"(off2) : "f"(-8388616.f));
+  uint32_t s1[2], s2[2];
+  split_scale(__low2float(sh), s1[0], s2[0]);
+  split_scale(__high2float(sh), s1[1], s2[1]);
+  // A store instruction of 16 lanes covers four rows, 32 bytes each; in the order of the k they would meet in two of the row's four
+  // 32-byte banks groups.  A lane starts with another 32-k step and nibble, by its row: all four are used.
+  const int turn = (g >> 1) ^ (g & 3);
+  const uint32_t wa[4] = {turn & 2 ? wv.z : wv.x, turn & 2 ? wv.w : wv.y, turn & 2 ? wv.x : wv.z, turn & 2 ? wv.y : wv.w};
+  const uint32_t mask0 = turn & 1 ? 0x00F000F0u : 0x000F000Fu, mul0 = turn & 1 ? 0x7d007d00u : 0x7f007f00u;      // 2^123 or 2^127
+  const uint32_t dst0 = sb + (b * 128 + j * 16 + g) * 128 + (((tq >> 1) ^ g ^ (2 * turn)) << 4) + (tq & 1) * 8;
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
-    const int row = b * 128 + j * 16 + g + 8 * (c & 1);
+    const uint32_t w01 = __byte_perm(wa[c], 0, 0x4140), w23 = __byte_perm(wa[c], 0, 0x4342);
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const uint32_t x = (wa[c] >> (4 * e)) & 0x0F0F0F0Fu;
-      // bytes -> floats through the 2^23 trick: 0x4B0000qq is 8388608 + q; q - 8 (exact) and the product with
-      // the scale run as packed pairs (add.f32x2 / mul.f32x2), the same floats as the scalar form
-      uint64_t f01, f23;
-      asm("mov.b64 %0, {%1, %2};" : "=l"(f01) : "r"(__byte_perm(x, 0x4B000000u, 0x7440)), "r"(__byte_perm(x, 0x4B000000u, 0x7441)));
-      asm("mov.b64 %0, {%1, %2};" : "=l"(f23) : "r"(__byte_perm(x, 0x4B000000u, 0x7442)), "r"(__byte_perm(x, 0x4B000000u, 0x7443)));
-      asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(off2));
-      asm("add.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(off2));
-      asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f01) : "l"(sc2x[c & 1]));
-      asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(f23) : "l"(sc2x[c & 1]));
-      float g0, g1, g2, g3;
-      asm("mov.b64 {%0, %1}, %2;" : "=f"(g0), "=f"(g1) : "l"(f01));
-      asm("mov.b64 {%0, %1}, %2;" : "=f"(g2), "=f"(g3) : "l"(f23));
-      const uint32_t p01 = pack_bf16(g0, g1);
-      const uint32_t p23 = pack_bf16(g2, g3);
-      const int k0 = 32 * (c >> 1) + 16 * e + 4 * tq;
-      const uint32_t dst = sb + row * 128 + ((((uint32_t)k0 >> 3) ^ ((uint32_t)row & 7u)) << 4) + (k0 & 7) * 2;
-      asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst), "r"(p01), "r"(p23) : "memory");
+      const uint32_t mask = e ? mask0 ^ 0x00FF00FFu : mask0, mul = e ? mul0 ^ 0x02000200u : mul0;
+      uint32_t p[2] = {w01 & mask, w23 & mask};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        uint32_t t;
+        asm("fma.rn.bf16x2 %0, %0, %1, %2;" : "+r"(p[i]) : "r"(mul), "r"(0xbe00be00u));      // -1/8
+        asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(t) : "r"(p[i]), "r"(s2[c & 1]));
+        asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(p[i]) : "r"(p[i]), "r"(s1[c & 1]), "r"(t));
+      }
+      const uint32_t dst = (dst0 ^ (uint32_t)((4 * (c >> 1) + 2 * e) << 4)) + (c & 1) * 1024;
+      asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(dst), "r"(p[0]), "r"(p[1]) : "memory");
     }
   }
 }
@@ -223,13 +240,14 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   using C = Cfg<BN, W4>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::STAGES * C::STAGE);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + C::TILES);
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + C::STAGES);
   const uint32_t tfull0 = smem_u32(bars + 2 * C::STAGES), tempty0 = smem_u32(bars + 2 * C::STAGES + 2);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * C::STAGES + 4);
   const uint32_t rawfull0 = smem_u32(bars + 2 * C::STAGES + 6), rawempty0 = rawfull0 + 8 * C::RAWS;   // W4 form: ring of W4B blocks
-  const uint32_t smem_base = smem_u32(smem);
-  const uint32_t push_base = smem_base + C::STAGES * C::STAGE + C::BARS;
+  const uint32_t afull0 = rawempty0 + 8 * C::RAWS, aempty0 = afull0 + 8 * C::ASTAGES;                                         // and of tiles of A
+  const uint32_t smem_base = smem_u32(smem), a_base = smem_base + C::STAGES * C::B_BYTES;
+  const uint32_t push_base = smem_base + C::TILES + C::BARS;
   const uint32_t raw_base = push_base + C::PUSH_STAGE;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -237,16 +255,24 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int tiles_n = (p.N + BN - 1) / BN;
   const int tiles_m = grouped ? min(*p.n_blk, p.max_blk) : (p.M + BM - 1) / BM;
   const int n_tiles = tiles_m * tiles_n;
+  // dense: tiles that run together share weights.  Grouped: they share rows -- with the experts' blocks innermost, 256 blocks of 4 KB rows
+  // (134 MB with their padding) went through L2 and from HBM again for every column of tiles
+  const auto mt_of = [&](int t) { return grouped ? t / tiles_n : (t % tiles_m + p.mt_rot) % tiles_m; };
+  const auto nt_of = [&](int t) { return grouped ? t % tiles_n : t / tiles_m; };
   const int KB = (p.K * (I8 ? 1 : 2) + BKB - 1) / BKB;  // k blocks
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::STAGES; ++i) {
-      mbar_init(full0 + 8 * i, W4 ? 1 + kDequantWarps : 1);   // W4: the A tile's copy and every expanding warp
+      mbar_init(full0 + 8 * i, W4 ? kGroupWarps : 1);
       mbar_init(empty0 + 8 * i, 1);
+    }
+    for (int i = 0; i < C::ASTAGES; ++i) {
+      mbar_init(afull0 + 8 * i, 1);
+      mbar_init(aempty0 + 8 * i, 1);
     }
     for (int i = 0; i < C::RAWS; ++i) {
       mbar_init(rawfull0 + 8 * i, 1);
-      mbar_init(rawempty0 + 8 * i, kDequantWarps);
+      mbar_init(rawempty0 + 8 * i, kGroupWarps);
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(tfull0 + 8 * i, 1);
@@ -271,11 +297,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       int it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-        const int mt = (t % tiles_m + p.mt_rot) % tiles_m, nt = t / tiles_m;
-        int row0 = mt * BM, expert = 0;
+        const int mt = mt_of(t), nt = nt_of(t);
+        int row0 = mt * BM, expert = 0, boxes = 0;
         if (grouped) {
           row0 = p.blk_row0[mt];
           expert = p.blk_expert[mt];
+          boxes = (min(BM, max(1, p.blk_rows[mt])) + kGroupBox - 1) / kGroupBox;
         }
         if (p.ag_cnt) {
           // rows of this m-tile arrive from their owner rank: bounded wait on the tile's counter in this
@@ -289,25 +316,30 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (!ok) break;
           asm volatile("fence.proxy.async;" ::: "memory");
         }
+        // W4: A alone; the last warp copies the weights' blocks, other warps expand them
+        constexpr int S = W4 ? C::ASTAGES : C::STAGES;
         for (int kb = 0; kb < KB; ++kb, ++it) {
-          const int s = it % C::STAGES;
-          if (it >= C::STAGES) ok = mbar_wait(empty0 + 8 * s, ((it / C::STAGES) - 1) & 1, ERR_GEMM_EMPTY_WAIT);
+          const int s = it % S;
+          const uint32_t full = (W4 ? afull0 : full0) + 8 * s;
+          if (it >= S) ok = mbar_wait((W4 ? aempty0 : empty0) + 8 * s, ((it / S) - 1) & 1, ERR_GEMM_EMPTY_WAIT);
           if (!ok) break;
-          const uint32_t sa = smem_base + s * C::STAGE, sb = sa + C::A_BYTES;
+          const uint32_t sa = W4 ? a_base + s * C::A_BYTES : smem_base + s * C::STAGE, sb = sa + C::A_BYTES;
           const int kx = kb * (I8 ? BKB : BKB / 2);
-          if (W4) {      // A alone; the last warp copies the weights' blocks, other warps expand them
-            mbar_expect_tx(full0 + 8 * s, C::A_BYTES);
-            tma_load_2d(sa, &map_a, kx, row0, full0 + 8 * s);
+          mbar_expect_tx(full, (W4 ? 0 : C::B_BYTES) + (grouped ? boxes * kGroupBox * BKB : C::A_BYTES));
+          if (grouped) {
+            for (int i = 0; i < boxes; ++i) tma_load_2d(sa + i * kGroupBox * BKB, &map_a, kx, row0 + i * kGroupBox, full);
           } else {
-            mbar_expect_tx(full0 + 8 * s, C::STAGE);
-            tma_load_2d(sa, &map_a, kx, row0, full0 + 8 * s);
-            if (grouped) tma_load_3d(sb, &map_b, kx, nt * BN, expert, full0 + 8 * s);
-            else tma_load_2d(sb, &map_b, kx, nt * BN, full0 + 8 * s);
+            tma_load_2d(sa, &map_a, kx, row0, full);
+          }
+          if (!W4) {
+            if (grouped) tma_load_3d(sb, &map_b, kx, nt * BN, expert, full);
+            else tma_load_2d(sb, &map_b, kx, nt * BN, full);
           }
         }
       }
       if (!ok) {  // drain what was issued and may never be consumed
-        for (int i = max(0, it - C::STAGES); i < it; ++i) mbar_wait(full0 + 8 * (i % C::STAGES), (i / C::STAGES) & 1, ERR_GEMM_FULL_WAIT);
+        constexpr int S = W4 ? C::ASTAGES : C::STAGES;
+        for (int i = max(0, it - S); i < it; ++i) mbar_wait((W4 ? afull0 : full0) + 8 * (i % S), (i / S) & 1, ERR_GEMM_FULL_WAIT);
       }
     }
   } else if (warp == 1) {
@@ -324,16 +356,20 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const uint32_t d_tmem = tmem_base + a * BN;
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % C::STAGES;
-          ok = mbar_wait(full0 + 8 * s, (it / C::STAGES) & 1, ERR_GEMM_FULL_WAIT);
+          constexpr int AS = W4 ? C::ASTAGES : 1;
+          const int as = it % AS;
+          ok = mbar_wait(full0 + 8 * s, (it / C::STAGES) & 1, ERR_GEMM_FULL_WAIT) &&
+               (!W4 || mbar_wait(afull0 + 8 * as, (it / AS) & 1, ERR_GEMM_FULL_WAIT));
           if (!ok) break;
           tc_fence_after();
-          const uint32_t sa = smem_base + s * C::STAGE, sb = sa + C::A_BYTES;
+          const uint32_t sa = W4 ? a_base + as * C::A_BYTES : smem_base + s * C::STAGE, sb = W4 ? smem_base + s * C::B_BYTES : sa + C::A_BYTES;
 #pragma unroll
           for (int k = 0; k < 4; ++k) {  // 4 x 32 bytes of K per stage
             const uint64_t da = make_desc_sw128(sa + k * 32), db = make_desc_sw128(sb + k * 32);
             if (I8) umma_i8(d_tmem, da, db, idesc, (kb | k) != 0);
             else umma_f16(d_tmem, da, db, idesc, (kb | k) != 0);
           }
+          if (W4) tc_commit(aempty0 + 8 * as);
           tc_commit(empty0 + 8 * s);  // stage is free once these MMAs have read it
         }
         if (ok) tc_commit(tfull0 + 8 * a);
@@ -345,7 +381,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       int slot = 0, round = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-        const int mt = (t % tiles_m + p.mt_rot) % tiles_m, nt = t / tiles_m, expert = grouped ? p.blk_expert[mt] : 0;
+        const int mt = mt_of(t), nt = nt_of(t), expert = grouped ? p.blk_expert[mt] : 0;
         const int nb0 = nt * (BN / 128), nblk = min(BN / 128, (p.N + 127) / 128 - nb0);
         const uint8_t* src = p.w4 + (size_t)expert * p.w4_expert_bytes + (size_t)nb0 * KB * kW4Block;
         for (int kb = 0; kb < KB; ++kb, src += kW4Block) {
@@ -365,21 +401,25 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else if (W4 && warp >= 6) {
     // ------------------------------------------------------------ W4 expansion (warps 6 .. 6 + kDequantWarps - 1)
-    const int dt = threadIdx.x - 6 * 32;   // 0 .. 32 * kDequantWarps - 1
+    const int grp = (warp - 6) / kGroupWarps, dt = threadIdx.x - 6 * 32 - grp * kGroupWarps * 32;
     int it = 0, slot = 0, par = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-      const int nt = t / tiles_m;
+      const int nt = nt_of(t);
       const int nb_total = (p.N + 127) / 128, nb0 = nt * (BN / 128);
       const int nblk = min(BN / 128, nb_total - nb0);
       for (int kb = 0; kb < KB; ++kb, ++it) {
+        if (it % kDequantGroups != grp) {      // the other groups'
+          if (++slot == C::RAWS) { slot = 0; par ^= 1; }
+          continue;
+        }
         const int s = it % C::STAGES;
         ok = __all_sync(0xffffffffu, mbar_wait(rawfull0 + 8 * slot, par, ERR_GEMM_FULL_WAIT));
         // the tile's last products are done
         if (ok && it >= C::STAGES) ok = __all_sync(0xffffffffu, mbar_wait(empty0 + 8 * s, ((it / C::STAGES) - 1) & 1, ERR_GEMM_EMPTY_WAIT));
         if (!ok) break;
-        const uint32_t sb = smem_base + s * C::STAGE + C::A_BYTES, raw = raw_base + slot * C::RAW;
-        for (int u = dt; u < nblk * 256; u += kDequantWarps * 32) expand_w4(u, raw, sb);
+        const uint32_t sb = smem_base + s * C::B_BYTES, raw = raw_base + slot * C::RAW;
+        for (int u = dt; u < nblk * 256; u += kGroupWarps * 32) expand_w4(u, raw, sb);
         fence_proxy_async_smem();   // the MMA reads the tile through the async proxy
         __syncwarp();
         if (lane == 0) {
@@ -396,7 +436,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool ok = true;
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++lt) {
       const int a = lt & 1;
-      const int mt = (t % tiles_m + p.mt_rot) % tiles_m, nt = t / tiles_m;
+      const int mt = mt_of(t), nt = nt_of(t);
       int row0 = mt * BM, rows = min(BM, p.M - row0), expert = 0;
       if (grouped) {
         row0 = p.blk_row0[mt];
@@ -881,7 +921,7 @@ extern "C" int b2_gemm_w4(const void* a, const void* w4b, void* c, int M, int N,
   p.w4_expert_bytes = (long long)((N + 127) / 128) * (K / 64) * kW4Block;
   if (bn != 128 && bn != 256) bn = (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
   CUtensorMap ma;
-  int rc = make_map(&ma, a, false, (uint64_t)M, (uint64_t)K, 0, BM);
+  int rc = make_map(&ma, a, false, (uint64_t)M, (uint64_t)K, 0, blk_expert ? kGroupBox : BM);
   if (rc) return rc;
   const int tiles_m = blk_expert ? max_blk : (M + BM - 1) / BM;
   const int n_tiles = tiles_m * ((N + bn - 1) / bn);
@@ -921,7 +961,7 @@ static int gemm_tc_impl(const void* a, const void* b, void* c, int M, int N, int
   }
   if (pair) bn = 128;       // B arrives in two halves
   CUtensorMap ma, mb;
-  int rc = make_map(&ma, a, i8 != 0, (uint64_t)M, (uint64_t)K, 0, BM);
+  int rc = make_map(&ma, a, i8 != 0, (uint64_t)M, (uint64_t)K, 0, blk_expert ? kGroupBox : BM);
   if (rc) return rc;
   rc = make_map(&mb, b, i8 != 0, (uint64_t)N, (uint64_t)K, blk_expert ? (uint64_t)n_experts : 0, (uint32_t)bn);
   if (rc) return rc;

@@ -124,6 +124,34 @@ def test_int4_block_ring(m, n, bn, kb):
     assert ((out[:m].double() - ref).abs() <= bound + 1e-9).all() and torch.isnan(out[m]).all()
 
 
+@pytest.mark.parametrize("n,k", [(256, 64), (1032, 320), (4096, 128)])
+def test_blocks_of_few_rows(n, k):
+    """Grouped products of blocks of every size around the copies of 32 rows, from int4 blocks and from bf16: unit rows give the weights'
+    bf16 bits, whatever their scales; rows beyond a block's last (not a number) reach nothing."""
+    rows = [1, 31, 32, 33, 64, 65, 96, 97, 127, 128]
+    e = len(rows)
+    w = torch.cat([Q.random_w4b(n, k, "cuda", i) for i in range(e)])
+    blocks = w.view(-1, 4352)
+    blocks[:, :4096] = torch.randint(0, 256, (len(blocks), 4096), device="cuda", dtype=torch.uint8)
+    scales = blocks[:, 4096:].view(torch.float16)
+    scales[:] = (torch.randn_like(scales, dtype=torch.float32) * 2.0 ** torch.randint(-24, 14, scales.shape, device="cuda")).half()
+    per = w.shape[0] // e
+    wb = [Q.dequant_w4b(w[i * per: (i + 1) * per], n).bfloat16() for i in range(e)]
+    tab = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")        # noqa: E731
+    table = (tab(range(e)), tab([128 * i for i in range(e)]), tab(rows), tab([e]), e + 3)
+    a = torch.full((128 * e, k), float("nan"), device="cuda").bfloat16()
+    for i, r in enumerate(rows):
+        a[128 * i: 128 * i + r] = torch.eye(k, device="cuda").repeat(128 // k + 1, 1)[:r]
+    for run in (lambda c: G.gemm_w4(a, w, n, k, c, blocks=table, n_experts=e), lambda c: G.gemm_grouped_bf16(a, torch.stack(wb), c, table)):
+        c = torch.full((128 * e, n), 7.0, device="cuda").bfloat16()
+        run(c)
+        torch.cuda.synchronize()
+        K.check_status()
+        for i, r in enumerate(rows):
+            got = c[128 * i: 128 * (i + 1)]
+            assert torch.equal(got[:r], wb[i].T.repeat(128 // k + 1, 1)[:r]) and (got[r:] == 7.0).all()
+
+
 @pytest.mark.parametrize("over", [-400, 0, 1])
 def test_experts_from_int4_or_copies(over, monkeypatch):
     """Prompt chunks on both sides of the rule: expanding a tile's blocks gives the bits of the bf16 copies."""
