@@ -182,6 +182,49 @@ __device__ __forceinline__ void group_mma(float (&acc)[T][4], uint32_t blk_addr,
   }
 }
 
+// The same for at most four tokens: an MMA's eight columns hold the high limbs of four tokens and the low limbs of the same four, so a k step takes one
+// MMA instead of two.  These MMAs are what the kernel is bound by otherwise: one takes some 25 cycles of a sub-core, four of them per 16 x 64
+// weights 100, the weights' HBM time is 90 (weights that are in L2 are no faster).  A lane's results are then both limbs' halves of the
+// sums: lanes t < 2 hold the high limbs, t >= 2 the low ones, of the same tokens; one exchange makes the former whole for row g, the latter for row
+// g + 8.  The integers, and what is done with them in fp32, are those of group_mma: so are the bits.  Two 16-row tiles.
+// 34816 x 5120 / 5120 x 17408, us: 1 row 20.5 / 11.3 -> 20.0 / 10.4, 4 rows 20.1 / 10.8 -> 19.1 / 9.9; 32 dense layers, one request 2.47 -> 2.40 ms.
+struct PackedLane {
+  bool low;          // t >= 2
+  int c_own, c_other;
+};
+template <int NG>
+__device__ __forceinline__ void group_mma_packed(float (&acc)[2][2], uint32_t blk_addr, uint32_t w_off, uint32_t sc_off, uint32_t x_addr, uint32_t gs_addr,
+                                                 const PackedLane& pl) {
+  constexpr uint32_t kMask = 0x0F0F0F0Fu;
+  uint4 wv[NG][2], x[NG], gs[NG];
+  unsigned short sc[NG][2];
+#pragma unroll
+  for (int q = 0; q < NG; ++q) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      wv[q][r] = lds128(blk_addr + q * kBlockBytes + w_off + 512 * r);
+      asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sc[q][r]) : "r"(blk_addr + q * kBlockBytes + sc_off + 32 * r));
+    }
+    x[q] = lds128(x_addr + q * 128);
+    gs[q] = lds128(gs_addr + q * 64);      // (scale, -8 sum X) of the lane's two tokens
+  }
+#pragma unroll
+  for (int q = 0; q < NG; ++q) {
+    const int m0 = pl.low ? (int)gs[q].y : 0, m1 = pl.low ? (int)gs[q].w : 0;
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const uint4 w = wv[q][r];
+      int d[4] = {m0, m1, m0, m1};
+      mma_u8s8_16832(d, w.x & kMask, w.y & kMask, (w.x >> 4) & kMask, (w.y >> 4) & kMask, x[q].x, x[q].y);
+      mma_u8s8_16832(d, w.z & kMask, w.w & kMask, (w.z >> 4) & kMask, (w.w >> 4) & kMask, x[q].z, x[q].w);
+      const int o0 = __shfl_xor_sync(0xffffffffu, pl.low ? d[0] : d[2], 2), o1 = __shfl_xor_sync(0xffffffffu, pl.low ? d[1] : d[3], 2);
+      const float sw = __half2float(__ushort_as_half(sc[q][r]));
+      acc[r][0] = fmaf(sw * __uint_as_float(gs[q].x), (float)((pl.low ? d[2] : d[0]) * pl.c_own + o0 * pl.c_other), acc[r][0]);
+      acc[r][1] = fmaf(sw * __uint_as_float(gs[q].z), (float)((pl.low ? d[3] : d[1]) * pl.c_own + o1 * pl.c_other), acc[r][1]);
+    }
+  }
+}
+
 // ---- activation staging, shared by the GEMV's own prologue and the stand-alone quantiser
 // Eight activations (one 16-byte vector of a row, k .. k + 7) as packed bf16, by input mode.
 __device__ __forceinline__ uint4 stage_load(const GemvParams& p, const uint8_t* xbase, int row, int k, float rinv) {
@@ -222,7 +265,8 @@ __device__ __forceinline__ uint4 stage_load(const GemvParams& p, const uint8_t* 
 // common.cuh: the attention merge uses them too.
 
 
-template <int T>
+// PACK: at most four tokens (T = 1)
+template <int T, bool PACK>
 __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(const GemvParams p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem0 = (smem_u32(smem_raw) + 127u) & ~127u;
@@ -362,7 +406,10 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
   uint32_t x_row[T];
 #pragma unroll
   for (int tt = 0; tt < T; ++tt) x_row[tt] = xs0 + min(tt * 8 + g, p.rows - 1) * strideB + t * 32;
-  const uint32_t gs_t = gs0 + 2 * t * 8;
+  if (PACK) x_row[0] = xs0 + min(g & 3, p.rows - 1) * strideB + t * 32 + (g >> 2) * 16;
+  const uint32_t gs_t = gs0 + 2 * (PACK ? t & 1 : t) * 8;
+  const PackedLane pl = {t >= 2, t >= 2 ? 1 : 128, t >= 2 ? 128 : 1};
+  float pacc[2][2] = {};      // PACK: row g (t < 2) or g + 8 of the warp's tiles, the lane's two tokens
 
   if (p.x_mode == 2) {
     // 1 / rms of each row from the per-block sums the producing kernel left (summed in block order)
@@ -433,7 +480,11 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
       constexpr int NGq = T == 1 ? 2 : 1;   // groups whose MMA chains are interleaved (two token tiles have chains enough, and no registers)
 #pragma unroll 1
       for (int q0 = 0; q0 < ng; q0 += NGq) {
-        if (kSplit) {
+        if (PACK) {
+          const uint32_t b = st + q0 * kBlockBytes, so = sc_off + (pl.low ? 2 : 0), ga = gsa + (gi + q0) * 64;
+          if (q0 + 1 < ng) group_mma_packed<2>(pacc, b, w_off, so, xa[0], ga, pl);
+          else group_mma_packed<1>(pacc, b, w_off, so, xa[0], ga, pl);
+        } else if (kSplit) {
           float (&a0)[T][4] = *reinterpret_cast<float (*)[T][4]>(&acc[0]);
           float (&a1)[T][4] = *reinterpret_cast<float (*)[T][4]>(&acc[T]);
           if (NGq == 2 && q0 + 1 < ng) {
@@ -458,7 +509,25 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
 
   // ---- write this split's partial sums
   float* outp = p.out + (size_t)blockIdx.z * p.out_batch + (size_t)split * p.M * p.ldo;
-  if (kSplit) {
+  if (PACK) {       // as below, with two sums a lane and tile
+    consumer_sync();
+    const uint32_t scr = ring + ((warp & 3) * 32 + lane) * 16;
+    if (wgrp == 1)
+      asm volatile("st.shared.v4.f32 [%0], {%1,%2,%3,%4};" ::"r"(scr), "f"(pacc[0][0]), "f"(pacc[0][1]), "f"(pacc[1][0]), "f"(pacc[1][1]) : "memory");
+    consumer_sync();
+    if (wgrp == 0) {
+      float4 o;
+      asm volatile("ld.shared.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(scr));
+      const float v[2][2] = {{pacc[0][0] + o.x, pacc[0][1] + o.y}, {pacc[1][0] + o.z, pacc[1][1] + o.w}};
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int n = nblk * 128 + (row16 + h) * 16 + g + (pl.low ? 8 : 0), m = 2 * (t & 1) + e;
+          if (m < p.M && n < p.N) outp[(size_t)m * p.ldo + n] = v[h][e];
+        }
+    }
+  } else if (kSplit) {
     // the two groups hold the sums of alternate stages of the same rows: they meet in shared memory (the ring is
     // free now: every stage has been waited for and consumed), group 0 first, so the order of the sum is fixed
     consumer_sync();
@@ -480,7 +549,7 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
   }
 #pragma unroll
   for (int h = 0; h < RT; ++h) {
-    if (kSplit && wgrp != 0) break;
+    if (PACK || (kSplit && wgrp != 0)) break;
     const int n_lo = nblk * 128 + (row16 + h) * 16 + g, n_hi = n_lo + 8;
 #pragma unroll
     for (int tt = 0; tt < T; ++tt) {
@@ -760,8 +829,11 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
   consumer_sync();
   const int g = lane >> 2, t = lane & 3, wgrp = warp >> 2, row16 = (warp & 3) * 2;
   const uint32_t w_off = row16 * 512 + lane * 16, sc_off = 4096 + (row16 * 16 + 2 * g) * 2;
-  const uint32_t x_row = xs0 + min(g, M - 1) * strideB + t * 32, gs_t = gs0 + 2 * t * 8;
-  float acc[2][1][4] = {};
+  const bool pack = M <= 4;         // nearly all groups: 48 rows of 8 in 256 experts make 1.7 a group
+  const uint32_t x_row = pack ? xs0 + min(g & 3, M - 1) * strideB + t * 32 + (g >> 2) * 16 : xs0 + min(g, M - 1) * strideB + t * 32;
+  const uint32_t gs_t = gs0 + 2 * (pack ? t & 1 : t) * 8;
+  const PackedLane pl = {t >= 2, t >= 2 ? 1 : 128, t >= 2 ? 128 : 1};
+  float acc[2][1][4] = {}, pacc[2][2] = {};
   for (int i = 0; i < nstage; ++i) {
     const int blk = block_of(i), q = part_of(i) * kG;
     if ((blk & 1) != wgrp) continue;
@@ -772,7 +844,11 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
     for (int q0 = 0; q0 < ng; q0 += 2) {
       const uint32_t xa[1] = {x_row + (q + q0) * 128};
       const uint32_t gsa = gs_t + (q + q0) * 64;
-      if (q0 + 1 < ng) {
+      if (pack) {
+        const uint32_t b = st + q0 * kBlockBytes, so = sc_off + (pl.low ? 2 : 0);
+        if (q0 + 1 < ng) group_mma_packed<2>(pacc, b, w_off, so, xa[0], gsa, pl);
+        else group_mma_packed<1>(pacc, b, w_off, so, xa[0], gsa, pl);
+      } else if (q0 + 1 < ng) {
         group_mma<1, 2>(acc[0], st + q0 * kBlockBytes, w_off, sc_off, xa, gsa);
         group_mma<1, 2>(acc[1], st + q0 * kBlockBytes, w_off + 512, sc_off + 32, xa, gsa);
       } else {
@@ -786,8 +862,15 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
       const int n0 = (nb0 + blk) * 128 + row16 * 16 + g;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int m = 2 * t + e;
-        if (m < M) {
+        const int m = 2 * (pack ? t & 1 : t) + e;
+        if (pack && m < M) {
+          float* o = p.out + (size_t)en.pair[m] * p.out_batch + n0 + (pl.low ? 8 : 0);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (n0 + (pl.low ? 8 : 0) + 16 * h < p.N) o[16 * h] = pacc[h][e];
+            pacc[h][e] = 0.f;
+          }
+        } else if (m < M) {
           float* o = p.out + (size_t)en.pair[m] * p.out_batch + n0;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -823,8 +906,9 @@ __global__ void __launch_bounds__(256) stage_rows_kernel(const GemvParams p, uin
   store_row_vec(xr, p.rows, row, v, stage_load(p, reinterpret_cast<const uint8_t*>(p.x), row, v * 8, p.x_mode == 2 ? s_rinv : 1.f));
 }
 
-template <int T>
+template <int T, bool PACK = false>
 int launch_t(GemvParams& p, cudaStream_t stream) {
+  if (T == 1 && !PACK && p.M <= 4) return launch_t<1, true>(p, stream);
   // staged rows and chunk length: as much of the split's k range as fits the activation budget
   int rows = 1;
   while (rows < p.M) rows *= 2;
@@ -845,12 +929,12 @@ int launch_t(GemvParams& p, cudaStream_t stream) {
     int want = 128 + kRingBytes + 128 + 256 + 16384 + kXBudget + 4096;
     if (want < smem) want = smem;   // many rows with two activation buffers of at least one stage's groups each
     if (want > 232448) return -7;
-    cudaError_t e = cudaFuncSetAttribute(gemv_w4_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
+    cudaError_t e = cudaFuncSetAttribute(gemv_w4_kernel<T, PACK>, cudaFuncAttributeMaxDynamicSharedMemorySize, want);
     if (e != cudaSuccess) return (int)e;
     configured[dev & 63] = want;
   }
   dim3 grid((p.N + 127) / 128, p.S, p.batches);
-  return b2_launch(gemv_w4_kernel<T>, grid, dim3(kThreads), smem, stream, true, p);
+  return b2_launch(gemv_w4_kernel<T, PACK>, grid, dim3(kThreads), smem, stream, true, p);
 }
 
 }  // namespace

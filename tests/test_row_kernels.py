@@ -208,6 +208,35 @@ def test_linears_on_rows_keep_every_weight(m, n, k):
     K.check_status()
 
 
+# one group, a stage and a lone group, unequal splits; n not a multiple of 128
+@pytest.mark.parametrize("n,k,splits", [(128, 64, 1), (300, 320, 1), (1000, 704, 3), (640, 1024, 2)])
+@pytest.mark.parametrize("fed", [False, True])
+def test_few_rows_have_the_bits_of_eight(n, k, splits, fed):
+    """Up to four rows put both limbs into the columns of one integer MMA: the sums of a step of eight rows, bit by bit."""
+    from b200serve.utils import quant as Q
+    torch.manual_seed(n)
+    w, x = Q.random_w4b(n, k, "cuda", 3), torch.randn(8, k, device="cuda").bfloat16()
+    x[2, 64:] = 0
+    x[1] *= 1e4
+
+    def sums(m):
+        out = torch.full((splits, m, n), float("nan"), device="cuda")
+        if fed:
+            xq, gs = torch.zeros(m * k * 2, dtype=torch.uint8, device="cuda"), torch.zeros(K.quant_slots(m) * (k // 64) * 2, dtype=torch.int32, device="cuda")
+            K.quant_x(x[:m].contiguous(), m, k, xq, gs)
+            K.gemv_w4_fused(w, xq, out, m, n, k, splits, x_mode=3, norm_ssq=gs)
+        else:
+            K.gemv_w4(w, x[:m].contiguous(), out, m, n, k, splits)
+        torch.cuda.synchronize()
+        K.check_status()
+        return out
+    want = sums(8)
+    ref = x.double() @ Q.dequant_w4b(w, n).double().T
+    assert (want.double().sum(0) - ref).norm() < 1e-4 * ref.norm()
+    for m in range(1, 6):
+        assert torch.equal(sums(m), want[:, :m])
+
+
 @pytest.mark.parametrize("m", [3, 16, 40])
 def test_staged_rows_of_every_kind(m):
     """SiLU(gate) * up of split sums, normalised residual rows, and the attention merge's own rows, each against a plain row form of the
