@@ -21,8 +21,8 @@
 // What bounds it is issue, the logic pipe first, beside a memory floor of 20 us with 136 pairs on 148 SMs: every instruction that the loops do not
 // hold counts, and their code has to fit the instruction caches (bounded waits inlined in them cost 14 of 48 us).
 // A row's bits do not depend on the other rows of the step; they are not those of the integer GEMV, whose activations are 15-bit integers.
-// 34816 x 5120 / 5120 x 17408, us: 9 - 16 rows 24.7 / 13.7 (integer GEMV 31.2 / 17.0), 17 - 32 rows 26.6 / 15.1, 33 - 48 rows 31.6 / 17.8, 64 rows
-// 35.7 / 20.0; with expanding and adding warps of two pipelines, as first built, 46.8 / 25.3, 59.4 / 32.3 and 65.9 / 36.2.  Measured and dropped: two CTAs of
+// 34816 x 5120 / 5120 x 17408, us: 9 - 16 rows 23.1 / 13.1 (integer GEMV 31.2 / 17.0), 17 - 32 rows 26.0 / 15.0, 33 - 48 rows 31.4 / 17.7, 64 rows
+// 35.0 / 19.5; with expanding and adding warps of two pipelines, as first built, 46.8 / 25.3, 59.4 / 32.3 and 65.9 / 36.2.  Measured and dropped: two CTAs of
 // eight workers per SM (24.5 / 28.8 / 33.2 / 40.3 for the four row counts: twice the splits, and 64 rows have no registers).
 #include "common.cuh"
 
@@ -160,23 +160,24 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
   if (warp == kWorkers + 2) {
     // ---------------------------------------------------------------- copies
     if (lane == 0) {
-      struct Cursor { int item, g, left; };
-      const auto at = [&](int item) { return Cursor{item, first_of(item), groups_of(item)}; };
+      struct Cursor { int item, left; bool two; const uint8_t *w, *x; };      // groups left of the item; the stage's blocks of the first n-block, its rows
+      const auto at = [&](int item) {
+        const int pair = item / p.S, g = (item - pair * p.S) * p.gps;
+        return Cursor{item, min(p.KG, g + p.gps) - g, 2 * pair + 1 < p.nb, p.w + ((size_t)(2 * pair) * p.KG + g) * kBlockBytes, p.x + (size_t)g * C::XT};
+      };
       const auto step = [&](Cursor& c) {
-        c.g += 2;
+        c.w += 2 * kBlockBytes;
+        c.x += 2 * C::XT;
         if ((c.left -= 2) <= 0) c = at(c.item + gridDim.x);
       };
+      const size_t next_block = (size_t)p.KG * kBlockBytes;
       const auto weights = [&](const Cursor& c, int slot) {
         const uint32_t ng = min(c.left, 2), bar = full0 + 8 * slot, dst = smem0 + slot * C::STAGE + 2 * C::XT;
-        const bool two = two_of(c.item);
-        mbar_expect_tx(bar, ng * ((two ? 2 : 1) * kBlockBytes + C::XT));
-        const uint8_t* src = p.w + ((size_t)(2 * (c.item / p.S)) * p.KG + c.g) * kBlockBytes;
-        bulk_g2s(dst, src, ng * kBlockBytes, bar);
-        if (two) bulk_g2s(dst + 2 * kBlockBytes, src + (size_t)p.KG * kBlockBytes, ng * kBlockBytes, bar);
+        mbar_expect_tx(bar, ng * ((c.two ? 2 : 1) * kBlockBytes + C::XT));
+        bulk_g2s(dst, c.w, ng * kBlockBytes, bar);
+        if (c.two) bulk_g2s(dst + 2 * kBlockBytes, c.w + next_block, ng * kBlockBytes, bar);
       };
-      const auto rows = [&](const Cursor& c, int slot) {
-        bulk_g2s(smem0 + slot * C::STAGE, p.x + (size_t)c.g * C::XT, min(c.left, 2) * C::XT, full0 + 8 * slot);
-      };
+      const auto rows = [&](const Cursor& c, int slot) { bulk_g2s(smem0 + slot * C::STAGE, c.x, min(c.left, 2) * C::XT, full0 + 8 * slot); };
       Cursor cw = at(blockIdx.x), cx = cw;
       int n = 0;
       for (; n < C::NS && cw.item < items; ++n, step(cw)) weights(cw, n);      // they depend on nothing: asked for before the previous kernel is done
@@ -241,7 +242,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
     uint32_t a = tmem + sub * 32 + lanes, afull = afull0;                             // weights' columns; alternate
     uint32_t d = tmem + 256 + sub * C::TW + lanes, done = done0, done_phase = 0;      // products' columns
     struct Scales { __half2 h[2]; };                                                  // the row's, two groups of each n-block
-    const auto expand = [&]() -> Scales {
+    const auto none = [] {};
+    // between: done while the expanded weights are on their way into tensor memory
+    const auto expand = [&](auto&& between) -> Scales {
       wait_all(full, phase, failed, ERR_GEMM_FULL_WAIT);
       uint4 v[2];
       unsigned short sc[4];
@@ -261,6 +264,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
           for (int hf = 0; hf < 2; ++hf) nibbles_bf16(w[2 * ks + hf], r[8 * ks + hf], r[8 * ks + 2 + hf], r[8 * ks + 4 + hf], r[8 * ks + 6 + hf]);
         B2_TMEM_ST_16X128_8(a + ((uint32_t)(16 * e) << 16), r);
       }
+      between();
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -278,58 +282,97 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
       for (int e = 0; e < 2; ++e) o.h[e] = __halves2half2(__ushort_as_half(sc[2 * e]), __ushort_as_half(sc[2 * e + 1]));
       return o;
     };
-    // groups: of the stage (1: its second one is not there); two: the pair has its second n-block
+    // One set of accumulators: an n-block's is handed back as soon as it is in registers, and its next products are made while the other n-block's are
+    // added up and a stage is expanded.  groups: of the stage (1: its second one is not there); two: the pair has its second n-block.
+    const auto fold = [&](const Scales& sc, int b, const uint32_t* v) {
+      const float2 f = __half22float2(sc.h[b >> 1]);
+      const float w = b & 1 ? f.y : f.x;
+      const uint64_t w2 = pack2(__float_as_uint(w), __float_as_uint(w));
+#pragma unroll
+      for (int i = 0; i < C::TW; i += 2)
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[b >> 1][i / 2]) : "l"(pack2(v[i], v[i + 1])), "l"(w2));
+    };
     const auto add = [&](const Scales& sc, int groups, bool two) {
-      // Two sets of accumulators: the next products are on their way into the other one.  One set: an n-block's is handed back as soon as it
-      // is in registers, and its next products are made while the other n-block's are added up and a stage is expanded.
-      constexpr int G = C::TW <= 8 ? 4 : 2;       // blocks whose loads are in flight together: what the registers hold
-      static_assert(C::TWO || G == 2);
 #pragma unroll
-      for (int b0 = 0; b0 < 4; b0 += G) {
-        if (b0 == 0 || !C::TWO) {
-          wait_all(C::TWO ? done : done0 + 4 * b0, done_phase, failed, ERR_GEMM_TMEM_FULL_WAIT);
-          tc_fence_after();
-        }
-        uint32_t v[G][C::TW];
+      for (int h = 0; h < 2; ++h) {
+        wait_all(done0 + 8 * h, done_phase, failed, ERR_GEMM_TMEM_FULL_WAIT);
+        tc_fence_after();
+        uint32_t v[2][C::TW];
 #pragma unroll
-        for (int b = 0; b < G; ++b) tmem_ld<C::TW>(d + (b0 + b) * C::DS, v[b]);
+        for (int j = 0; j < 2; ++j) tmem_ld<C::TW>(d + (2 * h + j) * C::DS, v[j]);
         tmem_ld_wait();
-        if (!C::TWO) {
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(free0 + 4 * b0);
-        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(free0 + 8 * h);
 #pragma unroll
-        for (int b = b0; b < b0 + G; ++b) {
-          if (((b & 1) && groups == 1) || ((b >> 1) && !two)) continue;      // a block that is not there
-          const float2 f = __half22float2(sc.h[b >> 1]);
-          const float w = b & 1 ? f.y : f.x;
-          const uint64_t w2 = pack2(__float_as_uint(w), __float_as_uint(w));
-#pragma unroll
-          for (int i = 0; i < C::TW; i += 2)
-            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[b >> 1][i / 2]) : "l"(pack2(v[b - b0][i], v[b - b0][i + 1])), "l"(w2));
-        }
+        for (int j = 0; j < 2; ++j)
+          if (!(j && groups == 1) && !(h && !two)) fold(sc, 2 * h + j, v[j]);      // else the block is not there
       }
-      if (C::TWO) {
-        d ^= 128;
-        done_phase ^= done != done0;
-        done ^= 8;
-      } else done_phase ^= 1;
+      done_phase ^= 1;
+    };
+    // Two sets: load() asks for a stage's products, sum() adds them up
+    uint32_t v2[4][C::TWO ? C::TW : 1];
+    const auto load = [&] {
+      wait_all(done, done_phase, failed, ERR_GEMM_TMEM_FULL_WAIT);
+      tc_fence_after();
+      if constexpr (C::TWO) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) tmem_ld<C::TW>(d + b * C::DS, v2[b]);
+      }
+      d ^= 128;
+      done_phase ^= done != done0;
+      done ^= 8;
+    };
+    const auto sum = [&](const Scales& sc, int groups, bool two) {
+      tmem_ld_wait();
+      if constexpr (C::TWO) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+          if (!((b & 1) && groups == 1) && !((b >> 1) && !two)) fold(sc, b, v2[b]);
+      }
     };
     for (int item = blockIdx.x; item < items; item += gridDim.x) {
       const int pair = item / p.S, split = item - pair * p.S;
       const bool two = two_of(item);
 #pragma unroll
       for (int i = 0; i < C::TW / 2; ++i) acc[0][i] = acc[1][i] = 0;
-      Scales scales = expand();
+      Scales scales = expand(none);
       int left = groups_of(item);
+      if (C::TWO) {
+        // up to 16 token rows the products of the stage before are on their way while a stage is expanded and the one before them is added up (24.7 -> 22.9 us;
+        // with 32 they are made in time: 26.6 / 27.4)
+        if (T > 16) {
 #pragma unroll 1
-      for (; left > 2; left -= 2) {
-        const Scales next = expand();
-        add(scales, 2, two);
-        scales = next;
+          for (; left > 2; left -= 2) {
+            const Scales next = expand(none);
+            load();
+            sum(scales, 2, two);
+            scales = next;
+          }
+        } else if (left > 2) {
+          Scales next = expand(none);
+#pragma unroll 1
+          for (left -= 2; left > 2; left -= 2) {
+            load();
+            const Scales after = expand([&] { sum(scales, 2, two); });
+            scales = next;
+            next = after;
+          }
+          load();
+          sum(scales, 2, two);
+          scales = next;
+        }
+        load();
+        sum(scales, left, two);
+      } else {
+#pragma unroll 1
+        for (; left > 2; left -= 2) {
+          const Scales next = expand(none);
+          add(scales, 2, two);
+          scales = next;
+        }
+        add(scales, left, two);
       }
-      add(scales, left, two);
       // ---- the item's sums
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
