@@ -149,7 +149,8 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float* __restrict_
 
 // ---------------------------------------------------------------- decode rows: router logits + routing in one launch
 // logits[m][r] = x[m] . W[r] for the R router rows (E experts, then the shared expert's gate row when there is one):
-// a warp per router row, eight token rows per pass over the weights.  The CTA that finishes last (a ticket) then
+// sixteen router rows a CTA, eight token rows per pass over the weights, on mma.sync, k spread over the warps (fp32 products of a
+// warp per router row were bound by issue: a layer of 48 rows took 20 us here, now 11.6).  The CTA that finishes last (a ticket) then
 // routes every token row.  With `shared_slot` each row gets one more slot: expert id E (the shared expert, see the
 // batched GEMV's alt weights) with weight sigmoid(gate logit), or 1 without a gate row; with shared_slot n > 1 (no gate
 // row) n more slots, ids E .. E + n - 1 with weight 1: runs of a shared expert's hidden columns.
@@ -175,21 +176,30 @@ __device__ void group_pairs(const int* topk_idx, int pairs, int* groups, int* s_
   __syncthreads();
   for (int i = tid; i < pairs; i += 256) atomicAdd(&s_count[__ldcg(topk_idx + i)], 1);
   __syncthreads();
-  if (tid < 32) {
-    int run = 0;
-    for (int i0 = 0; i0 < kGroupIds; i0 += 32) {
-      const int n = (s_count[i0 + tid] + 7) >> 3;
-      int x = n;
+  // groups before an expert's: three experts a thread, prefixes over the warp, the warps in turn
+  __shared__ int s_warp[8];
+  int n[3], mine = 0;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, x, o);
-        if (tid >= o) x += v;
-      }
-      s_first[i0 + tid] = run + x - n;
-      run += __shfl_sync(0xffffffffu, x, 31);
-    }
-    if (tid == 0) groups[0] = run;
+  for (int i = 0; i < 3; ++i) {
+    n[i] = 3 * tid + i < kGroupIds ? (s_count[3 * tid + i] + 7) >> 3 : 0;
+    mine += n[i];
   }
+  int x = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, x, o);
+    if ((tid & 31) >= o) x += v;
+  }
+  if ((tid & 31) == 31) s_warp[tid >> 5] = x;
+  __syncthreads();
+  int first = x - mine;
+  for (int i = 0; i < (tid >> 5); ++i) first += s_warp[i];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    if (3 * tid + i < kGroupIds) s_first[3 * tid + i] = first;
+    first += n[i];
+  }
+  if (tid == 255) groups[0] = first;
   __syncthreads();
   for (int e = tid; e < kGroupIds; e += 256) {
     const int c = s_count[e];
@@ -212,49 +222,45 @@ __global__ void __launch_bounds__(256) moe_router_rows_kernel(const RouterRowsPa
   __shared__ int s_last, s_count[kGroupIds], s_first[kGroupIds];
   pdl_wait();
   pdl_launch_dependents();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int r = blockIdx.x * 8 + warp;
+  __shared__ float s_red[8][16][9];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int r0 = blockIdx.x * 16;
   // token rows of this CTA: all of them, or the slice of eight that blockIdx.y names
   const int m_lo = gridDim.y > 1 ? blockIdx.y * 8 : 0, m_hi = gridDim.y > 1 ? min(p.M, m_lo + 8) : p.M;
-  if (r < p.R) {
-    const uint4* wr = reinterpret_cast<const uint4*>(p.w + (size_t)r * p.H);
-    const int chunks = p.H / 8;                 // 16-byte pieces of a row; a lane takes every 32nd
-    for (int m0 = m_lo; m0 < m_hi; m0 += 8) {
-      const int mt = min(8, m_hi - m0);
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int c0 = lane; c0 < chunks; c0 += 32 * 8) {
-        // eight pieces of the router row in flight, then the token rows against them
-        uint4 wv[8];
+  for (int m0 = m_lo; m0 < m_hi; m0 += 8) {
+    // A lane's 16 bytes of a row are eight k of a 32-k chunk: two MMAs take them as they are, since both operands have them in the same order.
+    // Chunks go round the warps; eight of a warp's are in flight together.
+    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    const auto piece = [&](const __nv_bfloat16* base, int row, int rows, int k) {
+      return row < rows && k < p.H ? __ldg(reinterpret_cast<const uint4*>(base + (size_t)row * p.H + k)) : make_uint4(0, 0, 0, 0);
+    };
+    for (int k0 = warp * 32 + t * 8; k0 - t * 8 < p.H; k0 += 8 * 8 * 32) {
+      uint4 u[8], v[8], x[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int c = c0 + 32 * u;
-          wv[u] = c < chunks ? __ldg(wr + c) : make_uint4(0, 0, 0, 0);
-        }
-        for (int mm = 0; mm < mt; ++mm) {
-          const uint4* xr = reinterpret_cast<const uint4*>(p.x + (size_t)(m0 + mm) * p.H);
-          uint4 xv[8];
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const int c = c0 + 32 * u;
-            xv[u] = c < chunks ? __ldg(xr + c) : make_uint4(0, 0, 0, 0);
-          }
-          float a = 0.f, b = 0.f;
-#pragma unroll
-          for (int u = 0; u < 8; ++u) {
-            const uint32_t ww[4] = {wv[u].x, wv[u].y, wv[u].z, wv[u].w}, xx[4] = {xv[u].x, xv[u].y, xv[u].z, xv[u].w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              a = fmaf(bf16_lo(ww[j]), bf16_lo(xx[j]), a);
-              b = fmaf(bf16_hi(ww[j]), bf16_hi(xx[j]), b);
-            }
-          }
-          acc[mm] += a + b;
-        }
+      for (int i = 0; i < 8; ++i) {
+        const int k = k0 + i * 8 * 32;
+        u[i] = piece(p.w, r0 + g, p.R, k);
+        v[i] = piece(p.w, r0 + g + 8, p.R, k);
+        x[i] = piece(p.x, m0 + g, m_hi, k);
       }
-      for (int mm = 0; mm < mt; ++mm) {
-        const float v = warp_sum(acc[mm]);
-        if (lane == 0) p.logits[(size_t)(m0 + mm) * p.ld + r] = v;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        mma_bf16_16816(c, u[i].x, v[i].x, u[i].y, v[i].y, x[i].x, x[i].y);
+        mma_bf16_16816(c, u[i].z, v[i].z, u[i].w, v[i].w, x[i].z, x[i].w);
       }
+    }
+    if (m0 > m_lo) __syncthreads();
+    s_red[warp][g][2 * t] = c[0];
+    s_red[warp][g][2 * t + 1] = c[1];
+    s_red[warp][g + 8][2 * t] = c[2];
+    s_red[warp][g + 8][2 * t + 1] = c[3];
+    __syncthreads();
+    const int row = threadIdx.x & 15, m = m0 + (threadIdx.x >> 4);
+    if (threadIdx.x < 128 && r0 + row < p.R && m < m_hi) {
+      float sum = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) sum += s_red[w][row][threadIdx.x >> 4];
+      p.logits[(size_t)m * p.ld + r0 + row] = sum;
     }
   }
   __threadfence();
@@ -490,7 +496,7 @@ extern "C" int b2_moe_router_rows(const void* w, const void* x, float* logits, i
   // Slices of eight token rows have CTAs of their own, which also route them (a router of 257 rows is 33 CTAs: 48 token rows
   // behind one another took 58 us of a layer's step).  Callers with a single ticket word keep one slice.
   const int slices = (M + 7) / 8 < n_tickets ? (M + 7) / 8 : 1;
-  return b2_launch(route_plain(rule) ? moe_router_rows_kernel<true> : moe_router_rows_kernel<false>, dim3((R + 7) / 8, slices), dim3(256), 0, (cudaStream_t)stream, true, p);
+  return b2_launch(route_plain(rule) ? moe_router_rows_kernel<true> : moe_router_rows_kernel<false>, dim3((R + 15) / 16, slices), dim3(256), 0, (cudaStream_t)stream, true, p);
 }
 
 // counts must hold E zeros on entry (the caller clears it on the stream).

@@ -208,6 +208,24 @@ def test_linears_on_rows_keep_every_weight(m, n, k):
     K.check_status()
 
 
+# router rows around the tiles of 16, rows around the slices of eight, widths that leave pieces of a 32-k chunk; slices side by side or one after another
+@pytest.mark.parametrize("tickets", [1, 16])
+@pytest.mark.parametrize("m,e,h", [(1, 8, 8), (7, 15, 200), (8, 16, 64), (9, 17, 2056), (33, 257, 2048), (64, 500, 136)])
+def test_router_logits(m, e, h, tickets):
+    from b200serve.ops import moe as M
+    torch.manual_seed(m + e)
+    w, x = (torch.randn(e, h, device="cuda") * h ** -0.5).bfloat16(), torch.randn(m, h, device="cuda").bfloat16()
+    ld, k = (e + 7) // 8 * 8, 4
+    lg = torch.full((m, ld), float("nan"), device="cuda")
+    idx, tw, tk = torch.zeros(m * k, dtype=torch.int32, device="cuda"), torch.zeros(m * k, device="cuda"), torch.zeros(tickets, dtype=torch.int32, device="cuda")
+    M.router_rows(w, x, lg, m, e, h, ld, e, k, False, False, idx, tw, tk)
+    torch.cuda.synchronize()
+    ref = x.double() @ w.double().T
+    # exact products, fp32 sums of h terms
+    assert ((lg[:, :e].double() - ref).abs() <= 16 * 2.0 ** -24 * (x.double().abs() @ w.double().abs().T) + 1e-12).all() and torch.isnan(lg[:, e:]).all()
+    assert torch.equal(idx.view(m, k).long(), torch.sort(lg[:, :e], dim=-1, descending=True, stable=True).indices[:, :k]) and int(tk.abs().sum()) == 0
+
+
 # one group, a stage and a lone group, unequal splits; n not a multiple of 128
 @pytest.mark.parametrize("n,k,splits", [(128, 64, 1), (300, 320, 1), (1000, 704, 3), (640, 1024, 2)])
 @pytest.mark.parametrize("fed", [False, True])
