@@ -746,7 +746,8 @@ __global__ void __launch_bounds__(256) quant_x_kernel(const GemvParams p, uint8_
 // weights stream past them.  Two groups of four consumer warps own alternate n-blocks, so a sum never leaves its warp and the
 // CTA has no barrier after the staging; a run is at most about 64 W4B blocks (280 KB), which keeps the fixed cost per CTA (table,
 // staging, ring fill: ~4 us with two CTAs per SM) below its stream time, and shorter where the groups would not fill a wave of 296
-// CTAs.  A step of 48 rows through 16 layers (hidden 2048, experts of 512): 11.5 -> 4.3 ms, with the router's slices (moe.cu); 4 layers, 8
+// CTAs.  Neither role divides per stage: a lone copying thread that did was behind (48 rows, 196 experts of 1024 x 2048 / 2048 x 512: 55 / 31 -> 49 / 28
+// us).  A step of 48 rows through 16 layers (hidden 2048, experts of 512): 11.5 -> 4.3 ms, with the router's slices (moe.cu); 4 layers, 8
 // rows, runs of 64 blocks whatever the groups / as here: experts of 512 500 / 496 us, hidden 512 with 16 of 256 (2 layers) 164 / 155.
 struct ExpertGroups {
   int n;           // groups in use
@@ -773,11 +774,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
   if ((int)blockIdx.y >= ep.groups->n) return;
   const ExpertGroups::Entry& en = ep.groups->e[blockIdx.y];
   const int M = en.rows, nb0 = blockIdx.x * ep.run, nbs = min(ep.run, ep.nb - nb0);
-  const int spb = (p.KG + kG - 1) / kG;                        // ring stages per n-block
   // stage order: the two warp groups' n-blocks in turn, a lone last block by itself
-  const int pairs2 = nbs / 2, nstage = nbs * spb;
-  auto block_of = [&](int i) { return i < pairs2 * 2 * spb ? i / (2 * spb) * 2 + (i & 1) : nbs - 1; };
-  auto part_of = [&](int i) { return i < pairs2 * 2 * spb ? i % (2 * spb) / 2 : i - pairs2 * 2 * spb; };
+  const int paired = nbs & ~1;
   if (tid == 0) {
     for (int i = 0; i < kStages; ++i) {
       mbar_init(full0 + 8 * i, 1);
@@ -791,16 +789,18 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
       const uint8_t* src = ((p.alt_w && en.expert == p.alt_id) ? p.alt_w : p.w + (size_t)en.expert * p.expert_bytes) +
                            (size_t)nb0 * p.KG * kBlockBytes;
       bool ok = true;
-      int issued = 0;
-      for (int i = 0; i < nstage && ok; ++i) {
-        if (i >= kStages) ok = mbar_wait(empty0 + 8 * (i % kStages), ((i / kStages) - 1) & 1, ERR_GEMV_EMPTY_WAIT);
-        if (!ok) break;
-        const int s = i % kStages, q = part_of(i) * kG;
-        const uint32_t bytes = min(kG, p.KG - q) * kBlockBytes;
-        mbar_expect_tx(full0 + 8 * s, bytes);
-        bulk_g2s(ring + s * kStageBytes, src + ((size_t)block_of(i) * p.KG + q) * kBlockBytes, bytes, full0 + 8 * s);
-        issued = i + 1;
-      }
+      int issued = 0, slot = 0, round = 0;
+      for (int blk0 = 0; blk0 < nbs && ok; blk0 += 2)
+        for (int q = 0; q < p.KG && ok; q += kG)
+          for (int blk = blk0; blk < min(blk0 + 2, nbs); ++blk) {
+            if (round > 0) ok = mbar_wait(empty0 + 8 * slot, (round - 1) & 1, ERR_GEMV_EMPTY_WAIT);
+            if (!ok) break;
+            const uint32_t bytes = min(kG, p.KG - q) * kBlockBytes;
+            mbar_expect_tx(full0 + 8 * slot, bytes);
+            bulk_g2s(ring + slot * kStageBytes, src + ((size_t)blk * p.KG + q) * kBlockBytes, bytes, full0 + 8 * slot);
+            ++issued;
+            if (++slot == kStages) { slot = 0; ++round; }
+          }
       if (!ok)   // wait (bounded) for the copies that were issued and possibly never consumed
         for (int i = max(0, issued - kStages); i < issued; ++i)
           mbar_wait(full0 + 8 * (i % kStages), (i / kStages) & 1, ERR_GEMV_FULL_WAIT);
@@ -829,14 +829,9 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
   consumer_sync();
   const int g = lane >> 2, t = lane & 3, wgrp = warp >> 2, row16 = (warp & 3) * 2;
   const uint32_t w_off = row16 * 512 + lane * 16, sc_off = 4096 + (row16 * 16 + 2 * g) * 2;
-  const bool pack = M <= 4;         // nearly all groups: 48 rows of 8 in 256 experts make 1.7 a group
-  const uint32_t x_row = pack ? xs0 + min(g & 3, M - 1) * strideB + t * 32 + (g >> 2) * 16 : xs0 + min(g, M - 1) * strideB + t * 32;
-  const uint32_t gs_t = gs0 + 2 * (pack ? t & 1 : t) * 8;
-  const PackedLane pl = {t >= 2, t >= 2 ? 1 : 128, t >= 2 ? 128 : 1};
-  float acc[2][1][4] = {}, pacc[2][2] = {};
-  for (int i = 0; i < nstage; ++i) {
-    const int blk = block_of(i), q = part_of(i) * kG;
-    if ((blk & 1) != wgrp) continue;
+  const uint32_t x_row = xs0 + min(g, M - 1) * strideB + t * 32, gs_t = gs0 + 2 * t * 8;
+  float acc[2][1][4] = {};
+  for (int blk = wgrp, q = 0, i = wgrp; blk < nbs;) {
     const int s = i % kStages, ng = min(kG, p.KG - q);
     if (!__all_sync(0xffffffffu, mbar_wait(full0 + 8 * s, (i / kStages) & 1, ERR_GEMV_FULL_WAIT))) return;   // the rest is not stored; the producer gives up too and drains its copies
     const uint32_t st = ring + s * kStageBytes;
@@ -844,11 +839,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
     for (int q0 = 0; q0 < ng; q0 += 2) {
       const uint32_t xa[1] = {x_row + (q + q0) * 128};
       const uint32_t gsa = gs_t + (q + q0) * 64;
-      if (pack) {
-        const uint32_t b = st + q0 * kBlockBytes, so = sc_off + (pl.low ? 2 : 0);
-        if (q0 + 1 < ng) group_mma_packed<2>(pacc, b, w_off, so, xa[0], gsa, pl);
-        else group_mma_packed<1>(pacc, b, w_off, so, xa[0], gsa, pl);
-      } else if (q0 + 1 < ng) {
+      if (q0 + 1 < ng) {
         group_mma<1, 2>(acc[0], st + q0 * kBlockBytes, w_off, sc_off, xa, gsa);
         group_mma<1, 2>(acc[1], st + q0 * kBlockBytes, w_off + 512, sc_off + 32, xa, gsa);
       } else {
@@ -862,15 +853,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
       const int n0 = (nb0 + blk) * 128 + row16 * 16 + g;
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int m = 2 * (pack ? t & 1 : t) + e;
-        if (pack && m < M) {
-          float* o = p.out + (size_t)en.pair[m] * p.out_batch + n0 + (pl.low ? 8 : 0);
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            if (n0 + (pl.low ? 8 : 0) + 16 * h < p.N) o[16 * h] = pacc[h][e];
-            pacc[h][e] = 0.f;
-          }
-        } else if (m < M) {
+        const int m = 2 * t + e;
+        if (m < M) {
           float* o = p.out + (size_t)en.pair[m] * p.out_batch + n0;
 #pragma unroll
           for (int h = 0; h < 2; ++h) {
@@ -882,6 +866,9 @@ __global__ void __launch_bounds__(kThreads, 2) gemv_w4_groups_kernel(const Exper
 #pragma unroll
       for (int h = 0; h < 2; ++h) acc[h][0][0] = acc[h][0][1] = acc[h][0][2] = acc[h][0][3] = 0.f;
     }
+    // on to the group's next stage
+    i += blk < paired ? 2 : 1;       // (the lone last block's stages follow one another)
+    if ((q += kG) >= p.KG) { q = 0; blk += 2; }
   }
 }
 
