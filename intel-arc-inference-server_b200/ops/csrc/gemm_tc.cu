@@ -87,6 +87,10 @@ struct GemmParams {
   const uint8_t* w4;
   long long w4_expert_bytes;
   Glu glu;           // EPI_GLU: SiLU(gate) * up with other constants
+  // ---- pair form: the tiles of the last, partly filled wave cut along K into `split` parts each
+  int split;         // 0 or 1: not
+  float* part;       // [tile of that wave][part][CTA][chunk of 32 columns][warp][8][lane] float4
+  int* part_tickets; // [tile of that wave][CTA][warp][half of the columns], zeroed, left zero
 };
 
 constexpr int kW4Block = 4352;     // one W4B block: 128 rows x 64 k of nibbles (4096 B) + 128 fp16 scales
@@ -548,6 +552,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 // stores and reads 16 KB of B instead of 32: six stages fit instead of four, and the tensor core's operand reads fall from 96 to
 // 64 bytes a cycle.  bf16 GEMMs that are not grouped, with the local epilogues; the loads carry no multicast.
 // 4096 rows x 34816 x 5120: 986 -> 908 us (1.61 PFLOP/s); x 5120 x 17408: 573 -> 504; 900 rows x 34816 x 5120: 272 -> 247.
+//
+// A last wave of a few tiles leaves most pairs idle for a whole tile's time (5120 columns at 900 rows: 80 tiles on 74 pairs).  Its tiles are cut along K, a
+// part per pair: a warp leaves its fp32 sums of half the columns in a workspace, and whichever part comes last for them adds the parts in order and goes
+// through the epilogue; every second part begins with the other half.  us without / with: 5120 x 17408,
+// 130 rows 128 / 68, 900 260 / 161, 4096 506 / 474; 5120 x 5120, 900 rows 58 / 49; 7168 x 5120, 2048 rows 118 / 110.  (Counted for each 32 columns, the fences took
+// what was gained: 5120 x 5120, 900 rows 58 / 55.)
 struct PairCfg {
   static constexpr int BN = 256, HALF = 128 * BKB, STAGE = 2 * HALF, STAGES = 6, BARS = 256;
   static constexpr int SMEM = STAGES * STAGE + 1024 + BARS;
@@ -620,6 +630,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, rank = (int)cluster_rank();
   const int tiles_m = (p.M + 2 * BM - 1) / (2 * BM), tiles_n = (p.N + C::BN - 1) / C::BN, n_tiles = tiles_m * tiles_n;
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, KB = p.K * 2 / BKB;
+  // work of this pair: whole tiles pair, pair + pairs, ..., then (split) a part of a tile of the last wave
+  const int whole = p.split > 1 ? n_tiles / pairs * pairs : n_tiles;
+  struct Work { int t, kb0, kb1, part; };      // part < 0: a whole tile
+  const auto work = [&](int i, Work& w) -> bool {
+    w.t = pair + i * pairs;
+    w.kb0 = 0; w.kb1 = KB; w.part = -1;
+    if (w.t < whole) return true;
+    if (p.split <= 1 || i != whole / pairs || pair >= (n_tiles - whole) * p.split) return false;
+    w.t = whole + pair / p.split;
+    w.part = pair % p.split;
+    w.kb0 = w.part * KB / p.split;
+    w.kb1 = (w.part + 1) * KB / p.split;
+    return true;
+  };
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < C::STAGES; ++i) {
@@ -650,9 +674,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       prefetch_tmap(&map_b);
       int it = 0;
       bool ok = true;
-      for (int t = pair; t < n_tiles && ok; t += pairs) {
-        const int row0 = (t % tiles_m) * 2 * BM + rank * BM, n0 = (t / tiles_m) * C::BN + rank * (C::BN / 2);
-        for (int kb = 0; kb < KB; ++kb, ++it) {
+      Work w;
+      for (int i = 0; ok && work(i, w); ++i) {
+        const int row0 = (w.t % tiles_m) * 2 * BM + rank * BM, n0 = (w.t / tiles_m) * C::BN + rank * (C::BN / 2);
+        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const int s = it % C::STAGES;
           if (it >= C::STAGES) ok = mbar_wait(empty0 + 8 * s, ((it / C::STAGES) - 1) & 1, ERR_GEMM_EMPTY_WAIT);
           if (!ok) break;
@@ -673,19 +698,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       constexpr uint32_t idesc = make_idesc(1, 1, 2 * BM, C::BN);
       int it = 0, lt = 0;
       bool ok = true;
-      for (int t = pair; t < n_tiles && ok; t += pairs, ++lt) {
+      Work w;
+      for (; ok && work(lt, w); ++lt) {
         const int a = lt & 1;
         if (lt >= 2) ok = mbar_wait_cluster(tempty0 + 8 * a, ((lt >> 1) - 1) & 1, ERR_GEMM_TMEM_EMPTY_WAIT);
         if (!ok) break;
         tc_fence_after();
-        for (int kb = 0; kb < KB; ++kb, ++it) {
+        for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const int s = it % C::STAGES;
           ok = mbar_wait_cluster(full0 + 8 * s, (it / C::STAGES) & 1, ERR_GEMM_FULL_WAIT);
           if (!ok) break;
           tc_fence_after();
           const uint64_t da = make_desc_sw128(smem + s * C::STAGE), db = make_desc_sw128(smem + s * C::STAGE + C::HALF);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) umma_f16_pair(tmem + a * C::BN, da + 2 * k, db + 2 * k, idesc, (kb | k) != 0);
+          for (int k = 0; k < 4; ++k) umma_f16_pair(tmem + a * C::BN, da + 2 * k, db + 2 * k, idesc, ((kb - w.kb0) | k) != 0);
           tc_commit_pair(empty0 + 8 * s);
         }
         if (ok) tc_commit_pair(tfull0 + 8 * a);
@@ -695,18 +721,75 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     // ------------------------------------------------------------ epilogue (warps 2..5): this CTA's 128 rows
     const int quarter = warp & 3;
     int lt = 0;
-    for (int t = pair; t < n_tiles; t += pairs, ++lt) {
-      const int a = lt & 1, nt = t / tiles_m;
-      const int grow = (t % tiles_m) * 2 * BM + rank * BM + quarter * 32 + lane;
-      if (!__all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * a, (lt >> 1) & 1, ERR_GEMM_TMEM_FULL_WAIT))) break;
+    bool ok = true;
+    Work w;
+    for (; work(lt, w); ++lt) {
+      const int a = lt & 1, nt = w.t / tiles_m;
+      const int grow = (w.t % tiles_m) * 2 * BM + rank * BM + quarter * 32 + lane;
+      if (ok) ok = __all_sync(0xffffffffu, mbar_wait(tfull0 + 8 * a, (lt >> 1) & 1, ERR_GEMM_TMEM_FULL_WAIT));
+      if (!ok && w.part < 0) continue;      // (a part is counted even if nothing arrived: the tickets go back to zero)
       tc_fence_after();
-#pragma unroll 1
-      for (int c = 0; c < C::BN / 32; ++c) {
-        uint32_t v[32];
+      const auto sums = [&](int c, uint32_t (&v)[32]) {
         B2_TMEM_LD_32(tmem + a * C::BN + c * 32 + ((uint32_t)(quarter * 32) << 16), v);
         tmem_ld_wait();
-        const int n0 = nt * C::BN + c * 32;
-        if (grow < p.M && n0 < p.N) store_chunk(p, v, grow, n0);
+      };
+      if (w.part < 0) {
+#pragma unroll 1
+        for (int c = 0; c < C::BN / 32; ++c) {
+          uint32_t v[32];
+          sums(c, v);
+          const int n0 = nt * C::BN + c * 32;
+          if (grow < p.M && n0 < p.N) store_chunk(p, v, grow, n0);
+        }
+      } else {
+        const int tail = w.t - whole;
+        constexpr int kHalf = C::BN / 64;                          // chunks of a half of the columns, which are counted together
+        constexpr size_t kPart = 2 * (C::BN / 32) * 4 * 256;       // float4 of a part of both CTAs
+        float4* mine = reinterpret_cast<float4*>(p.part) + (((size_t)tail * p.split * 2 + rank) * (C::BN / 32) * 4 + quarter) * 256 + lane;
+        for (int hh = 0; hh < 2; ++hh) {
+          const int half = (hh + w.part) & 1;
+#pragma unroll 1
+          for (int c = half * kHalf; c < (half + 1) * kHalf; ++c) {
+            uint32_t v[32];
+            sums(c, v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+              __stcg(mine + w.part * kPart + c * 1024 + 32 * j, make_float4(__uint_as_float(v[4 * j]), __uint_as_float(v[4 * j + 1]), __uint_as_float(v[4 * j + 2]), __uint_as_float(v[4 * j + 3])));
+          }
+          __threadfence();
+          __syncwarp();
+          int last = 0;
+          if (lane == 0) {
+            int* tk = p.part_tickets + ((tail * 2 + rank) * 4 + quarter) * 2 + half;
+            last = atomicAdd(tk, 1) == p.split - 1;
+            if (last) *tk = 0;
+          }
+          if (!__shfl_sync(0xffffffffu, last, 0)) continue;
+          __threadfence();
+#pragma unroll 1
+          for (int c = half * kHalf; c < (half + 1) * kHalf; ++c) {
+            float f[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) f[j] = 0.f;
+#pragma unroll 1
+            for (int q0 = 0; q0 < p.split; q0 += 4) {
+              float4 x[4][8];
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) x[q][j] = q0 + q < p.split ? __ldcg(mine + (q0 + q) * kPart + c * 1024 + 32 * j) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+              for (int q = 0; q < 4; ++q)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) { f[4 * j] += x[q][j].x; f[4 * j + 1] += x[q][j].y; f[4 * j + 2] += x[q][j].z; f[4 * j + 3] += x[q][j].w; }
+            }
+            uint32_t v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(f[j]);
+            const int n0 = nt * C::BN + c * 32;
+            if (grow < p.M && n0 < p.N) store_chunk(p, v, grow, n0);
+          }
+        }
       }
       tc_fence_before();
       __syncwarp();
@@ -884,22 +967,37 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& 
     configured[dev & 63] = true;
   }
   const int tiles = ((p.M + 2 * BM - 1) / (2 * BM)) * ((p.N + C::BN - 1) / C::BN), pairs = min(tiles, sm_count() / 2);
-  gemm_pair_kernel<<<2 * pairs, kThreads, C::SMEM, st>>>(ma, mb, p);
+  gemm_pair_kernel<<<p.split > 1 ? sm_count() / 2 * 2 : 2 * pairs, kThreads, C::SMEM, st>>>(ma, mb, p);
   return (int)cudaGetLastError();
+}
+
+// Parts along K of the pair form's last wave of tiles: the longest part, and what leaving, counting and adding parts costs (in k blocks of a tile, 0.27 us
+// each), against the whole tile; parts of 8 k blocks and more.  Behind more than six whole waves a last one is too little of the product to gain by
+// (34816 x 5120 at 900 rows, seven: 244 / 245 us; 3000 rows, 22: 676 / 682).
+int parts_of(int tiles, int kb) {
+  const int pairs = sm_count() / 2, rest = tiles % pairs;
+  int best = 1, cost = kb;
+  for (int s = 2; s <= 8 && rest > 0 && rest * s <= pairs && kb >= 8 * s && tiles / pairs <= 6; ++s) {
+    const int c = (kb + s - 1) / s + 24 + 2 * s;
+    if (c < cost) { cost = c; best = s; }
+  }
+  return best;
 }
 
 // Tile of a bf16 product that is not grouped: -256 the pair form, or 256 / 128 columns on one SM.  Waves of tiles times what a
 // wave takes (K = 5120, weights beyond L2): 256 x 256 on two SMs 30 us, 128 x 256 on one 33, 128 x 128 22; the narrow tile only
 // where it fits in one wave.  130 x 5120 x 17408: 110 / 78 us wide / narrow, 300 x 34816 x 5120: 128 / 116 pair / wide,
-// 512 x 5120 x 17408: 93 / 126, 4096 x 34816 x 5120: 908 / 986.
-int tile_of(int M, int N) {
-  const int sms = sm_count(), mt = (M + BM - 1) / BM, mp = (M + 2 * BM - 1) / (2 * BM);
+// 512 x 5120 x 17408: 93 / 126, 4096 x 34816 x 5120: 908 / 986.  parts: a workspace for cutting the last wave of pairs is there.
+int tile_of(int M, int N, int K, bool parts) {
+  const int sms = sm_count(), mt = (M + BM - 1) / BM, mp = (M + 2 * BM - 1) / (2 * BM), kb = K / 64;
   const int wide = (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
   if (N < 256) return wide;
   const auto waves = [](int tiles, int at_once) { return (tiles + at_once - 1) / at_once; };
-  const int n256 = (N + 255) / 256, n128 = (N + 127) / 128;
-  const int pair = waves(mp * n256, sms / 2) * 30, one = waves(mt * n256, sms) * 33;
-  if (mt * n128 <= sms && 22 < min(pair, one)) return 128;
+  const int n256 = (N + 255) / 256, n128 = (N + 127) / 128, s = parts ? parts_of(mp * n256, kb) : 1;
+  // in k blocks of a 256 x 256 tile
+  const int pair = s > 1 ? mp * n256 / (sms / 2) * kb + (kb + s - 1) / s + 24 + 2 * s : waves(mp * n256, sms / 2) * kb;
+  const int one = waves(mt * n256, sms) * kb * 11 / 10, narrow = kb * 11 / 15;
+  if (mt * n128 <= sms && narrow < min(pair, one)) return 128;
   return pair <= one ? -256 : wide;
 }
 
@@ -936,7 +1034,7 @@ static int gemm_tc_impl(const void* a, const void* b, void* c, int M, int N, int
                         const int* blk_row0, const int* blk_rows, const int* n_blk, int max_blk, int n_experts,
                         int bn, const void* rs_table, int rs_rank, int rs_world, int rs_tpr, const int* ag_cnt,
                         int ag_expect, const int* blk_wait, const int* row_src, const void* ret_table, void* stream,
-                        const Glu& glu = Glu{}) {
+                        const Glu& glu = Glu{}, float* part = nullptr, long long part_floats = 0, int* part_tickets = nullptr, int n_tickets = 0) {
   if (K % (i8 ? 128 : 64) != 0 || M < 1 || N % 8 != 0) return -1;
   if ((epi == EPI_SILU_MUL || epi == EPI_GLU) && N % 32 != 0) return -2;
   if (epi == EPI_RS_PUSH && (!rs_table || rs_world < 1 || rs_world > kMaxRanks || rs_rank < 0 || rs_rank >= rs_world ||
@@ -950,16 +1048,22 @@ static int gemm_tc_impl(const void* a, const void* b, void* c, int M, int N, int
   p.mt_rot = (epi == EPI_RS_PUSH) ? (rs_rank * rs_tpr) % ((M + BM - 1) / BM) : 0;
   p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.C = c; p.resid = (const __nv_bfloat16*)resid;
   p.a_scale = a_scale; p.b_scale = b_scale; p.epi = epi; p.glu = glu;
+  p.split = 0; p.part = part; p.part_tickets = part_tickets;
   p.blk_expert = blk_expert; p.blk_row0 = blk_row0; p.blk_rows = blk_rows; p.n_blk = n_blk; p.max_blk = max_blk;
   const bool local = !i8 && !blk_expert && !ag_cnt && epi != EPI_RS_PUSH && epi != EPI_EP_RETURN;
   bool pair = local && bn == -256;
   if (!pair && bn != 128 && bn != 256) {
-    bn = local ? tile_of(M, N) : (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
+    bn = local ? tile_of(M, N, K, part != nullptr) : (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
     // few rows: narrower tiles while they still fit in one wave
     if (!local && !blk_expert && ((M + BM - 1) / BM) * ((N + 127) / 128) <= sm_count()) bn = 128;
     pair = bn == -256;
   }
-  if (pair) bn = 128;       // B arrives in two halves
+  if (pair) {
+    bn = 128;       // B arrives in two halves
+    const int tiles = (M + 2 * BM - 1) / (2 * BM) * ((N + 255) / 256), rest = tiles % (sm_count() / 2);
+    if (part) p.split = parts_of(tiles, K / 64);
+    if (p.split > 1 && ((long long)rest * p.split * 65536 > part_floats || rest * 16 > n_tickets || ((uintptr_t)part & 15))) return -8;
+  }
   CUtensorMap ma, mb;
   int rc = make_map(&ma, a, i8 != 0, (uint64_t)M, (uint64_t)K, 0, blk_expert ? kGroupBox : BM);
   if (rc) return rc;
@@ -979,6 +1083,19 @@ extern "C" int b2_gemm_tc(const void* a, const void* b, void* c, int M, int N, i
                           int bn, void* stream) {
   return gemm_tc_impl(a, b, c, M, N, K, ldc, i8, epi, resid, a_scale, b_scale, blk_expert, blk_row0, blk_rows, n_blk,
                       max_blk, n_experts, bn, nullptr, 0, 1, 1, nullptr, 0, nullptr, nullptr, nullptr, stream);
+}
+
+// bf16 C = A * B^T with a workspace for cutting the last wave of tiles along K: b2_gemm_parts() floats and tickets, the latter zeroed once.  One product at a
+// time per workspace.
+extern "C" void b2_gemm_parts(long long* floats, int* tickets) {
+  *floats = (long long)(sm_count() / 2) * 65536;
+  *tickets = sm_count() / 2 * 16;
+}
+extern "C" int b2_gemm_tc_parts(const void* a, const void* b, void* c, int M, int N, int K, int ldc, int epi, const void* resid, int bn, float* part,
+                                long long part_floats, int* part_tickets, int n_tickets, void* stream) {
+  if (!part || !part_tickets || (epi != EPI_BF16 && epi != EPI_F32 && epi != EPI_SILU_MUL && epi != EPI_RESID_ADD && epi != EPI_RELU2)) return -1;
+  return gemm_tc_impl(a, b, c, M, N, K, ldc, 0, epi, resid, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 1, bn, nullptr, 0, 1, 1, nullptr, 0, nullptr,
+                      nullptr, nullptr, stream, Glu{}, part, part_floats, part_tickets, n_tickets);
 }
 
 // bf16 C [M][N / 2] = gated product of the interleave16 columns of A * B^T (common.cuh, Glu)

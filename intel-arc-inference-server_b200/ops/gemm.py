@@ -23,13 +23,24 @@ def _launch(a, b, c, m, n, k, ldc, i8, epi, resid=None, a_scale=None, b_scale=No
     K._check(rc, "gemm_tc")
 
 
+def gemm_parts(device) -> tuple:
+    """Workspace with which ``gemm_bf16`` cuts a last, partly filled wave of tiles along K: (fp32 partial sums, zeroed tickets) of a stream of products."""
+    floats, tickets = ctypes.c_longlong(0), ctypes.c_int(0)
+    K.lib().b2_gemm_parts(ctypes.byref(floats), ctypes.byref(tickets))
+    return (torch.empty(floats.value, dtype=torch.float32, device=device), torch.zeros(tickets.value, dtype=torch.int32, device=device))
+
+
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, epi: int = EPI_BF16,
-              resid: Optional[torch.Tensor] = None, bn: int = 0):
+              resid: Optional[torch.Tensor] = None, bn: int = 0, parts: Optional[tuple] = None):
     """``c = a @ b.T`` with ``a`` ``[M][K]``, ``b`` ``[N][K]`` bf16.  ``epi``: bf16 / fp32 store,
-    SiLU(gate)*up over interleave16 columns (``c`` is ``[M][N/2]``), ``resid + a b^T`` in bf16, or relu(x)^2 in bf16."""
+    SiLU(gate)*up over interleave16 columns (``c`` is ``[M][N/2]``), ``resid + a b^T`` in bf16, or relu(x)^2 in bf16.
+    ``parts``: a workspace of ``gemm_parts`` that no other product uses at the time."""
     m, k = a.shape
     n = b.shape[0]
-    _launch(a, b, c, m, n, k, c.stride(0), False, epi, resid=resid, bn=bn)
+    if parts is None:
+        return _launch(a, b, c, m, n, k, c.stride(0), False, epi, resid=resid, bn=bn)
+    K._check(K.lib().b2_gemm_tc_parts(K._p(a), K._p(b), K._p(c), m, n, k, c.stride(0), epi, K._p(resid), bn, K._p(parts[0]),
+                                      ctypes.c_longlong(parts[0].numel()), K._p(parts[1]), parts[1].numel(), K._stream()), "gemm_tc")
 
 
 def gemm_glu(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, limit: float, alpha: float, shift: float,

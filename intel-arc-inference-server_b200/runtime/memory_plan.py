@@ -113,6 +113,7 @@ def prefill_scratch_bytes(cfg: ModelConfig, chunk: int, backend: str) -> int:
         return 4 * step_scratch_elems(cfg, chunk, keys=2 * chunk)
     ffn = cfg.ffn if not cfg.is_moe else max(cfg.expert_ffn, cfg.shared_ffn)
     b = chunk * (2 * h * 2 + cfg.qkv_dim * 4 + 2 * cfg.q_dim * 2 + ffn * 2)
+    b += 20 << 20       # partial sums of a last wave of GEMM tiles
     biggest = max(cfg.qkv_dim * h, h * cfg.q_dim, 2 * ffn * h)
     if backend in ("bf16", "auto", "w4", "int4", "w4a16"):
         b += biggest * 2

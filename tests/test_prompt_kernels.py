@@ -152,6 +152,38 @@ def test_blocks_of_few_rows(n, k):
             assert torch.equal(got[:r], wb[i].T.repeat(128 // k + 1, 1)[:r]) and (got[r:] == 7.0).all()
 
 
+# one tile; a last wave of one, of a few and of half the pairs behind none, one and three whole ones; ragged rows and columns; parts of unequal length
+@pytest.mark.parametrize("m,n,k", [(300, 1000, 1088), (256, 19200, 1024), (900, 5120, 4160), (1000, 9728, 1536), (2048, 5640, 2048), (256, 256, 16384)])
+@pytest.mark.parametrize("epi", [G.EPI_BF16, G.EPI_F32, G.EPI_SILU_MUL, G.EPI_RESID_ADD])
+def test_last_wave_in_parts(m, n, k, epi):
+    if epi == G.EPI_SILU_MUL:
+        n = n // 32 * 32
+    torch.manual_seed(m + n)
+    a, b = torch.randn(m, k, device="cuda").bfloat16(), (torch.randn(n, k, device="cuda") * k ** -0.5).bfloat16()
+    shape = (m, n // 2 if epi == G.EPI_SILU_MUL else n)
+    dt = torch.float32 if epi == G.EPI_F32 else torch.bfloat16
+    resid = torch.randn(shape, device="cuda").bfloat16() if epi == G.EPI_RESID_ADD else None
+    parts = G.gemm_parts("cuda")
+    parts[0].fill_(float("nan"))
+    outs = []
+    for ws in (None, parts, parts):
+        c = torch.full((m + 1, shape[1]), float("nan"), dtype=dt, device="cuda")
+        G.gemm_bf16(a, b, c[:m], epi=epi, resid=resid, bn=-256, parts=ws)
+        torch.cuda.synchronize()
+        assert torch.isnan(c[m]).all() and int(parts[1].abs().sum()) == 0
+        outs.append(c[:m].double())
+    K.check_status()
+    assert torch.equal(outs[1], outs[2])                       # the same bits whichever part comes last
+    y = a.double() @ b.double().T
+    if epi == G.EPI_SILU_MUL:
+        v = y.view(m, n // 32, 2, 16)
+        y = (torch.nn.functional.silu(v[:, :, 0]) * v[:, :, 1]).reshape(shape)
+    y = y + resid.double() if resid is not None else y
+    # fp32 sums of k terms of about k ** -0.5, through the gate's slope; and the result's own rounding
+    err = lambda o: ((o - y).abs() - (0 if epi == G.EPI_F32 else 2.0 ** -8) * y.abs()).max()        # noqa: E731
+    assert err(outs[0]) < 2e-5 and err(outs[1]) < 2e-5
+
+
 @pytest.mark.parametrize("over", [-400, 0, 1])
 def test_experts_from_int4_or_copies(over, monkeypatch):
     """Prompt chunks on both sides of the rule: expanding a tile's blocks gives the bits of the bf16 copies."""
