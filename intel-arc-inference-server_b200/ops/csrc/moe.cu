@@ -342,47 +342,76 @@ __global__ void __launch_bounds__(1024) moe_plan_kernel(const int* __restrict__ 
 }
 
 // ---------------------------------------------------------------- scatter + gather
-// One CTA per (token, slot): writes the inverse map and copies the token's activation row to its
-// sorted position.
+// One CTA per token: writes the inverse map of its slots and copies its activation row to their sorted positions, each piece read
+// once (a CTA per slot: 2048 rows of 2048, eight slots, 26 -> 14 us; the bytes take 11.5).
+constexpr int kScatterSlots = 32;
 __global__ void __launch_bounds__(256) moe_scatter_kernel(const int* __restrict__ topk_idx, const int* __restrict__ rank,
                                                           const int* __restrict__ expert_base, int k,
                                                           const __nv_bfloat16* __restrict__ x, int H,
                                                           int* __restrict__ row_of, __nv_bfloat16* __restrict__ xs) {
-  const int i = blockIdx.x;  // token * k + slot
-  const int token = i / k;
-  const int pos = expert_base[topk_idx[i]] + rank[i];
-  if (threadIdx.x == 0) row_of[i] = pos;
-  const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)token * H);
-  uint4* dst = reinterpret_cast<uint4*>(xs + (size_t)pos * H);
-  for (int j = threadIdx.x; j < H / 8; j += blockDim.x) dst[j] = src[j];
+  __shared__ int s_pos[kScatterSlots];
+  const int token = blockIdx.x;
+  for (int s0 = 0; s0 < k; s0 += kScatterSlots) {
+    const int ns = min(kScatterSlots, k - s0);
+    if (s0) __syncthreads();
+    if ((int)threadIdx.x < ns) {
+      const int i = token * k + s0 + threadIdx.x;
+      row_of[i] = s_pos[threadIdx.x] = expert_base[topk_idx[i]] + rank[i];
+    }
+    __syncthreads();
+    const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)token * H);
+    for (int j = threadIdx.x; j < H / 8; j += blockDim.x) {
+      const uint4 v = src[j];
+      for (int s = 0; s < ns; ++s) reinterpret_cast<uint4*>(xs + (size_t)s_pos[s] * H)[j] = v;
+    }
+  }
 }
 
 // ---------------------------------------------------------------- combine (prefill): one CTA per token
-// out[token] = resid[token] + sum_slot w[slot] * y[row_of[token][slot]] + sigmoid(gate_logit[token]) * shared[token]
+// out[token] = resid[token] + sum_slot w[slot] * y[row_of[token][slot]] + sigmoid(gate_logit[token]) * shared[token], added in that order.
+// V: columns a thread takes at a time, 8 where rows begin on 16 bytes; up to eight slots' pieces are in flight together (one after another, two
+// columns a thread: 2048 rows of 2048, eight slots, 46 -> 25 us; the bytes take 14).
+template <int V>
 __global__ void __launch_bounds__(256) moe_combine_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ row_of,
                                                           const float* __restrict__ topk_w, int k, int H,
                                                           const __nv_bfloat16* __restrict__ shared_y,
                                                           const float* __restrict__ gate_logit, int gate_ld,
-                                                          const __nv_bfloat16* __restrict__ resid,
-                                                          __nv_bfloat16* __restrict__ out) {
+                                                          const __nv_bfloat16* resid,
+                                                          __nv_bfloat16* out) {
+  constexpr int W = V / 2;       // words
+  struct __align__(4 * W) Piece { uint32_t w[W]; };
+  const auto at = [](const __nv_bfloat16* p, size_t row, int H, int j) { return *reinterpret_cast<const Piece*>(p + row * H + (size_t)j * V); };
   const int token = blockIdx.x;
   float g = 0.f;
   if (shared_y) g = gate_logit ? 1.f / (1.f + __expf(-gate_logit[(size_t)token * gate_ld])) : 1.f;
-  for (int j = threadIdx.x; j < H / 2; j += blockDim.x) {
-    float2 acc = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(resid + (size_t)token * H)[j]);
-    for (int s = 0; s < k; ++s) {
-      const int row = row_of[token * k + s];
-      const float w = topk_w[token * k + s];
-      const float2 v = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(y + (size_t)row * H)[j]);
-      acc.x = fmaf(w, v.x, acc.x);
-      acc.y = fmaf(w, v.y, acc.y);
+  for (int j = threadIdx.x; j < H / V; j += blockDim.x) {
+    float acc[V];
+    const auto add = [&](float w, const Piece& v) {
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        acc[2 * i] = fmaf(w, bf16_lo(v.w[i]), acc[2 * i]);
+        acc[2 * i + 1] = fmaf(w, bf16_hi(v.w[i]), acc[2 * i + 1]);
+      }
+    };
+    const Piece r = at(resid, token, H, j);
+    Piece sh = {};
+    if (shared_y) sh = at(shared_y, token, H, j);
+#pragma unroll
+    for (int i = 0; i < W; ++i) { acc[2 * i] = bf16_lo(r.w[i]); acc[2 * i + 1] = bf16_hi(r.w[i]); }
+    for (int s0 = 0; s0 < k; s0 += 8) {
+      Piece v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (s0 + u < k) v[u] = at(y, row_of[token * k + s0 + u], H, j);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (s0 + u < k) add(topk_w[token * k + s0 + u], v[u]);
     }
-    if (shared_y) {
-      const float2 v = __bfloat1622float2(reinterpret_cast<const __nv_bfloat162*>(shared_y + (size_t)token * H)[j]);
-      acc.x = fmaf(g, v.x, acc.x);
-      acc.y = fmaf(g, v.y, acc.y);
-    }
-    reinterpret_cast<__nv_bfloat162*>(out + (size_t)token * H)[j] = __floats2bfloat162_rn(acc.x, acc.y);
+    if (shared_y) add(g, sh);
+    Piece o;
+#pragma unroll
+    for (int i = 0; i < W; ++i) o.w[i] = pack_bf16(acc[2 * i], acc[2 * i + 1]);
+    *reinterpret_cast<Piece*>(out + (size_t)token * H + (size_t)j * V) = o;
   }
 }
 
@@ -520,7 +549,7 @@ extern "C" int b2_moe_count(const int* topk_idx, int n, int* counts, int* rank, 
 extern "C" int b2_moe_scatter(const int* topk_idx, const int* rank, const int* expert_base, int T, int k, const void* x,
                               int H, int* row_of, void* xs, void* stream) {
   if (H % 8) return -1;
-  moe_scatter_kernel<<<T * k, 256, 0, (cudaStream_t)stream>>>(topk_idx, rank, expert_base, k, (const __nv_bfloat16*)x, H,
+  moe_scatter_kernel<<<T, 256, 0, (cudaStream_t)stream>>>(topk_idx, rank, expert_base, k, (const __nv_bfloat16*)x, H,
                                                                 row_of, (__nv_bfloat16*)xs);
   return (int)cudaGetLastError();
 }
@@ -529,7 +558,9 @@ extern "C" int b2_moe_combine(const void* y, const int* row_of, const float* top
                               const void* shared_y, const float* gate_logit, int gate_ld, const void* resid, void* out,
                               void* stream) {
   if (H % 2) return -1;
-  moe_combine_kernel<<<T, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)y, row_of, topk_w, k, H,
+  const bool wide = H % 8 == 0 && (((uintptr_t)y | (uintptr_t)shared_y | (uintptr_t)resid | (uintptr_t)out) & 15) == 0;
+  const auto kernel = wide ? moe_combine_kernel<8> : moe_combine_kernel<2>;
+  kernel<<<T, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)y, row_of, topk_w, k, H,
                                                            (const __nv_bfloat16*)shared_y, gate_logit, gate_ld,
                                                            (const __nv_bfloat16*)resid, (__nv_bfloat16*)out);
   return (int)cudaGetLastError();

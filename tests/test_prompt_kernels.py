@@ -186,6 +186,37 @@ def test_last_wave_in_parts(m, n, k, epi):
     assert all(((o - y).abs() <= bound).all() for o in outs)
 
 
+# slots around a pass of eight (combine) and of 32 (scatter), rows of pieces for some of a CTA and for several rounds; two columns a piece
+@pytest.mark.parametrize("h", [2, 130, 136, 2048, 4104])
+@pytest.mark.parametrize("k", [1, 7, 8, 9, 33])
+@pytest.mark.parametrize("shared", [None, "plain", "gated"])
+def test_scatter_and_combine(h, k, shared):
+    from b200serve.ops import moe as M
+    torch.manual_seed(h + k)
+    t, e = 37, 64
+    idx = torch.stack([torch.randperm(e, device="cuda")[:k] for _ in range(t)]).int()
+    x, resid, sh = (torch.randn(t, h, device="cuda").bfloat16() for _ in range(3))
+    w, gate = torch.rand(t, k, device="cuda"), torch.randn(t, 3, device="cuda")
+    row_of, blocks = torch.randperm(t * k + 5, device="cuda")[: t * k].int(), torch.randn(t * k + 5, h, device="cuda").bfloat16()
+    if h % 8 == 0:
+        base = torch.arange(e, device="cuda").int() * t
+        rank = torch.zeros(t * k, dtype=torch.int32, device="cuda")
+        for i in range(e):
+            rank[(idx.view(-1) == i).nonzero().flatten()] = torch.arange(int((idx == i).sum()), device="cuda").int()
+        at, xs = torch.zeros(t * k, dtype=torch.int32, device="cuda"), torch.full((e * t, h), float("nan"), device="cuda").bfloat16()
+        M.scatter(idx.view(-1), rank, base, t, k, x, h, at, xs)
+        assert torch.equal(at, base[idx.view(-1).long()] + rank) and torch.equal(xs[at.long()], x.repeat_interleave(k, 0))
+        assert int(xs.isnan().all(-1).sum()) == e * t - t * k
+    out = torch.empty_like(resid)
+    M.combine(blocks, row_of, w, t, k, h, sh if shared else None, gate if shared == "gated" else None, 3, resid, out)
+    torch.cuda.synchronize()
+    want = resid.double() + (blocks.double()[row_of.long()].view(t, k, h) * w.double()[..., None]).sum(1)
+    if shared:
+        want += sh.double() * (torch.sigmoid(gate[:, :1].double()) if shared == "gated" else 1.0)
+    size = resid.double().abs() + (blocks.double().abs()[row_of.long()].view(t, k, h) * w.double()[..., None]).sum(1) + sh.double().abs()
+    assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + (k + 2) * 2.0 ** -22 * size).all()       # rounded once; fp32 sums, the gate by a fast exponential
+
+
 @pytest.mark.parametrize("over", [-400, 0, 1])
 def test_experts_from_int4_or_copies(over, monkeypatch):
     """Prompt chunks on both sides of the rule: expanding a tile's blocks gives the bits of the bf16 copies."""
