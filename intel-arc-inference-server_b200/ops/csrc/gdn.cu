@@ -81,7 +81,10 @@ __device__ __forceinline__ bool first_of_slot(const int* ctrl, int m, int slot) 
   return true;
 }
 
+// ONE: a single slice, whose loads (unlike a loop's) go out together
+template <bool ONE>
 __device__ __forceinline__ float4 conv_in(const GdnConvParams& p, int m, int n) {
+  if (ONE) return *reinterpret_cast<const float4*>(p.part + (size_t)m * p.N + n);
   float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
   for (int s = 0; s < p.splits; ++s) {
@@ -122,7 +125,10 @@ struct ConvTaps {
 // 16480-wide projection, each a chain of 3000 dependent row visits: 2070 us where the bytes take 60 (a 3000-token prompt
 // through 12 such layers and 4 of attention: 61.1 -> 41.7 ms).
 // Rows of a step (ctrl): the CTAs of a slot's first row walk that slot's rows; the others leave.
+// The eight rows that a thread takes at a time are in flight together (ONE; with the loop over slices one after another: 3000 rows of 16480
+// 175 -> 69 us; the bytes take 60).
 constexpr int CONV_R = 16, CONV_T = 128, CONV_U = 8;
+template <bool ONE>
 __global__ void __launch_bounds__(CONV_T) gdn_conv_rows_kernel(const GdnConvParams p) {
   pdl_wait();
   pdl_launch_dependents();
@@ -140,7 +146,7 @@ __global__ void __launch_bounds__(CONV_T) gdn_conv_rows_kernel(const GdnConvPara
     }
     for (int m = blockIdx.y; m < p.M; ++m) {
       if (p.ctrl[CTRL_ROW_REQ + m] != slot) continue;
-      const float4 x = conv_in(p, m, n);
+      const float4 x = conv_in<ONE>(p, m, n);
       *reinterpret_cast<float4*>(p.act + (size_t)m * p.N + n) = conv ? t.step(x) : x;
     }
     if (conv) t.store(st);
@@ -155,25 +161,25 @@ __global__ void __launch_bounds__(CONV_T) gdn_conv_rows_kernel(const GdnConvPara
     if (m0 == 0) {
       t.load(st);
     } else {
-      t.a = conv_in(p, m0 - 3, n);
-      t.b = conv_in(p, m0 - 2, n);
-      t.c = conv_in(p, m0 - 1, n);
+      t.a = conv_in<ONE>(p, m0 - 3, n);
+      t.b = conv_in<ONE>(p, m0 - 2, n);
+      t.c = conv_in<ONE>(p, m0 - 1, n);
     }
   }
   for (int m = m0; m < m1; m += CONV_U) {
     float4 x[CONV_U];
 #pragma unroll
     for (int u = 0; u < CONV_U; ++u)
-      if (m + u < m1) x[u] = conv_in(p, m + u, n);
+      if (m + u < m1) x[u] = conv_in<ONE>(p, m + u, n);
 #pragma unroll
     for (int u = 0; u < CONV_U; ++u)
       if (m + u < m1) *reinterpret_cast<float4*>(p.act + (size_t)(m + u) * p.N + n) = conv ? t.step(x[u]) : x[u];
   }
   // the chunk's last three inputs become the slot's state: written by the CTA that read the old one
   if (conv && m0 == 0) {
-    t.a = conv_in(p, p.M - 3, n);
-    t.b = conv_in(p, p.M - 2, n);
-    t.c = conv_in(p, p.M - 1, n);
+    t.a = conv_in<ONE>(p, p.M - 3, n);
+    t.b = conv_in<ONE>(p, p.M - 2, n);
+    t.c = conv_in<ONE>(p, p.M - 1, n);
     t.store(st);
   }
 }
@@ -376,7 +382,9 @@ __global__ void __launch_bounds__(256) gdn_gate_kernel(const GdnChunkParams p) {
 // gdn_wy_prep_kernel  grid (chunks, n_v), all chunks at once: the products K K^T and Q K^T (bf16 split in two
 //                     limbs where the triangular solve amplifies errors), the solve by forward substitution in
 //                     fp32 (thread = one column of [Wk | Wv], its 64 values in registers), and the operand images
-//                     of the scan, padded for conflict-free ldmatrix, in a workspace block per (chunk, head);
+//                     of the scan, padded for conflict-free ldmatrix, in a workspace block per (chunk, head).  3000 rows, 48 heads:
+//                     312 -> 256 us with the decay factors' exponentials once per chunk instead of once per thread, packed FMAs, and
+//                     images stored by whole sectors (the bytes take 57);
 // gdn_wy_scan_kernel  grid (n_v, 2), four warps: walks the chunks; a warp owns 16 value columns of the state, S^T[16][128] fp32 in
 //                     MMA accumulator registers for the whole walk.  Every product is written with the value
 //                     dimension as M, so accumulators turn into the next product's A operand in registers
@@ -385,12 +393,12 @@ __global__ void __launch_bounds__(256) gdn_gate_kernel(const GdnChunkParams p) {
 constexpr int WY_C = 64;
 constexpr int WY_LDK = 136;                       // bf16 per row of a [64][128] image
 constexpr int WY_LDP = 72;                        // bf16 per row of a [..][64] image
-constexpr int WY_LDV = 68;                        // fp32 per row of Wv^T [128][64]
+constexpr int WY_LDV = 68;                        // fp32 per row of Wv [2 halves of the value columns][64][64], and of A [64][64]
 constexpr int WY_OFF_WK = 0;                      // Wk   [64][136] bf16  (row s, column dk)
 constexpr int WY_OFF_QG = WY_OFF_WK + WY_C * WY_LDK * 2;     // Qg   [64][136] bf16  gamma_s q_s
 constexpr int WY_OFF_KGT = WY_OFF_QG + WY_C * WY_LDK * 2;    // Kg^T [128][72] bf16  (row dk, column s) (gamma_63 / gamma_s) k_s
 constexpr int WY_OFF_P = WY_OFF_KGT + DH * WY_LDP * 2;       // P    [64][72]  bf16  (row t, column s)
-constexpr int WY_OFF_WVT = WY_OFF_P + WY_C * WY_LDP * 2;     // Wv^T [128][68] fp32  (row dv, column s)
+constexpr int WY_OFF_WVT = WY_OFF_P + WY_C * WY_LDP * 2;     // Wv   [2][64][68] fp32 (half of dv, row s, column dv): a warp stores whole sectors
 constexpr int WY_OFF_GC = WY_OFF_WVT + DH * WY_LDV * 4;      // gamma_63 (fp32) + padding
 constexpr int WY_BLOCK = WY_OFF_GC + 16;
 static_assert(WY_BLOCK % 16 == 0 && WY_OFF_WVT % 16 == 0, "bulk copies move multiples of 16 bytes");
@@ -415,7 +423,7 @@ __device__ __forceinline__ uint32_t ldsm_b_addr(uint32_t base, int ld, int n0, i
   return base + (uint32_t)(((n0 + (lane & 7) + ((lane >> 4) << 3)) * ld + k0 + (((lane >> 3) & 1) << 3)) * 2);
 }
 
-constexpr int WYA_SMEM = 3 * WY_C * WY_LDK * 2 + WY_C * WY_LDV * 4 + 2 * WY_C * 4;
+constexpr int WYA_SMEM = 3 * WY_C * WY_LDK * 2 + WY_C * WY_LDV * 4 + 4 * WY_C * 4;
 
 __global__ void __launch_bounds__(256, 2) gdn_wy_prep_kernel(const GdnWyParams p) {
   extern __shared__ __align__(16) uint8_t wy_smem[];
@@ -425,6 +433,8 @@ __global__ void __launch_bounds__(256, 2) gdn_wy_prep_kernel(const GdnWyParams p
   float* As = reinterpret_cast<float*>(Qhi + WY_C * WY_LDK);      // [64][68]
   float* lg = As + WY_C * WY_LDV;                                 // log gamma_s
   float* bet = lg + WY_C;
+  float* eg = bet + WY_C;                                         // gamma_s, and gamma_63 / gamma_s
+  float* ek = eg + WY_C;
   pdl_wait();
   pdl_launch_dependents();
   const int c = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -450,13 +460,19 @@ __global__ void __launch_bounds__(256, 2) gdn_wy_prep_kernel(const GdnWyParams p
       const float v = __shfl_up_sync(0xffffffffu, run, o);
       if (lane >= o) run += v;
     }
+    const float l63 = __shfl_sync(0xffffffffu, run, 31);
     lg[s1] = run;
     lg[s0] = run - l1;
+    eg[s1] = __expf(run);
+    eg[s0] = __expf(run - l1);
+    ek[s1] = __expf(l63 - run);
+    ek[s0] = __expf(l63 - (run - l1));
     bet[s0] = b0;
     bet[s1] = b1;
   }
-  // rows of K and Q into shared memory as bf16 limbs; 16 rows' loads are in flight per thread at a time
+  // rows of K and Q into shared memory as bf16 limbs, and gamma_s q_s into its image; 16 rows' loads are in flight per thread at a time
   {
+    __nv_bfloat16* Qg = reinterpret_cast<__nv_bfloat16*>(blk + WY_OFF_QG);
     const int col = tid & 127, sh = tid >> 7;      // this thread: column col of rows sh, sh + 2, ...
 #pragma unroll
     for (int s0 = 0; s0 < WY_C; s0 += 32) {
@@ -467,9 +483,11 @@ __global__ void __launch_bounds__(256, 2) gdn_wy_prep_kernel(const GdnWyParams p
         kv[u] = s < valid ? a0[(size_t)s * p.N + kd + hk * DH + col] : 0.f;
         qv[u] = s < valid ? a0[(size_t)s * p.N + hk * DH + col] : 0.f;
       }
+      if (s0 == 0) __syncthreads();      // the decay factors are there
 #pragma unroll
       for (int u = 0; u < 16; ++u) {
         const int s = s0 + 2 * u + sh;
+        Qg[s * WY_LDK + col] = __float2bfloat16(qv[u] * eg[s]);
         const __nv_bfloat16 kh = __float2bfloat16(kv[u]);
         Khi[s * WY_LDK + col] = kh;
         Klo[s * WY_LDK + col] = __float2bfloat16(kv[u] - __bfloat162float(kh));
@@ -525,64 +543,65 @@ __global__ void __launch_bounds__(256, 2) gdn_wy_prep_kernel(const GdnWyParams p
 #pragma unroll
     for (int s = 0; s < WY_C; ++s) w[s] = s < valid ? src[(size_t)s * p.N] : 0.f;
 #pragma unroll
-    for (int s = 0; s < WY_C; ++s) w[s] *= tid < DH ? bet[s] * __expf(lg[s]) : bet[s];
+    for (int s = 0; s < WY_C; ++s) w[s] *= tid < DH ? bet[s] * eg[s] : bet[s];
   }
   __syncthreads();
 #pragma unroll
   for (int s = 1; s < WY_C; ++s) {
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    uint64_t acc01 = 0, acc23 = 0;        // four sums, as packed pairs
 #pragma unroll
-    for (int r = 0; r < s; r += 4) {      // A[s][r] is zero from r = s on: whole float4 groups
+    for (int r = 0; r < s; r += 4) {      // A[s][r] is zero from r = s on: whole pairs
       const float4 a4 = *reinterpret_cast<const float4*>(As + s * WY_LDV + r);
-      acc[0] = fmaf(a4.x, w[r], acc[0]);
-      if (r + 1 < s) acc[1] = fmaf(a4.y, w[r + 1], acc[1]);
-      if (r + 2 < s) acc[2] = fmaf(a4.z, w[r + 2], acc[2]);
-      if (r + 3 < s) acc[3] = fmaf(a4.w, w[r + 3], acc[3]);
+      const auto madd = [](uint64_t& acc, float a0, float a1, float w0, float w1) {
+        uint64_t a2, w2;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(a2) : "f"(a0), "f"(a1));
+        asm("mov.b64 %0, {%1, %2};" : "=l"(w2) : "f"(w0), "f"(w1));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a2), "l"(w2));
+      };
+      madd(acc01, a4.x, a4.y, w[r], w[r + 1]);
+      if (r + 2 < s) madd(acc23, a4.z, a4.w, w[r + 2], w[r + 3]);
     }
-    w[s] -= (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    float f0, f1, f2, f3;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f0), "=f"(f1) : "l"(acc01));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f2), "=f"(f3) : "l"(acc23));
+    w[s] -= (f0 + f1) + (f2 + f3);
   }
   if (tid < DH) {
     __nv_bfloat16* Wk = reinterpret_cast<__nv_bfloat16*>(blk + WY_OFF_WK);
 #pragma unroll
     for (int s = 0; s < WY_C; ++s) Wk[s * WY_LDK + tid] = __float2bfloat16(w[s]);
-    // Kg^T row dk = tid: (gamma_63 / gamma_s) k_s[dk]
-    uint32_t* Kg = reinterpret_cast<uint32_t*>(blk + WY_OFF_KGT) + tid * (WY_LDP / 2);
-    const float l63 = lg[WY_C - 1];
-#pragma unroll
-    for (int s = 0; s < WY_C; s += 2) {
-      const float k0 = __bfloat162float(Khi[s * WY_LDK + tid]) + __bfloat162float(Klo[s * WY_LDK + tid]);
-      const float k1 = __bfloat162float(Khi[(s + 1) * WY_LDK + tid]) + __bfloat162float(Klo[(s + 1) * WY_LDK + tid]);
-      Kg[s >> 1] = pack_bf16(k0 * __expf(l63 - lg[s]), k1 * __expf(l63 - lg[s + 1]));
-    }
   } else {
-    float4* Wv = reinterpret_cast<float4*>(blk + WY_OFF_WVT) + (tid - DH) * (WY_LDV / 4);
+    float* Wv = reinterpret_cast<float*>(blk + WY_OFF_WVT) + ((tid - DH) >> 6) * (WY_C * WY_LDV) + (tid & 63);
 #pragma unroll
-    for (int s = 0; s < WY_C; s += 4) Wv[s >> 2] = make_float4(w[s], w[s + 1], w[s + 2], w[s + 3]);
+    for (int s = 0; s < WY_C; ++s) Wv[s * WY_LDV] = w[s];
   }
-  // Qg = gamma_s q_s (from the fp32 rows)
-  __nv_bfloat16* Qg = reinterpret_cast<__nv_bfloat16*>(blk + WY_OFF_QG);
+  // Kg^T: (gamma_63 / gamma_s) k_s[dk] in row dk, pairs of s from transposed 8 x 8 tiles: a quad stores 16 bytes of a row (a thread per row: 32
+  // sectors a store instruction)
   {
-    const int col = tid & 127, sh = tid >> 7;
+    const int g = lane >> 2, t = lane & 3;
+    const uint32_t kh_b = smem_u32(Khi), kl_b = smem_u32(Klo);
+    uint32_t* Kg = reinterpret_cast<uint32_t*>(blk + WY_OFF_KGT);
 #pragma unroll
-    for (int s0 = 0; s0 < WY_C; s0 += 32) {
-      float qv[16];
+    for (int i = 0; i < 2; ++i)
 #pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int s = s0 + 2 * u + sh;
-        qv[u] = s < valid ? a0[(size_t)s * p.N + hk * DH + col] : 0.f;
+      for (int sb = 0; sb < WY_C; sb += 32) {
+        const int dk = 16 * warp + 8 * i;
+        const uint32_t off = (uint32_t)(((sb + lane) * WY_LDK + dk) * 2);
+        uint32_t hi[4], lo[4];
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(hi[0]), "=r"(hi[1]), "=r"(hi[2]), "=r"(hi[3]) : "r"(kh_b + off));
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(lo[0]), "=r"(lo[1]), "=r"(lo[2]), "=r"(lo[3]) : "r"(kl_b + off));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int s = sb + 8 * q + 2 * t;
+          Kg[(dk + g) * (WY_LDP / 2) + (s >> 1)] = pack_bf16((bf16_lo(hi[q]) + bf16_lo(lo[q])) * ek[s], (bf16_hi(hi[q]) + bf16_hi(lo[q])) * ek[s + 1]);
+        }
       }
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int s = s0 + 2 * u + sh;
-        Qg[s * WY_LDK + col] = __float2bfloat16(qv[u] * __expf(lg[s]));
-      }
-    }
   }
-  if (tid == 0) *reinterpret_cast<float*>(blk + WY_OFF_GC) = __expf(lg[WY_C - 1]);
+  if (tid == 0) *reinterpret_cast<float*>(blk + WY_OFF_GC) = eg[WY_C - 1];
 }
 
-// the scan's stage: the block's images up to Wv^T, this CTA's half of Wv^T (64 value columns), gamma_63
-constexpr int WYB_WV_HALF = (DH / 2) * WY_LDV * 4;
+// the scan's stage: the block's images up to Wv^T, this CTA's half of Wv (64 value columns), gamma_63
+constexpr int WYB_WV_HALF = WY_C * WY_LDV * 4;
 constexpr int WYB_STAGE = WY_OFF_WVT + WYB_WV_HALF + 16;
 constexpr int WYB_SMEM = 2 * WYB_STAGE + 64;
 static_assert(WYB_STAGE % 128 == 0 || WYB_STAGE % 16 == 0, "stages start on 16-byte boundaries");
@@ -673,8 +692,8 @@ __global__ void __launch_bounds__(128, 1) gdn_wy_scan_kernel(const GdnWyParams p
       const float* wv = reinterpret_cast<const float*>(wy_smem + b * WYB_STAGE + WY_OFF_WVT);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float2 v0 = *reinterpret_cast<const float2*>(wv + dvl * WY_LDV + 8 * j + 2 * t);
-        const float2 v1 = *reinterpret_cast<const float2*>(wv + (dvl + 8) * WY_LDV + 8 * j + 2 * t);
+        const float* w = wv + (8 * j + 2 * t) * WY_LDV + dvl;
+        const float2 v0 = make_float2(w[0], w[WY_LDV]), v1 = make_float2(w[8], w[WY_LDV + 8]);
         const float u0 = v0.x - r1[j][0], u1 = v0.y - r1[j][1], u2 = v1.x - r1[j][2], u3 = v1.y - r1[j][3];
         // tile j is the k-half (j & 1) of k-step j >> 1: regs 0, 1 (rows g, g + 8) or 2, 3
         split2(u0, u1, uh[j >> 1][2 * (j & 1)], ul[j >> 1][2 * (j & 1)]);
@@ -777,7 +796,7 @@ extern "C" int b2_gdn_conv(const float* part, int splits, int M, int N, int conv
   const uintptr_t at = (uintptr_t)part | (uintptr_t)conv_w | (uintptr_t)conv_state | (uintptr_t)act;
   if (N % 4 == 0 && conv_ch % 4 == 0 && at % 16 == 0 && (ctrl || (M >= 3 && apart))) {
     const dim3 grid((N / 4 + CONV_T - 1) / CONV_T, ctrl ? M : (M + CONV_R - 1) / CONV_R);
-    if (grid.y <= 65535u) return b2_launch(gdn_conv_rows_kernel, grid, dim3(CONV_T), 0, (cudaStream_t)stream, true, p);
+    if (grid.y <= 65535u) return b2_launch(splits == 1 ? gdn_conv_rows_kernel<true> : gdn_conv_rows_kernel<false>, grid, dim3(CONV_T), 0, (cudaStream_t)stream, true, p);
   }
   return b2_launch(gdn_conv_kernel, dim3((N + 255) / 256), dim3(256), 0, (cudaStream_t)stream, true, p);
 }
