@@ -988,16 +988,18 @@ int parts_of(int tiles, int kb) {
 // wave takes (K = 5120, weights beyond L2): 256 x 256 on two SMs 30 us, 128 x 256 on one 33, 128 x 128 22; the narrow tile only
 // where it fits in one wave.  130 x 5120 x 17408: 110 / 78 us wide / narrow, 300 x 34816 x 5120: 128 / 116 pair / wide,
 // 512 x 5120 x 17408: 93 / 126, 4096 x 34816 x 5120: 908 / 986.  parts: a workspace for cutting the last wave of pairs is there.
-int tile_of(int M, int N, int K, bool parts) {
+// cost: the estimate, in k blocks of a 256 x 256 tile (0.375 us while all SMs work).
+int tile_of(int M, int N, int K, bool parts, int* cost = nullptr) {
   const int sms = sm_count(), mt = (M + BM - 1) / BM, mp = (M + 2 * BM - 1) / (2 * BM), kb = K / 64;
   const int wide = (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
-  if (N < 256) return wide;
   const auto waves = [](int tiles, int at_once) { return (tiles + at_once - 1) / at_once; };
   const int n256 = (N + 255) / 256, n128 = (N + 127) / 128, s = parts ? parts_of(mp * n256, kb) : 1;
-  // in k blocks of a 256 x 256 tile
   const int pair = s > 1 ? mp * n256 / (sms / 2) * kb + (kb + s - 1) / s + 24 + 2 * s : waves(mp * n256, sms / 2) * kb;
   const int one = waves(mt * n256, sms) * kb * 11 / 10, narrow = kb * 11 / 15;
-  if (mt * n128 <= sms && narrow < min(pair, one)) return 128;
+  const bool fits = mt * n128 <= sms && (N < 256 || narrow < min(pair, one));
+  if (cost) *cost = fits ? narrow : min(pair, one);
+  if (N < 256) return wide;
+  if (fits) return 128;
   return pair <= one ? -256 : wide;
 }
 
@@ -1017,7 +1019,11 @@ extern "C" int b2_gemm_w4(const void* a, const void* w4b, void* c, int M, int N,
   p.rs_world = 1; p.rs_tpr = 1;
   p.w4 = (const uint8_t*)w4b;
   p.w4_expert_bytes = (long long)((N + 127) / 128) * (K / 64) * kW4Block;
-  if (bn != 128 && bn != 256) bn = (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
+  if (bn != 128 && bn != 256) {
+    bn = (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
+    // narrow tiles while they fit in one wave (100 x 7168 x 5120: 57 / 46 us wide / narrow, x 5120 x 17408 166 / 137)
+    if (!blk_expert && (M + BM - 1) / BM * ((N + 127) / 128) <= sm_count()) bn = 128;
+  }
   CUtensorMap ma;
   int rc = make_map(&ma, a, false, (uint64_t)M, (uint64_t)K, 0, blk_expert ? kGroupBox : BM);
   if (rc) return rc;
@@ -1083,6 +1089,23 @@ extern "C" int b2_gemm_tc(const void* a, const void* b, void* c, int M, int N, i
                           int bn, void* stream) {
   return gemm_tc_impl(a, b, c, M, N, K, ldc, i8, epi, resid, a_scale, b_scale, blk_expert, blk_row0, blk_rows, n_blk,
                       max_blk, n_experts, bn, nullptr, 0, 1, 1, nullptr, 0, nullptr, nullptr, nullptr, stream);
+}
+
+// 1: a product of M rows with an int4 weight is estimated to be faster from the blocks (b2_gemm_w4) than from an expanded copy that has to be made first
+// (b2_dequant_w4b and b2_gemm_tc_parts).  Expanding takes 0.46 us for a million weights, reading the blocks 0.56 us (128 x 128 tiles) or 0.68 (128 x 256) for a k block and wave.
+// us, blocks / copy: 100 x 5120 x 17408 137 / 91, x 5120 x 5120 44 / 35, x 7168 x 5120 46 / 48, x 16480 x 5120 47 / 76, x 34816 x 5120 65 / 152, 200 x 34816 x
+// 5120 113 / 159, x 16480 x 5120 60 / 81.  Small weights (below 16 M; behind a row of tiles, whose blocks are expanded again, 32 M) stay where the rows put
+// them: 100 x 3072 x 2048 22 / 20.  8 layers, 80 / 128 / 200 / 256 rows, by rows alone and so: dense 27B shape 2.98 -> 2.62, 3.01 -> 2.66, 3.46 -> 3.09,
+// 3.49 -> 3.11 ms, hybrid 3.31 -> 2.91, 3.35 -> 2.96, 4.03 -> 3.48, 4.04 -> 3.50.
+extern "C" int b2_gemm_w4_blocks(int M, int N, int K) {
+  const int mt = (M + BM - 1) / BM, kb = K / 64, sms = sm_count();
+  const bool narrow = mt * ((N + 127) / 128) <= sms;
+  const double blocks = narrow ? 0.56 * kb : 0.68 * kb * ((mt * ((N + 255) / 256) + sms - 1) / sms);
+  int cost = 0;
+  tile_of(M, N, K, true, &cost);
+  const double copy = (double)N * K * 4.6e-7 + 0.375 * cost + 4.0;
+  const double weights = (double)N * K;
+  return mt == 1 ? blocks <= copy || weights < 16777216.0 : blocks <= 0.8 * copy && weights >= 33554432.0;
 }
 
 // bf16 C = A * B^T with a workspace for cutting the last wave of tiles along K: b2_gemm_parts() floats and tickets, the latter zeroed once.  One product at a

@@ -2,6 +2,7 @@
 from __future__ import annotations
 
 import ctypes
+import functools
 from typing import Optional
 
 import torch
@@ -72,6 +73,12 @@ def gemm_w4(a: torch.Tensor, w4b: torch.Tensor, n: int, k: int, c: torch.Tensor,
     rc = K.lib().b2_gemm_w4(K._p(a), K._p(w4b), K._p(c), a.shape[0], n, k, c.stride(0), epi, K._p(resid), K._p(be),
                             K._p(br0), K._p(brn), K._p(nb), max_blk, n_experts, bn, K._stream())
     K._check(rc, "gemm_w4")
+
+
+@functools.lru_cache(maxsize=4096)
+def w4_from_blocks(m: int, n: int, k: int) -> bool:
+    """``m`` rows against an int4 ``[n][k]`` weight are faster from its blocks (``gemm_w4``) than from a bf16 copy that has to be made first."""
+    return bool(K.lib().b2_gemm_w4_blocks(m, n, k))
 
 
 def gemm_tp(a, b, c, epi: int, *, rs=None, rs_tpr: int = 1, ag_cnt=None, ag_expect: int = 0, bn: int = 0,

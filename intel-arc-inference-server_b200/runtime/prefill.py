@@ -66,10 +66,10 @@ class PhaseProfile:
 
 
 # Backend ``w4`` keeps no bf16 copy of the model.  Up to this many rows (one row of GEMM tiles) the GEMM expands the int4 blocks
-# inside its tiles; beyond that every further row of tiles would expand them again, and the weight is expanded once into the
-# workspace that the two-pass form uses, which holds the largest matrix.  16 layers of the 27B shape, fused / expanded first:
-# 130 rows 7.6 / 6.8 ms, 900 rows 22.3 / 13.9, 4000 rows 67 / 41; in runs of 64 MB that stay in the L2 the products of a run are
-# too narrow to fill the GPU (900 rows: 16.7).
+# inside its tiles, unless that leaves most SMs idle; beyond that every further row of tiles would expand them again, and the weight is expanded once
+# into the workspace that the two-pass form uses, which holds the largest matrix, unless the blocks are still much faster: ``G.w4_from_blocks``.  16
+# layers of the 27B shape, one rule for all linears, fused / expanded first: 130 rows 7.6 / 6.8 ms, 900 rows 22.3 / 13.9, 4000 rows 67 / 41; in runs of 64
+# MB that stay in the L2 the products of a run are too narrow to fill the GPU (900 rows: 16.7).
 W4_FUSED_ROWS = 128
 
 
@@ -150,7 +150,7 @@ class PrefillRunner:
             G.quant_rows_i8(a, a8, self.a_scale[:rows])
             w8, ws = self._w_i8(ql)
             G.gemm_i8(a8, w8, self.a_scale[:rows], ws, out, epi=epi, resid=resid)
-        elif self.backend == "w4" and a.shape[0] <= W4_FUSED_ROWS:
+        elif self.backend == "w4" and a.shape[0] <= 2 * W4_FUSED_ROWS and G.w4_from_blocks(a.shape[0], ql.n, ql.k):
             G.gemm_w4(a, ql.w4b, ql.n, ql.k, out, epi=epi, resid=resid)
         else:
             G.gemm_bf16(a, self._w_bf16(ql), out, epi=epi, resid=resid, parts=self.parts)

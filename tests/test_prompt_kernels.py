@@ -217,6 +217,26 @@ def test_scatter_and_combine(h, k, shared):
     assert ((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + (k + 2) * 2.0 ** -22 * size).all()       # rounded once; fp32 sums, the gate by a fast exponential
 
 
+@pytest.mark.parametrize("m", [80, 128, 129, 256, 257])
+@pytest.mark.parametrize("n,k", [(1024, 1024), (5120, 5120), (5120, 17408), (16480, 5120)])
+def test_int4_linear_on_either_side_of_its_rule(m, n, k):
+    """A linear of backend ``w4`` is the product with the weight's bf16 copy, whichever way the rule sends it."""
+    from types import SimpleNamespace as N
+    from b200serve.runtime.prefill import PrefillRunner
+    torch.manual_seed(m)
+    w, a = Q.random_w4b(n, k, "cuda", 2), torch.randn(m, k, device="cuda").bfloat16()
+    runner = PrefillRunner.__new__(PrefillRunner)
+    runner.backend, runner.dev, runner._slab, runner.parts = "w4", torch.device("cuda"), None, G.gemm_parts("cuda")
+    out = torch.empty(m, n, device="cuda")
+    runner.linear(N(w4b=w, n=n, k=k, _w_bf16=None), a, out, G.EPI_F32)
+    torch.cuda.synchronize()
+    K.check_status()
+    assert (runner._slab is None) == (m <= 256 and G.w4_from_blocks(m, n, k)) and (m > 128 or n * k >= 1 << 24 or runner._slab is None)
+    wb = Q.dequant_w4b(w, n).bfloat16().double()
+    # as in the last wave's test: fp32 sums, and what the tensor core cuts off
+    assert ((out.double() - a.double() @ wb.T).abs() <= (16 + 0.4 * k ** 0.5) * 2.0 ** -24 * (a.double().abs() @ wb.abs().T) + 1e-9).all()
+
+
 @pytest.mark.parametrize("over", [-400, 0, 1])
 def test_experts_from_int4_or_copies(over, monkeypatch):
     """Prompt chunks on both sides of the rule: expanding a tile's blocks gives the bits of the bf16 copies."""
