@@ -1114,6 +1114,10 @@ extern "C" void b2_gemm_parts(long long* floats, int* tickets) {
   *floats = (long long)(sm_count() / 2) * 65536;
   *tickets = sm_count() / 2 * 16;
 }
+// 1: a product of this shape uses one
+extern "C" int b2_gemm_in_parts(int M, int N, int K) {
+  return tile_of(M, N, K, true) == -256 && parts_of((M + 2 * BM - 1) / (2 * BM) * ((N + 255) / 256), K / 64) > 1;
+}
 extern "C" int b2_gemm_tc_parts(const void* a, const void* b, void* c, int M, int N, int K, int ldc, int epi, const void* resid, int bn, float* part,
                                 long long part_floats, int* part_tickets, int n_tickets, void* stream) {
   if (!part || !part_tickets || (epi != EPI_BF16 && epi != EPI_F32 && epi != EPI_SILU_MUL && epi != EPI_RESID_ADD && epi != EPI_RELU2)) return -1;

@@ -31,6 +31,12 @@ def gemm_parts(device) -> tuple:
     return (torch.empty(floats.value, dtype=torch.float32, device=device), torch.zeros(tickets.value, dtype=torch.int32, device=device))
 
 
+@functools.lru_cache(maxsize=4096)
+def gemm_in_parts(m: int, n: int, k: int) -> bool:
+    """A product of this shape has a last wave of tiles worth cutting: it is faster with a workspace of ``gemm_parts``."""
+    return bool(K.lib().b2_gemm_in_parts(m, n, k))
+
+
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, epi: int = EPI_BF16,
               resid: Optional[torch.Tensor] = None, bn: int = 0, parts: Optional[tuple] = None):
     """``c = a @ b.T`` with ``a`` ``[M][K]``, ``b`` ``[N][K]`` bf16.  ``epi``: bf16 / fp32 store,

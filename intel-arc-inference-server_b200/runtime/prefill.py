@@ -115,7 +115,7 @@ class PrefillRunner:
         self.ids_stage = Staged((max_chunk,), torch.int64)   # ring of pinned buffers: the host runs a chunk ahead of the copies
         self.ids_dev = torch.empty(max_chunk, dtype=torch.int64, device=self.dev)
         self._slab: Optional[torch.Tensor] = None
-        self.parts = G.gemm_parts(self.dev) if self.dev.type == "cuda" and self.backend != "int8" else None     # this runner's GEMMs follow one another
+        self._parts: Optional[tuple] = None     # workspace of GEMMs whose last wave of tiles is cut; this runner's follow one another
         if self.backend == "int8":
             kmax = max(h, cfg.q_dim, ffn)
             self.a8 = torch.empty(c, kmax, dtype=torch.int8, device=self.dev)
@@ -153,7 +153,10 @@ class PrefillRunner:
         elif self.backend == "w4" and a.shape[0] <= 2 * W4_FUSED_ROWS and G.w4_from_blocks(a.shape[0], ql.n, ql.k):
             G.gemm_w4(a, ql.w4b, ql.n, ql.k, out, epi=epi, resid=resid)
         else:
-            G.gemm_bf16(a, self._w_bf16(ql), out, epi=epi, resid=resid, parts=self.parts)
+            cut = G.gemm_in_parts(a.shape[0], ql.n, ql.k)
+            if cut and self._parts is None:
+                self._parts = G.gemm_parts(self.dev)
+            G.gemm_bf16(a, self._w_bf16(ql), out, epi=epi, resid=resid, parts=self._parts if cut else None)
 
     # ------------------------------------------------------------------ one layer over a chunk
     def layer(self, lw, kv_index: int, slot: int, c: int, pos0: int, resid, x):

@@ -226,11 +226,12 @@ def test_int4_linear_on_either_side_of_its_rule(m, n, k):
     torch.manual_seed(m)
     w, a = Q.random_w4b(n, k, "cuda", 2), torch.randn(m, k, device="cuda").bfloat16()
     runner = PrefillRunner.__new__(PrefillRunner)
-    runner.backend, runner.dev, runner._slab, runner.parts = "w4", torch.device("cuda"), None, G.gemm_parts("cuda")
+    runner.backend, runner.dev, runner._slab, runner._parts = "w4", torch.device("cuda"), None, None
     out = torch.empty(m, n, device="cuda")
     runner.linear(N(w4b=w, n=n, k=k, _w_bf16=None), a, out, G.EPI_F32)
     torch.cuda.synchronize()
     K.check_status()
+    assert (runner._parts is not None) == (runner._slab is not None and G.gemm_in_parts(m, n, k))
     assert (runner._slab is None) == (m <= 256 and G.w4_from_blocks(m, n, k)) and (m > 128 or n * k >= 1 << 24 or runner._slab is None)
     wb = Q.dequant_w4b(w, n).bfloat16().double()
     # as in the last wave's test: fp32 sums, and what the tensor core cuts off
