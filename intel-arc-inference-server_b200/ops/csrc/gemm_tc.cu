@@ -185,13 +185,14 @@ __device__ __forceinline__ void store_chunk(const GemmParams& p, const uint32_t 
 }
 
 // A weight's scale, times 64, as two bf16 of five significant bits whose sum it is (an fp16 has eleven: the rest behind the first five is
-// at most half a unit of them, so five bits or a power of two), each in both halves of a word.
+// at most half a unit of them, so five bits or a power of two), each in both halves of a word.  One that is not finite stays as it is: the carry of
+// the rounding would make a NaN zero.
 __device__ __forceinline__ void split_scale(float s, uint32_t& hi, uint32_t& lo) {
   s *= 64.f;
-  const uint32_t h = (__float_as_uint(s) + 0x00040000u) & 0xFFF80000u;
-  const float rest = s - __uint_as_float(h);
+  const bool finite = fabsf(s) < __int_as_float(0x7f800000);
+  const uint32_t h = finite ? (__float_as_uint(s) + 0x00040000u) & 0xFFF80000u : __float_as_uint(s);
   hi = __byte_perm(h, 0, 0x3232);
-  lo = __byte_perm(__float_as_uint(fabsf(s) < __int_as_float(0x7f800000) ? rest : 0.f), 0, 0x3232);
+  lo = __byte_perm(__float_as_uint(finite ? s - __uint_as_float(h) : 0.f), 0, 0x3232);
 }
 
 // Vector `u` of a stage's W4B blocks (256 vectors a block) -> sixteen 8-byte pieces of the bf16 B tile.  A vector holds rows g and

@@ -152,6 +152,27 @@ def test_blocks_of_few_rows(n, k):
             assert torch.equal(got[:r], wb[i].T.repeat(128 // k + 1, 1)[:r]) and (got[r:] == 7.0).all()
 
 
+@pytest.mark.parametrize("bn", [128, 256])
+@pytest.mark.parametrize("grouped", [False, True])
+def test_every_scale_expands(bn, grouped):
+    """A row for every fp16 there is as its scale, each nibble four times: the bits of the dequantising pass, infinite and not a number
+    where that is."""
+    n = 65536
+    w = Q.random_w4b(n, 64, "cuda", 1)
+    blocks = w.view(-1, 4352)
+    blocks[:, :4096] = (torch.arange(4096, device="cuda") % 256).to(torch.uint8)
+    blocks[:, 4096:].view(torch.int16)[:] = torch.arange(n, device="cuda").to(torch.int16).view(-1, 128)
+    wb = G.dequant_w4b(w, n, 64)
+    assert int(wb.isnan().all(1).sum()) == 2046 and int(wb.isinf().any(1).sum()) == 2
+    finite = wb.isfinite().all(1)
+    tab = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")        # noqa: E731
+    out = torch.zeros(64, n, device="cuda").bfloat16()
+    G.gemm_w4(torch.eye(64, device="cuda").bfloat16(), w, n, 64, out, bn=bn, blocks=(tab([0]), tab([0]), tab([64]), tab([1]), 1) if grouped else None)
+    torch.cuda.synchronize()
+    K.check_status()
+    assert torch.equal(out[:, finite], wb[finite].T) and out[:, ~finite].isnan().all()      # (the zeros of a unit row times infinity are not numbers)
+
+
 # one tile; a last wave of one, of a few and of half the pairs behind none, one and three whole ones; ragged rows and columns; parts of unequal length
 @pytest.mark.parametrize("m,n,k", [(300, 1000, 1088), (256, 19200, 1024), (900, 5120, 4160), (1000, 9728, 1536), (2048, 5640, 2048), (256, 256, 16384)])
 @pytest.mark.parametrize("epi", [G.EPI_BF16, G.EPI_F32, G.EPI_SILU_MUL, G.EPI_RESID_ADD])
