@@ -39,6 +39,7 @@ struct RowsParams {
   const uint8_t* x;    // [KG][T][128]: stage_rows_kernel
   float* out;          // [S][M][N]
   int M, N, KG, S, gps, nb;
+  int stages;          // of a CTA that are copied (tests: the others' waits run out), or more than there are
   int* fold_tickets;                    // [nb] zeroed counters, or nullptr: no fold
   const __nv_bfloat16* fold_resid_in;   // [M][N]
   __nv_bfloat16* fold_resid_out;
@@ -53,7 +54,7 @@ struct Cfg {
   static constexpr bool TWO = T <= 32;                       // two sets of accumulators fit beside the two sets of weights
   static constexpr int DS = T <= 32 ? T : 64;                // columns from one block's accumulator to the next
   static constexpr int TW = T / 4;                           // token rows that a worker adds up
-  static constexpr int OFF_BAR = NS * STAGE, BARS = (2 * NS + 6) * 8 + 16;
+  static constexpr int OFF_BAR = NS * STAGE, BARS = (2 * NS + 8) * 8 + 16;
   static constexpr int SMEM = 1024 + OFF_BAR + BARS;
 };
 
@@ -64,8 +65,9 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 // A wait of a whole warp.  The first look is all that the hot loops hold: it costs 70 cycles where the bounded loop behind it, inlined, costs twice that
-// even if the phase is over, and the loops' code has to stay small.  After a failed wait (``failed``, a word of the CTA) nobody waits any more: the roles
-// finish on what is there.
+// even if the phase is over, and the loops' code has to stay small.  After a failed wait (``failed``, a word of the CTA) nobody waits for another role any
+// more: no copy is issued, workers and MMAs finish on what is there, so that the tickets are counted, and what is under way is waited for before the CTA ends.
+// (MMA warps that looked at the result of their waits cost 3 % at 16 rows.)
 __device__ __noinline__ void wait_long(uint32_t bar, uint32_t parity, uint32_t failed, unsigned int code) {
   uint32_t f;
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(f) : "r"(failed) : "memory");
@@ -127,19 +129,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
   const uint32_t bars = smem0 + C::OFF_BAR, full0 = bars, empty0 = full0 + 8 * C::NS;
   const uint32_t afull0 = empty0 + 8 * C::NS;                           // [stage parity]
   const uint32_t done0 = afull0 + 16, free0 = done0 + 16;               // two sets of accumulators: done of [stage parity]; one: done and free of [n-block]
-  const uint32_t misc = free0 + 16, failed = misc + 8;                  // TMEM address, "last" flag; a wait ran out
+  const uint32_t last0 = free0 + 16;                                    // all products of [n-block] are made
+  const uint32_t misc = last0 + 16, failed = misc + 8;                  // TMEM address, "last" flag; a wait ran out
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int pairs = (p.nb + 1) >> 1, items = pairs * p.S;
 
   if (tid == 0) {
     for (int i = 0; i < C::NS; ++i) {
       mbar_init(full0 + 8 * i, 1);
-      mbar_init(empty0 + 8 * i, kWorkers + 2);     // workers have read weights and scales, both MMA warps' products the token rows
+      mbar_init(empty0 + 8 * i, 2);     // both MMA warps' products have read the token rows; they were issued behind the workers' reading of weights and scales
     }
     for (int i = 0; i < 2; ++i) {
       mbar_init(afull0 + 8 * i, kWorkers);
       mbar_init(done0 + 8 * i, C::TWO ? 2 : 1);
       mbar_init(free0 + 8 * i, kWorkers);
+      mbar_init(last0 + 8 * i, 1);
     }
     mbar_fence_init();
     asm volatile("st.shared.u32 [%0], %1;" ::"r"(failed), "r"(0) : "memory");
@@ -180,20 +184,20 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
       const auto rows = [&](const Cursor& c, int slot) { bulk_g2s(smem0 + slot * C::STAGE, c.x, min(c.left, 2) * C::XT, full0 + 8 * slot); };
       Cursor cw = at(blockIdx.x), cx = cw;
       int n = 0;
-      for (; n < C::NS && cw.item < items; ++n, step(cw)) weights(cw, n);      // they depend on nothing: asked for before the previous kernel is done
+      for (; n < C::NS && n < p.stages && cw.item < items; ++n, step(cw)) weights(cw, n);      // they depend on nothing: asked for before the previous kernel is done
       pdl_wait();
       for (int i = 0; i < n; ++i, step(cx)) rows(cx, i);
       int slot = 0, round = 1;
-      bool ok = true;
-      for (; cw.item < items; step(cw)) {
-        ok = mbar_wait(empty0 + 8 * slot, (round - 1) & 1, ERR_GEMM_EMPTY_WAIT);
-        if (!ok) break;
+      for (int left = p.stages - n; left > 0 && cw.item < items; --left, step(cw)) {
+        uint32_t stop = !mbar_wait(empty0 + 8 * slot, (round - 1) & 1, ERR_GEMM_EMPTY_WAIT);
+        if (!stop) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(stop) : "r"(failed) : "memory");      // (a stage may then be "empty" that is still on its way)
+        if (stop) break;
         weights(cw, slot);
         rows(cw, slot);
         if (++slot == C::NS) { slot = 0; ++round; }
       }
-      if (!ok)   // wait (bounded) for the copies that were issued and possibly never consumed: those of the last round
-        for (int i = 0; i < C::NS; ++i) mbar_wait(full0 + 8 * i, (i < slot ? round : round - 1) & 1, ERR_GEMM_FULL_WAIT);
+      // every slot's last copies arrive (bounded) before the CTA ends, whether anybody else has waited for them or not
+      for (int i = 0; i < n; ++i) mbar_wait(full0 + 8 * i, (i < slot ? round : round - 1) & 1, ERR_GEMM_FULL_WAIT);
     }
   } else if (warp >= kWorkers) {
     // ---------------------------------------------------------------- MMAs of one n-block of the pair
@@ -222,12 +226,17 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
             }
           }
           tc_commit(empty0 + 8 * slot);
-          tc_commit(done0 + 8 * (C::TWO ? par : h));       // the last one that the CTA waits for
+          tc_commit(done0 + 8 * (C::TWO ? par : h));
         }
         __syncwarp();
         if (++slot == C::NS) { slot = 0; phase ^= 1; }
       }
     }
+    // what was issued is done (bounded) before tensor memory is given back
+    if (elect_one()) tc_commit(last0 + 8 * h);
+    __syncwarp();
+    if (lane == 0) mbar_wait(last0 + 8 * h, 0, ERR_GEMM_TMEM_FULL_WAIT);
+    __syncwarp();
   } else {
     // ---------------------------------------------------------------- expand a stage, add up the one before
     const int q = warp & 3, sub = warp >> 2;                   // quarter of the rows; block to expand and token rows to add up
@@ -268,10 +277,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(full + 8 * C::NS);         // the slot's "empty"
-        mbar_arrive(afull);
-      }
+      if (lane == 0) mbar_arrive(afull);
       st += C::STAGE;
       full += 8;
       if (full == empty0) { st = smem0; full = full0; phase ^= 1; }
@@ -456,8 +462,9 @@ int launch_rows(const RowsParams& p, cudaStream_t stream) {
 }  // namespace
 
 // ``x``: b2_stage_rows of the same M and K, whose rows are padded to 16, 32, 48 or 64 (decode steps come here from 9 rows on).  S <= 16 splits of whole fours of groups, none of them empty.
+// stages: of every CTA that are copied, for tests of what waits that run out leave behind (0: all).
 extern "C" int b2_gemm_w4_rows(const void* w4b, const void* x, float* out, int M, int N, int K, int S, int* fold_tickets,
-                               const void* fold_resid_in, void* fold_resid_out, float* fold_ssq, void* stream) {
+                               const void* fold_resid_in, void* fold_resid_out, float* fold_ssq, int stages, void* stream) {
   if (M < 1 || M > 64 || N < 1 || K < 64 || K % 64 != 0 || S < 1 || S > kMaxSplits) return -1;
   if ((((uintptr_t)w4b | (uintptr_t)x | (uintptr_t)out) & 15) || (((uintptr_t)fold_resid_in | (uintptr_t)fold_resid_out) & 7)) return -4;
   RowsParams p;
@@ -465,6 +472,7 @@ extern "C" int b2_gemm_w4_rows(const void* w4b, const void* x, float* out, int M
   p.M = M; p.N = N; p.KG = K / 64; p.S = S; p.nb = (N + 127) / 128;
   p.gps = ((p.KG + S - 1) / S + 3) / 4 * 4;
   if (p.gps * (S - 1) >= p.KG) return -2;                      // every split has groups
+  p.stages = stages > 0 ? stages : 1 << 30;
   p.fold_tickets = fold_tickets; p.fold_resid_in = (const __nv_bfloat16*)fold_resid_in;
   p.fold_resid_out = (__nv_bfloat16*)fold_resid_out; p.fold_ssq = fold_ssq;
   cudaStream_t st = (cudaStream_t)stream;

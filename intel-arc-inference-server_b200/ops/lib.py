@@ -226,11 +226,11 @@ def rows_splits(n: int, k: int) -> int:
     return best[1]
 
 
-def gemm_w4_rows(w4b, xr, out, m, n, k, splits, *, fold_tickets=None, fold_resid=None, fold_ssq=None):
+def gemm_w4_rows(w4b, xr, out, m, n, k, splits, *, fold_tickets=None, fold_resid=None, fold_ssq=None, stages=0):
     """``out[s][m][n]`` fp32 partial sums of staged rows (``stage_rows``) against a W4B weight, on tcgen05; ``fold_*`` as in
-    ``gemv_w4_fused``."""
+    ``gemv_w4_fused``.  ``stages``: how many stages of every CTA are copied, for tests of what waits that run out leave behind (0: all)."""
     rc = lib().b2_gemm_w4_rows(_p(w4b), _p(xr), _p(out), m, n, k, splits, _p(fold_tickets), _p(fold_resid), _p(fold_resid),
-                               _p(fold_ssq), _stream())
+                               _p(fold_ssq), stages, _stream())
     _check(rc, "gemm_w4_rows")
 
 

@@ -185,6 +185,33 @@ def test_linears_on_rows(m, n, k, splits, fold):
         assert (ssq.double() - sq).abs().max() < 1e-5 * sq.max()
 
 
+# each instance: copies that end before the ring is full, in its second turn, in a CTA's second item
+@pytest.mark.parametrize("m,n,k,splits,stages", [(9, 640, 2560, 1, 1), (24, 300, 2560, 2, 5), (40, 38100, 1280, 1, 11), (64, 2048, 5120, 2, 13)])
+def test_linears_on_rows_whose_waits_run_out(m, n, k, splits, stages):
+    """Copies that never come: the call ends, says so, counts its tickets, and gives tensor memory back: the next calls have the bits they had before."""
+    from b200serve.utils import quant as Q
+    torch.manual_seed(m)
+    w, x = Q.random_w4b(n, k, "cuda", 7), torch.randn(m, k, device="cuda").bfloat16()
+    nb = (n + 127) // 128
+    xr, tickets, ssq = torch.zeros(K.rows_pad(m) * k * 2, dtype=torch.uint8, device="cuda"), torch.zeros(nb, dtype=torch.int32, device="cuda"), torch.zeros(m, nb, device="cuda")
+    K.stage_rows(x, m, k, xr)
+
+    def sums(**how):
+        part, resid = torch.zeros(splits, m, n, device="cuda"), torch.zeros(m, n, device="cuda").bfloat16()
+        K.gemm_w4_rows(w, xr, part, m, n, k, splits, fold_tickets=tickets, fold_resid=resid, fold_ssq=ssq, **how)
+        torch.cuda.synchronize()
+        return part
+    want = sums()
+    K.check_status()
+    sums(stages=stages)
+    said = K.status()
+    K.status_clear()
+    assert set(said) == {"gemmrows"} and int(tickets.abs().sum()) == 0
+    for _ in range(3):
+        assert torch.equal(sums(), want)
+    K.check_status()
+
+
 @pytest.mark.parametrize("m,n,k", [(16, 38500, 192), (17, 19300, 64), (48, 19100, 320), (64, 38016, 128)])
 def test_linears_on_rows_keep_every_weight(m, n, k):
     """Unit rows give the weights themselves, bit by bit: all sixteen nibbles in every place, scales of any size; more pairs of blocks than
