@@ -93,11 +93,15 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // short system time limit passes, so the loop is not a hot spin.  The bound is kept on the SM's own
 // cycle counter (%clock64 costs a few cycles; %globaltimer is a slow read that, taken on every
 // wait, delayed each wake-up by most of a microsecond) and is only consulted after 256 failed
-// polls: about 4e9 cycles, i.e. roughly two seconds at 2 GHz.  The first look, without a time limit, is all that stays inline: it costs 70 cycles where the
-// loop takes twice that for a phase that is over, and hot loops that hold its code several times outgrow the instruction caches (32 dense layers, one
-// request 2.52 -> 2.47 ms).
+// polls: about 4e9 cycles, i.e. roughly two seconds at 2 GHz.
+// mbar_wait_lone: the loop inline, for a lone thread that issues copies or MMAs and nearly always has to wait.
+// mbar_wait: the first look, without a time limit, is all that stays inline, for warps whose phase usually is over: it costs 70 cycles where the loop takes
+// twice that, and hot loops that hold its code several times outgrow the instruction caches (32 dense layers, one request 2.52 -> 2.47 ms).  In the lone
+// threads of a GEMM that waits for HBM at every k block the look and the call behind it cost 27 ns each time: 17 x 4096 x 11008 54.6 us, with the loop 50.0;
+// 300 x 5120 x 17408 126 / 120; 17 requests of a 7B shape with unquantised weights (8 layers) 4 % of a step.  The copying threads of the GEMVs are better
+// off with mbar_wait (1 row, 5120 x 17408 11.1 / 10.8: their registers), those of prompt attention no different.
 constexpr long long kWaitCycles = 4000000000ll;
-static __device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, unsigned int code) {
+__device__ __forceinline__ bool mbar_wait_lone(uint32_t bar, uint32_t parity, unsigned int code) {
 #pragma unroll 1
   for (int i = 0; i < 256; ++i)
     if (mbar_try(bar, parity)) return true;
@@ -112,6 +116,7 @@ static __device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity
     }
   }
 }
+static __device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, unsigned int code) { return mbar_wait_lone(bar, parity, code); }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, unsigned int code) {
   uint32_t ok;
   asm volatile(

@@ -326,7 +326,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % S;
           const uint32_t full = (W4 ? afull0 : full0) + 8 * s;
-          if (it >= S) ok = mbar_wait((W4 ? aempty0 : empty0) + 8 * s, ((it / S) - 1) & 1, ERR_GEMM_EMPTY_WAIT);
+          if (it >= S) ok = mbar_wait_lone((W4 ? aempty0 : empty0) + 8 * s, ((it / S) - 1) & 1, ERR_GEMM_EMPTY_WAIT);
           if (!ok) break;
           const uint32_t sa = W4 ? a_base + s * C::A_BYTES : smem_base + s * C::STAGE, sb = sa + C::A_BYTES;
           const int kx = kb * (I8 ? BKB : BKB / 2);
@@ -355,7 +355,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++lt) {
         const int a = lt & 1;
-        if (lt >= 2) ok = mbar_wait(tempty0 + 8 * a, ((lt >> 1) - 1) & 1, ERR_GEMM_TMEM_EMPTY_WAIT);
+        if (lt >= 2) ok = mbar_wait_lone(tempty0 + 8 * a, ((lt >> 1) - 1) & 1, ERR_GEMM_TMEM_EMPTY_WAIT);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + a * BN;
@@ -363,8 +363,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           const int s = it % C::STAGES;
           constexpr int AS = W4 ? C::ASTAGES : 1;
           const int as = it % AS;
-          ok = mbar_wait(full0 + 8 * s, (it / C::STAGES) & 1, ERR_GEMM_FULL_WAIT) &&
-               (!W4 || mbar_wait(afull0 + 8 * as, (it / AS) & 1, ERR_GEMM_FULL_WAIT));
+          ok = mbar_wait_lone(full0 + 8 * s, (it / C::STAGES) & 1, ERR_GEMM_FULL_WAIT) &&
+               (!W4 || mbar_wait_lone(afull0 + 8 * as, (it / AS) & 1, ERR_GEMM_FULL_WAIT));
           if (!ok) break;
           tc_fence_after();
           const uint32_t sa = W4 ? a_base + as * C::A_BYTES : smem_base + s * C::STAGE, sb = W4 ? smem_base + s * C::B_BYTES : sa + C::A_BYTES;
@@ -390,7 +390,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         const int nb0 = nt * (BN / 128), nblk = min(BN / 128, (p.N + 127) / 128 - nb0);
         const uint8_t* src = p.w4 + (size_t)expert * p.w4_expert_bytes + (size_t)nb0 * KB * kW4Block;
         for (int kb = 0; kb < KB; ++kb, src += kW4Block) {
-          if (round > 0) ok = mbar_wait(rawempty0 + 8 * slot, (round - 1) & 1, ERR_GEMM_EMPTY_WAIT);
+          if (round > 0) ok = mbar_wait_lone(rawempty0 + 8 * slot, (round - 1) & 1, ERR_GEMM_EMPTY_WAIT);
           if (!ok) break;
           mbar_expect_tx(rawfull0 + 8 * slot, (uint32_t)nblk * kW4Block);
           for (int b = 0; b < nblk; ++b)
@@ -680,7 +680,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const int row0 = (w.t % tiles_m) * 2 * BM + rank * BM, n0 = (w.t / tiles_m) * C::BN + rank * (C::BN / 2);
         for (int kb = w.kb0; kb < w.kb1; ++kb, ++it) {
           const int s = it % C::STAGES;
-          if (it >= C::STAGES) ok = mbar_wait(empty0 + 8 * s, ((it / C::STAGES) - 1) & 1, ERR_GEMM_EMPTY_WAIT);
+          if (it >= C::STAGES) ok = mbar_wait_lone(empty0 + 8 * s, ((it / C::STAGES) - 1) & 1, ERR_GEMM_EMPTY_WAIT);
           if (!ok) break;
           const uint32_t sa = smem + s * C::STAGE, bar = map_rank0(full0 + 8 * s);
           if (rank == 0) mbar_expect_tx(full0 + 8 * s, 2 * C::STAGE);
