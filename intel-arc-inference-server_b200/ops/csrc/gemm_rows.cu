@@ -12,7 +12,7 @@
 // summed in its own fp32 accumulator, which the workers scale by the rows' fp16 scales and add up in registers: half a packed
 // FMA per row, token and group, no conversion, no quantised activation, no zero-point term.
 //
-// One persistent CTA per SM.  A stage of the ring is a pair of n-blocks x two groups and the groups' token rows, which both n-blocks share:
+// One persistent CTA per SM.  A stage of the ring is a pair of n-blocks (one where there are few) x two groups and the groups' token rows, which both share:
 //   warps 0-15    workers, one per TMEM quarter and block: expand a block's quarter, then add up a quarter of the token rows of all four blocks of the
 //                 stage before, whose products were made in the meantime;
 //   warps 16-17   issue an n-block's MMAs each;   warp 18  bulk copies.
@@ -121,7 +121,8 @@ __device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
   return v;
 }
 
-template <int T>
+// ONE: an item is a single n-block, the second of each pair is not there
+template <int T, bool ONE>
 __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams p) {
   using C = Cfg<T>;
   extern __shared__ uint8_t smem_raw[];
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
   const uint32_t last0 = free0 + 16;                                    // all products of [n-block] are made
   const uint32_t misc = last0 + 16, failed = misc + 8;                  // TMEM address, "last" flag; a wait ran out
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int pairs = (p.nb + 1) >> 1, items = pairs * p.S;
+  const int pairs = ONE ? p.nb : (p.nb + 1) >> 1, items = pairs * p.S;
 
   if (tid == 0) {
     for (int i = 0; i < C::NS; ++i) {
@@ -159,7 +160,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
   asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(misc));
   const auto first_of = [&](int item) { return item % p.S * p.gps; };
   const auto groups_of = [&](int item) { const int g = first_of(item); return min(p.KG, g + p.gps) - g; };
-  const auto two_of = [&](int item) { return 2 * (item / p.S) + 1 < p.nb; };       // the last of an odd number of n-blocks is alone
+  const auto two_of = [&](int item) { return !ONE && 2 * (item / p.S) + 1 < p.nb; };       // the last of an odd number of n-blocks is alone
 
   if (warp == kWorkers + 2) {
     // ---------------------------------------------------------------- copies
@@ -167,7 +168,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
       struct Cursor { int item, left; bool two; const uint8_t *w, *x; };      // groups left of the item; the stage's blocks of the first n-block, its rows
       const auto at = [&](int item) {
         const int pair = item / p.S, g = (item - pair * p.S) * p.gps;
-        return Cursor{item, min(p.KG, g + p.gps) - g, 2 * pair + 1 < p.nb, p.w + ((size_t)(2 * pair) * p.KG + g) * kBlockBytes, p.x + (size_t)g * C::XT};
+        return Cursor{item, min(p.KG, g + p.gps) - g, !ONE && 2 * pair + 1 < p.nb, p.w + ((size_t)(ONE ? pair : 2 * pair) * p.KG + g) * kBlockBytes, p.x + (size_t)g * C::XT};
       };
       const auto step = [&](Cursor& c) {
         c.w += 2 * kBlockBytes;
@@ -381,8 +382,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
       }
       // ---- the item's sums
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int col = (2 * pair + h) * 128 + row;
+      for (int h = 0; h < (ONE ? 1 : 2); ++h) {
+        const int col = ((ONE ? pair : 2 * pair) + h) * 128 + row;
         float* o = p.out + ((size_t)split * p.M + sub * C::TW) * p.N + col;
 #pragma unroll
         for (int i = 0; i < C::TW; ++i)
@@ -394,8 +395,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
       __threadfence();
       workers_sync();
       if (tid == 0) {
-        const int last = atomicAdd(&p.fold_tickets[2 * pair], 1) == p.S - 1;
-        if (last) p.fold_tickets[2 * pair] = 0;
+        const int last = atomicAdd(&p.fold_tickets[ONE ? pair : 2 * pair], 1) == p.S - 1;
+        if (last) p.fold_tickets[ONE ? pair : 2 * pair] = 0;
         asm volatile("st.shared.u32 [%0], %1;" ::"r"(misc + 4), "r"(last) : "memory");
       }
       workers_sync();
@@ -405,7 +406,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
       __threadfence();
       const int blocks = two ? 2 : 1;
       for (int t = warp; t < p.M * blocks; t += kWorkers) {       // a warp per row and n-block, four columns per lane, the slices' loads in flight together
-        const int m = t / blocks, nblk = 2 * pair + t % blocks, fn = nblk * 128 + lane * 4;
+        const int m = t / blocks, nblk = (ONE ? pair : 2 * pair) + t % blocks, fn = nblk * 128 + lane * 4;
         float f[4] = {0.f, 0.f, 0.f, 0.f};
         if (p.N % 4 == 0 && fn + 4 <= p.N) {
           const uint2 r = *reinterpret_cast<const uint2*>(p.fold_resid_in + (size_t)m * p.N + fn);
@@ -442,21 +443,36 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
   if (warp == kWorkers) tmem_dealloc(tmem, 512);
 }
 
+template <int T, bool ONE>
+int launch_items(const RowsParams& p, int items, cudaStream_t stream) {
+  using C = Cfg<T>;
+  static bool configured[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!configured[dev & 63]) {
+    const cudaError_t e = cudaFuncSetAttribute(gemm_rows_kernel<T, ONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    configured[dev & 63] = true;
+  }
+  return b2_launch(gemm_rows_kernel<T, ONE>, dim3(items), dim3(kThreads), C::SMEM, stream, true, p);
+}
+// While every n-block and split has an SM of its own, a CTA takes one n-block: half the stage, and a fold of half the columns, whose slices a lone SM reads at
+// 64 bytes a cycle.  us with fold, pairs / one, 17 / 32 / 64 rows: 2048 x 2048 in eight splits 9.2 / 7.3, 11.1 / 7.6, 17.0 / 11.0, 512 x 1408 in six 8.4 / 6.7,
+// 10.2 / 6.9, 15.7 / 10.3; without one 2816 x 512 3.1 / 2.8, 3.3 / 2.8, 4.4 / 3.5.  (The bits are the same: a block's sums do not know its neighbour.)
 template <int T>
 int launch_rows(const RowsParams& p, cudaStream_t stream) {
-  using C = Cfg<T>;
   static int sms[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
   if (!sms[dev & 63]) {
     int n = 0;
-    cudaError_t e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(gemm_rows_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    const cudaError_t e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     if (e != cudaSuccess) return (int)e;
     sms[dev & 63] = n;
   }
-  const int items = (p.nb + 1) / 2 * p.S, grid = items < sms[dev & 63] ? items : sms[dev & 63];
-  return b2_launch(gemm_rows_kernel<T>, dim3(grid), dim3(kThreads), C::SMEM, stream, true, p);
+  if (p.nb * p.S <= sms[dev & 63]) return launch_items<T, true>(p, p.nb * p.S, stream);
+  const int items = (p.nb + 1) / 2 * p.S;
+  return launch_items<T, false>(p, items < sms[dev & 63] ? items : sms[dev & 63], stream);
 }
 
 }  // namespace

@@ -149,7 +149,8 @@ def test_grouped_experts(m, k, e, shared, h, f):
 # rows at the edges of the three instances (32, 48 and 64 token rows); splits with unequal and lone groups: stages of which one pipeline has
 # no block; n not a multiple of 128; more items than SMs
 @pytest.mark.parametrize("m,n,k,splits", [(1, 128, 64, 1), (9, 256, 128, 2), (16, 300, 320, 1), (17, 128, 704, 3), (31, 1000, 1024, 4), (32, 5120, 640, 4),
-                                          (33, 640, 448, 7), (48, 128, 1088, 16), (49, 20480, 256, 2), (64, 384, 5120, 7)])
+                                          (33, 640, 448, 7), (48, 128, 1088, 16), (49, 20480, 256, 2), (64, 384, 5120, 7), (16, 9472, 512, 2), (17, 9473, 512, 2),
+                                          (40, 2048, 2048, 8), (64, 9601, 512, 2)])
 @pytest.mark.parametrize("fold", [False, True])
 def test_linears_on_rows(m, n, k, splits, fold):
     from b200serve.utils import quant as Q
