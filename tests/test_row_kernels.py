@@ -146,13 +146,25 @@ def test_grouped_experts(m, k, e, shared, h, f):
         assert (out[pick].double() - z).norm() < 2.0 ** -8 * z.norm()
 
 
-# rows at the edges of the three instances (32, 48 and 64 token rows); splits with unequal and lone groups: stages of which one pipeline has
-# no block; n not a multiple of 128; more items than SMs
+# rows at the edges of the four instances (16, 32, 48 and 64 token rows); splits with unequal and lone groups; n not a multiple of 128; n-blocks alone and in
+# pairs, whose last one is alone; more items than SMs
 @pytest.mark.parametrize("m,n,k,splits", [(1, 128, 64, 1), (9, 256, 128, 2), (16, 300, 320, 1), (17, 128, 704, 3), (31, 1000, 1024, 4), (32, 5120, 640, 4),
                                           (33, 640, 448, 7), (48, 128, 1088, 16), (49, 20480, 256, 2), (64, 384, 5120, 7), (16, 9472, 512, 2), (17, 9473, 512, 2),
                                           (40, 2048, 2048, 8), (64, 9601, 512, 2)])
 @pytest.mark.parametrize("fold", [False, True])
 def test_linears_on_rows(m, n, k, splits, fold):
+    _check_linears_on_rows(m, n, k, splits, fold)
+
+
+# rings of 8, 8, 7 and 6 stages that go round several times, n-blocks alone (21 stages) and in pairs (12 and 9), the last stage with one group and the last
+# pair with one block; two items a CTA, the ring's turn in the middle of one
+@pytest.mark.parametrize("m", [16, 32, 48, 64])
+@pytest.mark.parametrize("n,k,splits", [(300, 2624, 1), (10000, 2624, 2), (37890, 1344, 1)])
+def test_linears_on_rows_of_many_stages(m, n, k, splits):
+    _check_linears_on_rows(m, n, k, splits, n < 20000)
+
+
+def _check_linears_on_rows(m, n, k, splits, fold):
     from b200serve.utils import quant as Q
     torch.manual_seed(n + m)
     dev, per = "cuda", (-(-(k // 64) // splits) + 3) // 4 * 4
