@@ -28,7 +28,7 @@
 // experts of a whole tile of rows and more read such copies.  The role of the reference's direct-int4 GEMMs
 // (src/kernels/prefill/pf_gemm_q4.cl, src/kernels/prefill/pf_moe_q4gemm.cl:1-40).  The blocks have a ring of their own,
 // filled by a warp of its own, and so have the tiles of A: tied to the tiles of B, every trip from HBM was part of the loop.
-// 2048 rows over 256 experts (64 rows each), gate||up 1024 x 2048 / down 2048 x 512, us: 189 / 97 -> 157 / 89 with A apart, columns of tiles innermost, no rows fetched beyond
+// 2048 rows over 256 experts (64 rows each), gate||up 1024 x 2048 / down 2048 x 512, us: 186 / 102 -> 145 / 87 with A apart, tiles of eight blocks together, no rows fetched beyond
 // a block's last, and groups of expanding warps on alternate k blocks.
 #include "common.cuh"
 #include "wire.cuh"
@@ -44,7 +44,9 @@ namespace {
 constexpr int BM = 128;
 constexpr int BKB = 128;  // bytes of K per stage row (64 bf16 or 128 int8)
 constexpr int kThreads = 192;
-constexpr int kGroupBox = 32;   // grouped form: rows of a copy of A; a block's rows beyond its last such box are not fetched
+constexpr int kGroupRun = 8;    // grouped form: blocks whose tiles run together
+constexpr int kGroupBox = 32;   // grouped form: rows of a copy of A; a block's rows beyond its last such box are not fetched, four boxes are one copy (map_part: the
+                                // boxes; in four copies 8 x 256 rows of 4096 x 14336 took 231 us, in one 218)
 
 enum Epi : int { EPI_BF16 = 0, EPI_F32 = 1, EPI_SILU_MUL = 2, EPI_RESID_ADD = 3, EPI_RS_PUSH = 4, EPI_EP_RETURN = 5, EPI_GLU = 6, EPI_RELU2 = 7 };
 
@@ -240,7 +242,7 @@ __device__ __forceinline__ void expand_w4(int u, uint32_t raw, uint32_t sb) {
 
 template <int BN, bool I8, bool W4 = false>
 __global__ void __launch_bounds__(Cfg<BN, W4>::THREADS, 1)
-gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_part,
                const GemmParams p) {
   using C = Cfg<BN, W4>;
   extern __shared__ uint8_t smem_raw[];
@@ -260,10 +262,21 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   const int tiles_n = (p.N + BN - 1) / BN;
   const int tiles_m = grouped ? min(*p.n_blk, p.max_blk) : (p.M + BM - 1) / BM;
   const int n_tiles = tiles_m * tiles_n;
-  // dense: tiles that run together share weights.  Grouped: they share rows -- with the experts' blocks innermost, 256 blocks of 4 KB rows
-  // (134 MB with their padding) went through L2 and from HBM again for every column of tiles
-  const auto mt_of = [&](int t) { return grouped ? t / tiles_n : (t % tiles_m + p.mt_rot) % tiles_m; };
-  const auto nt_of = [&](int t) { return grouped ? t % tiles_n : t / tiles_m; };
+  // Dense: tiles that run together share weights.  Grouped: the columns of eight blocks of rows run together, which share both the rows and, where an expert has
+  // several blocks, its weights.  With all blocks innermost, 256 blocks of 4 KB rows (134 MB with their padding) came from HBM again for every column of tiles;
+  // with the columns of one block innermost, so did the weights of an expert of 1024 rows for every block.  us, all blocks / columns of one / of eight, bf16:
+  // 256 experts x 64 rows, 1024 x 2048 251 / 179 / 181; 8 x 1024, 28672 x 4096 1575 / 1926 / 1397; 1 x 8192, 16384 x 8192 1655 / 2035 / 1566 (four blocks
+  // 1767, sixteen 1647, both before whole blocks were one copy).
+  const auto at_of = [&](int t, int& mt, int& nt) {
+    if (grouped) {
+      const int run = t / (kGroupRun * tiles_n), first = run * kGroupRun, n = min(kGroupRun, tiles_m - first), i = t - first * tiles_n;
+      mt = first + i % n;
+      nt = i / n;
+    } else {
+      mt = (t % tiles_m + p.mt_rot) % tiles_m;
+      nt = t / tiles_m;
+    }
+  };
   const int KB = (p.K * (I8 ? 1 : 2) + BKB - 1) / BKB;  // k blocks
 
   if (threadIdx.x == 0) {
@@ -299,11 +312,13 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (lane == 0) {
       prefetch_tmap(&map_a);
       prefetch_tmap(&map_b);
+      if (grouped) prefetch_tmap(&map_part);
       int it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-        const int mt = mt_of(t), nt = nt_of(t);
-        int row0 = mt * BM, expert = 0, boxes = 0;
+        int mt, nt;
+        at_of(t, mt, nt);
+        int row0 = mt * BM, expert = 0, boxes = BM / kGroupBox;
         if (grouped) {
           row0 = p.blk_row0[mt];
           expert = p.blk_expert[mt];
@@ -330,12 +345,10 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           if (!ok) break;
           const uint32_t sa = W4 ? a_base + s * C::A_BYTES : smem_base + s * C::STAGE, sb = sa + C::A_BYTES;
           const int kx = kb * (I8 ? BKB : BKB / 2);
-          mbar_expect_tx(full, (W4 ? 0 : C::B_BYTES) + (grouped ? boxes * kGroupBox * BKB : C::A_BYTES));
-          if (grouped) {
-            for (int i = 0; i < boxes; ++i) tma_load_2d(sa + i * kGroupBox * BKB, &map_a, kx, row0 + i * kGroupBox, full);
-          } else {
-            tma_load_2d(sa, &map_a, kx, row0, full);
-          }
+          mbar_expect_tx(full, (W4 ? 0 : C::B_BYTES) + boxes * kGroupBox * BKB);
+          if (boxes == BM / kGroupBox) tma_load_2d(sa, &map_a, kx, row0, full);
+          else
+            for (int i = 0; i < boxes; ++i) tma_load_2d(sa + i * kGroupBox * BKB, &map_part, kx, row0 + i * kGroupBox, full);
           if (!W4) {
             if (grouped) tma_load_3d(sb, &map_b, kx, nt * BN, expert, full);
             else tma_load_2d(sb, &map_b, kx, nt * BN, full);
@@ -386,7 +399,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       int slot = 0, round = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-        const int mt = mt_of(t), nt = nt_of(t), expert = grouped ? p.blk_expert[mt] : 0;
+        int mt, nt;
+        at_of(t, mt, nt);
+        const int expert = grouped ? p.blk_expert[mt] : 0;
         const int nb0 = nt * (BN / 128), nblk = min(BN / 128, (p.N + 127) / 128 - nb0);
         const uint8_t* src = p.w4 + (size_t)expert * p.w4_expert_bytes + (size_t)nb0 * KB * kW4Block;
         for (int kb = 0; kb < KB; ++kb, src += kW4Block) {
@@ -410,7 +425,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     int it = 0, slot = 0, par = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
-      const int nt = nt_of(t);
+      int mt, nt;
+      at_of(t, mt, nt);
       const int nb_total = (p.N + 127) / 128, nb0 = nt * (BN / 128);
       const int nblk = min(BN / 128, nb_total - nb0);
       for (int kb = 0; kb < KB; ++kb, ++it) {
@@ -441,7 +457,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     bool ok = true;
     for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++lt) {
       const int a = lt & 1;
-      const int mt = mt_of(t), nt = nt_of(t);
+      int mt, nt;
+      at_of(t, mt, nt);
       int row0 = mt * BM, rows = min(BM, p.M - row0), expert = 0;
       if (grouped) {
         row0 = p.blk_row0[mt];
@@ -927,7 +944,7 @@ int sm_count() {
 }
 
 template <int BN, bool I8>
-int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, int n_tiles_max, cudaStream_t st) {
+int launch(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& part, const GemmParams& p, int n_tiles_max, cudaStream_t st) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -937,12 +954,12 @@ int launch(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& p, in
     configured[dev & 63] = true;
   }
   const int grid = min(n_tiles_max, sm_count());
-  gemm_tc_kernel<BN, I8><<<grid, kThreads, Cfg<BN>::SMEM, st>>>(ma, mb, p);
+  gemm_tc_kernel<BN, I8><<<grid, kThreads, Cfg<BN>::SMEM, st>>>(ma, mb, part, p);
   return (int)cudaGetLastError();
 }
 
 template <int BN>
-int launch_w4(const CUtensorMap& ma, const GemmParams& p, int n_tiles_max, cudaStream_t st) {
+int launch_w4(const CUtensorMap& ma, const CUtensorMap& part, const GemmParams& p, int n_tiles_max, cudaStream_t st) {
   static bool configured[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
@@ -953,7 +970,7 @@ int launch_w4(const CUtensorMap& ma, const GemmParams& p, int n_tiles_max, cudaS
     configured[dev & 63] = true;
   }
   const int grid = min(n_tiles_max, sm_count());
-  gemm_tc_kernel<BN, false, true><<<grid, Cfg<BN, true>::THREADS, Cfg<BN, true>::SMEM, st>>>(ma, ma, p);
+  gemm_tc_kernel<BN, false, true><<<grid, Cfg<BN, true>::THREADS, Cfg<BN, true>::SMEM, st>>>(ma, ma, part, p);
   return (int)cudaGetLastError();
 }
 
@@ -1025,14 +1042,15 @@ extern "C" int b2_gemm_w4(const void* a, const void* w4b, void* c, int M, int N,
     // narrow tiles while they fit in one wave (100 x 7168 x 5120: 57 / 46 us wide / narrow, x 5120 x 17408 166 / 137)
     if (!blk_expert && (M + BM - 1) / BM * ((N + 127) / 128) <= sm_count()) bn = 128;
   }
-  CUtensorMap ma;
-  int rc = make_map(&ma, a, false, (uint64_t)M, (uint64_t)K, 0, blk_expert ? kGroupBox : BM);
+  CUtensorMap ma, part;
+  int rc = make_map(&ma, a, false, (uint64_t)M, (uint64_t)K, 0, BM);
+  if (!rc) rc = make_map(&part, a, false, (uint64_t)M, (uint64_t)K, 0, kGroupBox);
   if (rc) return rc;
   const int tiles_m = blk_expert ? max_blk : (M + BM - 1) / BM;
   const int n_tiles = tiles_m * ((N + bn - 1) / bn);
   (void)n_experts;
   cudaStream_t st = (cudaStream_t)stream;
-  return bn == 256 ? launch_w4<256>(ma, p, n_tiles, st) : launch_w4<128>(ma, p, n_tiles, st);
+  return bn == 256 ? launch_w4<256>(ma, part, p, n_tiles, st) : launch_w4<128>(ma, part, p, n_tiles, st);
 }
 
 // C = A * B^T.  a: [M][K], b: [N][K] (or [E][N][K] when blk_* are given), both bf16 (i8 = 0) or int8 (i8 = 1).
@@ -1071,8 +1089,11 @@ static int gemm_tc_impl(const void* a, const void* b, void* c, int M, int N, int
     if (part) p.split = parts_of(tiles, K / 64);
     if (p.split > 1 && ((long long)rest * p.split * 65536 > part_floats || rest * 16 > n_tickets || ((uintptr_t)part & 15))) return -8;
   }
-  CUtensorMap ma, mb;
-  int rc = make_map(&ma, a, i8 != 0, (uint64_t)M, (uint64_t)K, 0, blk_expert ? kGroupBox : BM);
+  CUtensorMap ma, mb, mp;
+  int rc = make_map(&ma, a, i8 != 0, (uint64_t)M, (uint64_t)K, 0, BM);
+  if (rc) return rc;
+  mp = ma;
+  if (blk_expert) rc = make_map(&mp, a, i8 != 0, (uint64_t)M, (uint64_t)K, 0, kGroupBox);
   if (rc) return rc;
   rc = make_map(&mb, b, i8 != 0, (uint64_t)N, (uint64_t)K, blk_expert ? (uint64_t)n_experts : 0, (uint32_t)bn);
   if (rc) return rc;
@@ -1080,8 +1101,8 @@ static int gemm_tc_impl(const void* a, const void* b, void* c, int M, int N, int
   const int n_tiles = tiles_m * ((N + bn - 1) / bn);
   cudaStream_t st = (cudaStream_t)stream;
   if (pair) return launch_pair(ma, mb, p, st);
-  if (bn == 256) return i8 ? launch<256, true>(ma, mb, p, n_tiles, st) : launch<256, false>(ma, mb, p, n_tiles, st);
-  return i8 ? launch<128, true>(ma, mb, p, n_tiles, st) : launch<128, false>(ma, mb, p, n_tiles, st);
+  if (bn == 256) return i8 ? launch<256, true>(ma, mb, mp, p, n_tiles, st) : launch<256, false>(ma, mb, mp, p, n_tiles, st);
+  return i8 ? launch<128, true>(ma, mb, mp, p, n_tiles, st) : launch<128, false>(ma, mb, mp, p, n_tiles, st);
 }
 
 extern "C" int b2_gemm_tc(const void* a, const void* b, void* c, int M, int N, int K, int ldc, int i8, int epi,

@@ -173,6 +173,30 @@ def test_every_scale_expands(bn, grouped):
     assert torch.equal(out[:, finite], wb[finite].T) and out[:, ~finite].isnan().all()      # (the zeros of a unit row times infinity are not numbers)
 
 
+# blocks around the eight whose tiles run together, experts of one block and of several, the last one short; one column of tiles and several
+@pytest.mark.parametrize("blocks", [1, 7, 8, 9, 19])
+@pytest.mark.parametrize("n,bn", [(200, 128), (648, 128), (1288, 256)])
+def test_blocks_in_runs(blocks, n, bn):
+    torch.manual_seed(blocks)
+    e, k, rows = (blocks + 2) // 3, 192, [128, 97, 33] * 7
+    w = torch.cat([Q.random_w4b(n, k, "cuda", i) for i in range(e)])
+    per = w.shape[0] // e
+    wb = torch.stack([G.dequant_w4b(w[i * per: (i + 1) * per], n, k) for i in range(e)])
+    tab = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")        # noqa: E731
+    table = (tab([i // 3 for i in range(blocks)]), tab([128 * i for i in range(blocks)]), tab(rows[:blocks]), tab([blocks]), blocks + 2)
+    a = torch.randn(128 * blocks, k, device="cuda").bfloat16()
+    ref = torch.stack([a[128 * i: 128 * i + 128].double() @ wb[i // 3].double().T for i in range(blocks)])
+    bound = 16 * 2.0 ** -24 * torch.stack([a[128 * i: 128 * i + 128].double().abs() @ wb[i // 3].double().abs().T for i in range(blocks)])
+    for run in (lambda c: G.gemm_w4(a, w, n, k, c, epi=G.EPI_F32, blocks=table, n_experts=e, bn=bn), lambda c: G.gemm_grouped_bf16(a, wb, c, table, epi=G.EPI_F32, bn=bn)):
+        c = torch.full((128 * blocks, n), 7.0, device="cuda")
+        run(c)
+        torch.cuda.synchronize()
+        K.check_status()
+        for i, r in enumerate(rows[:blocks]):
+            got = c[128 * i: 128 * (i + 1)]
+            assert ((got[:r].double() - ref[i, :r]).abs() <= bound[i, :r] + 1e-9).all() and (got[r:] == 7.0).all()
+
+
 # one tile; a last wave of one, of a few and of half the pairs behind none, one and three whole ones; ragged rows and columns; parts of unequal length
 @pytest.mark.parametrize("m,n,k", [(300, 1000, 1088), (256, 19200, 1024), (900, 5120, 4160), (1000, 9728, 1536), (2048, 5640, 2048), (256, 256, 16384)])
 @pytest.mark.parametrize("epi", [G.EPI_BF16, G.EPI_F32, G.EPI_SILU_MUL, G.EPI_RESID_ADD])
