@@ -146,25 +146,11 @@ def test_grouped_experts(m, k, e, shared, h, f):
         assert (out[pick].double() - z).norm() < 2.0 ** -8 * z.norm()
 
 
-# rows at the edges of the four instances (16, 32, 48 and 64 token rows); splits with unequal and lone groups; n not a multiple of 128; n-blocks alone and in
-# pairs, whose last one is alone; more items than SMs
+# rows at the edges of the four instances (16, 32, 48 and 64 token rows); splits with unequal and lone groups; n not a multiple of 128; more items than SMs
 @pytest.mark.parametrize("m,n,k,splits", [(1, 128, 64, 1), (9, 256, 128, 2), (16, 300, 320, 1), (17, 128, 704, 3), (31, 1000, 1024, 4), (32, 5120, 640, 4),
-                                          (33, 640, 448, 7), (48, 128, 1088, 16), (49, 20480, 256, 2), (64, 384, 5120, 7), (16, 9472, 512, 2), (17, 9473, 512, 2),
-                                          (40, 2048, 2048, 8), (64, 9601, 512, 2)])
+                                          (33, 640, 448, 7), (48, 128, 1088, 16), (49, 20480, 256, 2), (64, 384, 5120, 7)])
 @pytest.mark.parametrize("fold", [False, True])
 def test_linears_on_rows(m, n, k, splits, fold):
-    _check_linears_on_rows(m, n, k, splits, fold)
-
-
-# rings of 8, 8, 7 and 6 stages that go round several times, n-blocks alone (21 stages) and in pairs (12 and 9), the last stage with one group and the last
-# pair with one block; two items a CTA, the ring's turn in the middle of one
-@pytest.mark.parametrize("m", [16, 32, 48, 64])
-@pytest.mark.parametrize("n,k,splits", [(300, 2624, 1), (10000, 2624, 2), (37890, 1344, 1)])
-def test_linears_on_rows_of_many_stages(m, n, k, splits):
-    _check_linears_on_rows(m, n, k, splits, n < 20000)
-
-
-def _check_linears_on_rows(m, n, k, splits, fold):
     from b200serve.utils import quant as Q
     torch.manual_seed(n + m)
     dev, per = "cuda", (-(-(k // 64) // splits) + 3) // 4 * 4
@@ -196,6 +182,21 @@ def _check_linears_on_rows(m, n, k, splits, fold):
         assert ((resid.double() - want).abs() <= 2.0 ** -8 * want.abs() + bound + 1e-6).all() and int(tickets.abs().sum()) == 0
         sq = torch.nn.functional.pad(resid.double() ** 2, (0, nb * 128 - n)).view(m, nb, 128).sum(-1)
         assert (ssq.double() - sq).abs().max() < 1e-5 * sq.max()
+
+
+# n-blocks alone and in pairs, whose last one is alone
+@pytest.mark.parametrize("m,n,k,splits", [(16, 9472, 512, 2), (17, 9473, 512, 2), (40, 2048, 2048, 8), (64, 9601, 512, 2)])
+@pytest.mark.parametrize("fold", [False, True])
+def test_linears_on_rows_in_pairs_and_alone(m, n, k, splits, fold):
+    test_linears_on_rows(m, n, k, splits, fold)
+
+
+# rings of 8, 8, 7 and 6 stages that go round several times, n-blocks alone (21 stages) and in pairs (12 and 9), the last stage with one group and the last
+# pair with one block; two items a CTA, the ring's turn in the middle of one
+@pytest.mark.parametrize("m", [16, 32, 48, 64])
+@pytest.mark.parametrize("n,k,splits", [(300, 2624, 1), (10000, 2624, 2), (37890, 1344, 1)])
+def test_linears_on_rows_of_many_stages(m, n, k, splits):
+    test_linears_on_rows(m, n, k, splits, n < 20000)
 
 
 # each instance: copies that end before the ring is full, in its second turn, in a CTA's second item
