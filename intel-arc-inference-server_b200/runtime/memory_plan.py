@@ -91,6 +91,7 @@ def state_bytes_per_slot(cfg: ModelConfig) -> int:
 
 
 def step_scratch_bytes(cfg: ModelConfig, max_rows: int = 64, nsplit: int = 32) -> int:
+    from ..ops.lib import rows_pad
     h = cfg.hidden
     if cfg.layer_specs:
         from ..models.listed import step_scratch_elems
@@ -100,7 +101,7 @@ def step_scratch_bytes(cfg: ModelConfig, max_rows: int = 64, nsplit: int = 32) -
     b += 16 * max_rows * (cfg.qkv_dim + 2 * h + 2 * max(cfg.ffn, cfg.expert_ffn * max(cfg.top_k, 1))) * 4
     kmax = max(2 * h, cfg.q_dim, cfg.ffn, cfg.expert_ffn, cfg.shared_ffn, cfg.gdn_value_dim)
     b += max_rows * (kmax // 64) * (128 + 8) + (1 << 16)      # quantised rows + group scales, small control words
-    b += max(32, (max_rows + 15) // 16 * 16) * kmax * 2       # rows of the tcgen05 form
+    b += rows_pad(max_rows) * kmax * 2       # rows of the tcgen05 form
     if cfg.n_gdn_layers:
         b += max_rows * (cfg.gdn_proj_dim * 4 + cfg.gdn_value_dim * 2)
     return int(b)
@@ -113,7 +114,8 @@ def prefill_scratch_bytes(cfg: ModelConfig, chunk: int, backend: str) -> int:
         return 4 * step_scratch_elems(cfg, chunk, keys=2 * chunk)
     ffn = cfg.ffn if not cfg.is_moe else max(cfg.expert_ffn, cfg.shared_ffn)
     b = chunk * (2 * h * 2 + cfg.qkv_dim * 4 + 2 * cfg.q_dim * 2 + ffn * 2)
-    b += 20 << 20       # partial sums of a last wave of GEMM tiles
+    if backend not in ("int8", "l0-int8"):
+        b += 20 << 20       # partial sums of a last wave of bf16 GEMM tiles
     biggest = max(cfg.qkv_dim * h, h * cfg.q_dim, 2 * ffn * h)
     if backend in ("bf16", "auto", "w4", "int4", "w4a16"):
         b += biggest * 2

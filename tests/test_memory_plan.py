@@ -214,3 +214,14 @@ def test_collector_rests_until_the_last_capture_ends():
             assert gc.isenabled() == first
         finally:
             gc.enable()
+
+
+def test_scratch_of_row_linears_and_of_cut_waves():
+    """Rows for the tcgen05 linears are counted as they are padded, the workspace of bf16 products only where a backend makes them."""
+    from b200serve.models.config import preset
+    from b200serve.runtime import memory_plan as MP
+    cfg = preset("dense-27b")
+    row = [MP.step_scratch_bytes(cfg, m + 1) - MP.step_scratch_bytes(cfg, m) for m in (15, 16, 17, 32)]
+    assert row[0] == row[2] and row[1] == row[3] == row[0] + 16 * cfg.ffn * 2
+    biggest = 2 * cfg.ffn * cfg.hidden * 2
+    assert MP.prefill_scratch_bytes(cfg, 512, "w4") - MP.prefill_scratch_bytes(cfg, 512, "int8") == biggest + (20 << 20)
