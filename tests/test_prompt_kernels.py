@@ -231,6 +231,48 @@ def test_last_wave_in_parts(m, n, k, epi):
     assert all(((o - y).abs() <= bound).all() for o in outs)
 
 
+# a last wave that is cut: one tile, and few in eight parts; few behind three whole waves; half the pairs in two parts behind one; some in two behind four.
+# Ragged rows and columns, parts of unequal length
+@pytest.mark.parametrize("m,n,k", [(130, 200, 4928), (300, 1000, 4096), (900, 15000, 3072), (700, 9464, 4096), (1200, 16480, 5120)])
+@pytest.mark.parametrize("epi", [G.EPI_BF16, G.EPI_F32, G.EPI_SILU_MUL, G.EPI_RESID_ADD])
+def test_last_wave_that_is_cut(m, n, k, epi, monkeypatch):
+    made, make = [], G.gemm_parts
+    monkeypatch.setattr(G, "gemm_parts", lambda device: made.append(make(device)) or made[-1])
+    test_last_wave_in_parts(m, n, k, epi)
+    left = int((~made[0][0].isnan()).sum())          # whole parts of 256 x 256 sums, two and more
+    assert left % 65536 == 0 and left >= 2 * 65536
+
+
+# blocks around the eight whose tiles run together, short blocks among them
+@pytest.mark.parametrize("blocks", [1, 8, 9, 17])
+@pytest.mark.parametrize("n,bn", [(192, 128), (640, 256)])
+def test_blocks_that_arrive_and_return(blocks, n, bn):
+    """Blocks whose rows are counted as arrived, and rows that go back to where they came from (two buffers of this GPU): the bits of the plain form."""
+    torch.manual_seed(blocks)
+    e, k, rows = (blocks + 2) // 3, 192, ([128, 97, 33] * 6)[:blocks]
+    tab = lambda v: torch.tensor(v, dtype=torch.int32, device="cuda")        # noqa: E731
+    table = (tab([i // 3 for i in range(blocks)]), tab([128 * i for i in range(blocks)]), tab(rows), tab([blocks]), blocks + 2)
+    a, b = torch.randn(128 * blocks, k, device="cuda").bfloat16(), torch.randn(e, n, k, device="cuda").bfloat16()
+    live = torch.cat([128 * i + torch.arange(r) for i, r in enumerate(rows)]).cuda()
+    full = lambda m, n: torch.full((m, n), 7.0, device="cuda").bfloat16()        # noqa: E731
+    want, got = full(len(a), n // 2), full(len(a), n // 2)
+    G.gemm_grouped_bf16(a, b, want, table, epi=G.EPI_SILU_MUL, bn=bn)
+    G.gemm_grouped_ep(a, b, got, table, G.EPI_SILU_MUL, blk_wait=tab(rows), bn=bn)
+    assert torch.equal(want, got)
+    want, home = full(len(a), n), [full(len(live), n) for _ in range(2)]
+    G.gemm_grouped_bf16(a, b, want, table, bn=bn)
+    src = torch.randperm(2 * len(live), device="cuda")[: len(live)]          # buffer and slot of each row
+    meta = torch.zeros(len(a), dtype=torch.int32, device="cuda")
+    meta[live] = (src % 2 * (1 << 24) + src // 2).int()
+    ptrs = torch.tensor([h.data_ptr() for h in home], dtype=torch.int64, device="cuda")
+    G.gemm_grouped_ep(a, b, None, table, G.EPI_EP_RETURN, row_src=meta, ret_table=ptrs, bn=bn)
+    torch.cuda.synchronize()
+    K.check_status()
+    back = torch.stack([full(len(live), n), full(len(live), n)])
+    back[src % 2, src // 2] = want[live]
+    assert torch.equal(torch.stack(home), back)
+
+
 # slots around a pass of eight (combine) and of 32 (scatter), rows of pieces for some of a CTA and for several rounds; two columns a piece
 @pytest.mark.parametrize("h", [2, 130, 136, 2048, 4104])
 @pytest.mark.parametrize("k", [1, 7, 8, 9, 33])
