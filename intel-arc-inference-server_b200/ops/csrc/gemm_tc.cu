@@ -1114,20 +1114,20 @@ extern "C" int b2_gemm_tc(const void* a, const void* b, void* c, int M, int N, i
 }
 
 // 1: a product of M rows with an int4 weight is estimated to be faster from the blocks (b2_gemm_w4) than from an expanded copy that has to be made first
-// (b2_dequant_w4b and b2_gemm_tc_parts).  Expanding takes 0.46 us for a million weights, reading the blocks 0.56 us (128 x 128 tiles) or 0.68 (128 x 256) for a k block and wave.
-// us, blocks / copy: 100 x 5120 x 17408 137 / 91, x 5120 x 5120 44 / 35, x 7168 x 5120 46 / 48, x 16480 x 5120 47 / 76, x 34816 x 5120 65 / 152, 200 x 34816 x
-// 5120 113 / 159, x 16480 x 5120 60 / 81.  Small weights (below 16 M; behind a row of tiles, whose blocks are expanded again, 32 M) stay where the rows put
-// them: 100 x 3072 x 2048 22 / 20.  8 layers, 80 / 128 / 200 / 256 rows, by rows alone and so: dense 27B shape 2.98 -> 2.62, 3.01 -> 2.66, 3.46 -> 3.09,
-// 3.49 -> 3.11 ms, hybrid 3.31 -> 2.91, 3.35 -> 2.96, 4.03 -> 3.48, 4.04 -> 3.50.
+// (b2_dequant_w4b and b2_gemm_tc_parts).  us: 6 and 0.456 (128 x 128 tiles) or 0.6 (128 x 256) for a k block and wave; against 0.43 for a million weights expanded,
+// the product's tiles, or 0.31 for a million bf16 weights read where that is more, and 6.  Blocks / copy, device time, weights from HBM:
+//   100 rows  3072 x 2048 20.2 / 17.9, 2048 x 4096 34.4 / 26.4, 9216 x 2048 20.9 / 23.0, 5120 x 5120 43.6 / 39.3, 7168 x 5120 42.8 / 44.4, 8192 x 5120 42.5 / 45.0,
+//             16480 x 5120 42.4 / 73.3, 34816 x 5120 57 / 148, 4096 x 11008 83 / 48, 5120 x 17408 129 / 89
+//   160 rows  12288 x 2048 27.8 / 30.6, 7168 x 5120 42.8 / 44.8, 16480 x 5120 52 / 77, 22016 x 4096 84 / 95, 34816 x 5120 99 / 150, 5120 x 17408 128 / 89
+// Weights of up to four million always go from the blocks: both take less than the host needs for two launches (1024 x 1024, as issued 14.7 / 17.8).
 extern "C" int b2_gemm_w4_blocks(int M, int N, int K) {
   const int mt = (M + BM - 1) / BM, kb = K / 64, sms = sm_count();
   const bool narrow = mt * ((N + 127) / 128) <= sms;
-  const double blocks = narrow ? 0.56 * kb : 0.68 * kb * ((mt * ((N + 255) / 256) + sms - 1) / sms);
+  const double blocks = narrow ? 0.456 * kb : 0.6 * kb * ((mt * ((N + 255) / 256) + sms - 1) / sms);
   int cost = 0;
   tile_of(M, N, K, true, &cost);
-  const double copy = (double)N * K * 4.6e-7 + 0.375 * cost + 4.0;
-  const double weights = (double)N * K;
-  return mt == 1 ? blocks <= copy || weights < 16777216.0 : blocks <= 0.8 * copy && weights >= 33554432.0;
+  const double millions = 1e-6 * N * K, tiles = 0.375 * cost, read = 0.31 * millions;
+  return millions <= 4.2 || blocks <= 0.43 * millions + (tiles > read ? tiles : read);
 }
 
 // bf16 C = A * B^T with a workspace for cutting the last wave of tiles along K: b2_gemm_parts() floats and tickets, the latter zeroed once.  One product at a

@@ -67,7 +67,7 @@ class PhaseProfile:
 
 # Backend ``w4`` keeps no bf16 copy of the model.  Up to this many rows (one row of GEMM tiles) the GEMM expands the int4 blocks
 # inside its tiles, unless that leaves most SMs idle; beyond that every further row of tiles would expand them again, and the weight is expanded once
-# into the workspace that the two-pass form uses, which holds the largest matrix, unless the blocks are still much faster: ``G.w4_from_blocks``.  16
+# into the workspace that the two-pass form uses, which holds the largest matrix, unless the blocks are still faster: ``G.w4_from_blocks``.  16
 # layers of the 27B shape, one rule for all linears, fused / expanded first: 130 rows 7.6 / 6.8 ms, 900 rows 22.3 / 13.9, 4000 rows 67 / 41; in runs of 64
 # MB that stay in the L2 the products of a run are too narrow to fill the GPU (900 rows: 16.7).
 W4_FUSED_ROWS = 128
