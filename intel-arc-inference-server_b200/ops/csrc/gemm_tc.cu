@@ -989,8 +989,8 @@ int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const GemmParams& 
   return (int)cudaGetLastError();
 }
 
-// Parts along K of the pair form's last wave of tiles: the longest part, and what leaving, counting and adding parts costs (in k blocks of a tile, 0.27 us
-// each), against the whole tile; parts of 8 k blocks and more.  Behind more than six whole waves a last one is too little of the product to gain by
+// Parts along K of the pair form's last wave of tiles: the longest part, and what leaving, counting and adding parts costs (in k blocks of a tile, the unit
+// of tile_of), against the whole tile; parts of 8 k blocks and more.  Behind more than six whole waves a last one is too little of the product to gain by
 // (34816 x 5120 at 900 rows, seven: 244 / 245 us; 3000 rows, 22: 676 / 682).
 int parts_of(int tiles, int kb) {
   const int pairs = sm_count() / 2, rest = tiles % pairs;
@@ -1006,7 +1006,8 @@ int parts_of(int tiles, int kb) {
 // wave takes (K = 5120, weights beyond L2): 256 x 256 on two SMs 30 us, 128 x 256 on one 33, 128 x 128 22; the narrow tile only
 // where it fits in one wave.  130 x 5120 x 17408: 110 / 78 us wide / narrow, 300 x 34816 x 5120: 128 / 116 pair / wide,
 // 512 x 5120 x 17408: 93 / 126, 4096 x 34816 x 5120: 908 / 986.  parts: a workspace for cutting the last wave of pairs is there.
-// cost: the estimate, in k blocks of a 256 x 256 tile (0.375 us while all SMs work).
+// cost: the estimate, in k blocks of a 256 x 256 tile, 0.375 us each and a launch, cut or not (256 rows, estimate / us: 16480 x 5120 80 / 38, 22016 x 4096 111 / 57;
+// cut 2048 x 6144 52 / 22, 5120 x 5120 57 / 24, 4096 x 11008 75 / 32, 5120 x 17408 121 / 48).
 int tile_of(int M, int N, int K, bool parts, int* cost = nullptr) {
   const int sms = sm_count(), mt = (M + BM - 1) / BM, mp = (M + 2 * BM - 1) / (2 * BM), kb = K / 64;
   const int wide = (N >= 256 && (N % 256 == 0 || N > 2048)) ? 256 : 128;
