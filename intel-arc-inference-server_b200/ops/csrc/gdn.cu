@@ -398,10 +398,10 @@ constexpr int WY_OFF_WK = 0;                      // Wk   [64][136] bf16  (row s
 constexpr int WY_OFF_QG = WY_OFF_WK + WY_C * WY_LDK * 2;     // Qg   [64][136] bf16  gamma_s q_s
 constexpr int WY_OFF_KGT = WY_OFF_QG + WY_C * WY_LDK * 2;    // Kg^T [128][72] bf16  (row dk, column s) (gamma_63 / gamma_s) k_s
 constexpr int WY_OFF_P = WY_OFF_KGT + DH * WY_LDP * 2;       // P    [64][72]  bf16  (row t, column s)
-constexpr int WY_OFF_WVT = WY_OFF_P + WY_C * WY_LDP * 2;     // Wv   [2][64][68] fp32 (half of dv, row s, column dv): a warp stores whole sectors
-constexpr int WY_OFF_GC = WY_OFF_WVT + DH * WY_LDV * 4;      // gamma_63 (fp32) + padding
+constexpr int WY_OFF_WV = WY_OFF_P + WY_C * WY_LDP * 2;      // Wv   [2][64][68] fp32 (half of dv, row s, column dv): a warp stores whole sectors
+constexpr int WY_OFF_GC = WY_OFF_WV + DH * WY_LDV * 4;       // gamma_63 (fp32) + padding
 constexpr int WY_BLOCK = WY_OFF_GC + 16;
-static_assert(WY_BLOCK % 16 == 0 && WY_OFF_WVT % 16 == 0, "bulk copies move multiples of 16 bytes");
+static_assert(WY_BLOCK % 16 == 0 && WY_OFF_WV % 16 == 0, "bulk copies move multiples of 16 bytes");
 
 struct GdnWyParams {
   float* act;      // [M][N] after gdn_prep_kernel: q, k normalised; beta and the decay factor in place of b, a
@@ -571,7 +571,7 @@ __global__ void __launch_bounds__(256, 2) gdn_wy_prep_kernel(const GdnWyParams p
 #pragma unroll
     for (int s = 0; s < WY_C; ++s) Wk[s * WY_LDK + tid] = __float2bfloat16(w[s]);
   } else {
-    float* Wv = reinterpret_cast<float*>(blk + WY_OFF_WVT) + ((tid - DH) >> 6) * (WY_C * WY_LDV) + (tid & 63);
+    float* Wv = reinterpret_cast<float*>(blk + WY_OFF_WV) + ((tid - DH) >> 6) * (WY_C * WY_LDV) + (tid & 63);
 #pragma unroll
     for (int s = 0; s < WY_C; ++s) Wv[s * WY_LDV] = w[s];
   }
@@ -600,9 +600,9 @@ __global__ void __launch_bounds__(256, 2) gdn_wy_prep_kernel(const GdnWyParams p
   if (tid == 0) *reinterpret_cast<float*>(blk + WY_OFF_GC) = eg[WY_C - 1];
 }
 
-// the scan's stage: the block's images up to Wv^T, this CTA's half of Wv (64 value columns), gamma_63
+// the scan's stage: the block's images up to Wv, this CTA's half of it (64 value columns), gamma_63
 constexpr int WYB_WV_HALF = WY_C * WY_LDV * 4;
-constexpr int WYB_STAGE = WY_OFF_WVT + WYB_WV_HALF + 16;
+constexpr int WYB_STAGE = WY_OFF_WV + WYB_WV_HALF + 16;
 constexpr int WYB_SMEM = 2 * WYB_STAGE + 64;
 static_assert(WYB_STAGE % 128 == 0 || WYB_STAGE % 16 == 0, "stages start on 16-byte boundaries");
 
@@ -633,9 +633,9 @@ __global__ void __launch_bounds__(128, 1) gdn_wy_scan_kernel(const GdnWyParams p
     const uint32_t dst = stage0 + b * WYB_STAGE, bar = bar0 + 8 * b;
     const uint8_t* src = ws + (size_t)c * ws_step;
     mbar_expect_tx(bar, WYB_STAGE);
-    bulk_g2s(dst, src, WY_OFF_WVT, bar);
-    bulk_g2s(dst + WY_OFF_WVT, src + WY_OFF_WVT + half * WYB_WV_HALF, WYB_WV_HALF, bar);
-    bulk_g2s(dst + WY_OFF_WVT + WYB_WV_HALF, src + WY_OFF_GC, 16, bar);
+    bulk_g2s(dst, src, WY_OFF_WV, bar);
+    bulk_g2s(dst + WY_OFF_WV, src + WY_OFF_WV + half * WYB_WV_HALF, WYB_WV_HALF, bar);
+    bulk_g2s(dst + WY_OFF_WV + WYB_WV_HALF, src + WY_OFF_GC, 16, bar);
   };
   if (tid == 0)
     for (int c = 0; c < min(2, p.chunks); ++c) fetch(c, c);
@@ -689,7 +689,7 @@ __global__ void __launch_bounds__(128, 1) gdn_wy_scan_kernel(const GdnWyParams p
     // ---- U^T = Wv^T - R1^T, as A operand limbs over the chunk's rows (4 k-steps of 16)
     uint32_t uh[4][4], ul[4][4];
     {
-      const float* wv = reinterpret_cast<const float*>(wy_smem + b * WYB_STAGE + WY_OFF_WVT);
+      const float* wv = reinterpret_cast<const float*>(wy_smem + b * WYB_STAGE + WY_OFF_WV);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float* w = wv + (8 * j + 2 * t) * WY_LDV + dvl;
@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(128, 1) gdn_wy_scan_kernel(const GdnWyParams p
     }
     // ---- S^T <- gamma_63 S^T + U^T Kg  (B[k = row s][n = dk] from Kg^T [dk][s])
     {
-      const float gc = *reinterpret_cast<const float*>(wy_smem + b * WYB_STAGE + WY_OFF_WVT + WYB_WV_HALF);
+      const float gc = *reinterpret_cast<const float*>(wy_smem + b * WYB_STAGE + WY_OFF_WV + WYB_WV_HALF);
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         st[j][0] *= gc; st[j][1] *= gc; st[j][2] *= gc; st[j][3] *= gc;
