@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_rows_kernel(const RowsParams
       Scales scales = expand(none);
       int left = groups_of(item);
       if (C::TWO) {
-        // up to 16 token rows the products of the stage before are on their way while a stage is expanded and the one before them is added up (24.7 -> 22.9 us;
+        // up to 16 token rows the products of the stage before are on their way while a stage is expanded and the one before them is added up (24.7 -> 23.1 us;
         // with 32 they are made in time: 26.6 / 27.4)
         if (T > 16) {
 #pragma unroll 1

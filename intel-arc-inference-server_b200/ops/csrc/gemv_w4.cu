@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
   float pacc[2][2] = {};      // PACK: row g (t < 2) or g + 8 of the warp's tiles, the lane's two tokens
 
   if (p.x_mode == 2) {
-    // (in the quantiser's order, whatever the rows; by one thread a step of two small layers took 106.4 us, now 104.7)
+    // (in the quantiser's order, whatever the rows)
     for (int m = warp; m < p.M; m += 8) {
       const float r = row_rinv(p, m, lane);
       if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(rinv0 + m * 4), "f"(r) : "memory");
