@@ -98,8 +98,8 @@ __device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
 // mbar_wait: the first look, without a time limit, is all that stays inline, for warps whose phase usually is over: it costs 70 cycles where the loop takes
 // twice that, and hot loops that hold its code several times outgrow the instruction caches (32 dense layers, one request 2.52 -> 2.47 ms).  In the lone
 // threads of a GEMM that waits for HBM at every k block the look and the call behind it cost 27 ns each time: 17 x 4096 x 11008 54.6 us, with the loop 50.0;
-// 300 x 5120 x 17408 126 / 120; 17 requests of a 7B shape with unquantised weights (8 layers) 4 % of a step.  The copying threads of the GEMVs are better
-// off with mbar_wait (1 row, 5120 x 17408 11.1 / 10.8: their registers), those of prompt attention no different.
+// 300 x 5120 x 17408 126 / 120; 17 requests of a 7B shape with unquantised weights (8 layers) 4 % of a step.  The copying threads of the GEMVs of
+// up to four rows are better off with mbar_wait (1 row, 5120 x 17408 11.1 / 10.8: their registers), those of prompt attention no different.
 constexpr long long kWaitCycles = 4000000000ll;
 __device__ __forceinline__ bool mbar_wait_lone(uint32_t bar, uint32_t parity, unsigned int code) {
 #pragma unroll 1

@@ -296,6 +296,9 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
   // layers of the 27B shape, 2.17 -> 2.13 / 2.42 -> 2.36 ms; with four tiles a warp has no registers for a second row tile.)
   constexpr bool kSplit = T <= 2;
   constexpr int RT = kSplit ? 2 : 1;   // row tiles per warp
+  // With more than four tokens the ring's waits keep their loops inline (16 layers of the 27B shape, 8 rows, out of line / inline 1573 / 1563 us), with fewer the
+  // loops' code is in the way (common.cuh).
+  const auto ring_wait = [](uint32_t bar, uint32_t parity, unsigned int code) { return PACK ? mbar_wait(bar, parity, code) : mbar_wait_lone(bar, parity, code); };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int nblk = blockIdx.x, split = blockIdx.y;
   if (p.skip_negative) {   // the ids are the previous kernel's output
@@ -369,7 +372,7 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
           }
           if (!ok) break;
           if (i >= kStages) {
-            ok = mbar_wait(empty0 + 8 * (i % kStages), ((i / kStages) - 1) & 1, ERR_GEMV_EMPTY_WAIT);
+            ok = ring_wait(empty0 + 8 * (i % kStages), ((i / kStages) - 1) & 1, ERR_GEMV_EMPTY_WAIT);
             if (!ok) break;
             issue_w(i);
           }
@@ -378,7 +381,7 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
           for (int c = max(0, next_chunk - 2); c < next_chunk; ++c) mbar_wait(xfull0 + 8 * (c & 1), (c >> 1) & 1, ERR_GEMV_FULL_WAIT);
       } else {
         for (int i = 0; i < nstage && ok; ++i) {
-          if (i >= kStages) ok = mbar_wait(empty0 + 8 * (i % kStages), ((i / kStages) - 1) & 1, ERR_GEMV_EMPTY_WAIT);
+          if (i >= kStages) ok = ring_wait(empty0 + 8 * (i % kStages), ((i / kStages) - 1) & 1, ERR_GEMV_EMPTY_WAIT);
           if (!ok) break;
           issue_w(i);
         }
@@ -475,7 +478,7 @@ __global__ void __launch_bounds__(kThreads, (T <= 2 ? 2 : 1)) gemv_w4_kernel(con
       const int i = (c0 + gi) / kG;  // stage index since kernel start
       if (kSplit && (i & 1) != wgrp) continue;   // the other group's stage
       const int s = i % kStages;
-      if (ok) ok = mbar_wait(full0 + 8 * s, (i / kStages) & 1, ERR_GEMV_FULL_WAIT);
+      if (ok) ok = ring_wait(full0 + 8 * s, (i / kStages) & 1, ERR_GEMV_FULL_WAIT);
       if (!ok) continue;
       const uint32_t st = ring + s * kStageBytes;
       uint32_t xa[T];
