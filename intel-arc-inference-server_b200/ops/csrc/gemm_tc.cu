@@ -1120,7 +1120,8 @@ extern "C" int b2_gemm_tc(const void* a, const void* b, void* c, int M, int N, i
 //   100 rows  3072 x 2048 20.2 / 17.9, 2048 x 4096 34.4 / 26.4, 9216 x 2048 20.9 / 23.0, 5120 x 5120 43.6 / 39.3, 7168 x 5120 42.8 / 44.4, 8192 x 5120 42.5 / 45.0,
 //             16480 x 5120 42.4 / 73.3, 34816 x 5120 57 / 148, 4096 x 11008 83 / 48, 5120 x 17408 129 / 89
 //   160 rows  12288 x 2048 27.8 / 30.6, 7168 x 5120 42.8 / 44.8, 16480 x 5120 52 / 77, 22016 x 4096 84 / 95, 34816 x 5120 99 / 150, 5120 x 17408 128 / 89
-// Weights of up to four million always go from the blocks: both take less than the host needs for two launches (1024 x 1024, as issued 14.7 / 17.8).
+// Weights of up to four million stay where the rows put them, from the blocks up to one row of tiles: the forms differ by a microsecond (1024 x 1024, 100 rows
+// 12.7 / 11.8, but 14.7 / 17.8 as issued from the host, 160 rows 12.7 / 11.9).
 extern "C" int b2_gemm_w4_blocks(int M, int N, int K) {
   const int mt = (M + BM - 1) / BM, kb = K / 64, sms = sm_count();
   const bool narrow = mt * ((N + 127) / 128) <= sms;
@@ -1128,7 +1129,7 @@ extern "C" int b2_gemm_w4_blocks(int M, int N, int K) {
   int cost = 0;
   tile_of(M, N, K, true, &cost);
   const double millions = 1e-6 * N * K, tiles = 0.375 * cost, read = 0.31 * millions;
-  return millions <= 4.2 || blocks <= 0.43 * millions + (tiles > read ? tiles : read);
+  return millions <= 4.2 ? mt == 1 : blocks <= 0.43 * millions + (tiles > read ? tiles : read);
 }
 
 // bf16 C = A * B^T with a workspace for cutting the last wave of tiles along K: b2_gemm_parts() floats and tickets, the latter zeroed once.  One product at a

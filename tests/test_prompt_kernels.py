@@ -327,9 +327,9 @@ def test_int4_linear_on_either_side_of_its_rule(m, n, k):
 
 def test_rule_of_int4_linears_follows_what_was_measured():
     """Shapes whose two forms were measured 4 % and more apart, and those too small for two launches."""
-    blocks = [(20, 1024, 1024), (256, 2048, 2048), (100, 9216, 2048), (160, 9216, 2048), (128, 12288, 2048), (160, 12288, 2048), (100, 7168, 5120), (160, 7168, 5120),
+    blocks = [(20, 1024, 1024), (128, 2048, 2048), (100, 9216, 2048), (160, 9216, 2048), (128, 12288, 2048), (160, 12288, 2048), (100, 7168, 5120), (160, 7168, 5120),
               (128, 8192, 5120), (256, 8192, 5120), (20, 16480, 5120), (256, 16480, 5120), (128, 22016, 4096), (160, 22016, 4096), (20, 34816, 5120), (256, 34816, 5120)]
-    copies = [(20, 3072, 2048), (100, 3072, 2048), (128, 2048, 4096), (256, 2048, 4096), (100, 4096, 4096), (160, 4096, 4096), (20, 2048, 6144), (100, 5120, 5120),
+    copies = [(129, 1024, 1024), (20, 3072, 2048), (100, 3072, 2048), (128, 2048, 4096), (256, 2048, 4096), (100, 4096, 4096), (160, 4096, 4096), (20, 2048, 6144), (100, 5120, 5120),
               (256, 5120, 5120), (128, 5120, 6144), (20, 4096, 11008), (256, 4096, 11008), (100, 5120, 17408), (256, 5120, 17408)]
     assert [s for s in blocks if not G.w4_from_blocks(*s)] == [] and [s for s in copies if G.w4_from_blocks(*s)] == []
 
