@@ -21,8 +21,8 @@
 // What bounds it is issue, the logic pipe first, beside a memory floor of 20 us with 136 pairs on 148 SMs: every instruction that the loops do not
 // hold counts, and their code has to fit the instruction caches (bounded waits inlined in them cost 14 of 48 us).
 // A row's bits do not depend on the other rows of the step; they are not those of the integer GEMV, whose activations are 15-bit integers.
-// 34816 x 5120 / 5120 x 17408, us: 9 - 16 rows 23.1 / 13.1 (integer GEMV 31.2 / 17.0), 17 - 32 rows 26.0 / 15.0, 33 - 48 rows 31.4 / 17.7, 64 rows
-// 35.0 / 19.5; with expanding and adding warps of two pipelines, as first built, 46.8 / 25.3, 59.4 / 32.3 and 65.9 / 36.2.  Measured and dropped: two CTAs of
+// 34816 x 5120 / 5120 x 17408, us: 9 - 16 rows 23.3 / 12.9 (integer GEMV 31.2 / 17.0), 17 - 32 rows 26.0 / 15.0, 33 - 48 rows 31.0 / 17.7, 64 rows
+// 34.5 / 19.6; with expanding and adding warps of two pipelines, as first built, 46.8 / 25.3, 59.4 / 32.3 and 65.9 / 36.2.  Measured and dropped: two CTAs of
 // eight workers per SM (24.5 / 28.8 / 33.2 / 40.3 for the four row counts: twice the splits, and 64 rows have no registers).
 #include "common.cuh"
 
