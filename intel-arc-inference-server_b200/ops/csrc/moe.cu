@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256) moe_route_kernel(const float* __restrict_
 // ---------------------------------------------------------------- decode rows: router logits + routing in one launch
 // logits[m][r] = x[m] . W[r] for the R router rows (E experts, then the shared expert's gate row when there is one):
 // sixteen router rows a CTA, eight token rows per pass over the weights, on mma.sync, k spread over the warps (fp32 products of a
-// warp per router row were bound by issue: a layer of 48 rows took 20 us here, now 11.6).  The CTA that finishes last (a ticket) then
+// warp per router row were bound by issue: 257 x 2048, the launch for 1 / 8 / 48 rows 6.2 / 10.6 / 13.3 us, now 6.9 / 7.9 / 8.0).  The CTA that finishes last (a ticket) then
 // routes every token row.  With `shared_slot` each row gets one more slot: expert id E (the shared expert, see the
 // batched GEMV's alt weights) with weight sigmoid(gate logit), or 1 without a gate row; with shared_slot n > 1 (no gate
 // row) n more slots, ids E .. E + n - 1 with weight 1: runs of a shared expert's hidden columns.
@@ -217,50 +217,67 @@ __device__ void group_pairs(const int* topk_idx, int pairs, int* groups, int* s_
   }
 }
 
+// Groups of eight router rows a CTA.  With one the launch alone is faster up to 16 rows (8 rows 7.3 us where it is 7.9), but its 33 CTAs are in the way of the experts' CTAs
+// that start behind it: 4 requests, 16 layers 1165 us where it is 1090.
+constexpr int kRouterTiles = 2;
+
 template <bool PLAIN>
 __global__ void __launch_bounds__(256) moe_router_rows_kernel(const RouterRowsParams p) {
   __shared__ int s_last, s_count[kGroupIds], s_first[kGroupIds];
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ float s_red[8][16][9];
+  constexpr int RT = kRouterTiles, RR = 8 * RT;      // router rows of the CTA
+  __shared__ float s_red[8][8][RR + 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int r0 = blockIdx.x * 16;
+  const int r0 = blockIdx.x * RR;
   // token rows of this CTA: all of them, or the slice of eight that blockIdx.y names
   const int m_lo = gridDim.y > 1 ? blockIdx.y * 8 : 0, m_hi = gridDim.y > 1 ? min(p.M, m_lo + 8) : p.M;
   for (int m0 = m_lo; m0 < m_hi; m0 += 8) {
     // A lane's 16 bytes of a row are eight k of a 32-k chunk: two MMAs take them as they are, since both operands have them in the same order.
-    // Chunks go round the warps; eight of a warp's are in flight together.
-    float c[4] = {0.f, 0.f, 0.f, 0.f};
+    // Chunks go round the warps; eight of a warp's are in flight together.  Token rows are the MMA's rows (the upper eight are zero).  A tensor core cuts off
+    // where it adds, so every MMA starts from zero and their results are added as a tree in fp32: errors of 7.5e-8 of the logits at 2048, as fp32 FMAs made (one chain
+    // of MMAs a warp: 2.4e-7, and 4.7e-7 at 4096).
+    float c[RT][2] = {};
     const auto piece = [&](const __nv_bfloat16* base, int row, int rows, int k) {
       return row < rows && k < p.H ? __ldg(reinterpret_cast<const uint4*>(base + (size_t)row * p.H + k)) : make_uint4(0, 0, 0, 0);
     };
     for (int k0 = warp * 32 + t * 8; k0 - t * 8 < p.H; k0 += 8 * 8 * 32) {
-      uint4 u[8], v[8], x[8];
+      uint4 w[RT][8], x[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int k = k0 + i * 8 * 32;
-        u[i] = piece(p.w, r0 + g, p.R, k);
-        v[i] = piece(p.w, r0 + g + 8, p.R, k);
+#pragma unroll
+        for (int r = 0; r < RT; ++r) w[r][i] = piece(p.w, r0 + 8 * r + g, p.R, k);
         x[i] = piece(p.x, m0 + g, m_hi, k);
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        mma_bf16_16816(c, u[i].x, v[i].x, u[i].y, v[i].y, x[i].x, x[i].y);
-        mma_bf16_16816(c, u[i].z, v[i].z, u[i].w, v[i].w, x[i].z, x[i].w);
+      for (int r = 0; r < RT; ++r) {
+        float d[8][2];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          float lo[4] = {0.f, 0.f, 0.f, 0.f}, hi[4] = {0.f, 0.f, 0.f, 0.f};
+          mma_bf16_16816(lo, x[i].x, 0u, x[i].y, 0u, w[r][i].x, w[r][i].y);
+          mma_bf16_16816(hi, x[i].z, 0u, x[i].w, 0u, w[r][i].z, w[r][i].w);
+          d[i][0] = lo[0] + hi[0];
+          d[i][1] = lo[1] + hi[1];
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) c[r][j] += ((d[0][j] + d[1][j]) + (d[2][j] + d[3][j])) + ((d[4][j] + d[5][j]) + (d[6][j] + d[7][j]));
       }
     }
     if (m0 > m_lo) __syncthreads();
-    s_red[warp][g][2 * t] = c[0];
-    s_red[warp][g][2 * t + 1] = c[1];
-    s_red[warp][g + 8][2 * t] = c[2];
-    s_red[warp][g + 8][2 * t + 1] = c[3];
-    __syncthreads();
-    const int row = threadIdx.x & 15, m = m0 + (threadIdx.x >> 4);
-    if (threadIdx.x < 128 && r0 + row < p.R && m < m_hi) {
-      float sum = 0.f;
 #pragma unroll
-      for (int w = 0; w < 8; ++w) sum += s_red[w][row][threadIdx.x >> 4];
-      p.logits[(size_t)m * p.ld + r0 + row] = sum;
+    for (int r = 0; r < RT; ++r) {
+      s_red[warp][g][8 * r + 2 * t] = c[r][0];
+      s_red[warp][g][8 * r + 2 * t + 1] = c[r][1];
+    }
+    __syncthreads();
+    const int row = threadIdx.x % RR, m = m0 + threadIdx.x / RR;
+    if (threadIdx.x < 8 * RR && r0 + row < p.R && m < m_hi) {
+      float w[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w[i] = s_red[i][threadIdx.x / RR][row];
+      p.logits[(size_t)m * p.ld + r0 + row] = ((w[0] + w[1]) + (w[2] + w[3])) + ((w[4] + w[5]) + (w[6] + w[7]));
     }
   }
   __threadfence();
@@ -522,10 +539,11 @@ extern "C" int b2_moe_router_rows(const void* w, const void* x, float* logits, i
   RouterRowsParams p{(const __nv_bfloat16*)w, (const __nv_bfloat16*)x, logits, M, R, H, ld, E, k, shared_slot, has_gate,
                      rule, topk_idx, topk_w, ticket, table};
   if (table && E + shared_slot > kGroupIds) return -1;
-  // Slices of eight token rows have CTAs of their own, which also route them (a router of 257 rows is 33 CTAs: 48 token rows
+  // Slices of eight token rows have CTAs of their own, which also route them (a router of 257 rows is 17 CTAs: 48 token rows
   // behind one another took 58 us of a layer's step).  Callers with a single ticket word keep one slice.
   const int slices = (M + 7) / 8 < n_tickets ? (M + 7) / 8 : 1;
-  return b2_launch(route_plain(rule) ? moe_router_rows_kernel<true> : moe_router_rows_kernel<false>, dim3((R + 15) / 16, slices), dim3(256), 0, (cudaStream_t)stream, true, p);
+  return b2_launch(route_plain(rule) ? moe_router_rows_kernel<true> : moe_router_rows_kernel<false>, dim3((R + 8 * kRouterTiles - 1) / (8 * kRouterTiles), slices), dim3(256), 0,
+                   (cudaStream_t)stream, true, p);
 }
 
 // counts must hold E zeros on entry (the caller clears it on the stream).

@@ -267,6 +267,26 @@ def test_router_logits(m, e, h, tickets):
     assert torch.equal(idx.view(m, k).long(), torch.sort(lg[:, :e], dim=-1, descending=True, stable=True).indices[:, :k]) and int(tk.abs().sum()) == 0
 
 
+@pytest.mark.parametrize("m,e,h", [(1, 256, 2048), (48, 257, 2048), (64, 64, 4096), (5, 64, 512), (20, 33, 1000)])
+def test_router_logits_are_fp32_sums(m, e, h):
+    """Errors of the size that additions in fp32 make, not a chain of additions that cut off.  Root mean squares in units of 2^-24: a chunk of 32 k is two MMAs that may cut
+    off up to 2 units of it each, at most 2 * 4 / 3 over all chunks; three levels of a tree in a warp, three over the warps and a chain of two below 7 / 3."""
+    from b200serve.ops import moe as M
+    torch.manual_seed(m + e)
+    w, x = (torch.randn(e, h, device="cuda") * h ** -0.5).bfloat16(), torch.randn(m, h, device="cuda").bfloat16()
+    ld, k = (e + 7) // 8 * 8, 4
+    lg = torch.zeros(m, ld, device="cuda")
+    idx, tw, tk = torch.zeros(m * k, dtype=torch.int32, device="cuda"), torch.zeros(m * k, device="cuda"), torch.zeros(16, dtype=torch.int32, device="cuda")
+    M.router_rows(w, x, lg, m, e, h, ld, e, k, False, False, idx, tw, tk)
+    torch.cuda.synchronize()
+    ref = x.double() @ w.double().T
+    assert (lg[:, :e].double() - ref).norm() <= 5 ** 0.5 * 2.0 ** -24 * ref.norm()
+    alone = torch.zeros_like(lg)
+    for i in range(m):
+        M.router_rows(w, x[i:], alone[i:], 1, e, h, ld, e, k, False, False, idx, tw, tk)
+    assert torch.equal(lg, alone)          # whatever the company
+
+
 # one group, a stage and a lone group, unequal splits; n not a multiple of 128
 @pytest.mark.parametrize("n,k,splits", [(128, 64, 1), (300, 320, 1), (1000, 704, 3), (640, 1024, 2)])
 @pytest.mark.parametrize("fed", [False, True])
